@@ -22,7 +22,7 @@ struct KronosCudaContext {
     cudaStream_t stream = nullptr;
     uint64_t launches = 0;
     std::string err;
-    DeviceBuffer x, q, xs, xsum, out, dots, inv, normw;
+    DeviceBuffer x, q, xs, xsum, out, dots, inv, normw, half, half_xs;
     uint32_t *d_err = nullptr;      // device word kernels set when a bounded wait gives up
 };
 

@@ -99,7 +99,10 @@ bool count(KronosCudaEngine *e, cudaError_t err, const char *what, uint32_t n = 
 bool gemv_from(KronosCudaEngine *e, const KronosCudaMatrix *m, const int8_t *q, const float *sc, const int32_t *sums, float *out, const char *what,
                uint32_t n_tok) {
     uint32_t launched = 0;
-    cudaError_t err = launch_gemv_batch(e->ctx->stream, m->dm, q, sc, sums, n_tok, out, m->dm.geom.rows, nullptr, e->ctx->sm_count, e->ctx->d_err, &launched, e->pdl);
+    const uint32_t min_tok = gemm_tc_min_tokens();
+    cudaError_t err = min_tok != 0 && n_tok >= min_tok
+                          ? launch_gemm_f16(e->ctx->stream, m->dm, q, sc, n_tok, e->act_half, out, m->dm.geom.rows, e->ctx->sm_count, e->ctx->d_err, &launched, e->pdl)
+                          : launch_gemv_batch(e->ctx->stream, m->dm, q, sc, sums, n_tok, out, m->dm.geom.rows, nullptr, e->ctx->sm_count, e->ctx->d_err, &launched, e->pdl);
     return count(e, err, what, launched);
 }
 bool gemv(KronosCudaEngine *e, const KronosCudaMatrix *m, float *out, const char *what, uint32_t n_tok = 1, size_t act_tok0 = 0) {
@@ -759,6 +762,8 @@ KronosCudaEngine *kronos_cuda_engine_create(KronosCudaContext *ctx, const Kronos
               dev_alloc(e, e->qkv, (size_t)e->max_batch * qkv_rows) && dev_alloc(e, e->gate_up, (size_t)e->max_batch * 2 * inter) &&
               dev_alloc(e, e->logits, (size_t)e->max_batch * (c.tp_size > 1 ? c.vocab_total : c.vocab_size)) && dev_alloc(e, e->act_q, (size_t)e->max_batch * act_n) &&
               dev_alloc(e, e->act_s, (size_t)e->max_batch * act_n / 64) && dev_alloc(e, e->act_m, (size_t)e->max_batch * act_n / 64) &&
+              dev_alloc(e, e->act_half.img, act_half_bytes(e->max_batch, std::max(act_n, e->sh_inter_max))) &&
+              dev_alloc(e, e->act_half.scales, act_half_scale_bytes(e->max_batch, std::max(act_n, e->sh_inter_max))) &&
               dev_alloc(e, e->q_i8, (size_t)e->max_batch * q_dim) && dev_alloc(e, e->attn_tap, q_dim) && dev_alloc(e, e->q_scale, (size_t)e->max_batch * n_q) &&
               dev_alloc(e, e->part_m, (size_t)n_q * e->n_split) && dev_alloc(e, e->part_l, (size_t)n_q * e->n_split) &&
               dev_alloc(e, e->part_o, (size_t)n_q * e->n_split * hd) &&

@@ -9,6 +9,7 @@
 
 #include "k2t_context.h"
 #include "k2t_dense.h"
+#include "k2t_gemm_f16.h"
 #include "k2t_model_kernels.h"
 
 using namespace k2t;
@@ -87,7 +88,7 @@ void kronos_cuda_context_destroy(KronosCudaContext *ctx) {
     if (!ctx) return;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
-    for (DeviceBuffer *b : {&ctx->x, &ctx->q, &ctx->xs, &ctx->xsum, &ctx->out, &ctx->dots, &ctx->inv, &ctx->normw}) release(*b);
+    for (DeviceBuffer *b : {&ctx->x, &ctx->q, &ctx->xs, &ctx->xsum, &ctx->out, &ctx->dots, &ctx->inv, &ctx->normw, &ctx->half, &ctx->half_xs}) release(*b);
     if (ctx->d_err) cudaFree(ctx->d_err);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     delete ctx;
@@ -314,9 +315,24 @@ static int32_t linear_impl(KronosCudaContext *ctx, const KronosCudaMatrix *m, co
     if (kronos_cuda_fwht_quant_dev(ctx, (const float *)ctx->x.p, n_tok, g.cols, nullptr, nullptr, 0, (int8_t *)ctx->q.p,
                                    (float *)ctx->xs.p, (int32_t *)ctx->xsum.p) != 0)
         return -1;
-    if (!run_gemv(ctx, m, (const int8_t *)ctx->q.p, (const float *)ctx->xs.p, (const int32_t *)ctx->xsum.p, n_tok,
-                  (float *)ctx->out.p, g.rows, nullptr))
+    uint32_t launched = 0;
+    const uint32_t min_tok = gemm_tc_min_tokens();
+    // prompt-sized calls: the activations are the library's own, so their chunk sums are consistent.  Without memory for the operand
+    // image the kernel that needs none serves the call.
+    bool half = min_tok != 0 && n_tok >= min_tok && n_tok <= 0xFFFFu * 32u;
+    if (half && (!reserve(ctx, ctx->half, act_half_bytes(n_tok, g.cols)) || !reserve(ctx, ctx->half_xs, act_half_scale_bytes(n_tok, g.cols)))) {
+        half = false;
+        ctx->err.clear();
+    }
+    if (half) {
+        const ActHalf h{(uint8_t *)ctx->half.p, (uint8_t *)ctx->half_xs.p};
+        if (!cuda_ok(ctx, launch_gemm_f16(s, m->dm, (const int8_t *)ctx->q.p, (const float *)ctx->xs.p, (uint32_t)n_tok, h, (float *)ctx->out.p, g.rows, ctx->sm_count,
+                                          ctx->d_err, &launched, true), "linear launch"))
+            return -1;
+        ctx->launches += launched;
+    } else if (!run_gemv(ctx, m, (const int8_t *)ctx->q.p, (const float *)ctx->xs.p, (const int32_t *)ctx->xsum.p, n_tok, (float *)ctx->out.p, g.rows, nullptr)) {
         return -1;
+    }
     if (!cuda_ok(ctx, cudaMemcpyAsync(out, ctx->out.p, n_out * 4, cudaMemcpyDeviceToHost, s), "copy out")) return -1;
     if (!wait) return 0;
     return sync_and_check(ctx, "linear") ? 0 : -1;

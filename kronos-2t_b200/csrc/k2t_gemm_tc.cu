@@ -508,15 +508,15 @@ cudaError_t launch_tc_fmt(cudaStream_t stream, const TcArgs &args, int sm_count,
     return cudaErrorNotSupported;
 }
 
-uint32_t tc_min_tokens() {
+}  // namespace
+
+uint32_t gemm_tc_min_tokens() {
     static const uint32_t v = [] {
         const char *s = std::getenv("KRONOS_CUDA_TC_MIN_TOKENS");          // 0 = never use the tensor-core path
         return s ? (uint32_t)std::atoi(s) : 16u;
     }();
     return v;
 }
-
-}  // namespace
 
 // y[t] = W x[t] for any number of tokens: batches of at least `KRONOS_CUDA_TC_MIN_TOKENS` (16) go to the tensor-core kernel in
 // one launch, shorter ones (and calls that ask for the integer dots) to the 4-token weight passes.
@@ -525,7 +525,7 @@ cudaError_t launch_gemv_batch(cudaStream_t stream, const DeviceMatrix &m, const 
                               uint32_t *launches, bool pdl) {
     if (launches) *launches = 0;
     const MatrixGeom &g = m.geom;
-    const uint32_t min_tok = tc_min_tokens();
+    const uint32_t min_tok = gemm_tc_min_tokens();
     if (min_tok != 0 && n_tok >= min_tok && n_tok <= 0xFFFFu * 16u && int_dots == nullptr && (g.max_odd == 0 || xsum != nullptr)) {
         TcArgs args;
         int fmt = fill_gemv_args(m, xsum != nullptr, args.g);

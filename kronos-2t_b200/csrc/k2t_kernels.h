@@ -32,6 +32,9 @@ cudaError_t launch_gemv_batch(cudaStream_t stream, const DeviceMatrix &m, const 
                               size_t n_tok, float *out, size_t out_stride, int32_t *int_dots, int sm_count, uint32_t *err_flag,
                               uint32_t *launches, bool pdl = false);
 
+// Fewest tokens of a call that the tensor cores take (KRONOS_CUDA_TC_MIN_TOKENS, 16; 0 = never).
+uint32_t gemm_tc_min_tokens();
+
 // Decode tables of one expert matrix (every expert of a MoE layer carries its own codebook): 64 bytes.
 struct ExpertCodebook {
     uint32_t cb[8];      // expanded codebook, 4 centroids per word
