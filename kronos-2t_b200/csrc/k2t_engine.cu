@@ -248,6 +248,7 @@ bool enqueue_attention_batch(KronosCudaEngine *e, uint32_t l, uint32_t T) {
     xa.max_seq = e->kv_stride; xa.layer = l; xa.sc_stride = e->kv_stride; xa.blk_stride = (e->kv_stride + 127) / 128;
     xa.ctx_cap = attn_ctx_cap(e); xa.ring = e->ring;
     xa.kv_bits = c.kv_bits; xa.attn_scale = 1.0f / sqrtf((float)hd); xa.err_flag = e->ctx->d_err; xa.trace = nullptr; xa.v_t = e->v_t;
+    if (attention_prompt_takes(xa, T)) return count(e, launch_attention_prompt(s, xa, e->pdl, T), "attention");
     return count(e, launch_attention_exact(s, xa, e->pdl, T), "attention", 2);
 }
 

@@ -152,6 +152,11 @@ cudaError_t launch_attention(cudaStream_t s, const AttnArgs &a, bool pdl);     /
 // [n_tok][n_q][sc_stride], block maxima [n_tok][n_q][blk_stride], o_proj activation rows [n_tok][n_q * head_dim] (scales and
 // sums [n_tok][n_q * head_dim / 64]); attn_out (optional) receives the last token's output.
 cudaError_t launch_attention_exact(cudaStream_t s, const ExactAttnArgs &a, bool pdl, uint32_t n_tok = 1);
+// the same for a prompt batch over the int8 cache with a full causal context: one kernel, rows of a kv head side by side
+// (k2t_attn_prompt.cu).  attention_prompt_takes: cache format, context (shared memory) and batch suit it.
+constexpr uint32_t PROMPT_ATTN_MIN_TOKENS = 16;
+bool attention_prompt_takes(const ExactAttnArgs &a, uint32_t n_tok);
+cudaError_t launch_attention_prompt(cudaStream_t s, const ExactAttnArgs &a, bool pdl, uint32_t n_tok);
 // longest context launch_attention_exact can serve (its value weights live in shared memory)
 size_t attention_exact_max_ctx(uint32_t head_dim, uint32_t kv_bits);
 // contexts of up to ATTN_EXACT_CTX positions: qkv_post + attention in one kernel (leaves longer contexts untouched)
