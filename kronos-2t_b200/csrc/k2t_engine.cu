@@ -365,11 +365,16 @@ bool enqueue_batch(KronosCudaEngine *e, uint32_t T, bool embed, Tail tail, bool 
             ra.n_experts = c.moe_num_experts; ra.hidden = h; ra.top_k = k; ra.norm_topk = (int32_t)(c.moe_norm_topk & 1u); ra.scoring = c.moe_norm_topk >> 8;
             ra.route_ids = L.d_route_ids; ra.route_w = L.d_route_w; ra.logits = e->router_logits; ra.done = e->router_done; ra.route_stride = 32; ra.err_flag = e->ctx->d_err;
             if (!count(e, launch_moe_router(s, ra, e->pdl, T), "router")) return false;
-            if (!count(e, launch_gemv_experts(s, L.gu_dm, L.gu_fmt, L.d_gu_books, L.d_gu_bases, L.d_route_ids, T * k, e->act_q, e->act_s, e->act_m, h, h / 64,
-                                              e->moe_gu, (size_t)2 * dff, e->ctx->sm_count, e->ctx->d_err, e->pdl, c.moe_num_experts, k, 32, k), "expert gate_up")) return false;
+            const uint32_t E = c.moe_num_experts;
+            const bool grouped = experts_grouped(T * k, E);
+            if (grouped && !count(e, launch_expert_tiles(s, L.d_route_ids, T, k, 32, E, L.d_gu_bases, e->tiles, e->ctx->d_err, e->pdl), "expert tiles")) return false;
+            if (!count(e, grouped ? launch_gemm_experts(s, L.gu_dm, L.gu_fmt, L.d_gu_books, L.d_gu_bases, E, e->tiles, T * k, k, e->act_q, e->act_s, e->moe_gu, e->ctx->d_err, e->pdl)
+                                  : launch_gemv_experts(s, L.gu_dm, L.gu_fmt, L.d_gu_books, L.d_gu_bases, L.d_route_ids, T * k, e->act_q, e->act_s, e->act_m, h, h / 64,
+                                                        e->moe_gu, (size_t)2 * dff, e->ctx->sm_count, e->ctx->d_err, e->pdl, E, k, 32, k), "expert gate_up")) return false;
             if (!count(e, launch_expert_swiglu_quant(s, e->moe_gu, dff, T * k, e->moe_q, e->moe_s, e->moe_m, e->pdl), "expert swiglu")) return false;
-            if (!count(e, launch_gemv_experts(s, L.dn_dm, L.dn_fmt, L.d_dn_books, L.d_dn_bases, L.d_route_ids, T * k, e->moe_q, e->moe_s, e->moe_m, dff, dff / 64,
-                                              e->moe_out, h, e->ctx->sm_count, e->ctx->d_err, e->pdl, c.moe_num_experts, k, 32, 1), "expert down")) return false;
+            if (!count(e, grouped ? launch_gemm_experts(s, L.dn_dm, L.dn_fmt, L.d_dn_books, L.d_dn_bases, E, e->tiles, T * k, 1, e->moe_q, e->moe_s, e->moe_out, e->ctx->d_err, e->pdl)
+                                  : launch_gemv_experts(s, L.dn_dm, L.dn_fmt, L.d_dn_books, L.d_dn_bases, L.d_route_ids, T * k, e->moe_q, e->moe_s, e->moe_m, dff, dff / 64,
+                                                        e->moe_out, h, e->ctx->sm_count, e->ctx->d_err, e->pdl, E, k, 32, 1), "expert down")) return false;
             if (!count(e, launch_moe_combine(s, e->moe_out, L.d_route_w, k, h, e->proj, e->pdl, L.d_route_ids, c.ep_size > 1 ? L.d_dn_bases : nullptr,
                                              c.moe_num_experts, T, 32, shared ? e->sh_out : nullptr, shared && L.sh_gate_w ? e->sh_scale : nullptr), "moe combine")) return false;
             continue;
@@ -799,6 +804,8 @@ KronosCudaEngine *kronos_cuda_engine_create(KronosCudaContext *ctx, const Kronos
              dev_alloc(e, e->moe_gu, (size_t)e->max_batch * k * 2 * dff) && dev_alloc(e, e->moe_out, (size_t)e->max_batch * k * h) &&
              dev_alloc(e, e->moe_q, (size_t)e->max_batch * k * dff) && dev_alloc(e, e->moe_s, (size_t)e->max_batch * k * dff / 64) &&
              dev_alloc(e, e->moe_m, (size_t)e->max_batch * k * dff / 64);
+        const uint32_t tiles = expert_tiles_max((size_t)e->max_batch * k, c.moe_num_experts);
+        ok = ok && dev_alloc(e, e->tiles.n_tiles, 1) && dev_alloc(e, e->tiles.expert, tiles) && dev_alloc(e, e->tiles.pairs, (size_t)tiles * 32);
         if (ok && e->sh_inter_max > 0) {
             const size_t si = e->sh_inter_max;
             ok = dev_alloc(e, e->sh_gu, (size_t)e->max_batch * 2 * si) && dev_alloc(e, e->sh_out, (size_t)e->max_batch * h) && dev_alloc(e, e->sh_scale, e->max_batch) &&

@@ -63,6 +63,7 @@ struct KronosCudaEngine {
     float *x_norm = nullptr, *moe_gu = nullptr, *moe_out = nullptr, *router_logits = nullptr;
     uint32_t *router_done = nullptr;
     int8_t *moe_q = nullptr; float *moe_s = nullptr; int32_t *moe_m = nullptr;
+    k2t::ExpertTiles tiles;                   // the batch's pairs sorted by expert (prompts)
     // shared-expert workspace, [max_batch] rows each: gate_up outputs, the down projection's activation, outputs, gate values
     uint32_t sh_inter_max = 0;
     float *sh_gu = nullptr, *sh_out = nullptr, *sh_scale = nullptr;

@@ -1,5 +1,6 @@
 // Prompt GEMM over half-precision operand images (k2t_gemm_f16.cu).
 #pragma once
+#include <algorithm>
 #include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -20,5 +21,27 @@ size_t act_half_scale_bytes(size_t n_tok, uint32_t cols);
 // two launches, the image and the product.
 cudaError_t launch_gemm_f16(cudaStream_t stream, const DeviceMatrix &m, const int8_t *xq, const float *xs, uint32_t n_tok, const ActHalf &h,
                             float *out, size_t out_stride, int sm_count, uint32_t *err_flag, uint32_t *launches, bool pdl);
+
+// The (token, route) pairs of a batch in tiles of 32 of one expert: device scratch of the caller.
+struct ExpertTiles {
+    uint32_t *n_tiles = nullptr;     // one word
+    uint32_t *expert = nullptr;      // [expert_tiles_max]
+    uint32_t *pairs = nullptr;       // [expert_tiles_max][32]: pair = token * k + route, 0xffffffff behind the expert's last one
+};
+constexpr uint32_t EXPERT_TILES_MAX_EXPERTS = 256;
+uint32_t expert_tiles_max(size_t n_pair, uint32_t n_experts);
+cudaError_t launch_expert_tiles(cudaStream_t stream, const uint32_t *route_ids, uint32_t n_tok, uint32_t k, uint32_t route_stride, uint32_t n_experts,
+                                const uint8_t *const *bases, const ExpertTiles &t, uint32_t *err_flag, bool pdl);
+
+// Prompts take the grouped form from three pairs per expert on.  A GEMV costs per pair (0.33 us each for gate_up and down of the 30B-A3B
+// shape: 128 experts, 2048 x 1536 and 768 x 2048, 3 bits), a tile per expert: 24 / 32 / 44 / 64 / 150 tokens with 8 routes through three
+// layers take 857 / 995 / 1238 / 1605 / 4024 us as GEMVs and 1113 / 1193 / 1271 / 1352 / 1498 us in tiles.  Few experts leave SMs
+// idle: 48 pairs at least.
+inline bool experts_grouped(uint32_t n_pair, uint32_t n_experts) { return n_pair >= std::max(3 * n_experts, 48u); }
+
+// The expert projections of all pairs of `t`, an expert's weights expanded once per 32 pairs; out = [n_pair][rows].  Same bits as
+// launch_gemv_experts, for activations in the form the library's own quantizers leave them.
+cudaError_t launch_gemm_experts(cudaStream_t stream, const DeviceMatrix &m0, int fmt, const ExpertCodebook *books, const uint8_t *const *bases, uint32_t n_experts,
+                                const ExpertTiles &t, uint32_t n_pair, uint32_t act_group, const int8_t *xq, const float *xs, float *out, uint32_t *err_flag, bool pdl);
 
 }  // namespace k2t
