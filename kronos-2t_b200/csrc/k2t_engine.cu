@@ -705,7 +705,7 @@ KronosCudaEngine *kronos_cuda_engine_create(KronosCudaContext *ctx, const Kronos
         const uint32_t want = (8u * (uint32_t)ctx->sm_count + c.num_key_value_heads - 1) / c.num_key_value_heads;
         e->n_split = std::min(128u, std::max(32u, (want + 3u) & ~3u));
     }
-    if (const char *v = std::getenv("KRONOS_CUDA_PROMPT_BATCH")) {                  // tokens per prompt batch (default 256: 1.7B-shape prompts 13.5k / 18.8k / 21.8k tok/s at 64 / 128 / 256)
+    if (const char *v = std::getenv("KRONOS_CUDA_PROMPT_BATCH")) {                  // tokens per prompt batch (default 512, the slack of a sliding window's ring)
         const uint32_t n = (uint32_t)std::strtoul(v, nullptr, 10);
         e->max_batch = std::min(512u, std::max(16u, (n + 15u) & ~15u));
     }
@@ -1248,8 +1248,13 @@ static int32_t forward_common(KronosCudaEngine *e, const float *embeds, const ui
     // prompt: batches of up to max_batch tokens (forward_prompt / forward_batch_sdot_impl, real_llm.rs:7407-7448, 7450-7860):
     // every projection as one tensor-core weight pass over the batch, the attention of the batch's tokens side by side
     if (!set_u32(e, e->d_pos, (uint32_t)pos_start)) return -1;
+    // As few batches as the workspace allows, of about the same size in whole tiles of 128 tokens: a short last one would pay for
+    // a batch's launches and its weights again (300 tokens of the 30B-A3B shape as 256 + 44 and as one: 2.86 and 1.86 ms; 1000 tokens
+    // of the 1.7B shape in batches of 256 and in two of 500: 11.9 and 9.7 ms).
+    const size_t n_batch = (n_tok + e->max_batch - 1) / e->max_batch;
+    const uint32_t T_even = (uint32_t)std::min<size_t>(e->max_batch, ((n_tok + n_batch - 1) / n_batch + 127) & ~(size_t)127);
     for (size_t t0 = 0, T_done = 0; t0 < n_tok; t0 += T_done) {
-        uint32_t T = (uint32_t)std::min<size_t>(e->max_batch, n_tok - t0);
+        uint32_t T = (uint32_t)std::min<size_t>(T_even, n_tok - t0);
         const size_t p0 = pos_start + t0;
         if (e->split_kv && p0 < ATTN_EXACT_CTX && p0 + T > ATTN_EXACT_CTX) T = (uint32_t)(ATTN_EXACT_CTX - p0);    // split-KV kernels: a batch stays on one side of the attention switch
         const bool last = t0 + T == n_tok;
