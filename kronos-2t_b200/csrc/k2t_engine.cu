@@ -17,6 +17,7 @@
 #include "k2t_dense.h"
 #include "k2t_engine.h"
 #include "k2t_gemv_fused.h"
+#include "k2t_prompt_ops.h"
 #include "k2t_prologue.cuh"
 
 using namespace k2t;
@@ -96,18 +97,20 @@ bool sync_vt(KronosCudaEngine *e) {
 bool count(KronosCudaEngine *e, cudaError_t err, const char *what, uint32_t n = 1) { return engine_count(e, err, what, n); }
 
 
+// batches the half-precision prompt GEMM takes; their small operators run as k2t_prompt_ops.cu
+bool wide_batch(uint32_t n_tok) { return gemm_tc_min_tokens() != 0 && n_tok >= gemm_tc_min_tokens(); }
+
 bool gemv_from(KronosCudaEngine *e, const KronosCudaMatrix *m, const int8_t *q, const float *sc, const int32_t *sums, float *out, const char *what,
-               uint32_t n_tok) {
+               uint32_t n_tok, bool image_ready = false) {
     uint32_t launched = 0;
-    const uint32_t min_tok = gemm_tc_min_tokens();
-    cudaError_t err = min_tok != 0 && n_tok >= min_tok
-                          ? launch_gemm_f16(e->ctx->stream, m->dm, q, sc, n_tok, e->act_half, out, m->dm.geom.rows, e->ctx->sm_count, e->ctx->d_err, &launched, e->pdl)
+    cudaError_t err = wide_batch(n_tok)
+                          ? launch_gemm_f16(e->ctx->stream, m->dm, q, sc, n_tok, e->act_half, out, m->dm.geom.rows, e->ctx->sm_count, e->ctx->d_err, &launched, e->pdl, image_ready)
                           : launch_gemv_batch(e->ctx->stream, m->dm, q, sc, sums, n_tok, out, m->dm.geom.rows, nullptr, e->ctx->sm_count, e->ctx->d_err, &launched, e->pdl);
     return count(e, err, what, launched);
 }
-bool gemv(KronosCudaEngine *e, const KronosCudaMatrix *m, float *out, const char *what, uint32_t n_tok = 1, size_t act_tok0 = 0) {
+bool gemv(KronosCudaEngine *e, const KronosCudaMatrix *m, float *out, const char *what, uint32_t n_tok = 1, size_t act_tok0 = 0, bool image_ready = false) {
     const size_t cols = m->dm.geom.cols, nc = cols / 64;
-    return gemv_from(e, m, e->act_q + act_tok0 * cols, e->act_s + act_tok0 * nc, e->act_m + act_tok0 * nc, out, what, n_tok);
+    return gemv_from(e, m, e->act_q + act_tok0 * cols, e->act_s + act_tok0 * nc, e->act_m + act_tok0 * nc, out, what, n_tok, image_ready);
 }
 
 void fill_embed_args(const KronosCudaEngine *e, EmbedArgs &a);
@@ -124,6 +127,9 @@ bool tp_gather(KronosCudaEngine *e, const float *slice, float *all, uint32_t n) 
 }
 
 
+// the activation buffers of a wide batch, and the image
+PromptAct act_of(const KronosCudaEngine *e, uint32_t T) { return PromptAct{e->act_q, e->act_s, e->act_m, e->act_half, (uint32_t)act_half_tokens(T)}; }
+
 // Residual add + RMSNorm + activation of the next projection.  Under tensor parallelism `delta` is this rank's partial
 // output of a row-parallel projection: the kernel exchanges and sums the ranks' partials itself.
 // `partial`: delta holds this rank's share only (row-parallel projection under tensor parallelism, routed experts under
@@ -137,14 +143,26 @@ uint32_t attn_ctx_cap(const KronosCudaEngine *e) {
 }
 
 // expert parallelism).
-bool norm_quant(KronosCudaEngine *e, const float *delta, const float *w, float *x_norm, uint32_t T, bool pdl, bool partial) {
+// `image`: set when the kernel has also left the operand image of a wide batch.
+bool norm_quant(KronosCudaEngine *e, const float *delta, const float *w, float *x_norm, uint32_t T, bool pdl, bool partial, bool &image) {
     const KronosCudaEngineConfig &c = e->cfg;
+    image = false;
     if (partial && delta != nullptr) {
         if (!e->tp_ready) return fail(e->ctx, "tensor-parallel engine used before kronos_cuda_engine_tp_attach");
         return count(e, launch_rmsnorm_quant_tp(e->ctx->stream, e->hidden, delta, w, c.hidden_size, c.rms_norm_eps, e->act_q, e->act_s, e->act_m, x_norm, T, pdl,
                                                 e->tp, e->tp_done), "rmsnorm");
     }
+    if (wide_batch(T)) {
+        image = true;
+        return count(e, launch_norm_batch(e->ctx->stream, e->hidden, delta, w, c.hidden_size, c.rms_norm_eps, x_norm, T, e->signs, act_of(e, T), pdl), "rmsnorm");
+    }
     return count(e, launch_rmsnorm_quant_x(e->ctx->stream, e->hidden, delta, w, c.hidden_size, c.rms_norm_eps, e->act_q, e->act_s, e->act_m, x_norm, T, pdl), "rmsnorm");
+}
+
+bool expert_swiglu(KronosCudaEngine *e, const float *gate_up, uint32_t d_ff, uint32_t n_slot, int8_t *q, float *sc, int32_t *sums, bool wide, const char *what) {
+    cudaStream_t s = e->ctx->stream;
+    return count(e, wide ? launch_swiglu_batch(s, true, gate_up, d_ff, n_slot, 0, e->signs, PromptAct{q, sc, sums}, e->pdl)
+                         : launch_expert_swiglu_quant(s, gate_up, d_ff, n_slot, q, sc, sums, e->pdl), what);
 }
 
 bool enqueue_attention(KronosCudaEngine *e, uint32_t l, uint32_t t, uint32_t T, bool long_ctx);
@@ -238,7 +256,7 @@ bool enqueue_attention_batch(KronosCudaEngine *e, uint32_t l, uint32_t T) {
     qa.q_i8 = e->q_i8; qa.q_scale = e->q_scale; qa.k_q8 = e->k_q8; qa.v_q8 = e->v_q8; qa.k_scale = e->k_scale; qa.v_scale = e->v_scale;
     qa.n_q = c.num_attention_heads; qa.n_kv = c.num_key_value_heads; qa.head_dim = hd; qa.max_seq = e->kv_stride; qa.layer = l;
     qa.eps = c.rms_norm_eps; qa.qk_norm_after_rope = c.qk_norm_after_rope; qa.kv_bits = c.kv_bits; qa.ring = e->ring; qa.v_t = e->v_t;
-    if (!count(e, launch_qkv_post(s, qa, e->pdl, T), "qkv_post")) return false;
+    if (!count(e, wide_batch(T) && heads_batch_takes(qa) ? launch_heads_batch(s, qa, T, e->signs, e->pdl) : launch_qkv_post(s, qa, e->pdl, T), "qkv_post")) return false;
     ExactAttnArgs xa{};
     xa.q_i8 = e->q_i8; xa.q_scale = e->q_scale; xa.k_q8 = e->k_q8; xa.v_q8 = e->v_q8; xa.k_scale = e->k_scale; xa.v_scale = e->v_scale;
     xa.pos = e->d_pos; xa.pos_offset = 0;
@@ -326,17 +344,19 @@ bool enqueue_batch(KronosCudaEngine *e, uint32_t T, bool embed, Tail tail, bool 
     if (e->blocks) return blocks_enqueue(e, T, embed, tail);
     if (T == 1 && e->fused && tail != Tail::None) return enqueue_fused_step(e, embed, tail, long_ctx);
     e->final_hidden = nullptr;
+    if (wide_batch(T) && !cuda_ok(e->ctx, cudaMemsetAsync(e->act_half.zero, 0, 4, s), "clear image word")) return false;
     if (embed) {
         EmbedArgs a{};
         fill_embed_args(e, a);
         if (!count(e, launch_embed(s, a, T, false), "embed")) return false;
     }
+    bool image = false;
     for (uint32_t l = 0; l < c.num_layers; ++l) {
         const EngineLayer &L = e->layers[l];
         // the FFN output of the layer before: partial sums under tensor parallelism, and after a MoE block under expert parallelism
         const bool ffn_partial = c.tp_size > 1 || (c.ep_size > 1 && l > 0 && e->layers[l - 1].moe);
-        if (!norm_quant(e, l == 0 ? nullptr : e->proj, L.input_norm, nullptr, T, e->pdl && (embed || l > 0), ffn_partial)) return false;
-        if (!gemv(e, L.qkv, e->qkv, "gemv qkv", T)) return false;
+        if (!norm_quant(e, l == 0 ? nullptr : e->proj, L.input_norm, nullptr, T, e->pdl && (embed || l > 0), ffn_partial, image)) return false;
+        if (!gemv(e, L.qkv, e->qkv, "gemv qkv", T, 0, image)) return false;
         if (T > 1 && !e->split_kv) {
             if (!enqueue_attention_batch(e, l, T)) return false;
         } else {
@@ -349,14 +369,14 @@ bool enqueue_batch(KronosCudaEngine *e, uint32_t T, bool embed, Tail tail, bool 
             // (forward_layer_coalesced_batch, 1090-1352, gives each token the same sums: its routes are visited in ascending
             // expert order either way): routes of all tokens, then the expert projections over the (token, route) pairs -
             // slot = token * k + route; two tokens that picked the same expert read its image twice, the second time from L2.
-            if (!norm_quant(e, e->proj, L.post_norm, e->x_norm, T, e->pdl, c.tp_size > 1)) return false;
+            if (!norm_quant(e, e->proj, L.post_norm, e->x_norm, T, e->pdl, c.tp_size > 1, image)) return false;
             const uint32_t k = std::min(c.moe_top_k, c.moe_num_experts), dff = c.moe_d_ff;
             // shared expert (every token; under expert parallelism rank 0's partial sum carries it): two plain projections
             // around the experts' SwiGLU kernel, and its sigmoid gate
             const bool shared = L.gate_up != nullptr && (c.ep_size <= 1 || c.ep_rank == 0);
             if (shared) {
-                if (!gemv(e, L.gate_up, e->sh_gu, "shared gate_up", T)) return false;
-                if (!count(e, launch_expert_swiglu_quant(s, e->sh_gu, L.sh_inter, T, e->sh_q, e->sh_s, e->sh_m, e->pdl), "shared swiglu")) return false;
+                if (!gemv(e, L.gate_up, e->sh_gu, "shared gate_up", T, 0, image)) return false;
+                if (!expert_swiglu(e, e->sh_gu, L.sh_inter, T, e->sh_q, e->sh_s, e->sh_m, wide_batch(T), "shared swiglu")) return false;
                 if (!gemv_from(e, L.down, e->sh_q, e->sh_s, e->sh_m, e->sh_out, "shared down", T)) return false;
                 if (L.sh_gate_w && !count(e, launch_shared_gate(s, L.sh_gate_w, e->x_norm, h, T, e->sh_scale, e->pdl), "shared gate")) return false;
             }
@@ -371,7 +391,7 @@ bool enqueue_batch(KronosCudaEngine *e, uint32_t T, bool embed, Tail tail, bool 
             if (!count(e, grouped ? launch_gemm_experts(s, L.gu_dm, L.gu_fmt, L.d_gu_books, L.d_gu_bases, E, e->tiles, T * k, k, e->act_q, e->act_s, e->moe_gu, e->ctx->d_err, e->pdl)
                                   : launch_gemv_experts(s, L.gu_dm, L.gu_fmt, L.d_gu_books, L.d_gu_bases, L.d_route_ids, T * k, e->act_q, e->act_s, e->act_m, h, h / 64,
                                                         e->moe_gu, (size_t)2 * dff, e->ctx->sm_count, e->ctx->d_err, e->pdl, E, k, 32, k), "expert gate_up")) return false;
-            if (!count(e, launch_expert_swiglu_quant(s, e->moe_gu, dff, T * k, e->moe_q, e->moe_s, e->moe_m, e->pdl), "expert swiglu")) return false;
+            if (!expert_swiglu(e, e->moe_gu, dff, T * k, e->moe_q, e->moe_s, e->moe_m, wide_batch(T), "expert swiglu")) return false;
             if (!count(e, grouped ? launch_gemm_experts(s, L.dn_dm, L.dn_fmt, L.d_dn_books, L.d_dn_bases, E, e->tiles, T * k, 1, e->moe_q, e->moe_s, e->moe_out, e->ctx->d_err, e->pdl)
                                   : launch_gemv_experts(s, L.dn_dm, L.dn_fmt, L.d_dn_books, L.d_dn_bases, L.d_route_ids, T * k, e->moe_q, e->moe_s, e->moe_m, dff, dff / 64,
                                                         e->moe_out, h, e->ctx->sm_count, e->ctx->d_err, e->pdl, E, k, 32, 1), "expert down")) return false;
@@ -379,17 +399,19 @@ bool enqueue_batch(KronosCudaEngine *e, uint32_t T, bool embed, Tail tail, bool 
                                              c.moe_num_experts, T, 32, shared ? e->sh_out : nullptr, shared && L.sh_gate_w ? e->sh_scale : nullptr), "moe combine")) return false;
             continue;
         }
-        if (!norm_quant(e, e->proj, L.post_norm, nullptr, T, e->pdl, c.tp_size > 1)) return false;
-        if (!gemv(e, L.gate_up, e->gate_up, "gemv gate_up", T)) return false;
-        if (!count(e, launch_swiglu_quant(s, e->gate_up, inter, e->act_q, e->act_s, e->act_m, nullptr, c.down_chunk0, T, e->pdl), "swiglu")) return false;
-        if (!gemv(e, L.down, e->proj, "gemv down", T)) return false;
+        if (!norm_quant(e, e->proj, L.post_norm, nullptr, T, e->pdl, c.tp_size > 1, image)) return false;
+        if (!gemv(e, L.gate_up, e->gate_up, "gemv gate_up", T, 0, image)) return false;
+        image = wide_batch(T);
+        if (!count(e, image ? launch_swiglu_batch(s, false, e->gate_up, inter, T, c.down_chunk0, e->signs, act_of(e, T), e->pdl)
+                            : launch_swiglu_quant(s, e->gate_up, inter, e->act_q, e->act_s, e->act_m, nullptr, c.down_chunk0, T, e->pdl), "swiglu")) return false;
+        if (!gemv(e, L.down, e->proj, "gemv down", T, 0, image)) return false;
     }
     // the last residual is folded into `hidden` by the final norm even when no logits are wanted
-    if (!norm_quant(e, e->proj, e->final_norm, nullptr, T, e->pdl, c.tp_size > 1 || (c.ep_size > 1 && e->layers.back().moe))) return false;
+    if (!norm_quant(e, e->proj, e->final_norm, nullptr, T, e->pdl, c.tp_size > 1 || (c.ep_size > 1 && e->layers.back().moe), image)) return false;
     const uint32_t vocab_all = c.tp_size > 1 ? c.vocab_total : c.vocab_size;
     float *lg = c.tp_size > 1 ? e->logits_local : e->logits;        // under tp: this rank's slice, then gathered into `logits`
     if (tail == Tail::AllLogits || tail == Tail::Greedy) {
-        if (!gemv(e, e->lm_head, lg, "gemv lm_head", T)) return false;
+        if (!gemv(e, e->lm_head, lg, "gemv lm_head", T, 0, image)) return false;
         for (uint32_t t = 0; t < T && c.tp_size > 1; ++t)
             if (!tp_gather(e, lg + (size_t)t * c.vocab_size, e->logits + (size_t)t * vocab_all, c.vocab_size)) return false;
     } else if (tail == Tail::LastLogits) {
@@ -761,6 +783,8 @@ KronosCudaEngine *kronos_cuda_engine_create(KronosCudaContext *ctx, const Kronos
     if (!e->lm_head) return bad("engine_create: lm_head: " + ctx->err);
     e->weight_bytes += e->lm_head->dm.geom.file_bytes;
     const uint32_t act_n = std::max(std::max(h, q_dim), inter), n_q = c.num_attention_heads;
+    // rotations of the small prompt operators: the residual stream, SwiGLU from its first chunk on, experts and shared experts, two blocks of a head
+    const uint32_t sign_chunks = std::max(std::max(h / 64, inter / 64 + c.down_chunk0), std::max(std::max(e->sh_inter_max, e->has_moe ? c.moe_d_ff : 0u) / 64, 2u));
     bool ok = dev_alloc(e, e->final_norm, h, final_norm) && dev_alloc(e, e->rope, (size_t)c.max_seq_len * hd, rope) &&
               (embed_bf16 == nullptr || dev_alloc(e, e->embed_bf16, (size_t)(c.tp_size > 1 ? c.vocab_total : c.vocab_size) * h, embed_bf16)) &&   // every rank keeps the whole table
               // per-token vectors hold max_batch tokens (prompt batches), [token][n]
@@ -768,7 +792,8 @@ KronosCudaEngine *kronos_cuda_engine_create(KronosCudaContext *ctx, const Kronos
               dev_alloc(e, e->qkv, (size_t)e->max_batch * qkv_rows) && dev_alloc(e, e->gate_up, (size_t)e->max_batch * 2 * inter) &&
               dev_alloc(e, e->logits, (size_t)e->max_batch * (c.tp_size > 1 ? c.vocab_total : c.vocab_size)) && dev_alloc(e, e->act_q, (size_t)e->max_batch * act_n) &&
               dev_alloc(e, e->act_s, (size_t)e->max_batch * act_n / 64) && dev_alloc(e, e->act_m, (size_t)e->max_batch * act_n / 64) &&
-              dev_alloc(e, e->act_half.img, act_half_bytes(e->max_batch, std::max(act_n, e->sh_inter_max))) &&
+              dev_alloc(e, e->signs, sign_table_bytes(sign_chunks)) && cuda_ok(ctx, launch_sign_table(ctx->stream, e->signs, sign_chunks), "sign table") &&
+              dev_alloc(e, e->act_half.zero, 1) && dev_alloc(e, e->act_half.img, act_half_bytes(e->max_batch, std::max(act_n, e->sh_inter_max))) &&
               dev_alloc(e, e->act_half.scales, act_half_scale_bytes(e->max_batch, std::max(act_n, e->sh_inter_max))) &&
               dev_alloc(e, e->q_i8, (size_t)e->max_batch * q_dim) && dev_alloc(e, e->attn_tap, q_dim) && dev_alloc(e, e->q_scale, (size_t)e->max_batch * n_q) &&
               dev_alloc(e, e->part_m, (size_t)n_q * e->n_split) && dev_alloc(e, e->part_l, (size_t)n_q * e->n_split) &&

@@ -48,6 +48,7 @@ struct KronosCudaEngine {
     float *attn_sc = nullptr, *attn_bmax = nullptr;      // long contexts in CPU order: scores [n_q][kv_stride], block maxima [n_q][kv_stride / 128]
     bool split_kv = false;                    // long contexts by the split-KV kernels instead (config flag, or the cache is too long for the exact path)
     int32_t *act_m = nullptr;
+    uint8_t *signs = nullptr;                 // rotation signs by chunk (k2t_prompt_ops.cu)
     k2t::ActHalf act_half;                    // operand image of a prompt batch's activations, rewritten by every projection
     int8_t *k_q8 = nullptr, *v_q8 = nullptr;
     int8_t *v_t = nullptr;      // int8 cache without a window: the value rows once more, transposed in 16-position blocks for the value chains

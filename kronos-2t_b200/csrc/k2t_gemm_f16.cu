@@ -28,9 +28,8 @@
 // What bounds it: instruction issue (0.59 per scheduler and cycle, 3000 warp instructions per chunk of 128 rows x 128 tokens, half of
 // them chain steps and expansion, the rest waits and hand-overs).
 #include <algorithm>
-#include <cuda_fp16.h>
 
-#include "k2t_gemm_f16.h"
+#include "k2t_act_image.cuh"
 #include "k2t_gemv_core.cuh"
 
 namespace k2t {
@@ -44,7 +43,6 @@ constexpr uint32_t HF_SLOTS = 8;             // chunks whose scales (weights and
 constexpr uint32_t HF_WAIT_LIMIT = 1u << 21;
 constexpr uint32_t HF_HEADER = 1024;
 constexpr uint32_t HF_A_STAGE = HF_M * 128;
-constexpr uint32_t HF_REC = 144;             // bytes per (chunk, 32 tokens) of the scale image: 32 scales, a flag, padding
 
 // EXP: a tile of an expert's (token, route) pairs, few chunks deep.  Half the warps and 113 KB at most, so that two CTAs share an SM and
 // one's start and end run under the other's chunks.
@@ -75,6 +73,7 @@ template <int FMT, int N, bool EXP = false> struct HfLayout {
 struct HfArgs {
     GemvArgs g;
     const uint8_t *img, *xs_img;
+    const uint32_t *zero;              // image left by the kernel that quantized: not zero where any of its scales is; else null
     uint32_t n_tok, tok_pad;
 };
 
@@ -154,14 +153,6 @@ __device__ __forceinline__ bool hf_wait(uint32_t bar, uint32_t parity, volatile 
     }
     *abort_w = 1;
     return false;
-}
-
-// four bytes (each 0..255, standing for byte - 1024 - add) -> four halves: 0x6400 | b is the half 1024 + b
-__device__ __forceinline__ void hf_widen(uint32_t bytes, __half2 add, uint32_t &h0, uint32_t &h1) {
-    const uint32_t a = prmt(bytes, 0x64646464u, 0x4140u), b = prmt(bytes, 0x64646464u, 0x4342u);
-    const __half2 x = __hadd2(*reinterpret_cast<const __half2 *>(&a), add), y = __hadd2(*reinterpret_cast<const __half2 *>(&b), add);
-    h0 = *reinterpret_cast<const uint32_t *>(&x);
-    h1 = *reinterpret_cast<const uint32_t *>(&y);
 }
 
 // A row's cell -> 64 halves in column order.  Bit-planes: 2 code - (2^B - 1), codebooks: the centroid.
@@ -247,9 +238,18 @@ __global__ void __launch_bounds__(HfRoles<N, EXP>::THREADS, EXP ? 2 : 1) gemm_f1
 #pragma unroll
         for (uint32_t t = 0; t < NQ / 2; ++t) f[t] = 0;
         const uint32_t rec = (part * NQ) / 32, xs_sa = sbase + L::XS + rec * HF_REC + ((part * NQ) % 32) * 4, flag_sa = sbase + L::XS + rec * HF_REC + 128;
+        // zero scales: a flag per record, or (image_ready) one word for the whole image and, where that is set, a look at the scales
+        // themselves; a token behind the batch then has no scale of its own (its column is never stored)
+        bool own_behind = false, all_plain = false, ready = false;
+        const uint32_t xs_own = xs_sa + (lane % NQ) * 4;
         const uint32_t ws_sa = sbase + L::WS + (quarter * 32 + lane) * 4;
         const uint32_t taddr0 = tmem + ((quarter * 32u) << 16) + part * NQ;
-        if (!EXP) pdl_wait();
+        if constexpr (!EXP) {
+            pdl_wait();
+            own_behind = tok0 + part * NQ + lane % NQ >= args.n_tok;
+            ready = args.zero != nullptr;
+            all_plain = ready && __ldcg(args.zero) == 0;
+        }
         bool ok = true;
         uint32_t s = 0, ph = 0;
 #pragma unroll 1
@@ -258,13 +258,20 @@ __global__ void __launch_bounds__(HfRoles<N, EXP>::THREADS, EXP ? 2 : 1) gemm_f1
             ok = hf_wait(bar_done + 8 * s, ph, s_abort) && hf_wait(bar_full + 8 * s, ph, s_abort);
             if (!ok) break;
             hf_fence_after();
+            uint32_t ws_bits[2], any[2];          // of both chunks, requested together (a second chunk that does not exist: old ones, not used)
+#pragma unroll
+            for (uint32_t k = 0; k < 2; ++k) {
+                const uint32_t slot = (c0 + k) % HF_SLOTS;
+                ws_bits[k] = hf_lds32(ws_sa + slot * (HF_M * 4));
+                any[k] = all_plain ? 0u : hf_lds32((ready ? xs_own : flag_sa) + slot * ((N / 32) * HF_REC));
+            }
 #pragma unroll
             for (uint32_t k = 0; k < 2; ++k) {
                 if (c0 + k < nc) {
-                    const uint32_t slot = (c0 + k) % HF_SLOTS, xo = slot * ((N / 32) * HF_REC);
-                    const uint32_t wsb = hf_lds32(ws_sa + slot * (HF_M * 4));
-                    const unsigned long long ws2 = hf_pack(wsb, wsb);
-                    const bool plain = hf_lds32(flag_sa + xo) != 0;
+                    const uint32_t xo = ((c0 + k) % HF_SLOTS) * ((N / 32) * HF_REC);
+                    const unsigned long long ws2 = hf_pack(ws_bits[k], ws_bits[k]);
+                    bool plain = all_plain;
+                    if (!plain) plain = ready ? __all_sync(0xffffffffu, own_behind || __uint_as_float(any[k]) != 0.0f) : any[k] != 0;
 #pragma unroll
                     for (uint32_t h = 0; h < NQ / 16; ++h) {
                         uint32_t v[16];
@@ -536,16 +543,9 @@ __global__ void __launch_bounds__(256) act_half_kernel(const int8_t *q, const fl
                 v[0] = __ldcg(p);
                 v[1] = __ldcg(p + 1);
             }
-            const __half2 add = __half2half2(__int2half_rn(-1152));
-            uint8_t *dst = img + ((size_t)c * tok_pad + t) * 128;
 #pragma unroll
-            for (uint32_t k = 0; k < 4; ++k) {          // eight columns per 16-byte piece
-                const uint32_t x = (k & 1u) ? v[k >> 1].z : v[k >> 1].x, y = (k & 1u) ? v[k >> 1].w : v[k >> 1].y;
-                uint4 h;
-                hf_widen(x ^ 0x80808080u, add, h.x, h.y);
-                hf_widen(y ^ 0x80808080u, add, h.z, h.w);
-                *reinterpret_cast<uint4 *>(dst + (((part * 4 + k) ^ (t & 7u)) << 4)) = h;
-            }
+            for (uint32_t k = 0; k < 4; ++k)
+                image_piece(img, tok_pad, c, t, part * 4 + k, (k & 1u) ? make_uint2(v[k >> 1].z, v[k >> 1].w) : make_uint2(v[k >> 1].x, v[k >> 1].y));
         }
     }
     if (tid < 128) {
@@ -553,9 +553,8 @@ __global__ void __launch_bounds__(256) act_half_kernel(const int8_t *q, const fl
         const float s = (t < n_tok && c < nc) ? __ldcg(xs + (size_t)t * nc + c) : 1.0f;
         const bool plain = __all_sync(0xffffffffu, s != 0.0f);
         if (c < nc) {
-            uint8_t *rec = xs_img + ((size_t)c * (tok_pad / 32) + blockIdx.y) * HF_REC;
-            reinterpret_cast<float *>(rec)[lane] = s;
-            if (lane < 4) reinterpret_cast<uint32_t *>(rec + 128)[lane] = plain ? 1u : 0u;
+            image_scale(xs_img, tok_pad, c, t, s);
+            if (lane == 0) *reinterpret_cast<uint32_t *>(xs_img + ((size_t)c * (tok_pad / 32) + blockIdx.y) * HF_REC + 128) = plain ? 1u : 0u;
         }
     }
 }
@@ -661,19 +660,19 @@ cudaError_t launch_gemm_experts(cudaStream_t stream, const DeviceMatrix &m0, int
     }
 }
 
-size_t act_half_bytes(size_t n_tok, uint32_t cols) { return ((n_tok + 127) & ~(size_t)127) * cols * 2; }
-size_t act_half_scale_bytes(size_t n_tok, uint32_t cols) { return ((n_tok + 127) & ~(size_t)127) / 32 * (cols / 64) * HF_REC; }
+size_t act_half_bytes(size_t n_tok, uint32_t cols) { return act_half_tokens(n_tok) * cols * 2; }
+size_t act_half_scale_bytes(size_t n_tok, uint32_t cols) { return act_half_tokens(n_tok) / 32 * (cols / 64) * HF_REC; }
 
 cudaError_t launch_gemm_f16(cudaStream_t stream, const DeviceMatrix &m, const int8_t *xq, const float *xs, uint32_t n_tok, const ActHalf &h,
-                            float *out, size_t out_stride, int sm_count, uint32_t *err_flag, uint32_t *launches, bool pdl) {
+                            float *out, size_t out_stride, int sm_count, uint32_t *err_flag, uint32_t *launches, bool pdl, bool image_ready) {
     if (launches) *launches = 0;
-    const uint32_t tok_pad = (n_tok + 127u) & ~127u;
-    if (n_tok == 0 || n_tok > 0xFFFFu * 32u) return cudaErrorInvalidValue;
+    const uint32_t tok_pad = (uint32_t)act_half_tokens(n_tok);
+    if (n_tok == 0 || n_tok > 0xFFFFu * 32u || (image_ready && h.zero == nullptr)) return cudaErrorInvalidValue;
     HfArgs args;
     const int fmt = fill_gemv_args(m, true, args.g);
     args.g.out = out; args.g.err_flag = err_flag; args.g.out_stride = out_stride;
-    args.img = h.img; args.xs_img = h.scales; args.n_tok = n_tok; args.tok_pad = tok_pad;
-    cudaError_t e = launch_kernel(act_half_kernel, dim3((m.geom.nc + 3) / 4, tok_pad / 32), dim3(256), 0, stream, pdl, xq, xs, n_tok, m.geom.nc, tok_pad, h.img, h.scales);
+    args.img = h.img; args.xs_img = h.scales; args.zero = image_ready ? h.zero : nullptr; args.n_tok = n_tok; args.tok_pad = tok_pad;
+    cudaError_t e = image_ready ? cudaSuccess : launch_kernel(act_half_kernel, dim3((m.geom.nc + 3) / 4, tok_pad / 32), dim3(256), 0, stream, pdl, xq, xs, n_tok, m.geom.nc, tok_pad, h.img, h.scales);
     if (e != cudaSuccess) return e;
     switch (fmt) {
         case FMT_BP4: e = launch_hf_fmt<FMT_BP4>(stream, args, sm_count, pdl); break;
@@ -686,7 +685,7 @@ cudaError_t launch_gemm_f16(cudaStream_t stream, const DeviceMatrix &m, const in
         case FMT_E8Q2: e = launch_hf_fmt<FMT_E8Q2>(stream, args, sm_count, pdl); break;
         default: return cudaErrorNotSupported;
     }
-    if (e == cudaSuccess && launches) *launches = 2;
+    if (e == cudaSuccess && launches) *launches = image_ready ? 1 : 2;
     return e;
 }
 

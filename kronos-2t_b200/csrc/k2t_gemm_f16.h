@@ -13,14 +13,16 @@ namespace k2t {
 struct ActHalf {
     uint8_t *img = nullptr;          // act_half_bytes, 1024-byte aligned
     uint8_t *scales = nullptr;       // act_half_scale_bytes, 16-byte aligned
+    uint32_t *zero = nullptr;        // images of k2t_prompt_ops.cu: set when a chunk without a scale was written since the caller cleared it
 };
+inline size_t act_half_tokens(size_t n_tok) { return (n_tok + 127) & ~(size_t)127; }
 size_t act_half_bytes(size_t n_tok, uint32_t cols);
 size_t act_half_scale_bytes(size_t n_tok, uint32_t cols);
 
 // y[t] = W x[t] for activations in the form the library's own quantizers leave them (the sums of a chunk are those of its values):
-// two launches, the image and the product.
+// two launches, the image and the product; image_ready: the kernel that quantized them has left the image (k2t_prompt_ops.cu).
 cudaError_t launch_gemm_f16(cudaStream_t stream, const DeviceMatrix &m, const int8_t *xq, const float *xs, uint32_t n_tok, const ActHalf &h,
-                            float *out, size_t out_stride, int sm_count, uint32_t *err_flag, uint32_t *launches, bool pdl);
+                            float *out, size_t out_stride, int sm_count, uint32_t *err_flag, uint32_t *launches, bool pdl, bool image_ready = false);
 
 // The (token, route) pairs of a batch in tiles of 32 of one expert: device scratch of the caller.
 struct ExpertTiles {
