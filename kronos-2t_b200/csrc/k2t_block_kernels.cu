@@ -84,6 +84,80 @@ __global__ void __launch_bounds__(1024) block_norm_kernel(const NormArgs a) {
     }
 }
 
+// The same for many tokens: 128 threads per token with VPT quadruples each, all requested at once and kept in registers.  One
+// quadruple per thread leaves an SM waiting at the barriers of a few large CTAs: 2048 tokens of 2048 columns 16.3 -> 14.5 us (4.0 TB/s).
+constexpr uint32_t NW_THREADS = 128;
+template <bool F32, bool ADD, bool PRE, int VPT>
+__global__ void __launch_bounds__(NW_THREADS) block_norm_wide_kernel(const NormArgs a) {
+    __shared__ float scratch[32];
+    const uint32_t t = blockIdx.x, n = a.n;
+    float *xr = a.x + t * a.x_stride, *yr = ADD ? a.y + t * a.y_stride : nullptr;
+    float4 x[VPT], v[VPT];
+    float ss[1] = {0.0f};
+    pdl_wait();
+    pdl_trigger();
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+        const uint32_t k = (threadIdx.x + i * NW_THREADS) * 4;
+        x[i] = v[i] = make_float4(0, 0, 0, 0);
+        if (k < n) {
+            x[i] = load4(xr, k, n);
+            if (ADD) v[i] = load4(yr, k, n);
+        }
+    }
+    if (ADD) {
+        for (uint32_t j = 0; j < a.top; ++j) {
+            const float w = __ldcg(a.weight + t * a.top + j);
+            const float *pr = a.pairs + (size_t)__ldcg(a.row + t * a.top + j) * a.pair_stride;
+#pragma unroll
+            for (int i = 0; i < VPT; ++i) {
+                const uint32_t k = (threadIdx.x + i * NW_THREADS) * 4;
+                if (k < n) {
+                    const float4 q = load4(pr, k, n);
+                    v[i] = make_float4(__fmaf_rn(w, q.x, v[i].x), __fmaf_rn(w, q.y, v[i].y), __fmaf_rn(w, q.z, v[i].z), __fmaf_rn(w, q.w, v[i].w));
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < VPT; ++i) ss[0] = sq4(v[i], ss[0]);
+        block_sum<1>(ss, scratch);
+        const float inv = 1.0f / sqrtf(ss[0] / (float)n + a.eps);
+        ss[0] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < VPT; ++i) {
+            const uint32_t k = (threadIdx.x + i * NW_THREADS) * 4;
+            if (k < n) {
+                const float4 g = __ldg(reinterpret_cast<const float4 *>(a.post + k)), o = x[i];
+                x[i] = make_float4(o.x + a.mult * (v[i].x * inv * g.x), o.y + a.mult * (v[i].y * inv * g.y), o.z + a.mult * (v[i].z * inv * g.z), o.w + a.mult * (v[i].w * inv * g.w));
+                *reinterpret_cast<float4 *>(xr + k) = x[i];
+                if (!PRE) act_store4<F32>(a.out, t, k, n, x[i]);
+            }
+        }
+    }
+    if (PRE) {
+#pragma unroll
+        for (int i = 0; i < VPT; ++i) {
+            const uint32_t k = (threadIdx.x + i * NW_THREADS) * 4;
+            if (k < n) ss[0] = sq4(x[i], ss[0]);
+        }
+        block_sum<1>(ss, scratch);
+        const float inv = 1.0f / sqrtf(ss[0] / (float)n + a.eps);
+#pragma unroll
+        for (int i = 0; i < VPT; ++i) {
+            const uint32_t k = (threadIdx.x + i * NW_THREADS) * 4;
+            if (k < n) {
+                const float4 g = __ldg(reinterpret_cast<const float4 *>(a.pre + k));
+                act_store4<F32>(a.out, t, k, n, make_float4(x[i].x * inv * g.x, x[i].y * inv * g.y, x[i].z * inv * g.z, x[i].w * inv * g.w));
+            }
+        }
+    }
+}
+template <int VPT> cudaError_t launch_norm_wide(cudaStream_t s, bool f32, const NormArgs &a, uint32_t n_tok, bool pdl) {
+    auto k = f32 ? (a.y == nullptr ? block_norm_wide_kernel<true, false, true, VPT> : a.pre == nullptr ? block_norm_wide_kernel<true, true, false, VPT> : block_norm_wide_kernel<true, true, true, VPT>)
+                 : (a.y == nullptr ? block_norm_wide_kernel<false, false, true, VPT> : a.pre == nullptr ? block_norm_wide_kernel<false, true, false, VPT> : block_norm_wide_kernel<false, true, true, VPT>);
+    return launch_kernel(k, dim3(n_tok), dim3(NW_THREADS), 0, s, pdl, a);
+}
+
 // A cluster of `cs` CTAs per token; CTA r holds the panels [r np / cs, (r + 1) np / cs) of the vector.  Two exchanges over
 // distributed shared memory: the sublayer's sum of squares together with the partial gate products - of x and of y w apart, so
 // that the products need not wait for the norm: gate (x + y w / rms) = gate x + gate (y w) / rms - and the token input's sum of
@@ -274,6 +348,10 @@ cudaError_t launch_block_embed(cudaStream_t s, bool f32, const uint16_t *table, 
 
 cudaError_t launch_block_norm(cudaStream_t s, bool f32, const NormArgs &a, uint32_t n_tok, bool pdl) {
     if (a.y == nullptr && a.pre == nullptr) return cudaErrorInvalidValue;
+    // as many tokens as keep every SM in several CTAs: a prompt of 300 tokens took 1.91 ms with large CTAs and 1.95 ms this way, one of
+    // 1000 tokens (1024 columns) 2.13 and 2.11 ms
+    if (n_tok >= 5 * 148 && a.n > 4 * NW_THREADS && a.n <= 32 * NW_THREADS)
+        return a.n <= 8 * NW_THREADS ? launch_norm_wide<2>(s, f32, a, n_tok, pdl) : a.n <= 16 * NW_THREADS ? launch_norm_wide<4>(s, f32, a, n_tok, pdl) : launch_norm_wide<8>(s, f32, a, n_tok, pdl);
     const uint32_t threads = std::min(n_tok > 64 ? 512u : 1024u, std::max(32u, ((a.n + 3) / 4 + 31u) & ~31u));
     auto k = f32 ? (a.y == nullptr ? block_norm_kernel<true, false, true> : a.pre == nullptr ? block_norm_kernel<true, true, false> : block_norm_kernel<true, true, true>)
                  : (a.y == nullptr ? block_norm_kernel<false, false, true> : a.pre == nullptr ? block_norm_kernel<false, true, false> : block_norm_kernel<false, true, true>);
