@@ -84,16 +84,41 @@ __global__ void __launch_bounds__(1024) block_norm_kernel(const NormArgs a) {
     }
 }
 
-// The same for many tokens: 128 threads per token with VPT quadruples each, all requested at once and kept in registers.  One
-// quadruple per thread leaves an SM waiting at the barriers of a few large CTAs: 2048 tokens of 2048 columns 16.3 -> 14.5 us (4.0 TB/s).
-constexpr uint32_t NW_THREADS = 128;
+// The same for many tokens, to the same bits: 128 threads per token with VPT quadruples each, all requested at once and kept in
+// registers; an SM holds sixteen tokens where it holds four of the large CTAs.  Whole prompts through four blocks, large CTAs -> this
+// form: 2048 tokens of Folizen medium (2048 columns) 2321 -> 2289 us, of Zasesun small (1024 columns) 901 -> 882 us.
+constexpr uint32_t NW_THREADS = 128, NW_MIN_TOKENS = 592;
+// The sum block_sum gives min(512, VPT * 128) threads with one quadruple each (from the 512th quadruple on a second one, already
+// added to part[i - 4]): the quadruples of this kernel's warp w are those of warps 4 i + w there, each summed over its lanes by itself.
+template <int CHAINS> __device__ __forceinline__ float wide_sum(float (&part)[CHAINS], float *scratch) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float v;
+    if constexpr (CHAINS == 4) {          // warp_sum of four values at once: a lane passes half of its sums on at each of the first two steps
+        const bool up16 = (lane & 16u) != 0, up8 = (lane & 8u) != 0;
+        const float k0 = up16 ? part[2] : part[0], k1 = up16 ? part[3] : part[1], g0 = up16 ? part[0] : part[2], g1 = up16 ? part[1] : part[3];
+        const float s0 = __fadd_rn(k0, __shfl_xor_sync(0xffffffffu, g0, 16)), s1 = __fadd_rn(k1, __shfl_xor_sync(0xffffffffu, g1, 16));
+        v = __fadd_rn(up8 ? s1 : s0, __shfl_xor_sync(0xffffffffu, up8 ? s0 : s1, 8));
+    } else {
+        const bool up16 = (lane & 16u) != 0;
+        v = __fadd_rn(up16 ? part[1] : part[0], __shfl_xor_sync(0xffffffffu, up16 ? part[0] : part[1], 16));
+        v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 8));
+    }
+#pragma unroll
+    for (int m = 4; m > 0; m >>= 1) v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, m));
+    __syncthreads();
+    const uint32_t chain = CHAINS == 4 ? ((lane >> 4) << 1) | ((lane >> 3) & 1u) : lane >> 4;
+    if ((lane & (CHAINS == 4 ? 7u : 15u)) == 0) scratch[4 * chain + warp] = v;
+    __syncthreads();
+    return warp_sum(lane < 4 * CHAINS ? scratch[lane] : 0.0f);
+}
 template <bool F32, bool ADD, bool PRE, int VPT>
 __global__ void __launch_bounds__(NW_THREADS) block_norm_wide_kernel(const NormArgs a) {
-    __shared__ float scratch[32];
+    constexpr int CHAINS = VPT < 4 ? VPT : 4;
+    __shared__ float scratch[16];
     const uint32_t t = blockIdx.x, n = a.n;
     float *xr = a.x + t * a.x_stride, *yr = ADD ? a.y + t * a.y_stride : nullptr;
     float4 x[VPT], v[VPT];
-    float ss[1] = {0.0f};
+    float part[CHAINS];
     pdl_wait();
     pdl_trigger();
 #pragma unroll
@@ -119,10 +144,8 @@ __global__ void __launch_bounds__(NW_THREADS) block_norm_wide_kernel(const NormA
             }
         }
 #pragma unroll
-        for (int i = 0; i < VPT; ++i) ss[0] = sq4(v[i], ss[0]);
-        block_sum<1>(ss, scratch);
-        const float inv = 1.0f / sqrtf(ss[0] / (float)n + a.eps);
-        ss[0] = 0.0f;
+        for (int i = 0; i < VPT; ++i) part[i % CHAINS] = sq4(v[i], i < CHAINS ? 0.0f : part[i % CHAINS]);
+        const float inv = 1.0f / sqrtf(wide_sum(part, scratch) / (float)n + a.eps);
 #pragma unroll
         for (int i = 0; i < VPT; ++i) {
             const uint32_t k = (threadIdx.x + i * NW_THREADS) * 4;
@@ -136,12 +159,8 @@ __global__ void __launch_bounds__(NW_THREADS) block_norm_wide_kernel(const NormA
     }
     if (PRE) {
 #pragma unroll
-        for (int i = 0; i < VPT; ++i) {
-            const uint32_t k = (threadIdx.x + i * NW_THREADS) * 4;
-            if (k < n) ss[0] = sq4(x[i], ss[0]);
-        }
-        block_sum<1>(ss, scratch);
-        const float inv = 1.0f / sqrtf(ss[0] / (float)n + a.eps);
+        for (int i = 0; i < VPT; ++i) part[i % CHAINS] = sq4(x[i], i < CHAINS ? 0.0f : part[i % CHAINS]);
+        const float inv = 1.0f / sqrtf(wide_sum(part, scratch) / (float)n + a.eps);
 #pragma unroll
         for (int i = 0; i < VPT; ++i) {
             const uint32_t k = (threadIdx.x + i * NW_THREADS) * 4;
@@ -348,9 +367,9 @@ cudaError_t launch_block_embed(cudaStream_t s, bool f32, const uint16_t *table, 
 
 cudaError_t launch_block_norm(cudaStream_t s, bool f32, const NormArgs &a, uint32_t n_tok, bool pdl) {
     if (a.y == nullptr && a.pre == nullptr) return cudaErrorInvalidValue;
-    // as many tokens as keep every SM in several CTAs: a prompt of 300 tokens took 1.91 ms with large CTAs and 1.95 ms this way, one of
-    // 1000 tokens (1024 columns) 2.13 and 2.11 ms
-    if (n_tok >= 5 * 148 && a.n > 4 * NW_THREADS && a.n <= 32 * NW_THREADS)
+    // from about as many tokens on as the SMs hold large CTAs at once (4 x 148).  Prompts of Folizen and Zasesun, small and medium, this form
+    // against large CTAs: 450 tokens 0.5 to 1.4% slower, 600 tokens 0.5 to 0.8% faster, 740 tokens 0 to 1.1%, 2048 tokens 0.6 to 2.1% faster
+    if (n_tok >= NW_MIN_TOKENS && a.n > 4 * NW_THREADS && a.n <= 32 * NW_THREADS)
         return a.n <= 8 * NW_THREADS ? launch_norm_wide<2>(s, f32, a, n_tok, pdl) : a.n <= 16 * NW_THREADS ? launch_norm_wide<4>(s, f32, a, n_tok, pdl) : launch_norm_wide<8>(s, f32, a, n_tok, pdl);
     const uint32_t threads = std::min(n_tok > 64 ? 512u : 1024u, std::max(32u, ((a.n + 3) / 4 + 31u) & ~31u));
     auto k = f32 ? (a.y == nullptr ? block_norm_kernel<true, false, true> : a.pre == nullptr ? block_norm_kernel<true, true, false> : block_norm_kernel<true, true, true>)

@@ -19,3 +19,24 @@ def test_long_prompt_and_portions(engine, design, width):  # noqa: F811
     eng = engine(model, "float32")
     whole = eng.forward_token_ids(toks, want_all=True).astype(np.float64)
     assert fm.error(portions(eng, toks, [380]), whole).max() < 2 * TOL["float32"]          # either stays within TOL of the exact values
+
+
+# sublayers whose own results do not depend on the portion (window attention in bfloat16 has tiles of the batch)
+BLOCKS = {
+    "folizen": lambda width: fm.make(width, 40, [fm.delta(2, 16, ff=64), fm.delta(1, 16)]),
+    "zasesun": lambda width: zm.make(width, 40, [zm.latent(2, 16, 8, 16, 24, 32, zm.moe(5, 2, 32, 16)), zm.latent(2, 16, 8, 16, 24, 32, zm.dense(64))]),
+}
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("width", [516, 1024, 1092, 2048, 2052, 4096])
+@pytest.mark.parametrize("design", ["folizen", "zasesun"])
+def test_bits_of_the_other_form(engine, design, width, dtype):  # noqa: F811
+    """Either form sums in the same order: the residual stream of a prompt's last token does not depend on the portion that it is in."""
+    model = BLOCKS[design](width)
+    toks = tokens_of(model, 743)
+    eng = engine(model, dtype)
+    whole = eng.forward_token_ids(toks, want_all=True)
+    stream = eng.read_hidden()
+    assert np.array_equal(portions(eng, toks, [372, 371]), whole)
+    assert np.array_equal(eng.read_hidden(), stream)
