@@ -133,6 +133,20 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok;
 }
+// Bounded wait of one thread on an mbarrier phase; gives up after `limit` polls or once another role has set the CTA's abort word.
+__device__ __forceinline__ bool mbar_wait_thread(uint32_t bar, uint32_t parity, uint32_t limit, volatile uint32_t *abort_w) {
+    for (uint32_t spin = 0; spin < limit; ++spin) {
+        if (mbar_try_wait(bar, parity)) return true;
+        if ((spin & 255u) == 255u && *abort_w != 0) return false;
+    }
+    *abort_w = 1;
+    return false;
+}
+// The same for a whole warp, one answer for its lanes: they poll at different times and may see the phase, the abort word or the limit
+// apart, and a lane that left alone would leave the others at the warp's next collective (a vote, __syncwarp, tcgen05.ld) for good.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, uint32_t limit, volatile uint32_t *abort_w) {
+    return __all_sync(0xffffffffu, mbar_wait_thread(bar, parity, limit, abort_w));
+}
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");

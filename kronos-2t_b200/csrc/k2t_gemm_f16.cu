@@ -146,15 +146,6 @@ __device__ __forceinline__ unsigned long long hf_step2(unsigned long long dot, u
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(p), "l"(ws), "l"(f));
     return r;
 }
-__device__ __forceinline__ bool hf_wait(uint32_t bar, uint32_t parity, volatile uint32_t *abort_w) {
-    for (uint32_t spin = 0; spin < HF_WAIT_LIMIT; ++spin) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((spin & 255u) == 255u && *abort_w != 0) return false;
-    }
-    *abort_w = 1;
-    return false;
-}
-
 // A row's cell -> 64 halves in column order.  Bit-planes: 2 code - (2^B - 1), codebooks: the centroid.
 struct HfTables { uint32_t cb[8], tab[4]; __half2 add; };
 template <int FMT, typename T> __device__ __forceinline__ HfTables hf_tables(const T &a) {          // T: GemvArgs or ExpertCodebook
@@ -255,7 +246,7 @@ __global__ void __launch_bounds__(HfRoles<N, EXP>::THREADS, EXP ? 2 : 1) gemm_f1
 #pragma unroll 1
         for (uint32_t c0 = 0; c0 < nc; c0 += 2) {
             // `full` has completed by the time of `done`: waiting for it orders this thread after the scales' stores and copies
-            ok = hf_wait(bar_done + 8 * s, ph, s_abort) && hf_wait(bar_full + 8 * s, ph, s_abort);
+            ok = mbar_wait_warp(bar_done + 8 * s, ph, HF_WAIT_LIMIT, s_abort) && mbar_wait_warp(bar_full + 8 * s, ph, HF_WAIT_LIMIT, s_abort);
             if (!ok) break;
             hf_fence_after();
             uint32_t ws_bits[2], any[2];          // of both chunks, requested together (a second chunk that does not exist: old ones, not used)
@@ -389,7 +380,7 @@ __global__ void __launch_bounds__(HfRoles<N, EXP>::THREADS, EXP ? 2 : 1) gemm_f1
             uint32_t h[32];
             hf_expand<FMT>(w, tables, h);
             if (p >= S) {
-                ok = hf_wait(bar_drained + 8 * s, ((p / S) - 1u) & 1u, s_abort);          // the products of the stage are done by then
+                ok = mbar_wait_warp(bar_drained + 8 * s, ((p / S) - 1u) & 1u, HF_WAIT_LIMIT, s_abort);          // the products of the stage are done by then
                 if (!ok) break;
             }
             if (c < nc) {
@@ -413,7 +404,7 @@ __global__ void __launch_bounds__(HfRoles<N, EXP>::THREADS, EXP ? 2 : 1) gemm_f1
             bool ok = true;
             for (uint32_t p = 0; 2 * p < nc; ++p) {
                 const uint32_t s = p % S;
-                ok = hf_wait(bar_full + 8 * s, (p / S) & 1u, s_abort);
+                ok = mbar_wait_thread(bar_full + 8 * s, (p / S) & 1u, HF_WAIT_LIMIT, s_abort);
                 if (!ok) break;
                 hf_fence_after();
 #pragma unroll
@@ -463,7 +454,7 @@ __global__ void __launch_bounds__(HfRoles<N, EXP>::THREADS, EXP ? 2 : 1) gemm_f1
         for (uint32_t p = 0; 2 * p < nc; ++p) {
             const uint32_t s = p % S;
             if (p >= S) {
-                ok = hf_wait(bar_drained + 8 * s, ((p / S) - 1u) & 1u, s_abort);
+                ok = mbar_wait_warp(bar_drained + 8 * s, ((p / S) - 1u) & 1u, HF_WAIT_LIMIT, s_abort);
                 if (!ok) break;
             }
 #pragma unroll
@@ -504,7 +495,7 @@ __global__ void __launch_bounds__(HfRoles<N, EXP>::THREADS, EXP ? 2 : 1) gemm_f1
         for (; 2 * p < nc; ++p) {
             const uint32_t s = p % S, n = min(2u, nc - 2 * p);
             if (p >= S) {
-                ok = hf_wait(bar_drained + 8 * s, ((p / S) - 1u) & 1u, s_abort);
+                ok = mbar_wait_thread(bar_drained + 8 * s, ((p / S) - 1u) & 1u, HF_WAIT_LIMIT, s_abort);
                 if (!ok) break;
             }
             mbar_expect_tx(bar_full + 8 * s, n * (N * 128 + XB));
