@@ -350,8 +350,9 @@ __global__ void __launch_bounds__(VAL_THREADS) attn_values_kernel(const ExactAtt
     // tile i: rows of stage i % NST -> transposed tile i % VAL_TBUF; the producer lane refills the stage once all have read it
     auto transpose_tile = [&](uint32_t i) -> bool {
         const uint32_t st = i % NST, tb = i % VAL_TBUF, n = min(VAL_TILE, ctx - i * VAL_TILE);
-        if (!mbar_wait_bounded(bar_full + 8 * st, (i / NST) & 1u)) return false;
-        if (i >= VAL_TBUF && !mbar_wait_bounded(bar_t_free + 8 * tb, ((i / VAL_TBUF) - 1u) & 1u)) return false;
+        // one answer per warp: a lane that left alone would leave the others at the warp's next __syncwarp
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(bar_full + 8 * st, (i / NST) & 1u))) return false;
+        if (i >= VAL_TBUF && !__all_sync(0xffffffffu, mbar_wait_bounded(bar_t_free + 8 * tb, ((i / VAL_TBUF) - 1u) & 1u))) return false;
         value_rows_transpose<HD, KV4>((uint32_t)__cvta_generic_to_shared(stages + (size_t)st * Sm::STAGE), tiles_t + tb * Sm::TILE_T, VAL_TILE,
                                       (n + 15) / 16, tw, NTW, lane);
         __syncwarp();
@@ -407,12 +408,15 @@ __global__ void __launch_bounds__(VAL_THREADS) attn_values_kernel(const ExactAtt
             if (i + 2 >= n_tiles) pdl_trigger();       // one thread's call releases the CTA: only the chain warps call it
             const long long tw0 = clock64();
             const uint32_t st = i % NST;
-            if (direct) {          // the tile's weights (the weight warps run ahead through all tiles) and its bytes
+            bool in = true;
+            if (direct) {          // the tile's weights (the weight warps run ahead through all tiles); its bytes below
                 uint32_t spin = 0;
                 while (min(min(s_ready[0], s_ready[1]), min(s_ready[2], s_ready[3])) <= i && ++spin < EXACT_WAIT_LIMIT) {}
                 __threadfence_block();
-                if (spin >= EXACT_WAIT_LIMIT || !mbar_wait_bounded(bar_full + 8 * st, (i / NST) & 1u)) { failed = true; break; }
-            } else if (!mbar_wait_bounded(bar_t_full + 8 * tb, (i / VAL_TBUF) & 1u)) { failed = true; break; }
+                in = spin < EXACT_WAIT_LIMIT;
+            }
+            const uint32_t bar = direct ? bar_full + 8 * st : bar_t_full + 8 * tb, parity = (direct ? i / NST : i / VAL_TBUF) & 1u;
+            if (!__all_sync(0xffffffffu, in && mbar_wait_bounded(bar, parity))) { failed = true; break; }          // one answer per warp, as above
             t_wait += clock64() - tw0;
             const uint32_t wa = wa0 + 4 * tl;
             // transposed tile: row d, swizzled chunks; direct: the ring stage as it landed, block b = [dimension][16]

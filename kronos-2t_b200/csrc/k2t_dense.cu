@@ -132,14 +132,6 @@ struct GemmArgs {
     const uint32_t *n_items;
 };
 
-__device__ __forceinline__ bool gm_wait(uint32_t bar, uint32_t parity, volatile uint32_t *abort_w) {
-    for (uint32_t spin = 0; spin < GM_WAIT_LIMIT; ++spin) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((spin & 255u) == 255u && *abort_w != 0) return false;
-    }
-    *abort_w = 1;
-    return false;
-}
 __device__ __forceinline__ uint64_t gm_desc(uint32_t saddr) {
     // start address, (unused) leading offset 1, stride of eight rows 1024 bytes, descriptor version 1, 128-byte swizzle
     return (uint64_t)((saddr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024u >> 4) << 32) | (1ull << 46) | (2ull << 61);
@@ -260,7 +252,7 @@ __global__ void __launch_bounds__(GM_THREADS) dense_gemm_kernel(const GemmArgs a
             uint32_t issued = pre;
             for (uint32_t p = pre; p < a.np && ok; ++p) {
                 const uint32_t s = p % S;
-                ok = gm_wait(bar_empty + 8 * s, ((p / S) - 1u) & 1u, s_abort);
+                ok = mbar_wait_thread(bar_empty + 8 * s, ((p / S) - 1u) & 1u, GM_WAIT_LIMIT, s_abort);
                 if (!ok) break;
                 mbar_expect_tx(bar_full + 8 * s, GM_A + B_BYTES);
                 bulk_g2s(a_base + s * GM_A, wsrc + p * w_pitch, GM_A, bar_full + 8 * s);
@@ -280,7 +272,7 @@ __global__ void __launch_bounds__(GM_THREADS) dense_gemm_kernel(const GemmArgs a
             bool ok = true;
             for (uint32_t p = 0; p < a.np; ++p) {
                 const uint32_t s = p % S;
-                ok = gm_wait(bar_full + 8 * s, (p / S) & 1u, s_abort);
+                ok = mbar_wait_thread(bar_full + 8 * s, (p / S) & 1u, GM_WAIT_LIMIT, s_abort);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t da = gm_desc(a_base + s * GM_A), db = gm_desc(b_base + s * B_BYTES);
@@ -296,7 +288,7 @@ __global__ void __launch_bounds__(GM_THREADS) dense_gemm_kernel(const GemmArgs a
         bool ok = false;
         for (uint32_t spin = 0; spin < 8 * GM_WAIT_LIMIT && !ok; ++spin) ok = mbar_try_wait(bar_done, 0u);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        ok = ok && *s_abort == 0;
+        ok = __all_sync(0xffffffffu, ok && *s_abort == 0);          // one answer per warp: the loads below are the whole warp's
         if (!ok && lane == 0 && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
         const uint32_t quarter = warp & 3u, row = row0 + quarter * 32 + lane;          // a warp reaches the tensor-memory lanes of its number mod 4
 #pragma unroll 1

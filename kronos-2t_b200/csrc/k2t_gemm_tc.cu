@@ -154,15 +154,6 @@ template <int K> __device__ __forceinline__ void tc_ld(uint32_t taddr, int (&v)[
 #pragma unroll
     for (int k = 0; k < K / 8; ++k) tc_ld8(taddr + k * 8, *reinterpret_cast<int(*)[8]>(&v[k * 8]));
 }
-// Bounded wait on an mbarrier phase; gives up when the limit runs out or another role has given up.
-__device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, volatile uint32_t *abort_w) {
-    for (uint32_t spin = 0; spin < WAIT_LIMIT; ++spin) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((spin & 255u) == 255u && *abort_w != 0) return false;
-    }
-    *abort_w = 1;
-    return false;
-}
 #ifdef K2T_TC_TRACE
 // Build-time diagnostic: cycles CTA 0 spends in the phases of its three roles (lane 0 of the first warp of each).
 __device__ unsigned long long g_tc_trace[32];
@@ -289,8 +280,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs arg
             if (c + 1 < nc) {
                 TC_ACC_T(5);
                 // `done` (the products) and `full` (already complete by then: it orders this thread after the decode threads' stores of the chunk's scales)
-                if (!tc_wait(bar_done + 8 * ((c + 1) % TC_ACC), ((c + 1) / TC_ACC) & 1u, s_abort)) return false;
-                if (!tc_wait(bar_full + 8 * ((c + 1) % TC_ACC), ((c + 1) / TC_ACC) & 1u, s_abort)) return false;
+                if (!mbar_wait_warp(bar_done + 8 * ((c + 1) % TC_ACC), ((c + 1) / TC_ACC) & 1u, WAIT_LIMIT, s_abort)) return false;
+                if (!mbar_wait_warp(bar_full + 8 * ((c + 1) % TC_ACC), ((c + 1) / TC_ACC) & 1u, WAIT_LIMIT, s_abort)) return false;
                 TC_ACC_T(6);
                 tc_fence_after();
                 tc_ld<NQ>(taddr0 + ((c + 1) % TC_ACC) * N, nxt);
@@ -301,7 +292,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs arg
             return true;
         };
         int v0[NQ], v1[NQ];
-        ok = tc_wait(bar_done, 0u, s_abort) && tc_wait(bar_full, 0u, s_abort);
+        ok = mbar_wait_warp(bar_done, 0u, WAIT_LIMIT, s_abort) && mbar_wait_warp(bar_full, 0u, WAIT_LIMIT, s_abort);
         if (ok) {
             tc_fence_after();
             tc_ld<NQ>(taddr0, v0);
@@ -417,8 +408,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs arg
             decode<FMT>(w, a.cb, u);
             TC_ACC_T(2);
             if (c >= TC_STAGES) {
-                ok = tc_wait(bar_done + 8 * s, ((c / TC_STAGES) - 1u) & 1u, s_abort) &&
-                     tc_wait(bar_drained + 8 * s, ((c / TC_STAGES) - 1u) & 1u, s_abort);
+                ok = mbar_wait_warp(bar_done + 8 * s, ((c / TC_STAGES) - 1u) & 1u, WAIT_LIMIT, s_abort) &&
+                     mbar_wait_warp(bar_drained + 8 * s, ((c / TC_STAGES) - 1u) & 1u, WAIT_LIMIT, s_abort);
                 if (!ok) break;
             }
             TC_ACC_T(3);
@@ -453,6 +444,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs arg
         // instruction descriptor: int32 accumulators, signed 8-bit A and B, both K-major, N / 8, M / 16
         const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((TC_M >> 4) << 24);
         bool ok = true;
+        uint32_t issued = 0;
 #ifdef K2T_TC_TRACE
         unsigned long long trace_acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         long long _tl = clock64();
@@ -460,7 +452,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs arg
         for (uint32_t c = 0; c < nc; ++c) {
             const uint32_t s = c % TC_STAGES, b = c % TC_ACC;
             TC_ACC_T(0);
-            ok = tc_wait(bar_full + 8 * s, (c / TC_STAGES) & 1u, s_abort);
+            ok = mbar_wait_thread(bar_full + 8 * s, (c / TC_STAGES) & 1u, WAIT_LIMIT, s_abort);
             TC_ACC_T(1);
             if (!ok) break;
             tc_fence_after();
@@ -469,12 +461,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs arg
             tc_mma_i8(d, da, db, idesc, 0u);
             tc_mma_i8(d, da + ((2 * TC_LBO) >> 4), db + ((2 * TC_LBO) >> 4), idesc, 1u);      // columns 32..63: two core matrices on
             tc_commit(bar_done + 8 * s);
+            issued = c + 1;
             TC_ACC_T(3);
         }
 #ifdef K2T_TC_TRACE
         if (blockIdx.x == 0 && blockIdx.y == 0) for (int k = 0; k < 4; ++k) g_tc_trace[16 + k] = trace_acc[k];
 #endif
-        if (!ok && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
+        if (!ok) {          // what was issued ends before the tensor memory is given back
+            if (a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
+            for (uint32_t spin = 0; issued > 0 && spin < WAIT_LIMIT && !mbar_try_wait(bar_done + 8 * ((issued - 1) % TC_STAGES), ((issued - 1) / TC_STAGES) & 1u); ++spin) {}
+        }
     }
     tc_fence_before();
     __syncthreads();

@@ -575,14 +575,6 @@ __device__ __forceinline__ void tm_st_wait() { asm volatile("tcgen05.wait::st.sy
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
-__device__ __forceinline__ bool fl_wait(uint32_t bar, uint32_t parity, volatile uint32_t *abort_w) {
-    for (uint32_t spin = 0; spin < WAIT_LIMIT; ++spin) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((spin & 255u) == 255u && *abort_w != 0) return false;
-    }
-    *abort_w = 1;
-    return false;
-}
 
 // Warps 0 .. 3: softmax, one row (token) per thread; warp 4: bulk copies; warp 5: tensor-core issue.
 // Tensor memory: S of even and odd tiles (KT columns each, the softmax weights overwrite them as bf16 pairs), then O.
@@ -641,11 +633,11 @@ __global__ void __launch_bounds__(FL_THREADS, 1) latent_flash_kernel(const Flash
             bool ok = true;
             uint32_t nk = 0, nv = 0;          // tiles requested
             for (uint32_t j = 0; j < n_tiles && ok; ++j) {
-                if (j >= 2) ok = fl_wait(b_ke + 8 * (j & 1u), ((j >> 1) - 1u) & 1u, s_abort);
+                if (j >= 2) ok = mbar_wait_thread(b_ke + 8 * (j & 1u), ((j >> 1) - 1u) & 1u, WAIT_LIMIT, s_abort);
                 if (!ok) break;
                 keys(j);
                 nk = j + 1;
-                if (j >= 2) ok = fl_wait(b_ve + 8 * (j & 1u), ((j >> 1) - 1u) & 1u, s_abort);
+                if (j >= 2) ok = mbar_wait_thread(b_ve + 8 * (j & 1u), ((j >> 1) - 1u) & 1u, WAIT_LIMIT, s_abort);
                 if (!ok) break;
                 values(j);
                 nv = j + 1;
@@ -666,7 +658,7 @@ __global__ void __launch_bounds__(FL_THREADS, 1) latent_flash_kernel(const Flash
             const uint32_t steps_d = (d.dim + 15) / 16, steps_r = (d.rot_dim + 15) / 16;
             auto scores = [&](uint32_t j) {
                 const uint32_t b = j & 1u, kb = s_k + b * k_bytes;
-                if (!fl_wait(b_kf + 8 * b, (j >> 1) & 1u, s_abort)) return false;
+                if (!mbar_wait_thread(b_kf + 8 * b, (j >> 1) & 1u, WAIT_LIMIT, s_abort)) return false;
                 tc_fence_after();
                 for (uint32_t i = 0; i < steps_d + steps_r; ++i) {
                     const uint32_t col = i < steps_d ? i * 16 : p.pd * PANEL + (i - steps_d) * 16, panel = col / PANEL, in = (col % PANEL) * 2;
@@ -676,15 +668,15 @@ __global__ void __launch_bounds__(FL_THREADS, 1) latent_flash_kernel(const Flash
                 tc_commit(b_ke + 8 * b);
                 return true;
             };
-            bool ok = fl_wait(b_q, 0, s_abort) && scores(0);
+            bool ok = mbar_wait_thread(b_q, 0, WAIT_LIMIT, s_abort) && scores(0);
             for (uint32_t j = 0; j < n_tiles && ok; ++j) {
                 const uint32_t b = j & 1u;
                 if (j + 1 < n_tiles) {
-                    if (j >= 1) ok = fl_wait(b_o, (j - 1) & 1u, s_abort);      // the weights of tile j - 1 lie where S of tile j + 1 goes
+                    if (j >= 1) ok = mbar_wait_thread(b_o, (j - 1) & 1u, WAIT_LIMIT, s_abort);      // the weights of tile j - 1 lie where S of tile j + 1 goes
                     ok = ok && scores(j + 1);
                     if (!ok) break;
                 }
-                ok = fl_wait(b_p + 8 * b, (j >> 1) & 1u, s_abort) && fl_wait(b_vf + 8 * b, (j >> 1) & 1u, s_abort);
+                ok = mbar_wait_thread(b_p + 8 * b, (j >> 1) & 1u, WAIT_LIMIT, s_abort) && mbar_wait_thread(b_vf + 8 * b, (j >> 1) & 1u, WAIT_LIMIT, s_abort);
                 if (!ok) break;
                 tc_fence_after();
                 for (uint32_t k = 0; k < KT / 16; ++k)
@@ -703,7 +695,7 @@ __global__ void __launch_bounds__(FL_THREADS, 1) latent_flash_kernel(const Flash
         bool ok = true;
         for (uint32_t j = 0; j < n_tiles; ++j) {
             const uint32_t b = j & 1u, t_s = tmem + b * KT + lanes;
-            ok = __all_sync(0xffffffffu, fl_wait(b_s + 8 * b, (j >> 1) & 1u, s_abort));
+            ok = mbar_wait_warp(b_s + 8 * b, (j >> 1) & 1u, WAIT_LIMIT, s_abort);
             if (!ok) break;
             tc_fence_after();
             uint32_t v[KT];
@@ -722,7 +714,7 @@ __global__ void __launch_bounds__(FL_THREADS, 1) latent_flash_kernel(const Flash
             if (j == 0) {
                 m = m_new;
             } else if (__any_sync(0xffffffffu, m_new > m + 8.0f)) {
-                ok = __all_sync(0xffffffffu, fl_wait(b_o, (j - 1) & 1u, s_abort));
+                ok = mbar_wait_warp(b_o, (j - 1) & 1u, WAIT_LIMIT, s_abort);
                 if (!ok) break;
                 tc_fence_after();
                 const float al = exp2_approx(m - m_new);
@@ -752,7 +744,7 @@ __global__ void __launch_bounds__(FL_THREADS, 1) latent_flash_kernel(const Flash
             mbar_arrive(b_p + 8 * b);
         }
         // the last update by a barrier of its own: the phases of b_o may still be two behind here, and a parity tells only neighbours apart
-        if (ok) ok = __all_sync(0xffffffffu, fl_wait(b_end, 0u, s_abort) && *s_abort == 0);
+        if (ok) ok = __all_sync(0xffffffffu, mbar_wait_thread(b_end, 0u, WAIT_LIMIT, s_abort) && *s_abort == 0);
         tc_fence_after();
         if (ok) {
             const float inv = 1.0f / l;

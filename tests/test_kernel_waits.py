@@ -7,7 +7,7 @@ import re
 import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "kronos-2t_b200", "csrc")
-PER_THREAD = r"\bmbar_wait_thread\("
+PER_THREAD = r"\bmbar_wait_(?:thread|bounded)\("
 SOURCES = sorted(f for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh")) and f != "k2t_device.cuh" and re.search(PER_THREAD, open(os.path.join(CSRC, f)).read()))
 
 
