@@ -228,6 +228,18 @@ def test_ring_is_used_again(engine, monkeypatch, dtype):
     assert fm.error(got, want).max() < TOL[dtype]
 
 
+@pytest.mark.parametrize("n", [600, 850])
+def test_prompt_fills_its_batches(engine, monkeypatch, n):
+    """A prompt of more tokens than a batch is the same portions one after the other: full batches, then the rest, bit for bit (the tiles
+    of the window attention begin with the batch)."""
+    monkeypatch.setenv("KRONOS_CUDA_PROMPT_BATCH", "400")
+    model = fm.make(96, 60, [fm.attention(4, 2, 32, 32, 21, ff=80), fm.delta(2, 24)], seed=9)
+    toks = tokens_of(model, n)
+    eng = engine(model, "bfloat16", max_seq=1024)
+    whole = eng.forward_token_ids(toks, want_all=True)
+    assert np.array_equal(portions(eng, toks, [400]), whole)
+
+
 def test_sequences_follow_one_another(engine):
     """A new sequence starts from nothing, whatever ran before; the same sequence gives the same bits again."""
     import kronos_2t_b200 as k2
