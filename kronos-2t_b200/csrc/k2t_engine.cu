@@ -38,6 +38,12 @@ bool engine_count(KronosCudaEngine *e, cudaError_t err, const char *what, uint32
     return cuda_ok(e->ctx, err, what);
 }
 
+uint32_t prompt_batch(size_t left, uint32_t max_batch) {
+    const size_t tile = max_batch % 128 == 0 ? 128 : 16, most = max_batch / tile;
+    const size_t tiles = (left + tile - 1) / tile, batches = (tiles + most - 1) / most;
+    return batches == 0 ? 0u : (uint32_t)std::min(left, (tiles + batches - 1) / batches * tile);
+}
+
 }  // namespace k2t
 
 namespace {
@@ -1273,14 +1279,9 @@ static int32_t forward_common(KronosCudaEngine *e, const float *embeds, const ui
     // prompt: batches of up to max_batch tokens (forward_prompt / forward_batch_sdot_impl, real_llm.rs:7407-7448, 7450-7860):
     // every projection as one tensor-core weight pass over the batch, the attention of the batch's tokens side by side
     if (!set_u32(e, e->d_pos, (uint32_t)pos_start)) return -1;
-    // As few batches as the workspace allows, of about the same size in whole tiles of 128 tokens: a short last one would pay for
-    // a batch's launches and its weights again (300 tokens of the 30B-A3B shape as 256 + 44 and as one: 2.86 and 1.86 ms; 1000 tokens
-    // of the 1.7B shape in batches of 256 and in two of 500: 11.9 and 9.7 ms).
-    const size_t n_batch = (n_tok + e->max_batch - 1) / e->max_batch;
-    // Block models fill each batch: 2049 / 4097 tokens as two / three even batches took 2 to 14% longer than as full ones and a single token.
-    const uint32_t T_even = e->blocks ? e->max_batch : (uint32_t)std::min<size_t>(e->max_batch, ((n_tok + n_batch - 1) / n_batch + 127) & ~(size_t)127);
     for (size_t t0 = 0, T_done = 0; t0 < n_tok; t0 += T_done) {
-        uint32_t T = (uint32_t)std::min<size_t>(T_even, n_tok - t0);
+        // block models fill each batch: 2049 / 4097 tokens as two / three even batches took 2 to 14% longer than as full ones and a single token
+        uint32_t T = e->blocks ? (uint32_t)std::min<size_t>(e->max_batch, n_tok - t0) : prompt_batch(n_tok - t0, e->max_batch);
         const size_t p0 = pos_start + t0;
         if (e->split_kv && p0 < ATTN_EXACT_CTX && p0 + T > ATTN_EXACT_CTX) T = (uint32_t)(ATTN_EXACT_CTX - p0);    // split-KV kernels: a batch stays on one side of the attention switch
         const bool last = t0 + T == n_tok;

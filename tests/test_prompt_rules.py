@@ -1,0 +1,33 @@
+"""Rules of the prompt path that the host decides, without a device."""
+import ctypes as C
+
+import pytest
+
+from k2t_internal import internal
+
+
+def batches(n, max_batch):
+    prompt_batch = internal("prompt_batch", C.c_uint32, C.c_size_t, C.c_uint32)
+    out = []
+    while n:
+        out.append(prompt_batch(n, max_batch))
+        assert 0 < out[-1] <= min(n, max_batch)
+        n -= out[-1]
+    return out
+
+
+@pytest.mark.parametrize("n,want", [(2, [2]), (300, [300]), (512, [512]), (513, [384, 129]), (1000, [512, 488]), (1025, [384, 384, 257]), (1537, [512, 384, 384, 257]),
+                                    (1540, [512, 384, 384, 260]), (2049, [512, 512, 384, 384, 257])])
+def test_batches_of_a_prompt(n, want):
+    assert batches(n, 512) == want
+
+
+@pytest.mark.parametrize("max_batch", [16, 48, 128, 208, 256, 384, 512])
+def test_no_short_last_batch(max_batch):
+    """As few batches as there can be, alike but for one tile (the last may miss part of its own)."""
+    tile = 128 if max_batch % 128 == 0 else 16
+    for n in list(range(1, 3 * max_batch + 40)) + [4001, 8192, 20011]:
+        b = batches(n, max_batch)
+        assert sum(b) == n and len(b) == -(-n // max_batch)
+        tiles = [-(-x // tile) for x in b]
+        assert max(tiles) - min(tiles) <= 1 and all(x % tile == 0 for x in b[:-1])
