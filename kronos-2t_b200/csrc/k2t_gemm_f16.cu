@@ -561,14 +561,12 @@ __global__ void __launch_bounds__(1024) expert_tiles_kernel(const uint32_t *rout
     pdl_wait();
     pdl_trigger();
     __syncthreads();
-    auto expert_of = [&](uint32_t i) {
-        const uint32_t e = __ldcg(route_ids + (size_t)(i / k) * route_stride + i % k);
-        return e < n_experts && bases[e] == nullptr ? n_experts : e;
-    };
+    auto expert_of = [&](uint32_t i) { return __ldcg(route_ids + (size_t)(i / k) * route_stride + i % k); };
+    auto held = [&](uint32_t e) { return e < n_experts && bases[e] != nullptr; };
     for (uint32_t i = tid; i < n_pair; i += 1024) {
         const uint32_t e = expert_of(i);
-        if (e < n_experts) atomicAdd(&count[e], 1u);
-        else if (e > n_experts && err_flag != nullptr) atomicExch(err_flag, 4u);
+        if (held(e)) atomicAdd(&count[e], 1u);
+        else if (e >= n_experts && err_flag != nullptr) atomicExch(err_flag, 4u);
     }
     __syncthreads();
     if (tid < 32) {          // tiles in front of every expert's
@@ -594,7 +592,7 @@ __global__ void __launch_bounds__(1024) expert_tiles_kernel(const uint32_t *rout
     __syncthreads();
     for (uint32_t i = tid; i < n_pair; i += 1024) {
         const uint32_t e = expert_of(i);
-        if (e < n_experts) tile_pairs[first[e] * 32 + atomicAdd(&count[e], 1u)] = i;
+        if (held(e)) tile_pairs[first[e] * 32 + atomicAdd(&count[e], 1u)] = i;
     }
 }
 
