@@ -623,6 +623,10 @@ template <int FMT> cudaError_t launch_hf_fmt(cudaStream_t s, const HfArgs &args,
 
 }  // namespace
 
+bool experts_grouped(uint32_t n_tok, uint32_t n_pair, uint32_t n_experts) {
+    const uint32_t min_tok = gemm_tc_min_tokens();
+    return min_tok != 0 && n_tok >= min_tok && n_pair >= std::max(3 * n_experts, 48u);
+}
 uint32_t expert_tiles_max(size_t n_pair, uint32_t n_experts) { return (uint32_t)(n_pair / 32 + std::min<size_t>(n_pair, n_experts)); }
 
 cudaError_t launch_expert_tiles(cudaStream_t stream, const uint32_t *route_ids, uint32_t n_tok, uint32_t k, uint32_t route_stride, uint32_t n_experts,

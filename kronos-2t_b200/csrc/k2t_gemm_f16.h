@@ -1,6 +1,5 @@
 // Prompt GEMM over half-precision operand images (k2t_gemm_f16.cu).
 #pragma once
-#include <algorithm>
 #include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -38,8 +37,8 @@ cudaError_t launch_expert_tiles(cudaStream_t stream, const uint32_t *route_ids, 
 // Prompts take the grouped form from three pairs per expert on.  A GEMV costs per pair (0.33 us each for gate_up and down of the 30B-A3B
 // shape: 128 experts, 2048 x 1536 and 768 x 2048, 3 bits), a tile per expert: 24 / 32 / 44 / 64 / 150 tokens with 8 routes through three
 // layers take 857 / 995 / 1238 / 1605 / 4024 us as GEMVs and 1113 / 1193 / 1271 / 1352 / 1498 us in tiles.  Few experts leave SMs
-// idle: 48 pairs at least.
-inline bool experts_grouped(uint32_t n_pair, uint32_t n_experts) { return n_pair >= std::max(3 * n_experts, 48u); }
+// idle: 48 pairs at least.  It is a tensor-core form: only for batches that gemm_tc_min_tokens() hands to the tensor cores.
+bool experts_grouped(uint32_t n_tok, uint32_t n_pair, uint32_t n_experts);
 
 // The expert projections of all pairs of `t`, an expert's weights expanded once per 32 pairs; out = [n_pair][rows].  Same bits as
 // launch_gemv_experts, for activations in the form the library's own quantizers leave them.

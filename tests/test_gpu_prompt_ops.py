@@ -27,3 +27,30 @@ def test_small_operators_of_a_batch(oracle, head_dim, n_q, n_kv, hidden, inter, 
         assert np.array_equal(eng.forward_token_ids(tokens[:1], pos_start=n_tok), ref.forward_token(tokens[0], threads=4))          # the cache rows
     finally:
         eng.close(); ref.close(); ctx.close()
+
+
+SWITCH = """
+import sys, zlib
+import numpy as np
+import kronos_2t_b200 as k2
+from kronos_2t_b200 import synth
+cfg = dict(hidden=192, layers=2, n_q=4, n_kv=2, head_dim=64, inter=320, vocab=320, max_seq=160, eps=1e-6, theta=1e6)
+ctx, crc = k2.Context(0), 0
+for kv_bits in (8, 4):
+    for moe in (None, dict(n_experts=4, top_k=2, d_ff=128, bits=3, sgc=1)):
+        eng = k2.Engine(ctx, synth.random_model(dict(cfg, kv_bits=kv_bits), "nf4", seed=5, **(dict(moe=moe) if moe else {})))
+        tokens, pos = np.random.Generator(np.random.PCG64(1)).integers(0, 320, 120).astype(np.uint32), 0
+        for n in (60, 3, 1, 16, 1, 5):
+            crc = zlib.crc32(eng.forward_token_ids(tokens[pos:pos + n], pos_start=pos, want_all=True).tobytes(), crc)
+            pos += n
+        toks, logits = eng.decode_greedy(int(tokens[pos]), pos, 4, want_logits=True)
+        crc = zlib.crc32(logits.tobytes(), zlib.crc32(np.asarray(toks).tobytes(), crc))
+        eng.close()
+print(crc)
+"""
+
+
+def test_tensor_core_switch_changes_no_bits():
+    """KRONOS_CUDA_TC_MIN_TOKENS: never, from one token on (single steps included), as it is: prompts, short ones and decoding."""
+    from test_prompt_rules import in_process
+    assert len({in_process(SWITCH, KRONOS_CUDA_TC_MIN_TOKENS=v) for v in ("0", "1", "4", "16", "100")}) == 1

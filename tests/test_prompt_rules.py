@@ -1,5 +1,8 @@
 """Rules of the prompt path that the host decides, without a device."""
 import ctypes as C
+import os
+import subprocess
+import sys
 
 import pytest
 
@@ -31,3 +34,17 @@ def test_no_short_last_batch(max_batch):
         assert sum(b) == n and len(b) == -(-n // max_batch)
         tiles = [-(-x // tile) for x in b]
         assert max(tiles) - min(tiles) <= 1 and all(x % tile == 0 for x in b[:-1])
+
+
+def in_process(code, **env):
+    """stdout of a Python program with environment variables that the library reads once."""
+    return subprocess.run([sys.executable, "-c", code], check=True, capture_output=True, text=True, cwd=os.path.dirname(os.path.abspath(__file__)),
+                          env=dict(os.environ, PYTHONPATH=os.pathsep.join(sys.path), **env)).stdout.strip()
+
+
+@pytest.mark.parametrize("switch,want", [(None, "0 1 1"), ("0", "0 0 0"), ("200", "0 0 1")])
+def test_expert_tiles_obey_the_tensor_core_switch(switch, want):
+    """512 pairs of 8 experts as 8, 100 and 300 tokens: the grouped form is a tensor-core form."""
+    code = ("import ctypes as C; from k2t_internal import internal; f = internal('experts_grouped', C.c_bool, C.c_uint32, C.c_uint32, C.c_uint32); "
+            "print(*[int(f(t, 512, 8)) for t in (8, 100, 300)])")
+    assert in_process(code, **({} if switch is None else dict(KRONOS_CUDA_TC_MIN_TOKENS=switch))) == want
