@@ -653,6 +653,7 @@ cudaError_t launch_gemm_experts(cudaStream_t stream, const DeviceMatrix &m0, int
     }
 }
 
+bool gemm_f16_takes(size_t n_tok) { return n_tok != 0 && act_half_tokens(n_tok) / 32 <= 0xFFFFu; }
 size_t act_half_bytes(size_t n_tok, uint32_t cols) { return act_half_tokens(n_tok) * cols * 2; }
 size_t act_half_scale_bytes(size_t n_tok, uint32_t cols) { return act_half_tokens(n_tok) / 32 * (cols / 64) * HF_REC; }
 
@@ -660,7 +661,7 @@ cudaError_t launch_gemm_f16(cudaStream_t stream, const DeviceMatrix &m, const in
                             float *out, size_t out_stride, int sm_count, uint32_t *err_flag, uint32_t *launches, bool pdl, bool image_ready) {
     if (launches) *launches = 0;
     const uint32_t tok_pad = (uint32_t)act_half_tokens(n_tok);
-    if (n_tok == 0 || n_tok > 0xFFFFu * 32u || (image_ready && h.zero == nullptr)) return cudaErrorInvalidValue;
+    if (!gemm_f16_takes(n_tok) || (image_ready && h.zero == nullptr)) return cudaErrorInvalidValue;
     HfArgs args;
     const int fmt = fill_gemv_args(m, true, args.g);
     args.g.out = out; args.g.err_flag = err_flag; args.g.out_stride = out_stride;

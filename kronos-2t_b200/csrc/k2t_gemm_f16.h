@@ -15,6 +15,7 @@ struct ActHalf {
     uint32_t *zero = nullptr;        // images of k2t_prompt_ops.cu: set when a chunk without a scale was written since the caller cleared it
 };
 inline size_t act_half_tokens(size_t n_tok) { return (n_tok + 127) & ~(size_t)127; }
+bool gemm_f16_takes(size_t n_tok);          // batches whose padded tokens, 32 to a CTA of either launch, fit a grid
 size_t act_half_bytes(size_t n_tok, uint32_t cols);
 size_t act_half_scale_bytes(size_t n_tok, uint32_t cols);
 

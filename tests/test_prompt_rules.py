@@ -48,3 +48,11 @@ def test_expert_tiles_obey_the_tensor_core_switch(switch, want):
     code = ("import ctypes as C; from k2t_internal import internal; f = internal('experts_grouped', C.c_bool, C.c_uint32, C.c_uint32, C.c_uint32); "
             "print(*[int(f(t, 512, 8)) for t in (8, 100, 300)])")
     assert in_process(code, **({} if switch is None else dict(KRONOS_CUDA_TC_MIN_TOKENS=switch))) == want
+
+
+def test_largest_batch_of_the_prompt_gemm():
+    """The padded tokens of the operand image are 32 to a CTA along grid.y, which ends at 65535: 2 097 025 tokens pad to 65536 x 32."""
+    takes = internal("gemm_f16_takes", C.c_bool, C.c_size_t)
+    assert [takes(n) for n in (0, 1, 16, 512, 2097024, 2097025, 2097120, 2097121, 2 ** 32 + 16)] == [False, True, True, True, True, False, False, False, False]
+    for n in range(2096900, 2097200):
+        assert takes(n) == ((n + 127) // 128 * 4 <= 65535)
