@@ -36,17 +36,27 @@ inline bool cuda_ok(KronosCudaContext *ctx, cudaError_t e, const char *what) {
     if (e == cudaSuccess) return true;
     return fail(ctx, std::string(what) + ": " + cudaGetErrorString(e));
 }
-inline bool reserve(KronosCudaContext *ctx, DeviceBuffer &b, size_t bytes) {
-    if (bytes <= b.cap) return true;
-    if (b.p) { cudaFree(b.p); b.p = nullptr; b.cap = 0; }
-    size_t want = (bytes + 255) & ~(size_t)255;
-    if (!cuda_ok(ctx, cudaMalloc(&b.p, want), "cudaMalloc(scratch)")) return false;
-    b.cap = want;
-    return true;
-}
 inline void release(DeviceBuffer &b) {
     if (b.p) cudaFree(b.p);
     b.p = nullptr; b.cap = 0;
+}
+inline bool reserve(KronosCudaContext *ctx, DeviceBuffer &b, size_t bytes) {
+    if (bytes <= b.cap) return true;
+    release(b);
+    const size_t want = (bytes + 255) & ~(size_t)255;
+    cudaError_t e = cudaMalloc(&b.p, want);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        // the operand image is there for speed alone: a call that needs memory for anything else gets it back
+        if (&b != &ctx->half && &b != &ctx->half_xs && (ctx->half.p || ctx->half_xs.p)) {
+            release(ctx->half); release(ctx->half_xs);
+            e = cudaMalloc(&b.p, want);
+            if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+        }
+    }
+    if (!cuda_ok(ctx, e, "cudaMalloc(scratch)")) { b.p = nullptr; return false; }
+    b.cap = want;
+    return true;
 }
 // Waits for the stream and reports a kernel-side timeout (a bounded wait that gave up) as an error.
 inline bool sync_and_check(KronosCudaContext *ctx, const char *what) {

@@ -322,6 +322,7 @@ static int32_t linear_impl(KronosCudaContext *ctx, const KronosCudaMatrix *m, co
     bool half = min_tok != 0 && n_tok >= min_tok && gemm_f16_takes(n_tok);
     if (half && (!reserve(ctx, ctx->half, act_half_bytes(n_tok, g.cols)) || !reserve(ctx, ctx->half_xs, act_half_scale_bytes(n_tok, g.cols)))) {
         half = false;
+        release(ctx->half); release(ctx->half_xs);
         ctx->err.clear();
     }
     if (half) {
