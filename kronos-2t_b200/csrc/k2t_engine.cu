@@ -48,6 +48,10 @@ uint32_t prompt_batch(size_t left, uint32_t max_batch) {
 
 namespace {
 
+// Tokens per launch of the two-kernel attention: its scores take query heads x cache rows floats per token (3.7 MB with 28 heads at
+// 32 k positions), and 256 tokens of any shape are more CTAs than the SMs hold.
+constexpr uint32_t SCORE_TOKENS = 256;
+
 // (Re)builds the KV cache: format `bits` (8 / 4) and geometry - the full causal context, or the sliding-window ring of
 // QuantizedKvCache::new_with_opts (real_llm.rs:1235-1257): taken only when 8 <= window and window + 512 < max_seq_len, sinks
 // capped at window / 2, ring = window - sinks + 512 rows of slack for batches.  Also the scratch sized by the cache rows.
@@ -76,7 +80,8 @@ bool alloc_kv(KronosCudaEngine *e, uint32_t bits, uint32_t window, uint32_t sink
     e->split_kv = e->ring.window == 0 && ((c.flags & KRONOS_CUDA_ENGINE_SPLIT_KV_ATTENTION) != 0 || longest > attention_exact_max_ctx(hd, bits));
     if (e->ring.window && longest > attention_exact_max_ctx(hd, bits)) return fail(ctx, "kv_window is longer than the attention kernel can hold");
     const size_t slots = (size_t)c.num_layers * c.num_key_value_heads * e->kv_stride;
-    const bool ok = dev_alloc(e, e->attn_sc, (size_t)e->max_batch * n_q * e->kv_stride) && dev_alloc(e, e->attn_bmax, (size_t)e->max_batch * n_q * ((e->kv_stride + 127) / 128)) &&
+    e->score_tokens = std::min(e->max_batch, SCORE_TOKENS);
+    const bool ok = dev_alloc(e, e->attn_sc, (size_t)e->score_tokens * n_q * e->kv_stride) && dev_alloc(e, e->attn_bmax, (size_t)e->score_tokens * n_q * ((e->kv_stride + 127) / 128)) &&
                     dev_alloc(e, e->k_q8, bits == 4 ? slots * hd / 2 : slots * hd) && dev_alloc(e, e->v_q8, bits == 4 ? slots * hd / 2 : slots * hd) &&
                     dev_alloc(e, e->k_scale, bits == 4 ? (slots * (hd / 64) + 1) / 2 : slots) &&      // NF4: bf16 per 64 values
                     dev_alloc(e, e->v_scale, bits == 4 ? (slots * (hd / 64) + 1) / 2 : slots);
@@ -273,7 +278,15 @@ bool enqueue_attention_batch(KronosCudaEngine *e, uint32_t l, uint32_t T) {
     xa.ctx_cap = attn_ctx_cap(e); xa.ring = e->ring;
     xa.kv_bits = c.kv_bits; xa.attn_scale = 1.0f / sqrtf((float)hd); xa.err_flag = e->ctx->d_err; xa.trace = nullptr; xa.v_t = e->v_t;
     if (attention_prompt_takes(xa, T)) return count(e, launch_attention_prompt(s, xa, e->pdl, T), "attention");
-    return count(e, launch_attention_exact(s, xa, e->pdl, T), "attention", 2);
+    for (uint32_t t0 = 0; t0 < T; t0 += e->score_tokens) {
+        const uint32_t n = std::min(e->score_tokens, T - t0), n_q = c.num_attention_heads;
+        ExactAttnArgs part = xa;
+        part.q_i8 += (size_t)t0 * n_q * hd; part.q_scale += (size_t)t0 * n_q; part.pos_offset = t0;
+        part.out_q += (size_t)t0 * n_q * hd; part.out_scales += (size_t)t0 * n_q * (hd / 64); part.out_sums += (size_t)t0 * n_q * (hd / 64);
+        if (t0 + n < T) part.attn_out = nullptr;          // the last token's
+        if (!count(e, launch_attention_exact(s, part, e->pdl, n), "attention", 2)) return false;
+    }
+    return true;
 }
 
 // Attention of token t of a batch of T for layer l: the output becomes row t of the o_proj activation.

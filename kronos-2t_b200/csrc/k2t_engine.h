@@ -45,7 +45,7 @@ struct KronosCudaEngine {
     int8_t *act_q = nullptr, *q_i8 = nullptr;
     float *attn_tap = nullptr;                // attention output of the last layer (diagnostic)
     float *act_s = nullptr, *q_scale = nullptr, *part_m = nullptr, *part_l = nullptr, *part_o = nullptr;
-    float *attn_sc = nullptr, *attn_bmax = nullptr;      // long contexts in CPU order: scores [n_q][kv_stride], block maxima [n_q][kv_stride / 128]
+    float *attn_sc = nullptr, *attn_bmax = nullptr;      // long contexts in CPU order: scores [score_tokens][n_q][kv_stride], block maxima [..][n_q][kv_stride / 128]
     bool split_kv = false;                    // long contexts by the split-KV kernels instead (config flag, or the cache is too long for the exact path)
     int32_t *act_m = nullptr;
     uint8_t *signs = nullptr;                 // rotation signs by chunk (k2t_prompt_ops.cu)
@@ -56,6 +56,7 @@ struct KronosCudaEngine {
     uint32_t *d_token = nullptr, *d_pos = nullptr, *d_step = nullptr, *d_history = nullptr;
     uint32_t n_split = 32;
     uint32_t max_batch = 512;                 // tokens per prompt batch: their projections run on the tensor cores in one weight pass (k2t_gemm_tc.cu), their attention side by side; every per-token buffer holds this many rows (KRONOS_CUDA_PROMPT_BATCH, 16..512)
+    uint32_t score_tokens = 0;                // tokens of a batch whose scores the two-kernel attention holds at a time
     uint32_t ctx_bound = 0;                   // prompt batches (launched eagerly, position known on the host): no token of the batch sees more positions; 0 = size launches for the whole cache
     uint32_t kv_stride = 0;                   // cache rows per (layer, kv head): the rows the geometry needs (max_seq_len, or sinks + ring) rounded up to 32, so every 32-row tile of rows and scales starts on 16 bytes
     k2t::KvRing ring{};                       // sliding-window + sink ring (all zero: row = position)

@@ -53,3 +53,48 @@ def test_linear_gives_its_operand_image_back(oracle):
     finally:
         dm.free()
         ctx.close()
+
+
+@pytest.mark.parametrize("kv_bits,window", [(8, 0), (4, 0), (8, 900)])
+def test_scores_in_portions(kv_bits, window):
+    """Batches of more tokens than the score scratch holds: as batches of 256 give it, bit for bit, and no larger scratch."""
+    import kronos_2t_b200 as k2
+    from kronos_2t_b200 import synth
+    past, n = (7100, 512) if kv_bits == 8 and not window else (700, 512)          # contexts that the row-sharing attention leaves alone
+    cfg = dict(hidden=64, layers=2, n_q=4, n_kv=2, head_dim=64, inter=64, vocab=128, max_seq=past + n + 600, eps=1e-5, theta=1e4, kv_bits=kv_bits, kv_window=window, kv_sinks=4)
+    tokens = np.random.Generator(np.random.PCG64(n)).integers(0, 128, past + n).astype(np.uint32)
+    ctx = k2.Context(0)
+    a, b = (k2.Engine(ctx, synth.random_model(cfg, "b4", seed=4)) for _ in range(2))
+    try:
+        for e in (a, b):
+            e.forward_token_ids(tokens[:past])
+        got = a.forward_token_ids(tokens[past:], pos_start=past, want_all=True)
+        want = np.concatenate([b.forward_token_ids(tokens[p:p + 256], pos_start=p, want_all=True) for p in range(past, past + n, 256)])
+        assert np.array_equal(got, want)
+        assert np.array_equal(a.read_attention(), b.read_attention())
+        p = past + n
+        assert np.array_equal(a.forward_token_ids(tokens[:1], pos_start=p), b.forward_token_ids(tokens[:1], pos_start=p))
+    finally:
+        a.close(); b.close(); ctx.close()
+
+
+def test_score_scratch_of_a_long_cache():
+    """32 heads over 32768 positions: scores of 256 tokens (1.07 GB), whatever the batch."""
+    import torch
+
+    import kronos_2t_b200 as k2
+    from kronos_2t_b200 import synth
+    cfg = dict(hidden=64, layers=1, n_q=32, n_kv=4, head_dim=64, inter=64, vocab=128, max_seq=32768, eps=1e-5, theta=1e4)
+    spec = synth.random_model(cfg, "b4", seed=4)
+    ctx = k2.Context(0)
+    k2.Engine(ctx, synth.random_model(dict(cfg, max_seq=64), "b4", seed=4)).close()
+    torch.cuda.synchronize()
+    before, _ = torch.cuda.mem_get_info()
+    e = k2.Engine(ctx, spec)
+    try:
+        taken = before - torch.cuda.mem_get_info()[0]
+        scores, cache = 256 * 32 * (32768 + 256) * 4, 4 * 32768 * 64 * 3
+        rest = 512 * (4 * 40 * 64 * 4 + 2048 * 12 + 128 * 4)          # vectors, activations, image
+        assert taken < scores + cache + rest + 64 * MB
+    finally:
+        e.close(); ctx.close()
