@@ -51,6 +51,8 @@ namespace {
 // Tokens per launch of the two-kernel attention: its scores take query heads x cache rows floats per token (3.7 MB with 28 heads at
 // 32 k positions), and 256 tokens of any shape are more CTAs than the SMs hold.
 constexpr uint32_t SCORE_TOKENS = 256;
+// free memory that batches of more than 256 tokens must leave (their workspace of the 7B shape: 0.5 GB)
+constexpr size_t WORKSPACE_SPARE = 512u << 20;
 
 // (Re)builds the KV cache: format `bits` (8 / 4) and geometry - the full causal context, or the sliding-window ring of
 // QuantizedKvCache::new_with_opts (real_llm.rs:1235-1257): taken only when 8 <= window and window + 512 < max_seq_len, sinks
@@ -746,6 +748,7 @@ KronosCudaEngine *kronos_cuda_engine_create(KronosCudaContext *ctx, const Kronos
         const uint32_t want = (8u * (uint32_t)ctx->sm_count + c.num_key_value_heads - 1) / c.num_key_value_heads;
         e->n_split = std::min(128u, std::max(32u, (want + 3u) & ~3u));
     }
+    if (c.tp_size > 1 || c.ep_size > 1) e->max_batch = 256;          // the exchange buffers grow with it, on every rank alike
     if (const char *v = std::getenv("KRONOS_CUDA_PROMPT_BATCH")) {                  // tokens per prompt batch (default 512, the slack of a sliding window's ring)
         const uint32_t n = (uint32_t)std::strtoul(v, nullptr, 10);
         e->max_batch = std::min(512u, std::max(16u, (n + 15u) & ~15u));
@@ -804,60 +807,79 @@ KronosCudaEngine *kronos_cuda_engine_create(KronosCudaContext *ctx, const Kronos
     const uint32_t act_n = std::max(std::max(h, q_dim), inter), n_q = c.num_attention_heads;
     // rotations of the small prompt operators: the residual stream, SwiGLU from its first chunk on, experts and shared experts, two blocks of a head
     const uint32_t sign_chunks = std::max(std::max(h / 64, inter / 64 + c.down_chunk0), std::max(std::max(e->sh_inter_max, e->has_moe ? c.moe_d_ff : 0u) / 64, 2u));
-    bool ok = dev_alloc(e, e->final_norm, h, final_norm) && dev_alloc(e, e->rope, (size_t)c.max_seq_len * hd, rope) &&
-              (embed_bf16 == nullptr || dev_alloc(e, e->embed_bf16, (size_t)(c.tp_size > 1 ? c.vocab_total : c.vocab_size) * h, embed_bf16)) &&   // every rank keeps the whole table
-              // per-token vectors hold max_batch tokens (prompt batches), [token][n]
-              dev_alloc(e, e->hidden, (size_t)e->max_batch * h) && dev_alloc(e, e->hidden2, h) && dev_alloc(e, e->proj, (size_t)e->max_batch * h) &&
-              dev_alloc(e, e->qkv, (size_t)e->max_batch * qkv_rows) && dev_alloc(e, e->gate_up, (size_t)e->max_batch * 2 * inter) &&
-              dev_alloc(e, e->logits, (size_t)e->max_batch * (c.tp_size > 1 ? c.vocab_total : c.vocab_size)) && dev_alloc(e, e->act_q, (size_t)e->max_batch * act_n) &&
-              dev_alloc(e, e->act_s, (size_t)e->max_batch * act_n / 64) && dev_alloc(e, e->act_m, (size_t)e->max_batch * act_n / 64) &&
-              dev_alloc(e, e->signs, sign_table_bytes(sign_chunks)) && cuda_ok(ctx, launch_sign_table(ctx->stream, e->signs, sign_chunks), "sign table") &&
-              dev_alloc(e, e->act_half.zero, 1) && dev_alloc(e, e->act_half.img, act_half_bytes(e->max_batch, std::max(act_n, e->sh_inter_max))) &&
-              dev_alloc(e, e->act_half.scales, act_half_scale_bytes(e->max_batch, std::max(act_n, e->sh_inter_max))) &&
-              dev_alloc(e, e->q_i8, (size_t)e->max_batch * q_dim) && dev_alloc(e, e->attn_tap, q_dim) && dev_alloc(e, e->q_scale, (size_t)e->max_batch * n_q) &&
-              dev_alloc(e, e->part_m, (size_t)n_q * e->n_split) && dev_alloc(e, e->part_l, (size_t)n_q * e->n_split) &&
-              dev_alloc(e, e->part_o, (size_t)n_q * e->n_split * hd) &&
-              alloc_kv(e, c.kv_bits, c.kv_window, c.kv_sinks) &&
-              dev_alloc(e, e->d_token, e->max_batch) && dev_alloc(e, e->d_pos, 1) && dev_alloc(e, e->d_step, 1) &&
-              dev_alloc(e, e->d_history, c.max_seq_len) && dev_alloc(e, e->d_dbg, 32) && dev_alloc(e, e->argmax_scratch, ARGMAX_SCRATCH_WORDS);
-    const uint32_t xg = c.tp_size > 1 ? c.tp_size : c.ep_size, xr = c.tp_size > 1 ? c.tp_rank : c.ep_rank;     // exchange group
-    if (ok && xg > 1) {
-        if (e->has_moe && c.tp_size > 1) return bad("engine_create: sparse-MoE layers are not combined with tensor parallelism");
-        const size_t slot = std::max<size_t>((size_t)e->max_batch * h, c.vocab_size), floats = 2 * (size_t)xg * slot;
-        void *raw = nullptr;
-        // floats | 256 bytes of flags | (value, call number) words of the fused sums: [2][tp][max_batch * hidden] x 8 bytes
-        const size_t ll_slot = (size_t)e->max_batch * h, total = floats * 4 + 256 + 2 * (size_t)xg * ll_slot * 8;
-        ok = cuda_ok(ctx, cudaMalloc(&raw, total), "cudaMalloc(tp exchange)");
-        if (ok) {
-            e->allocs.push_back(raw);
-            e->tp_buf = static_cast<float *>(raw);
-            e->tp.ll_slot = (uint32_t)ll_slot;
-            e->tp.peer_ll[xr] = reinterpret_cast<unsigned long long *>(static_cast<uint8_t *>(raw) + floats * 4 + 256);
-            e->tp.wait_polls = TP_WAIT_POLLS_DEFAULT;
-            if (const char *v = std::getenv("KRONOS_CUDA_PEER_WAIT_POLLS")) e->tp.wait_polls = (uint32_t)std::strtoul(v, nullptr, 10);
-            ok = cuda_ok(ctx, cudaMemsetAsync(raw, 0, total, ctx->stream), "clear tp exchange") &&
-                 dev_alloc(e, e->tp.epoch, 1) && dev_alloc(e, e->tp_done, 1) && dev_alloc(e, e->logits_local, (size_t)e->max_batch * c.vocab_size);
-            e->tp.tp = xg; e->tp.rank = xr; e->tp.slot = (uint32_t)slot; e->tp.err = ctx->d_err;
-            e->tp.peer_data[xr] = e->tp_buf;
-            e->tp.peer_flags[xr] = reinterpret_cast<uint32_t *>(e->tp_buf + floats);
+    if (!dev_alloc(e, e->final_norm, h, final_norm) || !dev_alloc(e, e->rope, (size_t)c.max_seq_len * hd, rope) ||
+        (embed_bf16 != nullptr && !dev_alloc(e, e->embed_bf16, (size_t)(c.tp_size > 1 ? c.vocab_total : c.vocab_size) * h, embed_bf16)) ||   // every rank keeps the whole table
+        !dev_alloc(e, e->signs, sign_table_bytes(sign_chunks)) || !cuda_ok(ctx, launch_sign_table(ctx->stream, e->signs, sign_chunks), "sign table"))
+        return bad(ctx->err);
+    if (e->has_moe && c.tp_size > 1) return bad("engine_create: sparse-MoE layers are not combined with tensor parallelism");
+    const size_t kept = e->allocs.size();          // behind these: the workspace of a batch and the cache
+    auto workspace = [&]() {
+        // per-token vectors hold max_batch tokens (prompt batches), [token][n]
+        bool ok = dev_alloc(e, e->hidden, (size_t)e->max_batch * h) && dev_alloc(e, e->hidden2, h) && dev_alloc(e, e->proj, (size_t)e->max_batch * h) &&
+                  dev_alloc(e, e->qkv, (size_t)e->max_batch * qkv_rows) && dev_alloc(e, e->gate_up, (size_t)e->max_batch * 2 * inter) &&
+                  dev_alloc(e, e->logits, (size_t)e->max_batch * (c.tp_size > 1 ? c.vocab_total : c.vocab_size)) && dev_alloc(e, e->act_q, (size_t)e->max_batch * act_n) &&
+                  dev_alloc(e, e->act_s, (size_t)e->max_batch * act_n / 64) && dev_alloc(e, e->act_m, (size_t)e->max_batch * act_n / 64) &&
+                  dev_alloc(e, e->act_half.zero, 1) && dev_alloc(e, e->act_half.img, act_half_bytes(e->max_batch, std::max(act_n, e->sh_inter_max))) &&
+                  dev_alloc(e, e->act_half.scales, act_half_scale_bytes(e->max_batch, std::max(act_n, e->sh_inter_max))) &&
+                  dev_alloc(e, e->q_i8, (size_t)e->max_batch * q_dim) && dev_alloc(e, e->attn_tap, q_dim) && dev_alloc(e, e->q_scale, (size_t)e->max_batch * n_q) &&
+                  dev_alloc(e, e->part_m, (size_t)n_q * e->n_split) && dev_alloc(e, e->part_l, (size_t)n_q * e->n_split) &&
+                  dev_alloc(e, e->part_o, (size_t)n_q * e->n_split * hd) &&
+                  alloc_kv(e, c.kv_bits, c.kv_window, c.kv_sinks) &&
+                  dev_alloc(e, e->d_token, e->max_batch) && dev_alloc(e, e->d_pos, 1) && dev_alloc(e, e->d_step, 1) &&
+                  dev_alloc(e, e->d_history, c.max_seq_len) && dev_alloc(e, e->d_dbg, 32) && dev_alloc(e, e->argmax_scratch, ARGMAX_SCRATCH_WORDS);
+        const uint32_t xg = c.tp_size > 1 ? c.tp_size : c.ep_size, xr = c.tp_size > 1 ? c.tp_rank : c.ep_rank;     // exchange group
+        if (ok && xg > 1) {
+            const size_t slot = std::max<size_t>((size_t)e->max_batch * h, c.vocab_size), floats = 2 * (size_t)xg * slot;
+            void *raw = nullptr;
+            // floats | 256 bytes of flags | (value, call number) words of the fused sums: [2][tp][max_batch * hidden] x 8 bytes
+            const size_t ll_slot = (size_t)e->max_batch * h, total = floats * 4 + 256 + 2 * (size_t)xg * ll_slot * 8;
+            ok = cuda_ok(ctx, cudaMalloc(&raw, total), "cudaMalloc(tp exchange)");
+            if (ok) {
+                e->allocs.push_back(raw);
+                e->tp_buf = static_cast<float *>(raw);
+                e->tp.ll_slot = (uint32_t)ll_slot;
+                e->tp.peer_ll[xr] = reinterpret_cast<unsigned long long *>(static_cast<uint8_t *>(raw) + floats * 4 + 256);
+                e->tp.wait_polls = TP_WAIT_POLLS_DEFAULT;
+                if (const char *v = std::getenv("KRONOS_CUDA_PEER_WAIT_POLLS")) e->tp.wait_polls = (uint32_t)std::strtoul(v, nullptr, 10);
+                ok = cuda_ok(ctx, cudaMemsetAsync(raw, 0, total, ctx->stream), "clear tp exchange") &&
+                     dev_alloc(e, e->tp.epoch, 1) && dev_alloc(e, e->tp_done, 1) && dev_alloc(e, e->logits_local, (size_t)e->max_batch * c.vocab_size);
+                e->tp.tp = xg; e->tp.rank = xr; e->tp.slot = (uint32_t)slot; e->tp.err = ctx->d_err;
+                e->tp.peer_data[xr] = e->tp_buf;
+                e->tp.peer_flags[xr] = reinterpret_cast<uint32_t *>(e->tp_buf + floats);
+            }
         }
-    }
-    if (ok && e->has_moe) {
-        const uint32_t k = std::min(c.moe_top_k, c.moe_num_experts), dff = c.moe_d_ff;
-        ok = dev_alloc(e, e->x_norm, (size_t)e->max_batch * h) && dev_alloc(e, e->router_logits, (size_t)e->max_batch * 256) && dev_alloc(e, e->router_done, e->max_batch) &&
-             dev_alloc(e, e->moe_gu, (size_t)e->max_batch * k * 2 * dff) && dev_alloc(e, e->moe_out, (size_t)e->max_batch * k * h) &&
-             dev_alloc(e, e->moe_q, (size_t)e->max_batch * k * dff) && dev_alloc(e, e->moe_s, (size_t)e->max_batch * k * dff / 64) &&
-             dev_alloc(e, e->moe_m, (size_t)e->max_batch * k * dff / 64);
-        const uint32_t tiles = expert_tiles_max((size_t)e->max_batch * k, c.moe_num_experts);
-        ok = ok && dev_alloc(e, e->tiles.n_tiles, 1) && dev_alloc(e, e->tiles.expert, tiles) && dev_alloc(e, e->tiles.pairs, (size_t)tiles * 32);
-        if (ok && e->sh_inter_max > 0) {
-            const size_t si = e->sh_inter_max;
-            ok = dev_alloc(e, e->sh_gu, (size_t)e->max_batch * 2 * si) && dev_alloc(e, e->sh_out, (size_t)e->max_batch * h) && dev_alloc(e, e->sh_scale, e->max_batch) &&
-                 dev_alloc(e, e->sh_q, (size_t)e->max_batch * si) && dev_alloc(e, e->sh_s, (size_t)e->max_batch * si / 64) && dev_alloc(e, e->sh_m, (size_t)e->max_batch * si / 64);
+        if (ok && e->has_moe) {
+            const uint32_t k = std::min(c.moe_top_k, c.moe_num_experts), dff = c.moe_d_ff;
+            ok = dev_alloc(e, e->x_norm, (size_t)e->max_batch * h) && dev_alloc(e, e->router_logits, (size_t)e->max_batch * 256) && dev_alloc(e, e->router_done, e->max_batch) &&
+                 dev_alloc(e, e->moe_gu, (size_t)e->max_batch * k * 2 * dff) && dev_alloc(e, e->moe_out, (size_t)e->max_batch * k * h) &&
+                 dev_alloc(e, e->moe_q, (size_t)e->max_batch * k * dff) && dev_alloc(e, e->moe_s, (size_t)e->max_batch * k * dff / 64) &&
+                 dev_alloc(e, e->moe_m, (size_t)e->max_batch * k * dff / 64);
+            const uint32_t tiles = expert_tiles_max((size_t)e->max_batch * k, c.moe_num_experts);
+            ok = ok && dev_alloc(e, e->tiles.n_tiles, 1) && dev_alloc(e, e->tiles.expert, tiles) && dev_alloc(e, e->tiles.pairs, (size_t)tiles * 32);
+            if (ok && e->sh_inter_max > 0) {
+                const size_t si = e->sh_inter_max;
+                ok = dev_alloc(e, e->sh_gu, (size_t)e->max_batch * 2 * si) && dev_alloc(e, e->sh_out, (size_t)e->max_batch * h) && dev_alloc(e, e->sh_scale, e->max_batch) &&
+                     dev_alloc(e, e->sh_q, (size_t)e->max_batch * si) && dev_alloc(e, e->sh_s, (size_t)e->max_batch * si / 64) && dev_alloc(e, e->sh_m, (size_t)e->max_batch * si / 64);
+            }
         }
+        return ok && cuda_ok(ctx, cudaStreamSynchronize(ctx->stream), "engine_create sync") && setup_mega(e);
+    };
+    // Where memory is short the same with smaller batches: an engine that fitted with 256 tokens still does, with as much to spare
+    // for what its owner allocates next.  (The buffers of the exchanges are the same size on every rank: no smaller batch there.)
+    const bool may_shrink = c.tp_size <= 1 && c.ep_size <= 1;
+    for (;;) {
+        cudaGetLastError();
+        const bool ok = workspace();
+        size_t free_bytes = 0, total = 0;
+        if (ok && (!may_shrink || e->max_batch <= 256 || (cudaMemGetInfo(&free_bytes, &total) == cudaSuccess && free_bytes >= WORKSPACE_SPARE))) break;
+        if (!ok && (cudaGetLastError() != cudaErrorMemoryAllocation || e->max_batch <= 16 || !may_shrink)) return bad(ctx->err);
+        cudaStreamSynchronize(ctx->stream);
+        for (size_t i = kept; i < e->allocs.size(); ++i) cudaFree(e->allocs[i]);
+        e->allocs.resize(kept);
+        e->k_q8 = e->v_q8 = e->v_t = nullptr; e->k_scale = e->v_scale = e->attn_sc = e->attn_bmax = nullptr;          // alloc_kv frees what it finds
+        e->max_batch = std::max(16u, (e->max_batch / 2) & ~15u);
+        ctx->err.clear();
     }
-    if (!ok || !cuda_ok(ctx, cudaStreamSynchronize(ctx->stream), "engine_create sync")) return bad(ctx->err);
-    if (!setup_mega(e)) return bad(ctx->err);
     return e;
 }
 

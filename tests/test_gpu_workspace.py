@@ -98,3 +98,29 @@ def test_score_scratch_of_a_long_cache():
         assert taken < scores + cache + rest + 64 * MB
     finally:
         e.close(); ctx.close()
+
+
+@pytest.mark.parametrize("left_mb", [3000, 2200, 1400, 800])
+def test_engine_with_smaller_batches_where_memory_is_short(left_mb):
+    """Weights of 0.1 GB, a workspace of 1.74 GB for batches of 512 tokens, 0.87 for 256, 0.44 for 128.  3 GB hold 512 and the spare half;
+    2.2 GB not the spare half, 1.4 GB not 512, 0.8 GB not 256.  Same bits as an engine with all the memory."""
+    import torch
+
+    import kronos_2t_b200 as k2
+    from kronos_2t_b200 import synth
+    torch.zeros(1, device="cuda")
+    cfg = dict(hidden=64, layers=2, n_q=2, n_kv=1, head_dim=64, inter=64 * 2048, vocab=524288, max_seq=640, eps=1e-5, theta=1e4)
+    spec = synth.random_model(cfg, "b4", seed=4)
+    tokens = np.random.Generator(np.random.PCG64(3)).integers(0, 128, 600).astype(np.uint32)
+    ctx = k2.Context(0)
+    try:
+        e = k2.Engine(ctx, spec)
+        want = e.forward_token_ids(tokens), e.forward_token_ids(tokens[:1], pos_start=600)
+        e.close()
+        with Full(left_mb * MB):
+            e = k2.Engine(ctx, spec)
+            got = e.forward_token_ids(tokens), e.forward_token_ids(tokens[:1], pos_start=600)
+            e.close()
+        assert all(np.array_equal(a, b) for a, b in zip(got, want))
+    finally:
+        ctx.close()
