@@ -116,7 +116,7 @@ bool wide_batch(uint32_t n_tok) { return gemm_tc_min_tokens() != 0 && n_tok >= g
 bool gemv_from(KronosCudaEngine *e, const KronosCudaMatrix *m, const int8_t *q, const float *sc, const int32_t *sums, float *out, const char *what,
                uint32_t n_tok, bool image_ready = false) {
     uint32_t launched = 0;
-    cudaError_t err = wide_batch(n_tok)
+    cudaError_t err = wide_batch(n_tok) && (image_ready || gemm_f16_pays(m->dm.geom.rows, m->dm.geom.nc, n_tok, e->ctx->sm_count))
                           ? launch_gemm_f16(e->ctx->stream, m->dm, q, sc, n_tok, e->act_half, out, m->dm.geom.rows, e->ctx->sm_count, e->ctx->d_err, &launched, e->pdl, image_ready)
                           : launch_gemv_batch(e->ctx->stream, m->dm, q, sc, sums, n_tok, out, m->dm.geom.rows, nullptr, e->ctx->sm_count, e->ctx->d_err, &launched, e->pdl);
     return count(e, err, what, launched);

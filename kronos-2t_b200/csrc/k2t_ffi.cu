@@ -319,7 +319,7 @@ static int32_t linear_impl(KronosCudaContext *ctx, const KronosCudaMatrix *m, co
     const uint32_t min_tok = gemm_tc_min_tokens();
     // prompt-sized calls: the activations are the library's own, so their chunk sums are consistent.  Without memory for the operand
     // image the kernel that needs none serves the call.
-    bool half = min_tok != 0 && n_tok >= min_tok && gemm_f16_takes(n_tok);
+    bool half = min_tok != 0 && n_tok >= min_tok && gemm_f16_takes(n_tok) && gemm_f16_pays(g.rows, g.nc, n_tok, ctx->sm_count);
     if (half && (!reserve(ctx, ctx->half, act_half_bytes(n_tok, g.cols)) || !reserve(ctx, ctx->half_xs, act_half_scale_bytes(n_tok, g.cols)))) {
         half = false;
         release(ctx->half); release(ctx->half_xs);

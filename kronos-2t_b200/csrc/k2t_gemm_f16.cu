@@ -654,6 +654,10 @@ cudaError_t launch_gemm_experts(cudaStream_t stream, const DeviceMatrix &m0, int
 }
 
 bool gemm_f16_takes(size_t n_tok) { return n_tok != 0 && act_half_tokens(n_tok) / 32 <= 0xFFFFu; }
+bool gemm_f16_pays(uint32_t rows, uint32_t nc, size_t n_tok, int sm_count) {
+    const uint32_t tile = gemm_tc_tile(rows, n_tok, sm_count);
+    return tile == 64 || (tile == 32 && nc >= 16);
+}
 size_t act_half_bytes(size_t n_tok, uint32_t cols) { return act_half_tokens(n_tok) * cols * 2; }
 size_t act_half_scale_bytes(size_t n_tok, uint32_t cols) { return act_half_tokens(n_tok) / 32 * (cols / 64) * HF_REC; }
 

@@ -16,6 +16,13 @@ struct ActHalf {
 };
 inline size_t act_half_tokens(size_t n_tok) { return (n_tok + 127) & ~(size_t)127; }
 bool gemm_f16_takes(size_t n_tok);          // batches whose padded tokens, 32 to a CTA of either launch, fit a grid
+// Whether a batch of int8 activations is better off converted and multiplied here than by the integer GEMM, which needs no conversion
+// launch.  Rotation + product of both, integer -> this one: as long as the integer GEMM fills less than half the SMs with its tiles of
+// 16 tokens it is 8 to 25% faster (2048 columns x 2048 rows, 128 tokens 19.4 -> 21.3 us; 18944 x 3584, 64 tokens 127 -> 138 us; 576 x 960,
+// 100 tokens 8.4 -> 9.9 us), beyond that slower (2048 x 6144, 33 tokens 22.5 -> 20.4 us; 18944 x 3584, 65 tokens 165 -> 139 us; 2048 x
+// 49152, 512 tokens 528 -> 276 us) - but for few chunks, whose launches weigh more (576 x 960, 512 tokens 12.2 -> 13.5 us in tiles of 32;
+// 576 x 1536 12.9 -> 11.9 us in tiles of 64).
+bool gemm_f16_pays(uint32_t rows, uint32_t nc, size_t n_tok, int sm_count);
 size_t act_half_bytes(size_t n_tok, uint32_t cols);
 size_t act_half_scale_bytes(size_t n_tok, uint32_t cols);
 

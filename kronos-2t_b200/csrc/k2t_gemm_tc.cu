@@ -492,12 +492,7 @@ cudaError_t launch_tc_n(cudaStream_t stream, const TcArgs &args, bool pdl) {
 
 template <int FMT>
 cudaError_t launch_tc_fmt(cudaStream_t stream, const TcArgs &args, int sm_count, bool pdl) {
-    // the narrowest token tile that holds the batch, halved while the grid would leave half the SMs idle: a CTA's time per
-    // chunk is bounded by the expansion of its weights and the hand-offs between its roles, less by its tokens
-    const uint32_t row_tiles = (args.g.rows + TC_M - 1) / TC_M;
-    uint32_t n = args.n_tok > 32 ? 64 : args.n_tok > 16 ? 32 : 16;
-    while (n > 16 && 2 * row_tiles * ((args.n_tok + n - 1) / n) <= (uint32_t)sm_count) n /= 2;
-    for (; n >= 16; n /= 2) {          // a tile whose tables do not fit shared memory: try the next narrower one
+    for (uint32_t n = gemm_tc_tile(args.g.rows, args.n_tok, sm_count); n >= 16; n /= 2) {          // a tile whose tables do not fit shared memory: try the next narrower one
         cudaError_t e = n == 64 ? launch_tc_n<FMT, 64>(stream, args, pdl) : n == 32 ? launch_tc_n<FMT, 32>(stream, args, pdl) : launch_tc_n<FMT, 16>(stream, args, pdl);
         if (e != cudaErrorNotSupported) return e;
     }
@@ -505,6 +500,15 @@ cudaError_t launch_tc_fmt(cudaStream_t stream, const TcArgs &args, int sm_count,
 }
 
 }  // namespace
+
+uint32_t gemm_tc_tile(uint32_t rows, size_t n_tok, int sm_count) {
+    // the narrowest token tile that holds the batch, halved while the grid would leave half the SMs idle: a CTA's time per
+    // chunk is bounded by the expansion of its weights and the hand-offs between its roles, less by its tokens
+    const size_t row_tiles = (rows + TC_M - 1) / TC_M;
+    uint32_t n = n_tok > 32 ? 64 : n_tok > 16 ? 32 : 16;
+    while (n > 16 && 2 * row_tiles * ((n_tok + n - 1) / n) <= (size_t)sm_count) n /= 2;
+    return n;
+}
 
 uint32_t gemm_tc_min_tokens() {
     static const uint32_t v = [] {

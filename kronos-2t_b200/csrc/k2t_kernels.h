@@ -32,6 +32,8 @@ cudaError_t launch_gemv_batch(cudaStream_t stream, const DeviceMatrix &m, const 
                               size_t n_tok, float *out, size_t out_stride, int32_t *int_dots, int sm_count, uint32_t *err_flag,
                               uint32_t *launches, bool pdl = false);
 
+// Tokens per CTA of the integer GEMM for a call (16, 32 or 64).
+uint32_t gemm_tc_tile(uint32_t rows, size_t n_tok, int sm_count);
 // Fewest tokens of a call that the tensor cores take (KRONOS_CUDA_TC_MIN_TOKENS, 16; 0 = never).
 uint32_t gemm_tc_min_tokens();
 

@@ -1,5 +1,7 @@
 """The prompt GEMM over half-precision operand images (kronos_cuda_linear with sixteen tokens and more, prompt batches of the engine)
 against the oracle's batch forms, bit for bit."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -68,3 +70,39 @@ def test_largest_dots(ctx, oracle, fmt):
         book[:1 << bits] = np.linspace(-127, 127, 1 << bits).round()
         m = oracle.nf_pack(idx, np.full(oracle.lib().k2o_nf_scale_count(rows, cols, 1), 0x3F80, np.uint16), bits, 1, book)
     _check(ctx, oracle, m, x)
+
+
+class Image(C.Structure):
+    _fields_ = [("img", C.c_void_p), ("scales", C.c_void_p), ("zero", C.c_void_p)]
+
+
+@pytest.mark.parametrize("fmt", FORMATS)
+@pytest.mark.parametrize("rows,cols,n_tok", [(54, 64, 16), (71, 1536, 17), (300, 2112, 33), (129, 576, 128), (260, 4160, 100), (18944, 128, 64), (18944, 192, 131)])
+def test_product_of_converted_activations(ctx, oracle, fmt, rows, cols, n_tok):
+    """The same sizes by the launch itself: kronos_cuda_linear leaves batches that the integer GEMM multiplies faster to it."""
+    import torch
+
+    from k2t_internal import internal
+    launch = internal("launch_gemm_f16", C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_uint32, C.POINTER(Image), C.c_void_p, C.c_size_t, C.c_int, C.c_void_p,
+                      C.c_void_p, C.c_bool, C.c_bool)
+    x = normal(n_tok * 7 + rows, (n_tok, cols))
+    x[n_tok - 1, cols - 64:] = 0.0
+    x[n_tok // 2, :] = 0.0
+    if cols > 1024:
+        x[:, 960:1024] = 0.0
+    m = _wide_matrix(oracle, fmt, rows, cols)
+    act = oracle.act_populate_fwht(x)
+    want = oracle.nibble4_gemv(oracle.nibble4_from_bipolar(m, False), act) if m.kind == 0 else oracle.nf_gemv(m, act)
+    q, s = torch.from_numpy(np.array(act.q)).cuda(), torch.from_numpy(np.array(act.scales)).cuda()
+    pad = (n_tok + 127) // 128 * 128
+    img, rec = (torch.full((n,), 0x7F, dtype=torch.uint8, device="cuda") for n in (pad * cols * 2 + 1024, pad // 32 * (cols // 64) * 144))
+    out, err = torch.zeros(n_tok, rows, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    image = Image((img.data_ptr() + 1023) // 1024 * 1024, rec.data_ptr(), None)
+    dm = upload(ctx, m)          # its handle: a KronosCudaMatrix, the DeviceMatrix first
+    try:
+        e = launch(torch.cuda.current_stream().cuda_stream, dm.handle, q.data_ptr(), s.data_ptr(), n_tok, C.byref(image), out.data_ptr(), rows, 148, err.data_ptr(), None, False, False)
+        torch.cuda.synchronize()
+    finally:
+        dm.free()
+    assert e == 0 and err.item() == 0
+    assert np.array_equal(out.cpu().numpy(), want)

@@ -56,3 +56,16 @@ def test_largest_batch_of_the_prompt_gemm():
     assert [takes(n) for n in (0, 1, 16, 512, 2097024, 2097025, 2097120, 2097121, 2 ** 32 + 16)] == [False, True, True, True, True, False, False, False, False]
     for n in range(2096900, 2097200):
         assert takes(n) == ((n + 127) // 128 * 4 <= 65535)
+
+
+# (rows, cols, tokens): the conversion launch pays / does not, as measured with 148 SMs
+CONVERTED = [(6144, 2048, 33), (16384, 2048, 17), (49152, 2048, 17), (49152, 2048, 512), (2048, 2048, 200), (3584, 18944, 65), (4608, 3584, 100), (1536, 576, 512)]
+DIRECT = [(64, 192, 16), (960, 576, 100), (1536, 576, 200), (960, 576, 512), (1024, 192, 512), (2048, 2048, 128), (2048, 8192, 128), (6144, 2048, 32), (16384, 2048, 16),
+          (49152, 2048, 16), (3584, 18944, 64), (4608, 3584, 64)]
+
+
+def test_which_batches_are_converted():
+    pays = internal("gemm_f16_pays", C.c_bool, C.c_uint32, C.c_uint32, C.c_size_t, C.c_int)
+    assert [x for x in CONVERTED if not pays(x[0], x[1] // 64, x[2], 148)] == []
+    assert [x for x in DIRECT if pays(x[0], x[1] // 64, x[2], 148)] == []
+    assert all(pays(rows, nc, n, 148) for rows in (64, 49152) for nc in (1, 300) for n in (16 * 0xFFFF + 1, 2000000))          # more than the integer GEMM takes
