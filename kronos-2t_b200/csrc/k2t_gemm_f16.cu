@@ -22,7 +22,7 @@
 // expert_tiles_kernel has gathered; a producer warp fetches the pairs' int8 rows where they lie and widens them on the way.  As one GEMV
 // per pair, 2048 pairs of 128 experts (1536 x 2048, 3 bits) took 686 us, bound by expanding the codes again for every pair; 2400 pairs
 // in tiles take 206 us, still bound by the expansion (203 tiles at most, 0.55 us per chunk and SM with two CTAs resident).
-// Every wait is bounded; a wait that gives up raises the context's error word and all roles leave.
+// Every wait is bounded; a wait that gives up raises the context's error word, and all roles come to their end.
 // Measured (B200, 256 tokens, image included): 16384 x 2048 nf4g128 55 us against 98 us with int32 accumulators, 2048 x 8192 57 against
 // 75; a 1000-token prompt through 12 layers of the 1.7B shape 21.5 -> 18.4 ms, 77 tokens through 4 layers of the 7B shape 2.09 -> 1.59 ms.
 // What bounds it: instruction issue (0.59 per scheduler and cycle, 3000 warp instructions per chunk of 128 rows x 128 tokens, half of
@@ -246,8 +246,7 @@ __global__ void __launch_bounds__(HfRoles<N, EXP>::THREADS, EXP ? 2 : 1) gemm_f1
 #pragma unroll 1
         for (uint32_t c0 = 0; c0 < nc; c0 += 2) {
             // `full` has completed by the time of `done`: waiting for it orders this thread after the scales' stores and copies
-            ok = mbar_wait_warp(bar_done + 8 * s, ph, HF_WAIT_LIMIT, s_abort) && mbar_wait_warp(bar_full + 8 * s, ph, HF_WAIT_LIMIT, s_abort);
-            if (!ok) break;
+            ok = ok && mbar_wait_thread(bar_done + 8 * s, ph, HF_WAIT_LIMIT, s_abort) && mbar_wait_thread(bar_full + 8 * s, ph, HF_WAIT_LIMIT, s_abort);
             hf_fence_after();
             uint32_t ws_bits[2], any[2];          // of both chunks, requested together (a second chunk that does not exist: old ones, not used)
 #pragma unroll
@@ -289,10 +288,10 @@ __global__ void __launch_bounds__(HfRoles<N, EXP>::THREADS, EXP ? 2 : 1) gemm_f1
             }
             hf_fence_before();
             __syncwarp();
-            if (lane == 0) hf_arrive(bar_drained + 8 * s);
+            if (lane == 0 && ok) hf_arrive(bar_drained + 8 * s);
             if (++s == S) { s = 0; ph ^= 1u; }
         }
-        if (!ok && lane == 0 && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
+        if (!ok && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
         if constexpr (EXP) {
             if (ok && row < a.rows) {
                 const uint32_t *pairs = args.tile_pairs + blockIdx.y * N + part * NQ;
@@ -379,10 +378,7 @@ __global__ void __launch_bounds__(HfRoles<N, EXP>::THREADS, EXP ? 2 : 1) gemm_f1
             asm volatile("cp.async.commit_group;" ::: "memory");
             uint32_t h[32];
             hf_expand<FMT>(w, tables, h);
-            if (p >= S) {
-                ok = mbar_wait_warp(bar_drained + 8 * s, ((p / S) - 1u) & 1u, HF_WAIT_LIMIT, s_abort);          // the products of the stage are done by then
-                if (!ok) break;
-            }
+            if (p >= S) ok = ok && mbar_wait_thread(bar_drained + 8 * s, ((p / S) - 1u) & 1u, HF_WAIT_LIMIT, s_abort);          // the products of the stage are done by then
             if (c < nc) {
                 const uint32_t dst = sbase + L::A + (2 * s + half) * HF_A_STAGE + i * 128;
 #pragma unroll
@@ -392,10 +388,10 @@ __global__ void __launch_bounds__(HfRoles<N, EXP>::THREADS, EXP ? 2 : 1) gemm_f1
             }
             fence_proxy_async();
             __syncwarp();
-            if (lane == 0) hf_arrive(bar_full + 8 * s);
+            if (lane == 0 && ok) hf_arrive(bar_full + 8 * s);
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
-        if (!ok && lane == 0 && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
+        if (!ok && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
     } else if (warp == EPI + DEC) {
         if (lane == 0) {
             // ------------------------------------------------------------------ issue
@@ -453,10 +449,7 @@ __global__ void __launch_bounds__(HfRoles<N, EXP>::THREADS, EXP ? 2 : 1) gemm_f1
 #pragma unroll 1
         for (uint32_t p = 0; 2 * p < nc; ++p) {
             const uint32_t s = p % S;
-            if (p >= S) {
-                ok = mbar_wait_warp(bar_drained + 8 * s, ((p / S) - 1u) & 1u, HF_WAIT_LIMIT, s_abort);
-                if (!ok) break;
-            }
+            if (p >= S) ok = ok && mbar_wait_thread(bar_drained + 8 * s, ((p / S) - 1u) & 1u, HF_WAIT_LIMIT, s_abort);
 #pragma unroll
             for (uint32_t h = 0; h < 2; ++h) {
                 const uint32_t dst = sbase + L::B + (2 * s + h) * (N * 128), rec = sbase + L::XS + ((2 * p + h) % HF_SLOTS) * HF_REC;
@@ -480,9 +473,9 @@ __global__ void __launch_bounds__(HfRoles<N, EXP>::THREADS, EXP ? 2 : 1) gemm_f1
             load(2 * p + 2);
             fence_proxy_async();
             __syncwarp();
-            if (lane == 0) hf_arrive(bar_full + 8 * s);
+            if (lane == 0 && ok) hf_arrive(bar_full + 8 * s);
         }
-        if (!ok && lane == 0 && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
+        if (!ok && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
     } else if (lane == 0) {
         // ------------------------------------------------------------------ activations and their scales
         constexpr uint32_t XB = (N / 32) * HF_REC;

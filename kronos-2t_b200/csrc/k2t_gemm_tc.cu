@@ -269,19 +269,19 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs arg
         };
         // one step of the software pipeline: the dots of chunk c are on their way into `cur`; once they are in, the buffer goes
         // back to the issuing thread, the dots of chunk c + 1 are requested into `nxt`, and the chains advance meanwhile
-        auto step = [&](uint32_t c, int (&cur)[NQ], int (&nxt)[NQ]) -> bool {
+        auto step = [&](uint32_t c, int (&cur)[NQ], int (&nxt)[NQ]) {
             TC_ACC_T(0);
             tc_ld_wait(cur);
             TC_ACC_T(1);
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar_drained + 8 * (c % TC_ACC));
+            if (lane == 0 && ok) mbar_arrive(bar_drained + 8 * (c % TC_ACC));
             TC_ACC_T(4);
             if (c + 1 < nc) {
                 TC_ACC_T(5);
                 // `done` (the products) and `full` (already complete by then: it orders this thread after the decode threads' stores of the chunk's scales)
-                if (!mbar_wait_warp(bar_done + 8 * ((c + 1) % TC_ACC), ((c + 1) / TC_ACC) & 1u, WAIT_LIMIT, s_abort)) return false;
-                if (!mbar_wait_warp(bar_full + 8 * ((c + 1) % TC_ACC), ((c + 1) / TC_ACC) & 1u, WAIT_LIMIT, s_abort)) return false;
+                ok = ok && mbar_wait_thread(bar_done + 8 * ((c + 1) % TC_ACC), ((c + 1) / TC_ACC) & 1u, WAIT_LIMIT, s_abort) &&
+                     mbar_wait_thread(bar_full + 8 * ((c + 1) % TC_ACC), ((c + 1) / TC_ACC) & 1u, WAIT_LIMIT, s_abort);
                 TC_ACC_T(6);
                 tc_fence_after();
                 tc_ld<NQ>(taddr0 + ((c + 1) % TC_ACC) * N, nxt);
@@ -289,22 +289,19 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs arg
             TC_ACC_T(2);
             advance(c, cur);
             TC_ACC_T(3);
-            return true;
         };
         int v0[NQ], v1[NQ];
-        ok = mbar_wait_warp(bar_done, 0u, WAIT_LIMIT, s_abort) && mbar_wait_warp(bar_full, 0u, WAIT_LIMIT, s_abort);
-        if (ok) {
-            tc_fence_after();
-            tc_ld<NQ>(taddr0, v0);
-            for (uint32_t c = 0; c < nc && ok; c += 2) {
-                ok = step(c, v0, v1);
-                if (ok && c + 1 < nc) ok = step(c + 1, v1, v0);
-            }
+        ok = ok && mbar_wait_thread(bar_done, 0u, WAIT_LIMIT, s_abort) && mbar_wait_thread(bar_full, 0u, WAIT_LIMIT, s_abort);
+        tc_fence_after();
+        tc_ld<NQ>(taddr0, v0);
+        for (uint32_t c = 0; c < nc; c += 2) {
+            step(c, v0, v1);
+            if (c + 1 < nc) step(c + 1, v1, v0);
         }
 #ifdef K2T_TC_TRACE
         if (tid == 0 && blockIdx.x == 0 && blockIdx.y == 0) for (int k = 0; k < 8; ++k) g_tc_trace[k] = trace_acc[k];
 #endif
-        if (!ok && lane == 0 && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
+        if (!ok && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
         if (ok && row < a.rows) {
 #pragma unroll
             for (uint32_t t = 0; t < NQ; ++t) {
@@ -407,11 +404,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs arg
             uint32_t u[16];
             decode<FMT>(w, a.cb, u);
             TC_ACC_T(2);
-            if (c >= TC_STAGES) {
-                ok = mbar_wait_warp(bar_done + 8 * s, ((c / TC_STAGES) - 1u) & 1u, WAIT_LIMIT, s_abort) &&
-                     mbar_wait_warp(bar_drained + 8 * s, ((c / TC_STAGES) - 1u) & 1u, WAIT_LIMIT, s_abort);
-                if (!ok) break;
-            }
+            if (c >= TC_STAGES)
+                ok = ok && mbar_wait_thread(bar_done + 8 * s, ((c / TC_STAGES) - 1u) & 1u, WAIT_LIMIT, s_abort) &&
+                     mbar_wait_thread(bar_drained + 8 * s, ((c / TC_STAGES) - 1u) & 1u, WAIT_LIMIT, s_abort);
             TC_ACC_T(3);
             const uint32_t a_dst = sbase + L.a + s * TC_A_STAGE + (i >> 3) * TC_SBO + (i & 7u) * 16;
 #pragma unroll
@@ -431,14 +426,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs arg
             }
             fence_proxy_async();
             __syncwarp();
-            if (lane == 0) mbar_arrive(bar_full + 8 * s);
+            if (lane == 0 && ok) mbar_arrive(bar_full + 8 * s);
             TC_ACC_T(4);
         }
 #ifdef K2T_TC_TRACE
         if (di == 0 && blockIdx.x == 0 && blockIdx.y == 0) for (int k = 0; k < 5; ++k) g_tc_trace[8 + k] = trace_acc[k];
 #endif
         cp_async_wait<0>();
-        if (!ok && lane == 0 && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
+        if (!ok && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
     } else if (lane == 0) {
         // ------------------------------------------------------------------ issue
         // instruction descriptor: int32 accumulators, signed 8-bit A and B, both K-major, N / 8, M / 16
