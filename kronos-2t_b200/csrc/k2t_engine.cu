@@ -407,7 +407,7 @@ bool enqueue_batch(KronosCudaEngine *e, uint32_t T, bool embed, Tail tail, bool 
             ra.route_ids = L.d_route_ids; ra.route_w = L.d_route_w; ra.logits = e->router_logits; ra.done = e->router_done; ra.route_stride = 32; ra.err_flag = e->ctx->d_err;
             if (!count(e, launch_moe_router(s, ra, e->pdl, T), "router")) return false;
             const uint32_t E = c.moe_num_experts;
-            const bool grouped = experts_grouped(T, T * k, E);
+            const bool grouped = experts_grouped(T, T * k, E, h, dff, c.moe_bits);
             if (grouped && !count(e, launch_expert_tiles(s, L.d_route_ids, T, k, 32, E, L.d_gu_bases, e->tiles, e->ctx->d_err, e->pdl), "expert tiles")) return false;
             if (!count(e, grouped ? launch_gemm_experts(s, L.gu_dm, L.gu_fmt, L.d_gu_books, L.d_gu_bases, E, e->tiles, T * k, k, e->act_q, e->act_s, e->moe_gu, e->ctx->d_err, e->pdl)
                                   : launch_gemv_experts(s, L.gu_dm, L.gu_fmt, L.d_gu_books, L.d_gu_bases, L.d_route_ids, T * k, e->act_q, e->act_s, e->act_m, h, h / 64,

@@ -28,6 +28,7 @@
 // What bounds it: instruction issue (0.59 per scheduler and cycle, 3000 warp instructions per chunk of 128 rows x 128 tokens, half of
 // them chain steps and expansion, the rest waits and hand-overs).
 #include <algorithm>
+#include <cmath>
 
 #include "k2t_act_image.cuh"
 #include "k2t_gemv_core.cuh"
@@ -616,9 +617,13 @@ template <int FMT> cudaError_t launch_hf_fmt(cudaStream_t s, const HfArgs &args,
 
 }  // namespace
 
-bool experts_grouped(uint32_t n_tok, uint32_t n_pair, uint32_t n_experts) {
+bool experts_grouped(uint32_t n_tok, uint32_t n_pair, uint32_t n_experts, uint32_t hidden, uint32_t d_ff, uint32_t bits) {
     const uint32_t min_tok = gemm_tc_min_tokens();
-    return min_tok != 0 && n_tok >= min_tok && n_pair >= std::max(3 * n_experts, 48u);
+    if (min_tok == 0 || n_tok < min_tok || n_experts == 0 || bits < 2 || bits > 5) return false;
+    // in units of a tile form's time per million weights (0.5 us)
+    constexpr float START = 120.0f, PAIR[4] = {6.0f, 1.4f, 2.2f, 4.2f}, PAIR_PER_WEIGHT[4] = {0.6f, 0.25f, 0.38f, 0.55f};          // 2 .. 5 bits
+    const float w = 3e-6f * (float)hidden * (float)d_ff, met = (float)n_experts * (1.0f - std::exp(-(float)n_pair / (float)n_experts));
+    return (float)n_pair * std::max(PAIR[bits - 2], PAIR_PER_WEIGHT[bits - 2] * w) >= START + met * w;
 }
 uint32_t expert_tiles_max(size_t n_pair, uint32_t n_experts) { return (uint32_t)(n_pair / 32 + std::min<size_t>(n_pair, n_experts)); }
 

@@ -42,11 +42,12 @@ uint32_t expert_tiles_max(size_t n_pair, uint32_t n_experts);
 cudaError_t launch_expert_tiles(cudaStream_t stream, const uint32_t *route_ids, uint32_t n_tok, uint32_t k, uint32_t route_stride, uint32_t n_experts,
                                 const uint8_t *const *bases, const ExpertTiles &t, uint32_t *err_flag, bool pdl);
 
-// Prompts take the grouped form from three pairs per expert on.  A GEMV costs per pair (0.33 us each for gate_up and down of the 30B-A3B
-// shape: 128 experts, 2048 x 1536 and 768 x 2048, 3 bits), a tile per expert: 24 / 32 / 44 / 64 / 150 tokens with 8 routes through three
-// layers take 857 / 995 / 1238 / 1605 / 4024 us as GEMVs and 1113 / 1193 / 1271 / 1352 / 1498 us in tiles.  Few experts leave SMs
-// idle: 48 pairs at least.  It is a tensor-core form: only for batches that gemm_tc_min_tokens() hands to the tensor cores.
-bool experts_grouped(uint32_t n_tok, uint32_t n_pair, uint32_t n_experts);
+// Whether the expert projections of a batch run in tiles (below) or as a GEMV per pair.  Tiles are a tensor-core form: only for batches that
+// gemm_tc_min_tokens() hands over.  Their time goes with the weights of the experts that the pairs meet, a GEMV's per pair, with the weights
+// of one expert and the cost of its decode.  Measured with 2048 columns, 2 layers: tokens at which tiles (first) and GEMVs take the same, by
+// experts / routes / width / bits: 128 / 8 / 768 / 3 60 (56: 953 and 909 us, 64: 962 and 1040), 4 39, 5 15; 64 / 6 / 768 / 3 47, 4 30, 5 and 2 fewer
+// than 16; 64 / 6 / 1408 / 3 54; 16 / 4 / 2816 / 3 20, 4 14; 8 / 2 / 4096 / 4 18; 4 / 2 / 2048 / 3 22; 256 / 8 / 768 / 2 fewer than 8.
+bool experts_grouped(uint32_t n_tok, uint32_t n_pair, uint32_t n_experts, uint32_t hidden, uint32_t d_ff, uint32_t bits);
 
 // The expert projections of all pairs of `t`, an expert's weights expanded once per 32 pairs; out = [n_pair][rows].  Same bits as
 // launch_gemv_experts, for activations in the form the library's own quantizers leave them.

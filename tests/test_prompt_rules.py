@@ -45,8 +45,8 @@ def in_process(code, **env):
 @pytest.mark.parametrize("switch,want", [(None, "0 1 1"), ("0", "0 0 0"), ("200", "0 0 1")])
 def test_expert_tiles_obey_the_tensor_core_switch(switch, want):
     """512 pairs of 8 experts as 8, 100 and 300 tokens: the grouped form is a tensor-core form."""
-    code = ("import ctypes as C; from k2t_internal import internal; f = internal('experts_grouped', C.c_bool, C.c_uint32, C.c_uint32, C.c_uint32); "
-            "print(*[int(f(t, 512, 8)) for t in (8, 100, 300)])")
+    code = ("import ctypes as C; from k2t_internal import internal; f = internal('experts_grouped', C.c_bool, *[C.c_uint32] * 6); "
+            "print(*[int(f(t, 512, 8, 2048, 4096, 4)) for t in (8, 100, 300)])")
     assert in_process(code, **({} if switch is None else dict(KRONOS_CUDA_TC_MIN_TOKENS=switch))) == want
 
 
@@ -69,3 +69,15 @@ def test_which_batches_are_converted():
     assert [x for x in CONVERTED if not pays(x[0], x[1] // 64, x[2], 148)] == []
     assert [x for x in DIRECT if pays(x[0], x[1] // 64, x[2], 148)] == []
     assert all(pays(rows, nc, n, 148) for rows in (64, 49152) for nc in (1, 300) for n in (16 * 0xFFFF + 1, 2000000))          # more than the integer GEMM takes
+
+
+# experts, routes, width, bits: tokens at which a GEMV per pair was faster, at which tiles were (2048 columns)
+@pytest.mark.parametrize("n_experts,k,d_ff,bits,gemv,tiles", [
+    (128, 8, 768, 3, (16, 32, 48, 56), (64, 72, 128)), (128, 8, 768, 4, (16, 32), (48, 64)), (128, 8, 768, 5, (), (20, 32, 64)), (128, 8, 768, 2, (), (16, 32, 64)),
+    (64, 6, 768, 3, (16, 32, 40), (56, 64)), (64, 6, 768, 4, (16, 24), (32, 48)), (64, 6, 768, 5, (), (16, 24)), (64, 6, 768, 2, (), (16, 24)),
+    (64, 6, 1408, 3, (16, 32, 48), (64, 80)), (16, 4, 2816, 3, (16,), (24, 32)), (16, 4, 2816, 4, (), (16, 20)), (16, 4, 2816, 5, (), (16,)),
+    (8, 2, 4096, 4, (16,), (20, 32)), (4, 2, 2048, 3, (16, 20), (32, 48)), (256, 8, 768, 2, (), (16, 32))])
+def test_experts_take_the_faster_form(n_experts, k, d_ff, bits, gemv, tiles):
+    grouped = internal("experts_grouped", C.c_bool, *[C.c_uint32] * 6)
+    form = {t: grouped(t, t * k, n_experts, 2048, d_ff, bits) for t in gemv + tiles}
+    assert form == {**dict.fromkeys(gemv, False), **dict.fromkeys(tiles, True)}
