@@ -347,16 +347,17 @@ __global__ void __launch_bounds__(VAL_THREADS) attn_values_kernel(const ExactAtt
     // the weights need the denominator).
     const bool is_tw = CW == 4 ? (warp >= 4 && warp < 8) : (warp == 2 || warp == 3 || warp == 6 || warp == 7);
     const uint32_t tw = CW == 4 ? warp - 4 : (warp < 4 ? warp - 2 : warp - 4);          // transposing warp index 0..3 (0 = warp CW, the producer's)
-    bool failed = false;          // a wait of this thread gave up
     // tile i: rows of stage i % NST -> transposed tile i % VAL_TBUF; the producer lane refills the stage once all have read it
-    auto transpose_tile = [&](uint32_t i) {          // a lane that has given up stays with its warp (see mbar_wait_thread) and waits no more
+    auto transpose_tile = [&](uint32_t i) -> bool {
         const uint32_t st = i % NST, tb = i % VAL_TBUF, n = min(VAL_TILE, ctx - i * VAL_TILE);
-        failed = failed || !mbar_wait_bounded(bar_full + 8 * st, (i / NST) & 1u);
-        if (i >= VAL_TBUF) failed = failed || !mbar_wait_bounded(bar_t_free + 8 * tb, ((i / VAL_TBUF) - 1u) & 1u);
+        // a lane that gives up keeps its warp's count of __syncwarp, here and behind the loops
+        if (!mbar_wait_bounded(bar_full + 8 * st, (i / NST) & 1u)) { __syncwarp(); return false; }
+        if (i >= VAL_TBUF && !mbar_wait_bounded(bar_t_free + 8 * tb, ((i / VAL_TBUF) - 1u) & 1u)) { __syncwarp(); return false; }
         value_rows_transpose<HD, KV4>((uint32_t)__cvta_generic_to_shared(stages + (size_t)st * Sm::STAGE), tiles_t + tb * Sm::TILE_T, VAL_TILE,
                                       (n + 15) / 16, tw, NTW, lane);
         __syncwarp();
-        if (lane == 0 && !failed) mbar_arrive(bar_rows_free + 8 * st);
+        if (lane == 0) mbar_arrive(bar_rows_free + 8 * st);
+        return true;
     };
     // producer (lane 0 of the ninth warp): tile i + NST goes into the stage of tile i once every transposing warp has read it
     auto refill_after = [&](uint32_t i) -> bool {
@@ -366,6 +367,7 @@ __global__ void __launch_bounds__(VAL_THREADS) attn_values_kernel(const ExactAtt
         return true;
     };
     constexpr uint32_t PRODUCER_WARP = VAL_THREADS / 32 - 1;
+    bool failed = false;
     const uint32_t li = tw * 32 + lane;                            // transposing warps: this lane's position within a tile (and li + NTW * 32)
     constexpr uint32_t PER = (VAL_TILE + NTW * 32 - 1) / (NTW * 32);
     float sc_first[4][PER];
@@ -385,7 +387,9 @@ __global__ void __launch_bounds__(VAL_THREADS) attn_values_kernel(const ExactAtt
                 sc_first[u][k] = (li + k * NTW * 32 < VAL_TILE && t < ctx) ? __ldcg(a.v_scale + slot0 + t) : 0.0f;
             }
     } else if (is_tw && !direct) {
-        for (uint32_t i = 0; i < VAL_TBUF && i < n_tiles; ++i) transpose_tile(i);
+        uint32_t i = 0;
+        for (; i < VAL_TBUF && i < n_tiles && !failed; ++i) failed = !transpose_tile(i);
+        for (; i < VAL_TBUF && i < n_tiles; ++i) __syncwarp();
     } else if (warp == PRODUCER_WARP && lane == 0 && !direct) {
         for (uint32_t i = 0; i < VAL_TBUF && i < n_tiles && !failed; ++i) failed = !refill_after(i);
     }
@@ -401,20 +405,18 @@ __global__ void __launch_bounds__(VAL_THREADS) attn_values_kernel(const ExactAtt
         const uint32_t d = tid, fd = vt_swz(d);                    // this thread's dimension
         const uint32_t cbfa = (uint32_t)__cvta_generic_to_shared(s_cb);
         const uint32_t wa0 = (uint32_t)__cvta_generic_to_shared(W + (KV4 ? (size_t)(d / 64) * w_stride : 0));
-        for (uint32_t i = 0; i < n_tiles; ++i) {
+        uint32_t i = 0;
+        for (; i < n_tiles; ++i) {
             const uint32_t tb = i % VAL_TBUF, tl = i * VAL_TILE, n = min(VAL_TILE, ctx - tl);
             if (i + 2 >= n_tiles) pdl_trigger();       // one thread's call releases the CTA: only the chain warps call it
             const long long tw0 = clock64();
             const uint32_t st = i % NST;
-            if (direct) {          // the tile's weights (the weight warps run ahead through all tiles); its bytes below
+            if (direct) {          // the tile's weights (the weight warps run ahead through all tiles) and its bytes
                 uint32_t spin = 0;
-                while (!failed && min(min(s_ready[0], s_ready[1]), min(s_ready[2], s_ready[3])) <= i && ++spin < EXACT_WAIT_LIMIT) {}
+                while (min(min(s_ready[0], s_ready[1]), min(s_ready[2], s_ready[3])) <= i && ++spin < EXACT_WAIT_LIMIT) {}
                 __threadfence_block();
-                failed = failed || spin >= EXACT_WAIT_LIMIT;
-            }
-            // a lane that has given up stays with its warp (see mbar_wait_thread) and waits no more
-            if (direct) failed = failed || !mbar_wait_bounded(bar_full + 8 * st, (i / NST) & 1u);
-            else failed = failed || !mbar_wait_bounded(bar_t_full + 8 * tb, (i / VAL_TBUF) & 1u);
+                if (spin >= EXACT_WAIT_LIMIT || !mbar_wait_bounded(bar_full + 8 * st, (i / NST) & 1u)) { failed = true; break; }
+            } else if (!mbar_wait_bounded(bar_t_full + 8 * tb, (i / VAL_TBUF) & 1u)) { failed = true; break; }
             t_wait += clock64() - tw0;
             const uint32_t wa = wa0 + 4 * tl;
             // transposed tile: row d, swizzled chunks; direct: the ring stage as it landed, block b = [dimension][16]
@@ -434,8 +436,9 @@ __global__ void __launch_bounds__(VAL_THREADS) attn_values_kernel(const ExactAtt
             }
             if (rem != 0) o = value_chain16<KV4>(o, x, w0, w1, w2, w3, cbfa, rem);
             __syncwarp();
-            if (lane == 0 && !failed) mbar_arrive(direct ? bar_rows_free + 8 * st : bar_t_free + 8 * tb);      // this warp is done with the tile
+            if (lane == 0) mbar_arrive(direct ? bar_rows_free + 8 * st : bar_t_free + 8 * tb);      // this warp is done with the tile
         }
+        for (; i < n_tiles; ++i) __syncwarp();          // of a lane that has given up
         if (failed) atomicExch(&s_fail, 1u);
         if (a.trace != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) a.trace[8] = (unsigned long long)t_wait;
         s_o[d] = o;
@@ -486,14 +489,15 @@ __global__ void __launch_bounds__(VAL_THREADS) attn_values_kernel(const ExactAtt
             }
         }
         if (n_tiles > 0 && !direct) load_scales(0);
-        for (uint32_t i = 0; i < n_tiles && !direct; ++i) {
+        uint32_t i = 0;
+        for (; i < n_tiles && !failed && !direct; ++i) {
             float sc_cur[PER][KV4 ? NB : 1];
 #pragma unroll
             for (uint32_t k = 0; k < PER; ++k)
 #pragma unroll
                 for (int g = 0; g < (KV4 ? NB : 1); ++g) sc_cur[k][g] = sc_next[k][g];
             if (i + 1 < n_tiles) load_scales(i + 1);
-            if (i >= VAL_TBUF) transpose_tile(i);
+            if (i >= VAL_TBUF) failed = !transpose_tile(i);
 #pragma unroll
             for (uint32_t k = 0; k < PER; ++k) {
                 const uint32_t t = i * VAL_TILE + li + k * NTW * 32;
@@ -508,7 +512,11 @@ __global__ void __launch_bounds__(VAL_THREADS) attn_values_kernel(const ExactAtt
                 }
             }
             __syncwarp();
-            if (lane == 0 && !failed) mbar_arrive(bar_t_full + 8 * (i % VAL_TBUF));
+            if (lane == 0) mbar_arrive(bar_t_full + 8 * (i % VAL_TBUF));
+        }
+        for (; i < n_tiles && !direct; ++i) {
+            if (i >= VAL_TBUF) __syncwarp();
+            __syncwarp();
         }
         if (failed) atomicExch(&s_fail, 1u);
     } else if (warp == PRODUCER_WARP && lane == 0) {

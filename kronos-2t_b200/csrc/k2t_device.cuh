@@ -135,10 +135,9 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
 }
 // Bounded wait of one thread on an mbarrier phase; gives up after `limit` polls or once another role has set the CTA's abort word.
 // The lanes of a warp poll at different times and may see the phase, the abort word or the limit apart.  A lane that left its role
-// alone would leave the others at the warp's next collective (a vote, __syncwarp, tcgen05.ld) for good, so a role of several lanes
-// either votes on the answer (mbar_wait_warp) or stays to its end with `ok = ok && mbar_wait_thread(..)`: no lane leaves, a lane
-// that has given up waits no more, and what the role hands over is only announced by a lane that is still ok.  (The second costs
-// nothing: a vote per stage made a prompt of 77 tokens through the 7B shape 3% slower, decoding at 4000 positions 1.5%.)
+// alone would leave the others at the warp's next collective for good, so a role of several lanes takes one of three forms: it votes
+// on the answer (mbar_wait_warp); or a lane stays to the end with `ok = ok && mbar_wait_thread(..)`, waits no more and announces nothing;
+// or, where the only collective is __syncwarp, it leaves the loop and then runs as many of them as the loop had left.
 __device__ __forceinline__ bool mbar_wait_thread(uint32_t bar, uint32_t parity, uint32_t limit, volatile uint32_t *abort_w) {
     for (uint32_t spin = 0; spin < limit; ++spin) {
         if (mbar_try_wait(bar, parity)) return true;

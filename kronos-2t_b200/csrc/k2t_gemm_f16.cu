@@ -360,8 +360,9 @@ __global__ void __launch_bounds__(HfRoles<N, EXP>::THREADS, EXP ? 2 : 1) gemm_f1
             asm volatile("cp.async.commit_group;" ::: "memory");
         }
         bool ok = true;
+        uint32_t p = pair0;
 #pragma unroll 1
-        for (uint32_t p = pair0; 2 * p < nc; p += PSTEP) {
+        for (; 2 * p < nc; p += PSTEP) {
             const uint32_t s = p % S, c = 2 * p + half;
             asm volatile("cp.async.wait_group %0;" ::"n"(L::PFG - 1) : "memory");
             Raw<FMT> w;
@@ -379,7 +380,10 @@ __global__ void __launch_bounds__(HfRoles<N, EXP>::THREADS, EXP ? 2 : 1) gemm_f1
             asm volatile("cp.async.commit_group;" ::: "memory");
             uint32_t h[32];
             hf_expand<FMT>(w, tables, h);
-            if (p >= S) ok = ok && mbar_wait_thread(bar_drained + 8 * s, ((p / S) - 1u) & 1u, HF_WAIT_LIMIT, s_abort);          // the products of the stage are done by then
+            if (p >= S) {
+                ok = mbar_wait_thread(bar_drained + 8 * s, ((p / S) - 1u) & 1u, HF_WAIT_LIMIT, s_abort);          // the products of the stage are done by then
+                if (!ok) break;
+            }
             if (c < nc) {
                 const uint32_t dst = sbase + L::A + (2 * s + half) * HF_A_STAGE + i * 128;
 #pragma unroll
@@ -389,8 +393,9 @@ __global__ void __launch_bounds__(HfRoles<N, EXP>::THREADS, EXP ? 2 : 1) gemm_f1
             }
             fence_proxy_async();
             __syncwarp();
-            if (lane == 0 && ok) hf_arrive(bar_full + 8 * s);
+            if (lane == 0) hf_arrive(bar_full + 8 * s);
         }
+        for (; 2 * p < nc; p += PSTEP) __syncwarp();          // of a lane that has given up
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         if (!ok && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
     } else if (warp == EPI + DEC) {

@@ -371,7 +371,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs arg
         unsigned long long trace_acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         long long _tl = clock64();
 #endif
-        for (uint32_t c = grp; c < nc; c += TC_GROUPS) {
+        uint32_t c = grp;
+        for (; c < nc; c += TC_GROUPS) {
             const uint32_t s = c % TC_STAGES;
             TC_ACC_T(0);
             cp_async_wait<TC_PFG - 1>();
@@ -404,9 +405,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs arg
             uint32_t u[16];
             decode<FMT>(w, a.cb, u);
             TC_ACC_T(2);
-            if (c >= TC_STAGES)
-                ok = ok && mbar_wait_thread(bar_done + 8 * s, ((c / TC_STAGES) - 1u) & 1u, WAIT_LIMIT, s_abort) &&
+            if (c >= TC_STAGES) {
+                ok = mbar_wait_thread(bar_done + 8 * s, ((c / TC_STAGES) - 1u) & 1u, WAIT_LIMIT, s_abort) &&
                      mbar_wait_thread(bar_drained + 8 * s, ((c / TC_STAGES) - 1u) & 1u, WAIT_LIMIT, s_abort);
+                if (!ok) break;
+            }
             TC_ACC_T(3);
             const uint32_t a_dst = sbase + L.a + s * TC_A_STAGE + (i >> 3) * TC_SBO + (i & 7u) * 16;
 #pragma unroll
@@ -426,9 +429,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(const TcArgs arg
             }
             fence_proxy_async();
             __syncwarp();
-            if (lane == 0 && ok) mbar_arrive(bar_full + 8 * s);
+            if (lane == 0) mbar_arrive(bar_full + 8 * s);
             TC_ACC_T(4);
         }
+        for (; c < nc; c += TC_GROUPS) __syncwarp();          // of a lane that has given up
 #ifdef K2T_TC_TRACE
         if (di == 0 && blockIdx.x == 0 && blockIdx.y == 0) for (int k = 0; k < 5; ++k) g_tc_trace[8 + k] = trace_acc[k];
 #endif

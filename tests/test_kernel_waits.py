@@ -31,6 +31,27 @@ def of_one_thread(text, at):
     return any(re.search(r"\b(?:lane|tid) == 0\b", h) for h in headers(text, at)) or re.search(r"\b(?:lane|tid) == 0\)\s*$", text[:at])
 
 
+def drained(text, at):
+    """The loop around a place is followed by the __syncwarps that it had left (its only collectives), or the place runs its own."""
+    if re.match(r"[^;{}]*\)\s*\{ __syncwarp\(\); return false; \}", text[at:]):
+        return True
+    depth = 0
+    for i in range(at - 1, -1, -1):
+        depth += {"}": 1, "{": -1}.get(text[i], 0)
+        if depth < 0:
+            depth = 0
+            if re.search(r"\bfor \([^{}]*$", text[max(text.rfind(c, 0, i) for c in "{}") + 1:i]):
+                break
+    else:
+        return False
+    for j in range(i, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[j], 0)
+        if depth == 0:
+            body = text[i:j]
+            return not re.search(r"__(all|any)_sync|shfl|tcgen05|hf_ld16|tc_ld", body) and bool(re.match(r"\}\s*for \(; [^)]*\) (?:\{\s*)?(?:if \([^)]*\) )?__syncwarp\(\);", text[j:]))
+    return False
+
+
 def splits(text):
     """Places of a role of several lanes where a lane takes its own answer and leaves, or takes one that it may leave by."""
     text = re.sub(r"//[^\n]*", "", text)
@@ -41,13 +62,17 @@ def splits(text):
         if re.search(r"bool mbar_wait\w+\($|__device__", statement) or "bool mbar_wait" in "".join(headers(text, m.start())[:1]) or of_one_thread(text, m.start()):
             continue
         stays = re.search(r"\bok = ok && |\bfailed = failed \|\| ", statement)
-        if not stays and not VOTE.search(statement + ";" + behind):
+        if not stays and not VOTE.search(statement + ";" + behind) and not drained(text, m.start()):
             bad.append(statement.strip())
     for m in LEAVE.finditer(text):
         name = next(g for g in m.groups() if g)
         before = re.findall(rf"\b{name} = ([^;]*);", text[:m.start()])
-        if not of_one_thread(text, m.start()) and not (before and VOTE.search(before[-1])):
-            bad.append(m.group(0))
+        loop = m.start() if m.group(0).startswith("if") else text.index("{" if ") {" in text[m.start():m.start() + 200] else ";", m.end()) + 1
+        if of_one_thread(text, m.start()) or (before and VOTE.search(before[-1])) or drained(text, loop):
+            continue
+        if m.group(0).startswith("for") and re.match(r"[^;{}]*\) [^;{}]*;\s*for \(; [^)]*\) __syncwarp\(\);", text[m.end():]):
+            continue          # a loop of one statement
+        bad.append(m.group(0))
     return bad
 
 
@@ -62,6 +87,8 @@ def test_a_wait_that_gives_up_does_not_split_its_warp(source):
     ("ok = ok && mbar_wait_thread(bar, 0, 9, s_abort); if (!ok) { failed = true; break; } __syncwarp();", True),
     ("ok = mbar_wait_warp(bar, 0, 9, s_abort); if (!ok) break; __syncwarp();", False),
     ("ok = ok && mbar_wait_thread(bar, 0, 9, s_abort); __syncwarp();", False),
+    ("ok = mbar_wait_thread(bar, 0, 9, s_abort); if (!ok) break; __syncwarp(); } for (; i < n; ++i) { __syncwarp();", False),
+    ("ok = mbar_wait_thread(bar, 0, 9, s_abort); if (!ok) break; tc_ld8(t, v); } for (; i < n; ++i) { __syncwarp();", True),
 ])
 def test_the_reading_itself(role, found):
     assert bool(splits("void kernel() { if (warp < 4) { for (;;) { " + role + " } } }")) is found
