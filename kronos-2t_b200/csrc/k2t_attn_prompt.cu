@@ -15,7 +15,7 @@
 // One token per CTA, as in decoding, converts every value byte for a single chain step and has four lanes busy with the
 // denominator while the others wait.
 // Sixteen rows: enough to share a value byte and to fill two warps with denominators, few enough that three CTAs fit an SM at a
-// thousand positions (64 bytes of scores per position).  From sixteen tokens on: below, a launch has too few CTAs.
+// thousand positions (64 bytes of scores per position).
 // Measured (B200): 256 tokens of 32 heads of 64 at 0 .. 1000 positions 58 us on average against 193 us (scores + values, a token and head
 // per CTA); a 1000-token prompt through 12 layers of the 1.7B shape 18.4 -> 11.9 ms.  Bound by shared memory (0.25 broadcast
 // wavefronts per chain step) and fp32 issue together.
@@ -285,17 +285,33 @@ constexpr size_t PROMPT_SMEM_MAX = 220 * 1024;
 
 }  // namespace
 
+bool attention_prompt_fits(uint32_t head_dim, uint32_t ctx) {
+    return head_dim == 64 ? PromptAttn<64, 8>::bytes(ctx) <= PROMPT_SMEM_MAX : head_dim == 128 && PromptAttn<128, 8>::bytes(ctx) <= PROMPT_SMEM_MAX;
+}
+uint32_t attention_prompt_rows(uint32_t head_dim, uint32_t ctx) {
+    if (!attention_prompt_fits(head_dim, ctx)) return 0;
+    return (head_dim == 64 ? PromptAttn<64, 16>::bytes(ctx) : PromptAttn<128, 16>::bytes(ctx)) <= PROMPT_SMEM_MAX ? 16 : 8;
+}
+bool attention_prompt_pays(uint32_t n_tok, uint32_t n_q, uint32_t n_kv, uint32_t head_dim, uint32_t ctx) {
+    const uint32_t rows = n_tok * n_q;
+    if (n_tok < PROMPT_ATTN_MIN_TOKENS) return false;
+    if (n_q == n_kv) return rows >= 1536 || ctx <= (rows >= 1024 ? 512u : 256u);
+    if (head_dim == 128) return rows >= 896 || ctx <= 768;
+    return rows >= 1152 || ctx <= (rows >= 576 ? 896u : 384u);
+}
 bool attention_prompt_takes(const ExactAttnArgs &a, uint32_t n_tok) {
-    if (a.kv_bits != 8 || a.v_t == nullptr || a.ring.window != 0 || n_tok < PROMPT_ATTN_MIN_TOKENS) return false;
-    return (a.head_dim == 64 ? PromptAttn<64, 8>::bytes(a.ctx_cap) : PromptAttn<128, 8>::bytes(a.ctx_cap)) <= PROMPT_SMEM_MAX && (a.head_dim == 64 || a.head_dim == 128);
+    return a.kv_bits == 8 && a.v_t != nullptr && a.ring.window == 0 && attention_prompt_fits(a.head_dim, a.ctx_cap) &&
+           attention_prompt_pays(n_tok, a.n_kv * a.group, a.n_kv, a.head_dim, a.ctx_cap);
 }
 
 cudaError_t launch_attention_prompt(cudaStream_t s, const ExactAttnArgs &args, bool pdl, uint32_t n_tok) {
-    if (!attention_prompt_takes(args, n_tok) || args.group == 0) return cudaErrorInvalidValue;
+    if (args.kv_bits != 8 || args.v_t == nullptr || args.ring.window != 0 || args.group == 0 || n_tok == 0) return cudaErrorInvalidValue;
+    const uint32_t rows = attention_prompt_rows(args.head_dim, args.ctx_cap);
+    if (rows == 0) return cudaErrorInvalidValue;
     ExactAttnArgs a = args;
     a.n_tok = n_tok;
-    if (a.head_dim == 64) return PromptAttn<64, 16>::bytes(a.ctx_cap) <= PROMPT_SMEM_MAX ? launch_prompt<64, 16>(s, a, pdl) : launch_prompt<64, 8>(s, a, pdl);
-    return PromptAttn<128, 16>::bytes(a.ctx_cap) <= PROMPT_SMEM_MAX ? launch_prompt<128, 16>(s, a, pdl) : launch_prompt<128, 8>(s, a, pdl);
+    if (a.head_dim == 64) return rows == 16 ? launch_prompt<64, 16>(s, a, pdl) : launch_prompt<64, 8>(s, a, pdl);
+    return rows == 16 ? launch_prompt<128, 16>(s, a, pdl) : launch_prompt<128, 8>(s, a, pdl);
 }
 
 }  // namespace k2t

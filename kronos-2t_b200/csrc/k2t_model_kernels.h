@@ -155,6 +155,17 @@ cudaError_t launch_attention_exact(cudaStream_t s, const ExactAttnArgs &a, bool 
 // the same for a prompt batch over the int8 cache with a full causal context: one kernel, rows of a kv head side by side
 // (k2t_attn_prompt.cu).  attention_prompt_takes: cache format, context (shared memory) and batch suit it.
 constexpr uint32_t PROMPT_ATTN_MIN_TOKENS = 16;
+// rows of a CTA for contexts of up to ctx positions: 16, 8 where their scores do not fit shared memory, 0 where eight do not either
+uint32_t attention_prompt_rows(uint32_t head_dim, uint32_t ctx);
+// A CTA walks through the context once for its rows, so few rows (tokens x heads) behind a long context leave the SMs to the two-kernel form,
+// which has a CTA per token and head.  Whole prompts of n tokens behind p positions, two kernels -> this one in us:
+//   a kv head per head (1.7B, 32 heads of 64, 4 layers): 48 + 600 776 -> 736, 64 + 6300 2437 -> 2174, 512 + 6300 16130 -> 9238 (any context from
+//     1536 rows on); 32 + 340 691 -> 675, + 600 718 -> 725; 16 + 220 633 -> 629, + 340 642 -> 656, + 6300 1085 -> 1637
+//   grouped heads of 128 (7B, 28 over 4, 2 layers): 32 + 1000 820 -> 783, + 3000 959 -> 967, + 6300 1170 -> 1155 (any from 896 rows on); 16 + 730
+//     779 -> 760, + 1500 797 -> 835, + 6300 958 -> 1151
+//   grouped heads of 64 (135M, 9 over 3, 10 layers): 128 + 2200 1393 -> 1320, 256 + 6300 5216 -> 4080 (any from 1152 rows on); 64 + 500 816 -> 764,
+//     + 1000 894 -> 906, + 3000 1225 -> 1466; 16 + 340 702 -> 687, + 470 718 -> 732, + 6300 1034 -> 2248
+bool attention_prompt_pays(uint32_t n_tok, uint32_t n_q, uint32_t n_kv, uint32_t head_dim, uint32_t ctx);
 bool attention_prompt_takes(const ExactAttnArgs &a, uint32_t n_tok);
 cudaError_t launch_attention_prompt(cudaStream_t s, const ExactAttnArgs &a, bool pdl, uint32_t n_tok);
 // longest context launch_attention_exact can serve (its value weights live in shared memory)

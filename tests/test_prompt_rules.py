@@ -81,3 +81,25 @@ def test_experts_take_the_faster_form(n_experts, k, d_ff, bits, gemv, tiles):
     grouped = internal("experts_grouped", C.c_bool, *[C.c_uint32] * 6)
     form = {t: grouped(t, t * k, n_experts, 2048, d_ff, bits) for t in gemv + tiles}
     assert form == {**dict.fromkeys(gemv, False), **dict.fromkeys(tiles, True)}
+
+
+# heads, kv heads, head size, tokens, context: where the row-sharing attention was slower, where it was faster
+SLOWER = [(32, 32, 64, 16, 384), (32, 32, 64, 32, 1024), (32, 32, 64, 16, 6400), (9, 3, 64, 16, 512), (9, 3, 64, 48, 640), (9, 3, 64, 64, 3072), (9, 3, 64, 64, 6400),
+          (28, 4, 128, 16, 1536), (28, 4, 128, 16, 6400)]
+FASTER = [(32, 32, 64, 16, 128), (32, 32, 64, 32, 384), (32, 32, 64, 48, 640), (32, 32, 64, 64, 6400), (32, 32, 64, 512, 6400), (9, 3, 64, 16, 384), (9, 3, 64, 64, 640),
+          (9, 3, 64, 128, 2432), (9, 3, 64, 256, 6400), (28, 4, 128, 16, 768), (28, 4, 128, 32, 1152), (28, 4, 128, 64, 6400), (28, 4, 128, 512, 6400), (32, 4, 128, 32, 3584)]
+
+
+def test_which_batches_share_rows():
+    pays = internal("attention_prompt_pays", C.c_bool, *[C.c_uint32] * 5)
+    ask = lambda q, kv, d, n, ctx: pays(n, q, kv, d, ctx)  # noqa: E731
+    assert [x for x in SLOWER if ask(*x)] == [] and [x for x in FASTER if not ask(*x)] == []
+    assert not any(ask(32, 4, 128, n, 128) for n in range(1, 16))
+
+
+def test_rows_of_an_attention_tile():
+    """Scores of 16 rows take 64 bytes per position (rounded up to 16), beside the queries and outputs, in 220 KB."""
+    rows = internal("attention_prompt_rows", C.c_uint32, C.c_uint32, C.c_uint32)
+    last = lambda d, r: max(ctx for ctx in range(128, 8192) if rows(d, ctx) >= r)  # noqa: E731
+    assert [last(64, 16), last(128, 16), last(64, 8), last(128, 8)] == [3424, 3344, 6944, 6864]
+    assert rows(96, 128) == 0
