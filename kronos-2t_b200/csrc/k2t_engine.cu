@@ -38,10 +38,18 @@ bool engine_count(KronosCudaEngine *e, cudaError_t err, const char *what, uint32
     return cuda_ok(e->ctx, err, what);
 }
 
-uint32_t prompt_batch(size_t left, uint32_t max_batch) {
-    const size_t tile = max_batch % 128 == 0 ? 128 : 16, most = max_batch / tile;
-    const size_t tiles = (left + tile - 1) / tile, batches = (tiles + most - 1) / most;
-    return batches == 0 ? 0u : (uint32_t)std::min(left, (tiles + batches - 1) / batches * tile);
+uint32_t prompt_batch(size_t n_tok, size_t done, uint32_t max_batch, bool experts) {
+    const size_t left = n_tok - done, batches = (n_tok + max_batch - 1) / max_batch, tail = n_tok % max_batch;
+    size_t n = max_batch;
+    if (tail > (experts ? 32u : 64u)) {
+        if (experts) {          // whole token tiles of the projections, dealt out evenly
+            const size_t tile = max_batch % 128 == 0 ? 128 : 16, tiles = (left + tile - 1) / tile, most = max_batch / tile, more = (tiles + most - 1) / most;
+            n = more == 0 ? 0 : (tiles + more - 1) / more * tile;
+        } else {
+            n = ((n_tok + batches - 1) / batches + 127) & ~(size_t)127;
+        }
+    }
+    return (uint32_t)std::min(std::min<size_t>(n, max_batch), left);
 }
 
 }  // namespace k2t
@@ -1316,7 +1324,7 @@ static int32_t forward_common(KronosCudaEngine *e, const float *embeds, const ui
     if (!set_u32(e, e->d_pos, (uint32_t)pos_start)) return -1;
     for (size_t t0 = 0, T_done = 0; t0 < n_tok; t0 += T_done) {
         // block models fill each batch: 2049 / 4097 tokens as two / three even batches took 2 to 14% longer than as full ones and a single token
-        uint32_t T = e->blocks ? (uint32_t)std::min<size_t>(e->max_batch, n_tok - t0) : prompt_batch(n_tok - t0, e->max_batch);
+        uint32_t T = e->blocks ? (uint32_t)std::min<size_t>(e->max_batch, n_tok - t0) : prompt_batch(n_tok, t0, e->max_batch, e->has_moe);
         const size_t p0 = pos_start + t0;
         if (e->split_kv && p0 < ATTN_EXACT_CTX && p0 + T > ATTN_EXACT_CTX) T = (uint32_t)(ATTN_EXACT_CTX - p0);    // split-KV kernels: a batch stays on one side of the attention switch
         const bool last = t0 + T == n_tok;

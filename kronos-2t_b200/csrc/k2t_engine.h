@@ -116,11 +116,14 @@ namespace k2t {
 // what a batch leaves behind: argmax of its (single) token, logits of the last token, of all tokens, nothing
 enum class Tail { Greedy, LastLogits, AllLogits, None };
 
-// Tokens of the next batch of a prompt with `left` tokens to go: as few batches as max_batch (a multiple of 16) allows, each of about
-// the same number of whole token tiles of the projections (128; 16 where max_batch is not a multiple of that).  A short last batch
-// would pay for a batch's launches and its weights again: 300 tokens of the 30B-A3B shape as 256 + 44 and as one: 2.86 and 1.86 ms;
-// 1000 tokens of the 1.7B shape in batches of 256 and as 512 + 488: 11.9 and 9.7 ms.
-uint32_t prompt_batch(size_t left, uint32_t max_batch);
+// Tokens of the next batch of a prompt of n_tok tokens, `done` of them behind it: as few batches as max_batch (a multiple of 16) allows.
+// Up to 64 tokens behind full batches (32 with experts) are cheap by themselves, a single one is a decode step: 513 tokens as 512 + 1
+// and as 384 + 129 took 1580 and 2055 us through 4 layers of the 1.7B shape, 1908 and 2415 through 2 of 7B, 1860 and 2277 through 2 of 30B-A3B;
+// 1537 as 3 x 512 + 1 and as 512 + 2 x 384 + 257 5380 and 5590, 5797 and 6437, 5722 and 5926.  More pay for a batch's launches and its
+// weights again: experts get whole token tiles of the projections dealt out evenly (580: 384 + 196 2404, 512 + 68 2635; 1600: 512 + 2 x 384 + 320
+// 6099, 3 x 512 + 64 6600), the others an even size rounded up to 128, which fills the batches of longer prompts (650: 384 + 266 2204, 512
+// + 138 2267 for 1.7B; 1700: 3 x 512 + 164 6590, 2 x 512 + 384 + 292 6693).
+uint32_t prompt_batch(size_t n_tok, size_t done, uint32_t max_batch, bool experts);
 
 // books `n` launches (and, while a step is profiled, an event behind them); false with the context's error set when err is one
 bool engine_count(KronosCudaEngine *e, cudaError_t err, const char *what, uint32_t n = 1);

@@ -9,31 +9,32 @@ import pytest
 from k2t_internal import internal
 
 
-def batches(n, max_batch):
-    prompt_batch = internal("prompt_batch", C.c_uint32, C.c_size_t, C.c_uint32)
-    out = []
-    while n:
-        out.append(prompt_batch(n, max_batch))
-        assert 0 < out[-1] <= min(n, max_batch)
-        n -= out[-1]
+def batches(n_tok, max_batch, experts):
+    prompt_batch = internal("prompt_batch", C.c_uint32, C.c_size_t, C.c_size_t, C.c_uint32, C.c_bool)
+    out, done = [], 0
+    while done < n_tok:
+        out.append(prompt_batch(n_tok, done, max_batch, experts))
+        assert 0 < out[-1] <= min(n_tok - done, max_batch)
+        done += out[-1]
     return out
 
 
-@pytest.mark.parametrize("n,want", [(2, [2]), (300, [300]), (512, [512]), (513, [384, 129]), (1000, [512, 488]), (1025, [384, 384, 257]), (1537, [512, 384, 384, 257]),
-                                    (1540, [512, 384, 384, 260]), (2049, [512, 512, 384, 384, 257])])
-def test_batches_of_a_prompt(n, want):
-    assert batches(n, 512) == want
+@pytest.mark.parametrize("n,dense,experts", [
+    (2, [2], None), (300, [300], None), (512, [512], None), (513, [512, 1], None), (544, [512, 32], None), (545, [512, 33], [384, 161]), (576, [512, 64], [384, 192]),
+    (577, [384, 193], None), (1000, [512, 488], None), (1025, [512, 512, 1], None), (1100, [384, 384, 332], None), (1537, [512, 512, 512, 1], None),
+    (1600, [512, 512, 512, 64], [512, 384, 384, 320]), (1700, [512, 512, 512, 164], [512, 512, 384, 292])])
+def test_batches_of_a_prompt(n, dense, experts):
+    assert batches(n, 512, False) == dense
+    assert batches(n, 512, True) == (experts or dense)
 
 
+@pytest.mark.parametrize("experts", [False, True])
 @pytest.mark.parametrize("max_batch", [16, 48, 128, 208, 256, 384, 512])
-def test_no_short_last_batch(max_batch):
-    """As few batches as there can be, alike but for one tile (the last may miss part of its own)."""
-    tile = 128 if max_batch % 128 == 0 else 16
+def test_as_few_batches_as_there_can_be(max_batch, experts):
     for n in list(range(1, 3 * max_batch + 40)) + [4001, 8192, 20011]:
-        b = batches(n, max_batch)
+        b = batches(n, max_batch, experts)
         assert sum(b) == n and len(b) == -(-n // max_batch)
-        tiles = [-(-x // tile) for x in b]
-        assert max(tiles) - min(tiles) <= 1 and all(x % tile == 0 for x in b[:-1])
+        assert all(x % 16 == 0 for x in b[:-1])
 
 
 def in_process(code, **env):
