@@ -57,8 +57,10 @@ uint32_t prompt_batch(size_t n_tok, size_t done, uint32_t max_batch, bool expert
 namespace {
 
 // Tokens per launch of the two-kernel attention: its scores take query heads x cache rows floats per token (3.7 MB with 28 heads at
-// 32 k positions), and 256 tokens of any shape are more CTAs than the SMs hold.
+// 32 k positions).  A whole batch where that is half a GB at most (300 tokens of the 135M shape over an NF4 cache as 256 + 44 took 14%
+// longer), 256 tokens where it is more.
 constexpr uint32_t SCORE_TOKENS = 256;
+constexpr size_t SCORE_BYTES = 512u << 20;
 // free memory that batches of more than 256 tokens must leave (their workspace of the 7B shape: 0.5 GB)
 constexpr size_t WORKSPACE_SPARE = 512u << 20;
 
@@ -90,7 +92,7 @@ bool alloc_kv(KronosCudaEngine *e, uint32_t bits, uint32_t window, uint32_t sink
     e->split_kv = e->ring.window == 0 && ((c.flags & KRONOS_CUDA_ENGINE_SPLIT_KV_ATTENTION) != 0 || longest > attention_exact_max_ctx(hd, bits));
     if (e->ring.window && longest > attention_exact_max_ctx(hd, bits)) return fail(ctx, "kv_window is longer than the attention kernel can hold");
     const size_t slots = (size_t)c.num_layers * c.num_key_value_heads * e->kv_stride;
-    e->score_tokens = std::min(e->max_batch, SCORE_TOKENS);
+    e->score_tokens = std::min(e->max_batch, std::max(SCORE_TOKENS, (uint32_t)std::min<size_t>(e->max_batch, SCORE_BYTES / ((size_t)n_q * e->kv_stride * 4))));
     const bool ok = dev_alloc(e, e->attn_sc, (size_t)e->score_tokens * n_q * e->kv_stride) && dev_alloc(e, e->attn_bmax, (size_t)e->score_tokens * n_q * ((e->kv_stride + 127) / 128)) &&
                     dev_alloc(e, e->k_q8, bits == 4 ? slots * hd / 2 : slots * hd) && dev_alloc(e, e->v_q8, bits == 4 ? slots * hd / 2 : slots * hd) &&
                     dev_alloc(e, e->k_scale, bits == 4 ? (slots * (hd / 64) + 1) / 2 : slots) &&      // NF4: bf16 per 64 values
@@ -288,8 +290,9 @@ bool enqueue_attention_batch(KronosCudaEngine *e, uint32_t l, uint32_t T) {
     xa.ctx_cap = attn_ctx_cap(e); xa.ring = e->ring;
     xa.kv_bits = c.kv_bits; xa.attn_scale = 1.0f / sqrtf((float)hd); xa.err_flag = e->ctx->d_err; xa.trace = nullptr; xa.v_t = e->v_t;
     if (attention_prompt_takes(xa, T)) return count(e, launch_attention_prompt(s, xa, e->pdl, T), "attention");
-    for (uint32_t t0 = 0; t0 < T; t0 += e->score_tokens) {
-        const uint32_t n = std::min(e->score_tokens, T - t0), n_q = c.num_attention_heads;
+    const uint32_t parts = (T + e->score_tokens - 1) / e->score_tokens, per = (T + parts - 1) / parts, n_q = c.num_attention_heads;
+    for (uint32_t t0 = 0; t0 < T; t0 += per) {
+        const uint32_t n = std::min(per, T - t0);
         ExactAttnArgs part = xa;
         part.q_i8 += (size_t)t0 * n_q * hd; part.q_scale += (size_t)t0 * n_q; part.pos_offset = t0;
         part.out_q += (size_t)t0 * n_q * hd; part.out_scales += (size_t)t0 * n_q * (hd / 64); part.out_sums += (size_t)t0 * n_q * (hd / 64);

@@ -55,13 +55,15 @@ def test_linear_gives_its_operand_image_back(oracle):
         ctx.close()
 
 
-@pytest.mark.parametrize("kv_bits,window", [(8, 0), (4, 0), (8, 900)])
-def test_scores_in_portions(kv_bits, window):
-    """Batches of more tokens than the score scratch holds: as batches of 256 give it, bit for bit, and no larger scratch."""
+@pytest.mark.parametrize("kv_bits,window,past,max_seq", [(8, 0, 7100, 8300), (4, 0, 700, 8300), (8, 8000, 8200, 9000)])
+def test_scores_in_portions(kv_bits, window, past, max_seq):
+    """Batches of more tokens than the score scratch holds (half a GB: 504 tokens of 32 heads over 8320 rows): as batches of 256 give it, bit for
+    bit.  Contexts that the row-sharing attention leaves alone."""
     import kronos_2t_b200 as k2
     from kronos_2t_b200 import synth
-    past, n = (7100, 512) if kv_bits == 8 and not window else (700, 512)          # contexts that the row-sharing attention leaves alone
-    cfg = dict(hidden=64, layers=2, n_q=4, n_kv=2, head_dim=64, inter=64, vocab=128, max_seq=past + n + 600, eps=1e-5, theta=1e4, kv_bits=kv_bits, kv_window=window, kv_sinks=4)
+    n = 512
+    cfg = dict(hidden=64, layers=2, n_q=32, n_kv=4, head_dim=64, inter=64, vocab=128, max_seq=max_seq, eps=1e-5, theta=1e4, kv_bits=kv_bits, kv_window=window, kv_sinks=4)
+    assert 256 <= (512 << 20) // (32 * (max_seq if not window else window + 512) * 4) < 512
     tokens = np.random.Generator(np.random.PCG64(n)).integers(0, 128, past + n).astype(np.uint32)
     ctx = k2.Context(0)
     a, b = (k2.Engine(ctx, synth.random_model(cfg, "b4", seed=4)) for _ in range(2))
