@@ -469,9 +469,9 @@ def run_b200(args, rank, world, local_rank):
                 roofline["sharded_parity"] = sharded_parity(ctx, rank, world, dist)
             except Exception as exc:
                 roofline["sharded_parity"] = {"error": f"{type(exc).__name__}: {exc}"}
-        roofline["prefill_note"] = ("prompt batches of 256 tokens: every dense projection is one launch of the tensor-core kernel (tcgen05.mma kind::i8 for the "
-                                    "exact chunk dots, fp32 chains on the CUDA cores in the reference's order), attention of the batch side by side; "
-                                    "int8_TOPs = 2 x multiply-adds of the projections x tok/s; the MoE experts still run as expert-batched GEMVs")
+        roofline["prefill_note"] = ("prompt batches of up to 512 tokens: every dense projection is one launch of the prompt GEMM (tcgen05.mma kind::f16 for the exact "
+                                    "chunk dots, fp32 chains on the CUDA cores in the reference's order), the rows of a kv head share its cached rows in attention; "
+                                    "int8_TOPs = 2 x multiply-adds of the projections x tok/s; MoE experts: the (token, route) pairs of an expert in tiles of 32")
         roofline["decode_note"] = ("frac = bytes_per_token * tok_s / (n_gpus * peak): weights of one step in the reference's file format + the cached "
                                    "rows the token attends to; n_gpus > 1: the Qwen2-7B shape tensor-parallel (tp) and the Qwen3-30B-A3B shape "
                                    "expert-parallel (ep) over all ranks - strong scaling of ONE token stream")
@@ -610,7 +610,7 @@ def decode_tok_s(ctx, stream, timed_region, world):
 
 
 def _prefill(eng, rng, vocab, lo, hi, timed_region=None):
-    """Prompt positions [lo, hi) of random token ids (batches of 256 tokens: every projection one tensor-core launch); returns
+    """Prompt positions [lo, hi) of random token ids (batches of up to 512 tokens: every projection one tensor-core launch); returns
     tok/s when timed - the second of two identical passes, so that no kernel is loaded inside the timed region."""
     toks = rng.integers(0, vocab, hi - lo).astype("uint32")
     eng.forward_token_ids(toks, pos_start=lo)

@@ -153,9 +153,6 @@ bool tp_gather(KronosCudaEngine *e, const float *slice, float *all, uint32_t n) 
 // the activation buffers of a wide batch, and the image
 PromptAct act_of(const KronosCudaEngine *e, uint32_t T) { return PromptAct{e->act_q, e->act_s, e->act_m, e->act_half, (uint32_t)act_half_tokens(T)}; }
 
-// Residual add + RMSNorm + activation of the next projection.  Under tensor parallelism `delta` is this rank's partial
-// output of a row-parallel projection: the kernel exchanges and sums the ranks' partials itself.
-// `partial`: delta holds this rank's share only (row-parallel projection under tensor parallelism, routed experts under
 // Context the attention launches beyond 512 positions are sized for (grid of the scores kernel, shared memory of the values
 // kernel): the cache's capacity (a captured decode step is replayed at any position), or, for a prompt batch whose last
 // position the host knows, that position rounded up - two values CTAs fit an SM then, and no scores CTA starts for nothing.
@@ -165,6 +162,9 @@ uint32_t attn_ctx_cap(const KronosCudaEngine *e) {
     return std::min(full, (e->ctx_bound + 127u) & ~127u);
 }
 
+// Residual add + RMSNorm + activation of the next projection.  Under tensor parallelism `delta` is this rank's partial
+// output of a row-parallel projection: the kernel exchanges and sums the ranks' partials itself.
+// `partial`: delta holds this rank's share only (row-parallel projection under tensor parallelism, routed experts under
 // expert parallelism).
 // `image`: set when the kernel has also left the operand image of a wide batch.
 bool norm_quant(KronosCudaEngine *e, const float *delta, const float *w, float *x_norm, uint32_t T, bool pdl, bool partial, bool &image) {
@@ -397,10 +397,11 @@ bool enqueue_batch(KronosCudaEngine *e, uint32_t T, bool embed, Tail tail, bool 
         }
         if (!gemv(e, L.o, e->proj, "gemv o", T)) return false;        // under tp: partial sums, exchanged by the norm kernel that follows
         if (L.moe) {
-            // SparseMoeRuntime::forward_layer_single (sparse_moe.rs:961-1084) for every token of the batch in five launches
-            // (forward_layer_coalesced_batch, 1090-1352, gives each token the same sums: its routes are visited in ascending
-            // expert order either way): routes of all tokens, then the expert projections over the (token, route) pairs -
-            // slot = token * k + route; two tokens that picked the same expert read its image twice, the second time from L2.
+            // SparseMoeRuntime::forward_layer_single (sparse_moe.rs:961-1084) for every token of the batch (forward_layer_coalesced_batch,
+            // 1090-1352, gives each token the same sums: its routes are visited in ascending expert order either way): routes of all
+            // tokens, then the expert projections over the (token, route) pairs - slot = token * k + route.  Many pairs are sorted into
+            // tiles of one expert, whose weights are then expanded once per 32 of them; few take a GEMV each, in which two tokens that
+            // picked the same expert read its image twice, the second time from L2 (experts_grouped).
             if (!norm_quant(e, e->proj, L.post_norm, e->x_norm, T, e->pdl, c.tp_size > 1, image)) return false;
             const uint32_t k = std::min(c.moe_top_k, c.moe_num_experts), dff = c.moe_d_ff;
             // shared expert (every token; under expert parallelism rank 0's partial sum carries it): two plain projections

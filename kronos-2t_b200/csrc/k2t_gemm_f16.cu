@@ -25,8 +25,8 @@
 // Every wait is bounded; a wait that gives up raises the context's error word, and all roles come to their end.
 // Measured (B200, 256 tokens, image included): 16384 x 2048 nf4g128 55 us against 98 us with int32 accumulators, 2048 x 8192 57 against
 // 75; a 1000-token prompt through 12 layers of the 1.7B shape 21.5 -> 18.4 ms, 77 tokens through 4 layers of the 7B shape 2.09 -> 1.59 ms.
-// What bounds it: instruction issue (0.59 per scheduler and cycle, 3000 warp instructions per chunk of 128 rows x 128 tokens, half of
-// them chain steps and expansion, the rest waits and hand-overs).
+// What bounds it: issue and latency together (0.53 to 0.59 instructions per scheduler and cycle, 3000 per chunk of 128 rows x 128
+// tokens and warp instruction: half of them chain steps and expansion, the rest waits and hand-overs; tensor pipe 8 to 15%).
 #include <algorithm>
 #include <cmath>
 

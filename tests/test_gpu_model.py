@@ -133,7 +133,7 @@ def test_sparse_moe_layers_match_oracle(ctx, oracle, mode, moe, kw):
 
 @pytest.mark.parametrize("batch", [16, 48, 112])
 def test_prompt_batch_size_does_not_change_results(ctx, oracle, monkeypatch, batch):
-    """The engine cuts a prompt into batches of KRONOS_CUDA_PROMPT_BATCH tokens (default 256): whatever the size - several batches
+    """The engine cuts a prompt into batches of KRONOS_CUDA_PROMPT_BATCH tokens (default 512): whatever the size - several batches
     per prompt, a ragged last one, a batch that crosses position 512 where the attention kernels change, token tiles of every
     width in the tensor-core launches - logits of every position and the cache rows equal the oracle's token-by-token run."""
     monkeypatch.setenv("KRONOS_CUDA_PROMPT_BATCH", str(batch))
