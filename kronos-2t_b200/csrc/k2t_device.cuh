@@ -138,13 +138,19 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
 // alone would leave the others at the warp's next collective for good, so a role of several lanes takes one of three forms: it votes
 // on the answer (mbar_wait_warp); or a lane stays to the end with `ok = ok && mbar_wait_thread(..)`, waits no more and announces nothing;
 // or, where the only collective is __syncwarp, it leaves the loop and then runs as many of them as the loop had left.
-__device__ __forceinline__ bool mbar_wait_thread(uint32_t bar, uint32_t parity, uint32_t limit, volatile uint32_t *abort_w) {
+// A phase that has passed costs one try: the polls follow behind a branch (a loop around the first try took 170 cycles of a
+// warp where this takes 100, and every role of the tensor-core kernels waits once or more per chunk).
+__device__ __forceinline__ bool mbar_poll(uint32_t bar, uint32_t parity, uint32_t limit, volatile uint32_t *abort_w) {
     for (uint32_t spin = 0; spin < limit; ++spin) {
         if (mbar_try_wait(bar, parity)) return true;
         if ((spin & 255u) == 255u && *abort_w != 0) return false;
     }
     *abort_w = 1;
     return false;
+}
+__device__ __forceinline__ bool mbar_wait_thread(uint32_t bar, uint32_t parity, uint32_t limit, volatile uint32_t *abort_w) {
+    if (__builtin_expect(mbar_try_wait(bar, parity), 1)) return true;
+    return mbar_poll(bar, parity, limit, abort_w);
 }
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, uint32_t limit, volatile uint32_t *abort_w) {
     return __all_sync(0xffffffffu, mbar_wait_thread(bar, parity, limit, abort_w));

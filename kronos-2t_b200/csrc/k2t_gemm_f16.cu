@@ -9,6 +9,8 @@
 // tokens per instruction: 1.3 instructions per (row, token, chunk) where the int32 accumulators of k2t_gemm_tc.cu take 4.75
 // (integer correction, conversion, multiply, fma).
 //
+// Rows of 32 chunks and more go to k2t_gemm_prompt.cu; here are the shorter ones, the conversion of the activations, and the experts.
+//
 // The activations come as an operand image (act_half_kernel below): per chunk 128 bytes per token in the 128-byte-swizzled
 // K-major layout, so a tile of tokens is one contiguous run, plus the tokens' scales.  One CTA = 128 rows x N tokens:
 //   * DECODE groups of 128 threads (thread = row) expand the row's cell of every chunk to 64 halves (A operand), from a ring
@@ -30,8 +32,7 @@
 #include <algorithm>
 #include <cmath>
 
-#include "k2t_act_image.cuh"
-#include "k2t_gemv_core.cuh"
+#include "k2t_gemm_half.cuh"
 
 namespace k2t {
 
@@ -57,8 +58,6 @@ template <int N, bool EXP = false> struct HfRoles {
     static constexpr uint32_t DEC_ARRIVALS = 8;                // decode warps that fill a stage: two groups, one per chunk
     static constexpr uint32_t TMEM = EXP ? 128 : N == 32 ? 256 : 512;      // columns (a power of two)
 };
-
-template <int FMT> __host__ __device__ constexpr uint32_t hf_cell() { return Cell<FMT>::B0 + Cell<FMT>::B1 + Cell<FMT>::B2; }
 
 template <int FMT, int N, bool EXP = false> struct HfLayout {
     static constexpr uint32_t PF = !EXP ? 8 : hf_cell<FMT>() <= 24 ? 6 : 4;          // ring slots of raw weights: chunks requested ahead
@@ -90,101 +89,6 @@ struct HfExperts {
 template <bool EXP> struct HfParam { using T = HfArgs; };
 template <> struct HfParam<true> { using T = HfExperts; };
 constexpr uint32_t HF_NO_PAIR = 0xffffffffu;
-
-__device__ __forceinline__ void hf_cp_async16(uint32_t dst, const void *src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
-__device__ __forceinline__ void hf_cp_async8(uint32_t dst, const void *src) { asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory"); }
-__device__ __forceinline__ void hf_cp_async4(uint32_t dst, const void *src) { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory"); }
-__device__ __forceinline__ uint32_t hf_lds32(uint32_t saddr) {
-    uint32_t v;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(saddr));
-    return v;
-}
-__device__ __forceinline__ void hf_lds64(uint32_t saddr, uint32_t &x, uint32_t &y) { asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(x), "=r"(y) : "r"(saddr)); }
-__device__ __forceinline__ void hf_lds128(uint32_t saddr, uint32_t *v) {
-    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(saddr));
-}
-__device__ __forceinline__ void hf_lds_pairs(uint32_t saddr, unsigned long long &x, unsigned long long &y) {
-    asm volatile("ld.shared.v2.b64 {%0,%1}, [%2];" : "=l"(x), "=l"(y) : "r"(saddr));
-}
-__device__ __forceinline__ void hf_sts128(uint32_t saddr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
-    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(saddr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
-}
-__device__ __forceinline__ void hf_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
-__device__ __forceinline__ void hf_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void hf_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void hf_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void hf_mma(uint32_t d_tmem, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t"
-        ".reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t"
-        "}\n" ::"r"(d_tmem), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
-}
-__device__ __forceinline__ uint64_t hf_desc(uint32_t saddr) {      // K-major, 128-byte swizzle, groups of eight rows 1024 bytes apart
-    return (uint64_t)((saddr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024u >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
-// sixteen accumulators of the lane's row, waited for
-__device__ __forceinline__ void hf_ld16(uint32_t taddr, uint32_t (&v)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
-        "tcgen05.wait::ld.sync.aligned;"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]),
-          "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-        : "r"(taddr) : "memory");
-}
-__device__ __forceinline__ unsigned long long hf_pack(uint32_t lo, uint32_t hi) {
-    unsigned long long d;
-    asm("mov.b64 %0, {%1,%2};" : "=l"(d) : "r"(lo), "r"(hi));
-    return d;
-}
-// two chain steps: f <- fma(dot * xs, ws, f) in both halves
-__device__ __forceinline__ unsigned long long hf_step2(unsigned long long dot, unsigned long long xs, unsigned long long ws, unsigned long long f) {
-    unsigned long long p, r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(p) : "l"(dot), "l"(xs));
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(p), "l"(ws), "l"(f));
-    return r;
-}
-// A row's cell -> 64 halves in column order.  Bit-planes: 2 code - (2^B - 1), codebooks: the centroid.
-struct HfTables { uint32_t cb[8], tab[4]; __half2 add; };
-template <int FMT, typename T> __device__ __forceinline__ HfTables hf_tables(const T &a) {          // T: GemvArgs or ExpertCodebook
-
-    HfTables t;
-    // codebook bytes are stored + 128 (sign bit flipped) so that they are unsigned
-#pragma unroll
-    for (int i = 0; i < 8; ++i) t.cb[i] = a.cb[i] ^ 0x80808080u;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) t.tab[i] = a.tab[i];
-    int c = FMT == FMT_NF4 ? -1152 + a.nf4_offset : -1152;
-    if constexpr (is_bitplane<FMT>()) c = -1024 - a.max_odd;
-    t.add = __half2half2(__int2half_rn(c));
-    return t;
-}
-template <int FMT> __device__ __forceinline__ void hf_expand(const Raw<FMT> &w, const HfTables &t, uint32_t (&h)[32]) {
-    if (FMT == FMT_BP4) {            // twice the code, straight from the nibbles
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            hf_widen((w.w[i] << 1) & 0x1E1E1E1Eu, t.add, h[4 * i], h[4 * i + 1]);
-            hf_widen((w.w[i] >> 3) & 0x1E1E1E1Eu, t.add, h[4 * i + 2], h[4 * i + 3]);
-        }
-        return;
-    }
-    if (FMT == FMT_NF4) {            // upper and lower half of the sorted codebook in two tables of non-negative bytes (see cell_dot)
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const uint32_t x = w.w[i], y = x ^ 0x88888888u;
-            hf_widen(0x80808080u + prmt(t.tab[0], t.tab[1], y) - prmt(t.tab[2], t.tab[3], x), t.add, h[4 * i], h[4 * i + 1]);
-            hf_widen(0x80808080u + prmt(t.tab[0], t.tab[1], y >> 16) - prmt(t.tab[2], t.tab[3], x >> 16), t.add, h[4 * i + 2], h[4 * i + 3]);
-        }
-        return;
-    }
-    uint32_t u[16];
-    decode<FMT>(w, t.cb, u);
-#pragma unroll
-    for (int j = 0; j < 16; ++j) hf_widen(is_bitplane<FMT>() ? u[j] << 1 : FMT == FMT_E8Q2 ? u[j] ^ 0x80808080u : u[j], t.add, h[2 * j], h[2 * j + 1]);
-}
 
 template <int FMT, int N, bool EXP>
 __global__ void __launch_bounds__(HfRoles<N, EXP>::THREADS, EXP ? 2 : 1) gemm_f16_kernel(const typename HfParam<EXP>::T args) {
@@ -675,6 +579,11 @@ cudaError_t launch_gemm_f16(cudaStream_t stream, const DeviceMatrix &m, const in
     args.img = h.img; args.xs_img = h.scales; args.zero = image_ready ? h.zero : nullptr; args.n_tok = n_tok; args.tok_pad = tok_pad;
     cudaError_t e = image_ready ? cudaSuccess : launch_kernel(act_half_kernel, dim3((m.geom.nc + 3) / 4, tok_pad / 32), dim3(256), 0, stream, pdl, xq, xs, n_tok, m.geom.nc, tok_pad, h.img, h.scales);
     if (e != cudaSuccess) return e;
+    if (gemm_prompt_takes(m.geom.nc)) {
+        e = launch_gemm_prompt(stream, args.g, fmt, h, image_ready, n_tok, sm_count, pdl);
+        if (e == cudaSuccess && launches) *launches = image_ready ? 1 : 2;
+        return e;
+    }
     switch (fmt) {
         case FMT_BP4: e = launch_hf_fmt<FMT_BP4>(stream, args, sm_count, pdl); break;
         case FMT_BP5: e = launch_hf_fmt<FMT_BP5>(stream, args, sm_count, pdl); break;

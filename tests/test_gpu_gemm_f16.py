@@ -76,10 +76,8 @@ class Image(C.Structure):
     _fields_ = [("img", C.c_void_p), ("scales", C.c_void_p), ("zero", C.c_void_p)]
 
 
-@pytest.mark.parametrize("fmt", FORMATS)
-@pytest.mark.parametrize("rows,cols,n_tok", [(54, 64, 16), (71, 1536, 17), (300, 2112, 33), (129, 576, 128), (260, 4160, 100), (18944, 128, 64), (18944, 192, 131)])
-def test_product_of_converted_activations(ctx, oracle, fmt, rows, cols, n_tok):
-    """The same sizes by the launch itself: kronos_cuda_linear leaves batches that the integer GEMM multiplies faster to it."""
+def _converted(ctx, oracle, fmt, rows, cols, n_tok, sm_count):
+    """The launch itself on a batch with chunks of zeros, and the oracle's product."""
     import torch
 
     from k2t_internal import internal
@@ -100,9 +98,27 @@ def test_product_of_converted_activations(ctx, oracle, fmt, rows, cols, n_tok):
     image = Image((img.data_ptr() + 1023) // 1024 * 1024, rec.data_ptr(), None)
     dm = upload(ctx, m)          # its handle: a KronosCudaMatrix, the DeviceMatrix first
     try:
-        e = launch(torch.cuda.current_stream().cuda_stream, dm.handle, q.data_ptr(), s.data_ptr(), n_tok, C.byref(image), out.data_ptr(), rows, 148, err.data_ptr(), None, False, False)
+        e = launch(torch.cuda.current_stream().cuda_stream, dm.handle, q.data_ptr(), s.data_ptr(), n_tok, C.byref(image), out.data_ptr(), rows, sm_count, err.data_ptr(), None, False, False)
         torch.cuda.synchronize()
     finally:
         dm.free()
     assert e == 0 and err.item() == 0
-    assert np.array_equal(out.cpu().numpy(), want)
+    return out.cpu().numpy(), want
+
+
+@pytest.mark.parametrize("fmt", FORMATS)
+@pytest.mark.parametrize("rows,cols,n_tok", [(54, 64, 16), (71, 1536, 17), (300, 2112, 33), (129, 576, 128), (260, 4160, 100), (18944, 128, 64), (18944, 192, 131)])
+def test_product_of_converted_activations(ctx, oracle, fmt, rows, cols, n_tok):
+    """The same sizes by the launch itself: kronos_cuda_linear leaves batches that the integer GEMM multiplies faster to it."""
+    got, want = _converted(ctx, oracle, fmt, rows, cols, n_tok, 148)
+    assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("fmt", FORMATS)
+@pytest.mark.parametrize("rows,cols,n_tok,sm_count", [
+    (54, 2048, 16, 148), (300, 2048, 20, 3), (129, 2560, 33, 1), (257, 4096, 64, 3), (300, 4608, 77, 3), (131, 2048, 128, 2), (300, 2048, 130, 3), (384, 2560, 500, 2), (1025, 2048, 97, 4)])
+def test_products_of_long_rows(ctx, oracle, fmt, rows, cols, n_tok, sm_count):
+    """Rows of 32 chunks and more, for as many CTAs as sm_count says: every width of a tile (32 to 192 tokens), the last one partly filled, several
+    tiles per CTA, ragged rows, last passes of 8 chunks and more."""
+    got, want = _converted(ctx, oracle, fmt, rows, cols, n_tok, sm_count)
+    assert np.array_equal(got, want)
