@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "k2t_context.h"
+#include "k2t_device.cuh"
 #include "k2t_dense.h"
 #include "k2t_gemm_f16.h"
 #include "k2t_model_kernels.h"
@@ -29,6 +30,41 @@ bool check_gemv_args(KronosCudaContext *ctx, const KronosCudaMatrix *m, const vo
     if (n_tok == 0) return fail(ctx, "gemv: n_tok is 0");
     if (out_stride < m->dm.geom.rows) return fail(ctx, "gemv: out_stride smaller than rows");
     return true;
+}
+
+// A result of up to COPY_OUT_BYTES to page-locked host memory.  The chain of a call's queue entries in one stream bounds a host that queues
+// projections: beside a copy engine's entry of some 7 us this one takes 4 (16 projections of one token, their four results of 196 KB by copy
+// engine all the same: 449 -> 270 us with the direct reads below; 2048 x 49152, one token, 41 us by kernel, 38 by copy engine).
+constexpr size_t COPY_OUT_BYTES = 64 * 1024;
+__global__ void __launch_bounds__(256) copy_out_kernel(const float *__restrict__ src, float *__restrict__ dst, uint32_t n) {
+    const uint32_t i = (blockIdx.x * 256 + threadIdx.x) * 4;
+    pdl_wait();
+    pdl_trigger();
+    if (i + 4 <= n) *reinterpret_cast<float4 *>(dst + i) = __ldcg(reinterpret_cast<const float4 *>(src + i));
+    else for (uint32_t k = i; k < n; ++k) dst[k] = __ldcg(src + k);
+}
+
+// The address at which the GPU reaches [p, p + bytes) itself, or null where that is not all of one page-locked, mapped host allocation (asked of
+// the driver on every call).  A kernel that reads an input of up to READ_IN_BYTES where it lies saves the copy's entry in the queue (the sixteen
+// projections above 449 -> 355 us, 4 x 8192 values 55 -> 51); of 200 x 8192 values both ways took 240 to 390 us from run to run: copied.
+constexpr size_t READ_IN_BYTES = 512 * 1024;
+void *host_on_device(const void *p, size_t bytes, size_t alignment) {
+    using GetAttributes = int (*)(unsigned, int *, void **, unsigned long long);
+    static const GetAttributes get = [] {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        const bool ok = cudaGetDriverEntryPoint("cuPointerGetAttributes", &fn, cudaEnableDefault, &found) == cudaSuccess && found == cudaDriverEntryPointSuccess;
+        return ok ? reinterpret_cast<GetAttributes>(fn) : nullptr;
+    }();
+    const unsigned long long at = reinterpret_cast<unsigned long long>(p);
+    if (get == nullptr || at % alignment != 0) return nullptr;
+    unsigned type = 0, managed = 0;
+    unsigned long long device = 0, start = 0;
+    size_t size = 0;
+    int which[5] = {2, 3, 8, 11, 12};          // memory type (1: host), device pointer, managed, the allocation's start and size
+    void *out[5] = {&type, &device, &managed, &start, &size};
+    if (get(5, which, out, at) != 0 || type != 1 || managed != 0 || device == 0 || start == 0 || at < start || bytes > size || at - start > size - bytes) return nullptr;
+    return reinterpret_cast<void *>(device);
 }
 
 // Runs the GEMV over n_tok tokens (tensor-core kernel for batches, 4-token weight passes otherwise).
@@ -308,11 +344,14 @@ static int32_t linear_impl(KronosCudaContext *ctx, const KronosCudaMatrix *m, co
         ctx->launches += 1 + launched;
         return !wait || sync_and_check(ctx, "linear") ? 0 : -1;
     }
-    if (!reserve(ctx, ctx->x, n * 4) || !reserve(ctx, ctx->q, n) || !reserve(ctx, ctx->xs, nch * 4) ||
-        !reserve(ctx, ctx->xsum, nch * 4) || !reserve(ctx, ctx->out, n_out * 4))
-        return -1;
-    if (!cuda_ok(ctx, cudaMemcpyAsync(ctx->x.p, x, n * 4, cudaMemcpyHostToDevice, s), "copy x")) return -1;
-    if (kronos_cuda_fwht_quant_dev(ctx, (const float *)ctx->x.p, n_tok, g.cols, nullptr, nullptr, 0, (int8_t *)ctx->q.p,
+    if (!reserve(ctx, ctx->q, n) || !reserve(ctx, ctx->xs, nch * 4) || !reserve(ctx, ctx->xsum, nch * 4) || !reserve(ctx, ctx->out, n_out * 4)) return -1;
+    const float *d_x = n * 4 <= READ_IN_BYTES ? (const float *)host_on_device(x, n * 4, 8) : nullptr;
+    float *d_out = n_out * 4 <= COPY_OUT_BYTES ? (float *)host_on_device(out, n_out * 4, 16) : nullptr;
+    if (d_x == nullptr) {
+        if (!reserve(ctx, ctx->x, n * 4) || !cuda_ok(ctx, cudaMemcpyAsync(ctx->x.p, x, n * 4, cudaMemcpyHostToDevice, s), "copy x")) return -1;
+        d_x = (const float *)ctx->x.p;
+    }
+    if (kronos_cuda_fwht_quant_dev(ctx, d_x, n_tok, g.cols, nullptr, nullptr, 0, (int8_t *)ctx->q.p,
                                    (float *)ctx->xs.p, (int32_t *)ctx->xsum.p) != 0)
         return -1;
     uint32_t launched = 0;
@@ -334,7 +373,12 @@ static int32_t linear_impl(KronosCudaContext *ctx, const KronosCudaMatrix *m, co
     } else if (!run_gemv(ctx, m, (const int8_t *)ctx->q.p, (const float *)ctx->xs.p, (const int32_t *)ctx->xsum.p, n_tok, (float *)ctx->out.p, g.rows, nullptr)) {
         return -1;
     }
-    if (!cuda_ok(ctx, cudaMemcpyAsync(out, ctx->out.p, n_out * 4, cudaMemcpyDeviceToHost, s), "copy out")) return -1;
+    if (d_out != nullptr) {
+        ctx->launches += 1;
+        if (!cuda_ok(ctx, launch_kernel(copy_out_kernel, dim3((unsigned)((n_out + 1023) / 1024)), dim3(256), 0, s, true, (const float *)ctx->out.p, d_out, (uint32_t)n_out), "copy out")) return -1;
+    } else if (!cuda_ok(ctx, cudaMemcpyAsync(out, ctx->out.p, n_out * 4, cudaMemcpyDeviceToHost, s), "copy out")) {
+        return -1;
+    }
     if (!wait) return 0;
     return sync_and_check(ctx, "linear") ? 0 : -1;
 }
