@@ -417,7 +417,7 @@ bool enqueue_batch(KronosCudaEngine *e, uint32_t T, bool embed, Tail tail, bool 
             ra.w = L.router_w; ra.bias = L.router_bias; ra.x = e->x_norm;
             ra.n_experts = c.moe_num_experts; ra.hidden = h; ra.top_k = k; ra.norm_topk = (int32_t)(c.moe_norm_topk & 1u); ra.scoring = c.moe_norm_topk >> 8;
             ra.route_ids = L.d_route_ids; ra.route_w = L.d_route_w; ra.logits = e->router_logits; ra.done = e->router_done; ra.route_stride = 32; ra.err_flag = e->ctx->d_err;
-            if (!count(e, launch_moe_router(s, ra, e->pdl, T), "router")) return false;
+            if (!count(e, launch_moe_router(s, ra, e->pdl, T), "router", router_in_two(ra, T) ? 2 : 1)) return false;
             const uint32_t E = c.moe_num_experts;
             const bool grouped = experts_grouped(T, T * k, E, h, dff, c.moe_bits);
             if (grouped && !count(e, launch_expert_tiles(s, L.d_route_ids, T, k, 32, E, L.d_gu_bases, e->tiles, e->ctx->d_err, e->pdl), "expert tiles")) return false;

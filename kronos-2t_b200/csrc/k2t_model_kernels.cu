@@ -182,6 +182,79 @@ __device__ __forceinline__ float exp_cr(float x) { return (float)exp((double)x);
 // equals - what select_topk_by_score's strict '>' insertion produces), optional renormalisation in that order, sort by id.
 constexpr uint32_t ROUTER_THREADS = 128, ROUTER_MAX_EXPERTS = 256, ROUTER_MAX_TOPK = 32;
 constexpr uint32_t ROUTER_EXPERTS_PER_CTA = ROUTER_THREADS / 16;
+// One token's routes from its logits, by a CTA of ROUTER_THREADS.
+__device__ __forceinline__ void router_select(const RouterArgs &a) {
+    __shared__ float s_z[ROUTER_MAX_EXPERTS];
+    __shared__ float s_sel_w[ROUTER_MAX_TOPK];
+    __shared__ uint32_t s_sel_e[ROUTER_MAX_TOPK];
+    __shared__ float s_max;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (uint32_t e = tid; e < a.n_experts; e += ROUTER_THREADS) s_z[e] = __ldcg(a.logits + e);
+    __syncthreads();
+    if (warp == 0) {
+        float m = -INFINITY;
+        for (uint32_t e = lane; e < a.n_experts; e += 32) m = fmaxf(m, s_z[e]);
+        m = warp_max(m);
+        if (lane == 0) s_max = m;
+    }
+    __syncthreads();
+    // scores: softmax numerators (normalised below), sigmoid values, or the raw logits (top-k softmax)
+    for (uint32_t e = tid; e < a.n_experts; e += ROUTER_THREADS) {
+        if (a.scoring == 0) s_z[e] = exp_cr(__fsub_rn(s_z[e], s_max));
+        else if (a.scoring == 2) s_z[e] = __fdiv_rn(1.0f, __fadd_rn(1.0f, exp_cr(-s_z[e])));
+    }
+    __syncthreads();
+    if (a.scoring == 0) {
+        if (tid == 0) {
+            float sum = 0.0f;
+            for (uint32_t e = 0; e < a.n_experts; ++e) sum = __fadd_rn(sum, s_z[e]);
+            s_max = sum > 0.0f ? __fdiv_rn(1.0f, sum) : __fdiv_rn(1.0f, (float)a.n_experts);
+        }
+        __syncthreads();
+        const float inv_all = s_max;
+        for (uint32_t e = tid; e < a.n_experts; e += ROUTER_THREADS) s_z[e] = __fmul_rn(s_z[e], inv_all);
+        __syncthreads();
+    }
+    const uint32_t k = min(min(a.top_k, a.n_experts), ROUTER_MAX_TOPK);
+    // Non-finite scores (a NaN ranks before nothing and after nothing) can leave ranks unassigned: every slot starts as
+    // a valid route (expert i, weight 0), so the expert kernels never see an id outside [0, n_experts).
+    if (tid < k) { s_sel_e[tid] = tid; s_sel_w[tid] = 0.0f; }
+    __syncthreads();
+    for (uint32_t e = tid; e < a.n_experts; e += ROUTER_THREADS) {       // rank of expert e in the descending order
+        const float sc = s_z[e];
+        uint32_t rank = 0;
+        for (uint32_t j = 0; j < a.n_experts; ++j) {
+            const float sj = s_z[j];
+            rank += (sj > sc || (sj == sc && j < e)) ? 1u : 0u;
+        }
+        if (rank < k) { s_sel_e[rank] = e; s_sel_w[rank] = sc; }
+    }
+    __syncthreads();
+    if (tid == 0) {
+        // in place in shared memory (k is small; private arrays indexed by loop variables would live in local memory)
+        uint32_t *ids = s_sel_e;
+        float *w = s_sel_w;
+        if (a.scoring == 1) {                 // k-way softmax over the selected logits, in selection order
+            float max_z = -INFINITY, sum = 0.0f;
+            for (uint32_t i = 0; i < k; ++i) max_z = fmaxf(max_z, w[i]);
+            for (uint32_t i = 0; i < k; ++i) { w[i] = exp_cr(__fsub_rn(w[i], max_z)); sum = __fadd_rn(sum, w[i]); }
+            const float inv = sum > 0.0f ? __fdiv_rn(1.0f, sum) : __fdiv_rn(1.0f, (float)k);
+            for (uint32_t i = 0; i < k; ++i) w[i] = __fmul_rn(w[i], inv);
+        } else if (a.norm_topk) {
+            float top_sum = 0.0f;
+            for (uint32_t i = 0; i < k; ++i) top_sum = __fadd_rn(top_sum, w[i]);
+            if (top_sum > 0.0f) { const float inv_top = __fdiv_rn(1.0f, top_sum); for (uint32_t i = 0; i < k; ++i) w[i] = __fmul_rn(w[i], inv_top); }
+        }
+        for (uint32_t i = 1; i < k; ++i) {
+            const uint32_t ce = ids[i]; const float cw = w[i];
+            uint32_t j = i;
+            while (j > 0 && ids[j - 1] > ce) { ids[j] = ids[j - 1]; w[j] = w[j - 1]; --j; }
+            ids[j] = ce; w[j] = cw;
+        }
+        for (uint32_t i = 0; i < k; ++i) { a.route_ids[i] = min(ids[i], a.n_experts - 1u); a.route_w[i] = w[i]; }
+    }
+}
+
 __global__ void __launch_bounds__(ROUTER_THREADS) moe_router_kernel(RouterArgs a) {
     extern __shared__ __align__(128) float s_dyn[];      // x [hidden], then (staged form) the CTA's eight router rows [8][hidden + 16]
     float *s_xr = s_dyn;
@@ -189,10 +262,6 @@ __global__ void __launch_bounds__(ROUTER_THREADS) moe_router_kernel(RouterArgs a
         const size_t t = blockIdx.y;
         a.x += t * a.hidden; a.logits += t * a.n_experts; a.done += t; a.route_ids += t * a.route_stride; a.route_w += t * a.route_stride;
     }
-    __shared__ float s_z[ROUTER_MAX_EXPERTS];
-    __shared__ float s_sel_w[ROUTER_MAX_TOPK];
-    __shared__ uint32_t s_sel_e[ROUTER_MAX_TOPK];
-    __shared__ float s_max;
     __shared__ uint32_t s_last;
     __shared__ __align__(8) uint64_t s_bar;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, half = lane >> 4, l16 = lane & 15;
@@ -263,70 +332,102 @@ __global__ void __launch_bounds__(ROUTER_THREADS) moe_router_kernel(RouterArgs a
     if (s_last == 0) return;
     __threadfence();
     if (tid == 0) *a.done = 0;               // ready for the next launch (launches of a stream do not overlap here)
-    for (uint32_t e = tid; e < a.n_experts; e += ROUTER_THREADS) s_z[e] = __ldcg(a.logits + e);
-    __syncthreads();
-    if (warp == 0) {
-        float m = -INFINITY;
-        for (uint32_t e = lane; e < a.n_experts; e += 32) m = fmaxf(m, s_z[e]);
-        m = warp_max(m);
-        if (lane == 0) s_max = m;
-    }
-    __syncthreads();
-    // scores: softmax numerators (normalised below), sigmoid values, or the raw logits (top-k softmax)
-    for (uint32_t e = tid; e < a.n_experts; e += ROUTER_THREADS) {
-        if (a.scoring == 0) s_z[e] = exp_cr(__fsub_rn(s_z[e], s_max));
-        else if (a.scoring == 2) s_z[e] = __fdiv_rn(1.0f, __fadd_rn(1.0f, exp_cr(-s_z[e])));
-    }
-    __syncthreads();
-    if (a.scoring == 0) {
-        if (tid == 0) {
-            float sum = 0.0f;
-            for (uint32_t e = 0; e < a.n_experts; ++e) sum = __fadd_rn(sum, s_z[e]);
-            s_max = sum > 0.0f ? __fdiv_rn(1.0f, sum) : __fdiv_rn(1.0f, (float)a.n_experts);
-        }
-        __syncthreads();
-        const float inv_all = s_max;
-        for (uint32_t e = tid; e < a.n_experts; e += ROUTER_THREADS) s_z[e] = __fmul_rn(s_z[e], inv_all);
-        __syncthreads();
-    }
-    const uint32_t k = min(min(a.top_k, a.n_experts), ROUTER_MAX_TOPK);
-    // Non-finite scores (a NaN ranks before nothing and after nothing) can leave ranks unassigned: every slot starts as
-    // a valid route (expert i, weight 0), so the expert kernels never see an id outside [0, n_experts).
-    if (tid < k) { s_sel_e[tid] = tid; s_sel_w[tid] = 0.0f; }
-    __syncthreads();
-    for (uint32_t e = tid; e < a.n_experts; e += ROUTER_THREADS) {       // rank of expert e in the descending order
-        const float sc = s_z[e];
-        uint32_t rank = 0;
-        for (uint32_t j = 0; j < a.n_experts; ++j) {
-            const float sj = s_z[j];
-            rank += (sj > sc || (sj == sc && j < e)) ? 1u : 0u;
-        }
-        if (rank < k) { s_sel_e[rank] = e; s_sel_w[rank] = sc; }
-    }
-    __syncthreads();
+    router_select(a);
+}
+
+// Prompt batches: the logits of 16 tokens x 16 experts per CTA, then the selection, a CTA per token.  Same sums: a lane owns four of the sixteen
+// accumulators of eight (token, expert) pairs, so six 16-byte loads feed 32 multiply-adds, where a CTA per token and eight experts read
+// the router matrix again for every token (300 tokens, 128 experts of 2048: 51 us in the one launch, 25 + 9 in two).
+constexpr uint32_t RL_TOKENS = 16, RL_EXPERTS = 16, RL_SLICE = 256, RL_PITCH = RL_SLICE + 8, RL_STAGES = 3;          // floats of a row per stage; rows two apart 16 banks apart
+constexpr uint32_t RL_SMEM = RL_STAGES * (RL_TOKENS + RL_EXPERTS) * RL_PITCH * 4;
+__global__ void __launch_bounds__(ROUTER_THREADS) router_logits_kernel(const RouterArgs a, uint32_t n_tok) {
+    extern __shared__ __align__(128) float s_dyn[];          // [stage][16 tokens, 16 experts][RL_PITCH]
+    __shared__ __align__(8) uint64_t s_bars[RL_STAGES];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, q = lane & 3u, tile = lane >> 2;
+    const uint32_t tok0 = blockIdx.y * RL_TOKENS, exp0 = blockIdx.x * RL_EXPERTS, slices = (a.hidden + RL_SLICE - 1) / RL_SLICE;
+    const uint32_t bar = (uint32_t)__cvta_generic_to_shared(s_bars), rows = (uint32_t)__cvta_generic_to_shared(s_dyn);
     if (tid == 0) {
-        // in place in shared memory (k is small; private arrays indexed by loop variables would live in local memory)
-        uint32_t *ids = s_sel_e;
-        float *w = s_sel_w;
-        if (a.scoring == 1) {                 // k-way softmax over the selected logits, in selection order
-            float max_z = -INFINITY, sum = 0.0f;
-            for (uint32_t i = 0; i < k; ++i) max_z = fmaxf(max_z, w[i]);
-            for (uint32_t i = 0; i < k; ++i) { w[i] = exp_cr(__fsub_rn(w[i], max_z)); sum = __fadd_rn(sum, w[i]); }
-            const float inv = sum > 0.0f ? __fdiv_rn(1.0f, sum) : __fdiv_rn(1.0f, (float)k);
-            for (uint32_t i = 0; i < k; ++i) w[i] = __fmul_rn(w[i], inv);
-        } else if (a.norm_topk) {
-            float top_sum = 0.0f;
-            for (uint32_t i = 0; i < k; ++i) top_sum = __fadd_rn(top_sum, w[i]);
-            if (top_sum > 0.0f) { const float inv_top = __fdiv_rn(1.0f, top_sum); for (uint32_t i = 0; i < k; ++i) w[i] = __fmul_rn(w[i], inv_top); }
-        }
-        for (uint32_t i = 1; i < k; ++i) {
-            const uint32_t ce = ids[i]; const float cw = w[i];
-            uint32_t j = i;
-            while (j > 0 && ids[j - 1] > ce) { ids[j] = ids[j - 1]; w[j] = w[j - 1]; --j; }
-            ids[j] = ce; w[j] = cw;
-        }
-        for (uint32_t i = 0; i < k; ++i) { a.route_ids[i] = min(ids[i], a.n_experts - 1u); a.route_w[i] = w[i]; }
+        for (uint32_t i = 0; i < RL_STAGES; ++i) mbar_init(bar + 8 * i, 1);
+        fence_mbar_init();
+        fence_proxy_async();
     }
+    pdl_wait();
+    pdl_trigger();
+    __syncthreads();
+    auto request = [&](uint32_t c) {          // by one warp, a row per lane; rows behind the last one repeat it
+        const uint32_t b = bar + 8 * (c % RL_STAGES), n = min(RL_SLICE, a.hidden - c * RL_SLICE) * 4;
+        if (lane == 0) mbar_expect_tx(b, (RL_TOKENS + RL_EXPERTS) * n);
+        __syncwarp();
+        const float *src = lane < RL_TOKENS ? a.x + (size_t)min(tok0 + lane, n_tok - 1) * a.hidden : a.w + (size_t)min(exp0 + lane - RL_TOKENS, a.n_experts - 1) * a.hidden;
+        bulk_g2s(rows + ((c % RL_STAGES) * 32 + lane) * RL_PITCH * 4, src + c * RL_SLICE, n, b);
+    };
+    static_assert(RL_TOKENS + RL_EXPERTS == 32, "a row per lane");
+    if (warp == 0)
+        for (uint32_t c = 0; c < min(RL_STAGES, slices); ++c) request(c);
+    const uint32_t t0 = tok0 + warp * 4 + (tile & 1u) * 2, e0 = exp0 + (tile >> 1) * 4;
+    float4 acc[2][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    bool ok = true;
+    for (uint32_t c = 0; c < slices; ++c) {
+        bool here = mbar_try_wait(bar + 8 * (c % RL_STAGES), (c / RL_STAGES) & 1u);
+        for (uint32_t spin = 0; ok && !here && spin < (1u << 22); ++spin) here = mbar_try_wait(bar + 8 * (c % RL_STAGES), (c / RL_STAGES) & 1u);
+        ok = ok && here;
+        const float *x = s_dyn + ((c % RL_STAGES) * 32 + warp * 4 + (tile & 1u) * 2) * RL_PITCH + 4 * q, *w = s_dyn + ((c % RL_STAGES) * 32 + RL_TOKENS + (tile >> 1) * 4) * RL_PITCH + 4 * q;
+        const uint32_t n = min(RL_SLICE, a.hidden - c * RL_SLICE);
+        float4 xv[2][2], wv[2][4];
+        auto load = [&](uint32_t s, uint32_t k) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) xv[k][i] = *reinterpret_cast<const float4 *>(x + i * RL_PITCH + s);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) wv[k][j] = *reinterpret_cast<const float4 *>(w + j * RL_PITCH + s);
+        };
+        auto step = [&](uint32_t k) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    float4 &v = acc[i][j];
+                    v.x = __fmaf_rn(wv[k][j].x, xv[k][i].x, v.x); v.y = __fmaf_rn(wv[k][j].y, xv[k][i].y, v.y);
+                    v.z = __fmaf_rn(wv[k][j].z, xv[k][i].z, v.z); v.w = __fmaf_rn(wv[k][j].w, xv[k][i].w, v.w);
+                }
+        };
+        load(0, 0);
+#pragma unroll 2
+        for (uint32_t s = 0; s < n; s += 32) {          // the next sixteen are on their way while sixteen are added
+            if (s + 16 < n) load(s + 16, 1);
+            step(0);
+            if (s + 16 < n) {
+                if (s + 32 < n) load(s + 32, 0);
+                step(1);
+            }
+        }
+        __syncthreads();
+        if (warp == 0 && c + RL_STAGES < slices) request(c + RL_STAGES);
+    }
+    if (!ok && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);          // every copy that was asked for has been waited for
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {          // accumulators r and r + 4, those of r + 8 and r + 12, then 0 + 1 and 2 + 3
+            float v[4] = {acc[i][j].x, acc[i][j].y, acc[i][j].z, acc[i][j].w};
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                v[r] = __fadd_rn(v[r], __shfl_down_sync(0xffffffffu, v[r], 1));
+                v[r] = __fadd_rn(v[r], __shfl_down_sync(0xffffffffu, v[r], 2));
+            }
+            const float z = __fadd_rn(__fadd_rn(v[0], v[1]), __fadd_rn(v[2], v[3]));
+            if (q == 0 && t0 + i < n_tok && e0 + j < a.n_experts) a.logits[(size_t)(t0 + i) * a.n_experts + e0 + j] = a.bias != nullptr ? __fadd_rn(z, __ldg(a.bias + e0 + j)) : z;
+        }
+}
+__global__ void __launch_bounds__(ROUTER_THREADS) router_select_kernel(RouterArgs a) {
+    const size_t t = blockIdx.x;
+    a.logits += t * a.n_experts; a.route_ids += t * a.route_stride; a.route_w += t * a.route_stride;
+    pdl_wait();
+    pdl_trigger();
+    router_select(a);
 }
 
 // SwiGLU of the routed experts' gate_up outputs [slot][2 * d_ff] (gate = rows [0, d_ff), up = the rest), chunk by chunk
@@ -975,6 +1076,9 @@ cudaError_t launch_rmsnorm_quant(cudaStream_t s, float *hidden, const float *del
                                  int8_t *q, float *scales, int32_t *sums, uint32_t n_tok, bool pdl) {
     return launch_rmsnorm_quant_x(s, hidden, delta, w, n, eps, q, scales, sums, nullptr, n_tok, pdl);
 }
+bool router_in_two(const RouterArgs &a, uint32_t n_tok) {
+    return n_tok >= 16 && a.hidden % 16 == 0 && (n_tok + RL_TOKENS - 1) / RL_TOKENS <= 0xFFFF && ((reinterpret_cast<uintptr_t>(a.w) | reinterpret_cast<uintptr_t>(a.x)) & 15u) == 0;
+}
 cudaError_t launch_moe_router(cudaStream_t s, const RouterArgs &a_in, bool pdl, uint32_t n_tok) {
     RouterArgs a = a_in;
     if (a.n_experts > ROUTER_MAX_EXPERTS || a.top_k > ROUTER_MAX_TOPK || a.hidden * 4 > 160 * 1024) return cudaErrorInvalidValue;
@@ -987,6 +1091,11 @@ cudaError_t launch_moe_router(cudaStream_t s, const RouterArgs &a_in, bool pdl, 
         if (e != cudaSuccess) return e;
     }
     if (a.logits == nullptr || a.done == nullptr) return cudaErrorInvalidValue;
+    if (router_in_two(a, n_tok)) {
+        cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(router_logits_kernel), RL_SMEM);
+        if (e == cudaSuccess) e = launch_kernel(router_logits_kernel, dim3((a.n_experts + RL_EXPERTS - 1) / RL_EXPERTS, (n_tok + RL_TOKENS - 1) / RL_TOKENS), dim3(ROUTER_THREADS), RL_SMEM, s, pdl, a, n_tok);
+        return e != cudaSuccess ? e : launch_kernel(router_select_kernel, dim3(n_tok), dim3(ROUTER_THREADS), 0, s, pdl, a);
+    }
     return launch_kernel(moe_router_kernel, dim3((a.n_experts + ROUTER_EXPERTS_PER_CTA - 1) / ROUTER_EXPERTS_PER_CTA, n_tok), dim3(ROUTER_THREADS), smem, s, pdl, a);
 }
 cudaError_t launch_expert_swiglu_quant(cudaStream_t s, const float *gate_up, uint32_t d_ff, uint32_t n_slot, int8_t *q, float *scales,

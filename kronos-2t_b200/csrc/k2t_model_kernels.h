@@ -187,6 +187,7 @@ cudaError_t launch_rmsnorm_quant_x(cudaStream_t s, float *hidden, const float *d
 cudaError_t launch_rmsnorm_quant_tp(cudaStream_t s, float *hidden, const float *delta, const float *w, uint32_t n, float eps,
                                     int8_t *q, float *scales, int32_t *sums, float *x_norm, uint32_t n_tok, bool pdl,
                                     const TpLink &tp, uint32_t *tp_done);
+bool router_in_two(const RouterArgs &a, uint32_t n_tok);          // batches whose router takes two launches
 cudaError_t launch_moe_router(cudaStream_t s, const RouterArgs &a, bool pdl, uint32_t n_tok = 1);
 // SwiGLU of n_slot expert outputs [n_slot][2 * d_ff] with the scalar-path exp (moe_800b.rs:1498-1517), then rotation + int8
 cudaError_t launch_expert_swiglu_quant(cudaStream_t s, const float *gate_up, uint32_t d_ff, uint32_t n_slot, int8_t *q, float *scales,

@@ -1,0 +1,23 @@
+"""The router of prompt batches (two launches from sixteen tokens on): experts and tokens on both sides of its tiles, against the oracle's token-by-token
+run, logits and routes bit for bit."""
+import numpy as np
+import pytest
+
+import k2t_models as km
+from test_gpu_model import ctx, make  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n_experts,n_tok", [(3, 15), (3, 16), (16, 17), (17, 33), (40, 31)])
+def test_routes_of_a_batch(ctx, oracle, n_experts, n_tok):  # noqa: F811
+    spec, eng, ref = make(ctx, oracle, km.MOE_TINY, "nf4g128", seed=5, moe=dict(layers=[0, 2], n_experts=n_experts, top_k=3, d_ff=64, bits=3, sgc=2, bias=n_experts == 17))
+    try:
+        tokens = np.random.Generator(np.random.PCG64(n_tok)).integers(0, km.MOE_TINY["vocab"], n_tok).tolist()
+        want = np.stack([ref.forward_token(t, threads=2) for t in tokens])
+        assert np.array_equal(eng.forward_token_ids(tokens, want_all=True), want)
+        for layer in (0, 2):
+            assert all(np.array_equal(g, w) for g, w in zip(eng.read_routes(layer), ref.last_routes(layer)))
+    finally:
+        eng.close()
+        ref.close()
