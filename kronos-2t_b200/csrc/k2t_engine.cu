@@ -421,11 +421,11 @@ bool enqueue_batch(KronosCudaEngine *e, uint32_t T, bool embed, Tail tail, bool 
             const uint32_t E = c.moe_num_experts;
             const bool grouped = experts_grouped(T, T * k, E, h, dff, c.moe_bits);
             if (grouped && !count(e, launch_expert_tiles(s, L.d_route_ids, T, k, 32, E, L.d_gu_bases, e->tiles, e->ctx->d_err, e->pdl), "expert tiles")) return false;
-            if (!count(e, grouped ? launch_gemm_experts(s, L.gu_dm, L.gu_fmt, L.d_gu_books, L.d_gu_bases, E, e->tiles, T * k, k, e->act_q, e->act_s, e->moe_gu, e->ctx->d_err, e->pdl)
+            if (!count(e, grouped ? launch_gemm_experts(s, L.gu_dm, L.gu_fmt, L.d_gu_books, L.d_gu_bases, E, e->tiles, T * k, k, e->act_q, e->act_s, e->moe_gu, e->ctx->sm_count, e->ctx->d_err, e->pdl)
                                   : launch_gemv_experts(s, L.gu_dm, L.gu_fmt, L.d_gu_books, L.d_gu_bases, L.d_route_ids, T * k, e->act_q, e->act_s, e->act_m, h, h / 64,
                                                         e->moe_gu, (size_t)2 * dff, e->ctx->sm_count, e->ctx->d_err, e->pdl, E, k, 32, k), "expert gate_up")) return false;
             if (!expert_swiglu(e, e->moe_gu, dff, T * k, e->moe_q, e->moe_s, e->moe_m, wide_batch(T), "expert swiglu")) return false;
-            if (!count(e, grouped ? launch_gemm_experts(s, L.dn_dm, L.dn_fmt, L.d_dn_books, L.d_dn_bases, E, e->tiles, T * k, 1, e->moe_q, e->moe_s, e->moe_out, e->ctx->d_err, e->pdl)
+            if (!count(e, grouped ? launch_gemm_experts(s, L.dn_dm, L.dn_fmt, L.d_dn_books, L.d_dn_bases, E, e->tiles, T * k, 1, e->moe_q, e->moe_s, e->moe_out, e->ctx->sm_count, e->ctx->d_err, e->pdl)
                                   : launch_gemv_experts(s, L.dn_dm, L.dn_fmt, L.d_dn_books, L.d_dn_bases, L.d_route_ids, T * k, e->moe_q, e->moe_s, e->moe_m, dff, dff / 64,
                                                         e->moe_out, h, e->ctx->sm_count, e->ctx->d_err, e->pdl, E, k, 32, 1), "expert down")) return false;
             if (!count(e, launch_moe_combine(s, e->moe_out, L.d_route_w, k, h, e->proj, e->pdl, L.d_route_ids, c.ep_size > 1 ? L.d_dn_bases : nullptr,

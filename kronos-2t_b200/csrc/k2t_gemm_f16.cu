@@ -9,7 +9,7 @@
 // tokens per instruction: 1.3 instructions per (row, token, chunk) where the int32 accumulators of k2t_gemm_tc.cu take 4.75
 // (integer correction, conversion, multiply, fma).
 //
-// Rows of 32 chunks and more go to k2t_gemm_prompt.cu; here are the shorter ones, the conversion of the activations, and the experts.
+// Rows of 32 chunks and more go to k2t_gemm_prompt.cu; here are the shorter ones, the conversion of the activations, and the sorting of the experts' pairs.
 //
 // The activations come as an operand image (act_half_kernel below): per chunk 128 bytes per token in the 128-byte-swizzled
 // K-major layout, so a tile of tokens is one contiguous run, plus the tokens' scales.  One CTA = 128 rows x N tokens:
@@ -20,10 +20,6 @@
 //   * EPILOGUE warps (lane = row, N / 4 or N / 2 tokens each) read the dots and advance their chains.
 // The roles hand over two chunks at a time (a stage): half the barrier traffic of single chunks.
 //
-// The experts of a prompt (EXP) run in the same kernel: a tile is 128 rows of one expert and up to 32 of its (token, route) pairs, which
-// expert_tiles_kernel has gathered; a producer warp fetches the pairs' int8 rows where they lie and widens them on the way.  As one GEMV
-// per pair, 2048 pairs of 128 experts (1536 x 2048, 3 bits) took 686 us, bound by expanding the codes again for every pair; 2400 pairs
-// in tiles take 206 us, still bound by the expansion (203 tiles at most, 0.55 us per chunk and SM with two CTAs resident).
 // Every wait is bounded; a wait that gives up raises the context's error word, and all roles come to their end.
 // Measured (B200, 256 tokens, image included): 16384 x 2048 nf4g128 55 us against 98 us with int32 accumulators, 2048 x 8192 57 against
 // 75; a 1000-token prompt through 12 layers of the 1.7B shape 21.5 -> 18.4 ms, 77 tokens through 4 layers of the 7B shape 2.09 -> 1.59 ms.
@@ -46,25 +42,23 @@ constexpr uint32_t HF_WAIT_LIMIT = 1u << 21;
 constexpr uint32_t HF_HEADER = 1024;
 constexpr uint32_t HF_A_STAGE = HF_M * 128;
 
-// EXP: a tile of an expert's (token, route) pairs, few chunks deep.  Half the warps and 113 KB at most, so that two CTAs share an SM and
-// one's start and end run under the other's chunks.
-template <int N, bool EXP = false> struct HfRoles {
-    static constexpr uint32_t EPI_WARPS = EXP ? 4 : N >= 64 ? 16 : 8;
-    static constexpr uint32_t GROUPS = N >= 64 || EXP ? 2 : 4;
-    static constexpr uint32_t STAGES = N == 128 || EXP ? 2 : 3;       // a stage holds two chunks, each with an accumulator buffer of N tensor-memory columns
+template <int N> struct HfRoles {
+    static constexpr uint32_t EPI_WARPS = N >= 64 ? 16 : 8;
+    static constexpr uint32_t GROUPS = N >= 64 ? 2 : 4;
+    static constexpr uint32_t STAGES = N == 128 ? 2 : 3;       // a stage holds two chunks, each with an accumulator buffer of N tensor-memory columns
     static constexpr uint32_t NQ = N / (EPI_WARPS / 4);        // tokens per epilogue warp
     static constexpr uint32_t DEC_WARPS = 4 * GROUPS;
     static constexpr uint32_t THREADS = (EPI_WARPS + DEC_WARPS + 2) * 32;
     static constexpr uint32_t DEC_ARRIVALS = 8;                // decode warps that fill a stage: two groups, one per chunk
-    static constexpr uint32_t TMEM = EXP ? 128 : N == 32 ? 256 : 512;      // columns (a power of two)
+    static constexpr uint32_t TMEM = N == 32 ? 256 : 512;      // columns (a power of two)
 };
 
-template <int FMT, int N, bool EXP = false> struct HfLayout {
-    static constexpr uint32_t PF = !EXP ? 8 : hf_cell<FMT>() <= 24 ? 6 : 4;          // ring slots of raw weights: chunks requested ahead
-    static constexpr uint32_t PFG = PF / HfRoles<N, EXP>::GROUPS;                    // of them by one decode group
+template <int FMT, int N> struct HfLayout {
+    static constexpr uint32_t PF = 8;          // ring slots of raw weights: chunks requested ahead
+    static constexpr uint32_t PFG = PF / HfRoles<N>::GROUPS;                    // of them by one decode group
     static constexpr uint32_t A = HF_HEADER;
-    static constexpr uint32_t B = A + HfRoles<N, EXP>::STAGES * 2 * HF_A_STAGE;
-    static constexpr uint32_t XS = B + HfRoles<N, EXP>::STAGES * 2 * N * 128;
+    static constexpr uint32_t B = A + HfRoles<N>::STAGES * 2 * HF_A_STAGE;
+    static constexpr uint32_t XS = B + HfRoles<N>::STAGES * 2 * N * 128;
     static constexpr uint32_t WS = XS + HF_SLOTS * (N / 32) * HF_REC;
     static constexpr uint32_t RING = WS + HF_SLOTS * HF_M * 4;
     static constexpr uint32_t TOTAL = RING + PF * HF_M * (hf_cell<FMT>() + 4) + 1024;      // the base is rounded up to 1024 bytes
@@ -77,34 +71,15 @@ struct HfArgs {
     uint32_t n_tok, tok_pad;
 };
 
-// The pairs of a batch sorted into tiles of one expert each (expert_tiles_kernel), and the experts' images.
-struct HfExperts {
-    GemvArgs g;                        // geometry and the first expert's planes; xq / xs = activation rows, out = one row per pair
-    const uint32_t *n_tiles, *tile_expert, *tile_pairs;
-    const ExpertCodebook *books;
-    const uint8_t *const *bases;
-    const uint8_t *base0;
-    uint32_t act_group;                // activation row of a pair = pair / act_group
-};
-template <bool EXP> struct HfParam { using T = HfArgs; };
-template <> struct HfParam<true> { using T = HfExperts; };
-constexpr uint32_t HF_NO_PAIR = 0xffffffffu;
-
-template <int FMT, int N, bool EXP>
-__global__ void __launch_bounds__(HfRoles<N, EXP>::THREADS, EXP ? 2 : 1) gemm_f16_kernel(const typename HfParam<EXP>::T args) {
+template <int FMT, int N>
+__global__ void __launch_bounds__(HfRoles<N>::THREADS, 1) gemm_f16_kernel(const HfArgs args) {
     extern __shared__ uint8_t smem_raw[];
-    using R = HfRoles<N, EXP>;
-    using L = HfLayout<FMT, N, EXP>;
+    using R = HfRoles<N>;
+    using L = HfLayout<FMT, N>;
     constexpr uint32_t EPI = R::EPI_WARPS, DEC = R::DEC_WARPS, S = R::STAGES, NQ = R::NQ, CELL = hf_cell<FMT>(), PF = L::PF;
     const GemvArgs &a = args.g;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nc = a.nc;
     const uint32_t row0 = blockIdx.x * HF_M, tok0 = blockIdx.y * N;
-    uint32_t expert = 0;
-    if constexpr (EXP) {          // the routes are the predecessor's: nothing can be requested before
-        pdl_wait();
-        if (blockIdx.y >= __ldcg(args.n_tiles)) return;
-        expert = __ldcg(args.tile_expert + blockIdx.y);
-    }
     const uint32_t raw = (uint32_t)__cvta_generic_to_shared(smem_raw), sbase = (raw + 1023u) & ~1023u;
     uint8_t *smem = smem_raw + (sbase - raw);
     // per stage: full (A written by a decode group, activations and scales landed), done (products in tensor memory), drained (the
@@ -140,12 +115,10 @@ __global__ void __launch_bounds__(HfRoles<N, EXP>::THREADS, EXP ? 2 : 1) gemm_f1
         const uint32_t xs_own = xs_sa + (lane % NQ) * 4;
         const uint32_t ws_sa = sbase + L::WS + (quarter * 32 + lane) * 4;
         const uint32_t taddr0 = tmem + ((quarter * 32u) << 16) + part * NQ;
-        if constexpr (!EXP) {
-            pdl_wait();
-            own_behind = tok0 + part * NQ + lane % NQ >= args.n_tok;
-            ready = args.zero != nullptr;
-            all_plain = ready && __ldcg(args.zero) == 0;
-        }
+        pdl_wait();
+        own_behind = tok0 + part * NQ + lane % NQ >= args.n_tok;
+        ready = args.zero != nullptr;
+        all_plain = ready && __ldcg(args.zero) == 0;
         bool ok = true;
         uint32_t s = 0, ph = 0;
 #pragma unroll 1
@@ -197,16 +170,7 @@ __global__ void __launch_bounds__(HfRoles<N, EXP>::THREADS, EXP ? 2 : 1) gemm_f1
             if (++s == S) { s = 0; ph ^= 1u; }
         }
         if (!ok && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
-        if constexpr (EXP) {
-            if (ok && row < a.rows) {
-                const uint32_t *pairs = args.tile_pairs + blockIdx.y * N + part * NQ;
-#pragma unroll
-                for (uint32_t t = 0; t < NQ; ++t) {
-                    const uint32_t pair = __ldcg(pairs + t);
-                    if (pair != HF_NO_PAIR) a.out[(size_t)pair * a.out_stride + row] = __uint_as_float((t & 1u) ? (uint32_t)(f[t / 2] >> 32) : (uint32_t)f[t / 2]);
-                }
-            }
-        } else if (ok && row < a.rows) {
+        if (ok && row < a.rows) {
             const uint32_t t_first = tok0 + part * NQ;
             float *p = a.out + (size_t)t_first * a.out_stride + row;
 #pragma unroll
@@ -226,14 +190,7 @@ __global__ void __launch_bounds__(HfRoles<N, EXP>::THREADS, EXP ? 2 : 1) gemm_f1
         }
         constexpr uint32_t B0 = Cell<FMT>::B0, B1 = Cell<FMT>::B1, B2 = Cell<FMT>::B2, SLOT = HF_M * (CELL + 4);
         const uint32_t ring = sbase + L::RING;
-        HfTables tables;
-        ptrdiff_t at = 0;          // this expert's image behind the first one's
-        if constexpr (EXP) {
-            tables = hf_tables<FMT>(args.books[expert]);
-            at = args.bases[expert] - args.base0;
-        } else {
-            tables = hf_tables<FMT>(a);
-        }
+        const HfTables tables = hf_tables<FMT>(a);
         uint32_t p_cur = 0xffffffffu, ws_g0 = 0;
         const uint8_t *wb0 = nullptr, *wb1 = nullptr, *wb2 = nullptr, *wsb = nullptr;
         auto request = [&](uint32_t c) {          // the row's cell of chunk c and the word with its scale -> ring slot c % PF
@@ -241,10 +198,10 @@ __global__ void __launch_bounds__(HfRoles<N, EXP>::THREADS, EXP ? 2 : 1) gemm_f1
             if (p != p_cur) {
                 p_cur = p;
                 const size_t r_n = (size_t)row_c * tile_chunks(nc, p);
-                wb0 = a.plane[0] + at + tile_code_off(a.rows_pad, B0, p) + r_n * B0;
-                if (B1) wb1 = a.plane[1] + at + tile_code_off(a.rows_pad, B1, p) + r_n * B1;
-                if (B2) wb2 = a.plane[2] + at + tile_code_off(a.rows_pad, B2, p) + r_n * B2;
-                wsb = reinterpret_cast<const uint8_t *>(a.scales) + at + tile_scale_off(a.rows_pad, p) + (size_t)row_c * tile_scale_pitch(nc, a.sgc, p);
+                wb0 = a.plane[0] + tile_code_off(a.rows_pad, B0, p) + r_n * B0;
+                if (B1) wb1 = a.plane[1] + tile_code_off(a.rows_pad, B1, p) + r_n * B1;
+                if (B2) wb2 = a.plane[2] + tile_code_off(a.rows_pad, B2, p) + r_n * B2;
+                wsb = reinterpret_cast<const uint8_t *>(a.scales) + tile_scale_off(a.rows_pad, p) + (size_t)row_c * tile_scale_pitch(nc, a.sgc, p);
                 ws_g0 = scale_group_of(a, p * 32);
             }
             const uint32_t cc = c & 31u, slot = ring + (c % PF) * SLOT;
@@ -328,64 +285,6 @@ __global__ void __launch_bounds__(HfRoles<N, EXP>::THREADS, EXP ? 2 : 1) gemm_f1
                 for (uint32_t spin = 0; spin < WAIT_LIMIT && !mbar_try_wait(bar_last, 0u); ++spin) {}
             }
         }
-    } else if constexpr (EXP) {
-        // ------------------------------------------------------------------ activations of the tile's pairs, widened on the way: eight
-        // tokens x four 16-byte pieces per load, the values of a stage requested one stage ahead
-        const uint32_t piece = lane & 3u, r8 = lane >> 2;
-        const uint32_t *pairs = args.tile_pairs + blockIdx.y * N;
-        const uint32_t own = __ldcg(pairs + lane);
-        const float *xs = own == HF_NO_PAIR ? nullptr : a.xs + (size_t)(own / args.act_group) * nc;
-        const uint8_t *xq[4];
-#pragma unroll
-        for (uint32_t j = 0; j < 4; ++j) {
-            const uint32_t pair = __shfl_sync(0xffffffffu, own, j * 8 + r8);
-            xq[j] = pair == HF_NO_PAIR ? nullptr : reinterpret_cast<const uint8_t *>(a.xq) + (size_t)(pair / args.act_group) * a.cols + piece * 16;
-        }
-        uint4 v[2][4];
-        float sc[2];
-        auto load = [&](uint32_t c0) {
-#pragma unroll
-            for (uint32_t h = 0; h < 2; ++h) {
-                const bool in = c0 + h < nc;
-                sc[h] = in && xs != nullptr ? __ldcg(xs + c0 + h) : 1.0f;
-#pragma unroll
-                for (uint32_t j = 0; j < 4; ++j)
-                    v[h][j] = in && xq[j] != nullptr ? __ldcg(reinterpret_cast<const uint4 *>(xq[j] + (size_t)(c0 + h) * 64)) : make_uint4(0, 0, 0, 0);
-            }
-        };
-        load(0);
-        const __half2 add = __half2half2(__int2half_rn(-1152));
-        bool ok = true;
-#pragma unroll 1
-        for (uint32_t p = 0; 2 * p < nc; ++p) {
-            const uint32_t s = p % S;
-            if (p >= S) ok = ok && mbar_wait_thread(bar_drained + 8 * s, ((p / S) - 1u) & 1u, HF_WAIT_LIMIT, s_abort);
-#pragma unroll
-            for (uint32_t h = 0; h < 2; ++h) {
-                const uint32_t dst = sbase + L::B + (2 * s + h) * (N * 128), rec = sbase + L::XS + ((2 * p + h) % HF_SLOTS) * HF_REC;
-#pragma unroll
-                for (uint32_t j = 0; j < 4; ++j) {
-                    const uint32_t t = j * 8 + r8;
-                    uint32_t o[8];
-                    hf_widen(v[h][j].x ^ 0x80808080u, add, o[0], o[1]);
-                    hf_widen(v[h][j].y ^ 0x80808080u, add, o[2], o[3]);
-                    hf_widen(v[h][j].z ^ 0x80808080u, add, o[4], o[5]);
-                    hf_widen(v[h][j].w ^ 0x80808080u, add, o[6], o[7]);
-                    hf_sts128(dst + t * 128 + (((2 * piece) ^ (t & 7u)) << 4), o[0], o[1], o[2], o[3]);
-                    hf_sts128(dst + t * 128 + (((2 * piece + 1) ^ (t & 7u)) << 4), o[4], o[5], o[6], o[7]);
-                }
-                const bool plain = __all_sync(0xffffffffu, sc[h] != 0.0f);
-                if (2 * p + h < nc) {          // a chunk beyond the end has no slot of its own
-                    asm volatile("st.shared.f32 [%0], %1;" ::"r"(rec + lane * 4), "f"(sc[h]) : "memory");
-                    if (lane == 0) asm volatile("st.shared.u32 [%0], %1;" ::"r"(rec + 128), "r"(plain ? 1u : 0u) : "memory");
-                }
-            }
-            load(2 * p + 2);
-            fence_proxy_async();
-            __syncwarp();
-            if (lane == 0 && ok) hf_arrive(bar_full + 8 * s);
-        }
-        if (!ok && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
     } else if (lane == 0) {
         // ------------------------------------------------------------------ activations and their scales
         constexpr uint32_t XB = (N / 32) * HF_REC;
@@ -499,20 +398,12 @@ __global__ void __launch_bounds__(1024) expert_tiles_kernel(const uint32_t *rout
     }
 }
 
-template <int FMT> cudaError_t launch_hf_experts(cudaStream_t s, const HfExperts &args, uint32_t max_tiles, bool pdl) {
-    constexpr uint32_t smem = HfLayout<FMT, 32, true>::TOTAL;
-    static_assert(smem <= 113u * 1024u, "two CTAs per SM");
-    cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(gemm_f16_kernel<FMT, 32, true>), smem);
-    if (e != cudaSuccess) return e;
-    return launch_kernel(gemm_f16_kernel<FMT, 32, true>, dim3((args.g.rows + HF_M - 1) / HF_M, max_tiles), dim3(HfRoles<32, true>::THREADS), smem, s, pdl, args);
-}
-
 template <int FMT, int N> cudaError_t launch_hf_n(cudaStream_t s, const HfArgs &args, bool pdl) {
     constexpr uint32_t smem = HfLayout<FMT, N>::TOTAL;
     static_assert(smem <= 227u * 1024u, "shared memory");
-    cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(gemm_f16_kernel<FMT, N, false>), smem);
+    cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(gemm_f16_kernel<FMT, N>), smem);
     if (e != cudaSuccess) return e;
-    return launch_kernel(gemm_f16_kernel<FMT, N, false>, dim3((args.g.rows + HF_M - 1) / HF_M, (args.n_tok + N - 1) / N), dim3(HfRoles<N>::THREADS), smem, s, pdl, args);
+    return launch_kernel(gemm_f16_kernel<FMT, N>, dim3((args.g.rows + HF_M - 1) / HF_M, (args.n_tok + N - 1) / N), dim3(HfRoles<N>::THREADS), smem, s, pdl, args);
 }
 
 template <int FMT> cudaError_t launch_hf_fmt(cudaStream_t s, const HfArgs &args, int sm_count, bool pdl) {
@@ -540,24 +431,6 @@ cudaError_t launch_expert_tiles(cudaStream_t stream, const uint32_t *route_ids, 
                                 const uint8_t *const *bases, const ExpertTiles &t, uint32_t *err_flag, bool pdl) {
     if (n_experts > EXPERT_TILES_MAX_EXPERTS || expert_tiles_max((size_t)n_tok * k, n_experts) > 0xFFFFu) return cudaErrorInvalidValue;
     return launch_kernel(expert_tiles_kernel, dim3(1), dim3(1024), 0, stream, pdl, route_ids, n_tok * k, k, route_stride, n_experts, bases, t.n_tiles, t.expert, t.pairs, err_flag);
-}
-
-cudaError_t launch_gemm_experts(cudaStream_t stream, const DeviceMatrix &m0, int fmt, const ExpertCodebook *books, const uint8_t *const *bases, uint32_t n_experts,
-                                const ExpertTiles &t, uint32_t n_pair, uint32_t act_group, const int8_t *xq, const float *xs, float *out, uint32_t *err_flag, bool pdl) {
-    HfExperts args;
-    if (fill_gemv_args(m0, true, args.g) < 0) return cudaErrorNotSupported;
-    args.g.xq = xq; args.g.xs = xs; args.g.out = out; args.g.out_stride = m0.geom.rows; args.g.err_flag = err_flag;
-    args.n_tiles = t.n_tiles; args.tile_expert = t.expert; args.tile_pairs = t.pairs;
-    args.books = books; args.bases = bases; args.base0 = m0.d_base; args.act_group = act_group;
-    const uint32_t tiles = expert_tiles_max(n_pair, n_experts);
-    switch (fmt) {
-        case FMT_NF4: return launch_hf_experts<FMT_NF4>(stream, args, tiles, pdl);
-        case FMT_NF4G: return launch_hf_experts<FMT_NF4G>(stream, args, tiles, pdl);
-        case FMT_NF3: return launch_hf_experts<FMT_NF3>(stream, args, tiles, pdl);
-        case FMT_NF5: return launch_hf_experts<FMT_NF5>(stream, args, tiles, pdl);
-        case FMT_E8Q2: return launch_hf_experts<FMT_E8Q2>(stream, args, tiles, pdl);
-        default: return cudaErrorNotSupported;       // experts are NF matrices (2..5 bits)
-    }
 }
 
 bool gemm_f16_takes(size_t n_tok) { return n_tok != 0 && act_half_tokens(n_tok) / 32 <= 0xFFFFu; }

@@ -52,6 +52,6 @@ bool experts_grouped(uint32_t n_tok, uint32_t n_pair, uint32_t n_experts, uint32
 // The expert projections of all pairs of `t`, an expert's weights expanded once per 32 pairs; out = [n_pair][rows].  Same bits as
 // launch_gemv_experts, for activations in the form the library's own quantizers leave them.
 cudaError_t launch_gemm_experts(cudaStream_t stream, const DeviceMatrix &m0, int fmt, const ExpertCodebook *books, const uint8_t *const *bases, uint32_t n_experts,
-                                const ExpertTiles &t, uint32_t n_pair, uint32_t act_group, const int8_t *xq, const float *xs, float *out, uint32_t *err_flag, bool pdl);
+                                const ExpertTiles &t, uint32_t n_pair, uint32_t act_group, const int8_t *xq, const float *xs, float *out, int sm_count, uint32_t *err_flag, bool pdl);
 
 }  // namespace k2t

@@ -8,6 +8,8 @@ namespace k2t {
 
 template <int FMT> __host__ __device__ constexpr uint32_t hf_cell() { return Cell<FMT>::B0 + Cell<FMT>::B1 + Cell<FMT>::B2; }
 
+constexpr uint32_t HF_NO_PAIR = 0xffffffffu;          // behind the last pair of an expert's tile
+
 __device__ __forceinline__ void hf_cp_async16(uint32_t dst, const void *src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
 __device__ __forceinline__ void hf_cp_async8(uint32_t dst, const void *src) { asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory"); }
 __device__ __forceinline__ void hf_cp_async4(uint32_t dst, const void *src) { asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory"); }

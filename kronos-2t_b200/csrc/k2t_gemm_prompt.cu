@@ -16,6 +16,9 @@
 // the rest of them expansion and waits).  Measured on B200, nf4g128, image ready, k2t_gemm_f16.cu -> here: 2048 x 6144, 512 tokens
 // 48.5 -> 32.5 us; 2048 x 16384 97.9 -> 82.6; 8192 x 2048 65.1 -> 59.3; b4, 77 tokens: 3584 x 37888 78.2 -> 57.7, 18944 x 3584 112.7 -> 104.1.
 // Bound: 0.6 instructions per scheduler and cycle; what a chunk needs at least, packed chain steps, is a quarter of its time.
+// The experts of a prompt (EXP) run in the same kernel: a tile is 128 rows of one expert and up to 32 of its (token, route) pairs, which
+// expert_tiles_kernel has gathered; two warps fetch the pairs' int8 rows where they lie and widen them on the way (one warp that did so
+// held two CTAs an SM to a tile's chunk per 0.59 us).  2400 pairs of 128 experts, 3 bits: 1536 x 2048 202 -> 158 us, 2048 x 768 131 -> 94.
 // Waits are bounded as in k2t_gemm_f16.cu.
 #include <algorithm>
 #include <type_traits>
@@ -24,6 +27,8 @@
 
 namespace k2t {
 
+int fill_gemv_args(const DeviceMatrix &m, bool has_xsum, GemvArgs &a);      // k2t_gemv.cu
+
 namespace {
 
 constexpr uint32_t GP_M = 128;               // rows per tile = UMMA M
@@ -31,14 +36,16 @@ constexpr uint32_t GP_WAIT_LIMIT = 1u << 21;
 constexpr uint32_t GP_HEADER = 1024;
 constexpr uint32_t GP_WS_SLOTS = 8;
 
-template <int FMT, int N> struct GpLayout {
+// EXP: the pairs of an expert; two warps fetch and widen their activations instead of one thread that copies an image.
+template <int FMT, int N, bool EXP = false> struct GpLayout {
     static constexpr uint32_t ND = N > 128 ? 2 : N > 64 ? 3 : 4;                     // accumulator buffers in tensor memory
     static constexpr uint32_t NA = 4;                                                // chunks of expanded weights there
     static constexpr uint32_t NB = N > 128 ? 4 : 6;                                  // chunks of activations in shared memory
     static constexpr uint32_t EPI = N > 128 ? 12 : 8, NG = N > 64 ? 2 : 4, DEC = 4 * NG, THREADS = (EPI + DEC + 4) * 32;          // warps: chains, expansion (groups of four)
     static constexpr uint32_t NQ = N > 128 ? 64 : N / 2;                             // tokens of a chain warp
     // registers a thread, at launch and by role
-    static constexpr int R_ALL = N > 128 ? 80 : N > 64 ? 96 : 72, R_EPI = N > 128 ? 112 : N > 64 ? 136 : 88, R_DEC = N > 128 ? 56 : N > 64 ? 80 : 72, R_MISC = N > 128 ? 32 : 40;
+    static constexpr int R_ALL = N > 128 ? 80 : N > 64 ? 96 : 72, R_EPI = EXP ? 64 : N > 128 ? 112 : N > 64 ? 136 : 88, R_DEC = N > 128 ? 56 : N > 64 ? 80 : 72,
+                         R_MISC = EXP ? 88 : N > 128 ? 32 : 40;
     static_assert(EPI * R_EPI + DEC * R_DEC + 4 * R_MISC <= (EPI + DEC + 4) * R_ALL && THREADS * R_ALL <= 65536, "registers");
     static constexpr uint32_t CELL = hf_cell<FMT>();
     static constexpr uint32_t GC = 4, NR = 4;                                        // chunks per slot of raw weights, slots
@@ -60,6 +67,22 @@ struct GpArgs {
     uint32_t n_tok, tok_pad, tok_tiles, tiles, width;          // width: tokens of a tile, a multiple of 16
 };
 
+// The pairs of a batch sorted into tiles of one expert each (k2t_gemm_f16.cu), and the experts' images.
+struct GpExperts {
+    GemvArgs g;                        // geometry and the first expert's planes; xq / xs = activation rows, out = one row per pair
+    const uint32_t *n_tiles, *tile_expert, *tile_pairs;
+    const ExpertCodebook *books;
+    const uint8_t *const *bases;
+    const uint8_t *base0;
+    uint32_t act_group, row_tiles;     // activation row of a pair = pair / act_group
+};
+template <bool EXP> struct GpParam { using T = GpArgs; };
+template <> struct GpParam<true> { using T = GpExperts; };
+
+template <int R_ALL, int R> __device__ __forceinline__ void gp_registers() {
+    if constexpr (R > R_ALL) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R));
+    else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R));
+}
 __device__ __forceinline__ void gp_arrive_n(uint32_t bar, uint32_t n) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(n) : "memory"); }
 __device__ __forceinline__ bool gp_elect() {
     uint32_t p;
@@ -102,10 +125,10 @@ __device__ __forceinline__ void gp_st32(uint32_t taddr, const uint32_t (&h)[32])
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
-template <int FMT, int N>
-__global__ void __launch_bounds__(GpLayout<FMT, N>::THREADS, 1) gemm_prompt_kernel(const GpArgs args) {
+template <int FMT, int N, bool EXP>
+__global__ void __launch_bounds__(GpLayout<FMT, N, EXP>::THREADS, 1) gemm_prompt_kernel(const typename GpParam<EXP>::T args) {
     extern __shared__ uint8_t smem_raw[];
-    using L = GpLayout<FMT, N>;
+    using L = GpLayout<FMT, N, EXP>;
     constexpr uint32_t GP_EPI = L::EPI, GP_DEC = L::DEC, NG = L::NG, ND = L::ND, NA = L::NA, NB = L::NB, NQ = L::NQ, GC = L::GC, NR = L::NR, CELL = L::CELL, B0 = Cell<FMT>::B0, B1 = Cell<FMT>::B1, B2 = Cell<FMT>::B2;
     const GemvArgs &a = args.g;
     const uint32_t tid = threadIdx.x, hw_warp = tid >> 5, warp = hw_warp < 4 ? hw_warp + GP_EPI + GP_DEC : hw_warp - 4, lane = tid & 31, nc = a.nc;
@@ -135,14 +158,25 @@ __global__ void __launch_bounds__(GpLayout<FMT, N>::THREADS, 1) gemm_prompt_kern
     __syncthreads();
     hf_fence_after();
     const uint32_t tmem = *s_tmem, tmem_a = tmem + ND * N;
-    const uint32_t my_tiles = (args.tiles - blockIdx.x + gridDim.x - 1) / gridDim.x, total = my_tiles * nc;
+    uint32_t tiles;
+    if constexpr (EXP) {          // the routes are the predecessor's: nothing can be requested before
+        pdl_wait();
+        tiles = __ldcg(args.n_tiles) * args.row_tiles;
+    } else {
+        tiles = args.tiles;
+    }
+    const uint32_t my_tiles = tiles > blockIdx.x ? (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0u, total = my_tiles * nc;
+    auto first_row = [&](uint32_t tile) {
+        if constexpr (EXP) return tile % args.row_tiles * GP_M;
+        else return tile / args.tok_tiles * GP_M;
+    };
 
     if (warp < GP_EPI) {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(L::R_EPI));
+        gp_registers<L::R_ALL, L::R_EPI>();
         // ------------------------------------------------------------------ chains: lane = four rows (8 apart), NQ / 8 blocks of two tokens
         constexpr uint32_t NBLK = NQ / 8;
         const uint32_t quarter = warp & 3u, part = warp >> 2;
-        pdl_wait();
+        if constexpr (!EXP) pdl_wait();
         uint32_t xs_at[NBLK];
 #pragma unroll
         for (uint32_t b = 0; b < NBLK; ++b) {
@@ -154,12 +188,21 @@ __global__ void __launch_bounds__(GpLayout<FMT, N>::THREADS, 1) gemm_prompt_kern
         uint32_t s8 = 0, ph = 0, f8 = (ND % NA) * 8, xo = 0, wo = 0, ta = tmem + ((quarter * 32u) << 16) + part * NQ;
         if (lane == 0)
             for (uint32_t i = 0; i < ND; ++i) hf_arrive(bar_full + 8 * (i % NA));          // nothing to read there yet
-        auto tiles = [&](auto plain_image) {
+        auto run = [&](auto plain_image) {
             constexpr bool PLAIN = decltype(plain_image)::value;
 #pragma unroll 1
-            for (uint32_t tile = blockIdx.x; tile < args.tiles; tile += gridDim.x) {
-                const uint32_t row0 = (tile / args.tok_tiles) * GP_M, tok0 = (tile % args.tok_tiles) * args.width, end = min(args.n_tok, tok0 + args.width);
-                const bool live = tok0 + part * NQ < end;          // any token of the warp
+            for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+                const uint32_t row0 = first_row(tile);
+                uint32_t tok0 = 0, end = 0;
+                bool live;          // any token of the warp
+                const uint32_t *pairs = nullptr;
+                if constexpr (EXP) {
+                    pairs = args.tile_pairs + tile / args.row_tiles * N + part * NQ;
+                    live = __ldcg(pairs) != HF_NO_PAIR;          // they fill their tile from the front
+                } else {
+                    tok0 = (tile % args.tok_tiles) * args.width; end = min(args.n_tok, tok0 + args.width);
+                    live = tok0 + part * NQ < end;
+                }
                 unsigned long long f[4][NBLK];
 #pragma unroll
                 for (uint32_t r = 0; r < 4; ++r)
@@ -225,7 +268,20 @@ __global__ void __launch_bounds__(GpLayout<FMT, N>::THREADS, 1) gemm_prompt_kern
                     if (xo == 2 * NB * L::XS_CHUNK) xo = 0;
                     wo = (wo + GP_M * 8) & (GP_WS_SLOTS * GP_M * 8 - 1);
                 }
-                if (ok) {
+                if constexpr (EXP) {
+                    if (ok && live) {
+#pragma unroll
+                        for (uint32_t b = 0; b < NBLK; ++b) {
+                            const uint2 pair = __ldcg(reinterpret_cast<const uint2 *>(pairs + 8 * b + 2 * (lane & 3u)));
+#pragma unroll
+                            for (uint32_t r = 0; r < 4; ++r) {
+                                const uint32_t row = row0 + quarter * 32 + (lane >> 2) + 8 * r;
+                                if (row < a.rows && pair.x != HF_NO_PAIR) a.out[(size_t)pair.x * a.out_stride + row] = __uint_as_float((uint32_t)f[r][b]);
+                                if (row < a.rows && pair.y != HF_NO_PAIR) a.out[(size_t)pair.y * a.out_stride + row] = __uint_as_float((uint32_t)(f[r][b] >> 32));
+                            }
+                        }
+                    }
+                } else if (ok) {
 #pragma unroll
                     for (uint32_t r = 0; r < 4; ++r) {
                         const uint32_t row = row0 + quarter * 32 + (lane >> 2) + 8 * r;
@@ -242,22 +298,31 @@ __global__ void __launch_bounds__(GpLayout<FMT, N>::THREADS, 1) gemm_prompt_kern
                 }
             }
         };
-        if (args.zero != nullptr && __ldcg(args.zero) == 0) tiles(std::true_type{});
-        else tiles(std::false_type{});
+        if constexpr (EXP) run(std::false_type{});
+        else if (args.zero != nullptr && __ldcg(args.zero) == 0) run(std::true_type{});
+        else run(std::false_type{});
         if (!ok && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
     } else if (warp < GP_EPI + GP_DEC) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(L::R_DEC));
+        gp_registers<L::R_ALL, L::R_DEC>();
         // ------------------------------------------------------------------ expansion: groups of four warps, chunk by chunk in turn; thread = row
         const uint32_t di = (warp - GP_EPI) * 32 + lane, grp = di >> 7, row = di & 127u, quarter = row >> 5;
-        const HfTables tables = hf_tables<FMT>(a);
+        HfTables tables;
+        auto table_of = [&](uint32_t tile) {
+            if constexpr (EXP) { if (tile < tiles) tables = hf_tables<FMT>(args.books[__ldcg(args.tile_expert + tile / args.row_tiles)]); }
+        };
+        if constexpr (EXP) table_of(blockIdx.x);
+        else tables = hf_tables<FMT>(a);
         const uint32_t ta = tmem_a + ((quarter * 32u) << 16), sw = (row >> 1) & (GC - 1), sw8 = ((row >> 2) & 1u) * 16, spt = (nc + GC - 1) / GC;
         // the four rows of an epilogue lane side by side, each scale twice
         const uint32_t ws_at = sbase + L::WS + (quarter * 32 + (lane & 7u) * 4 + (lane >> 3)) * 8;
         bool ok = true;
-        uint32_t c = grp, base = 0, s = grp, ph = 1;          // chunk in its tile, raw slots of the tiles before, weight buffer and its phase
+        uint32_t tile = blockIdx.x, c = grp, base = 0, s = grp, ph = 1;          // chunk in its tile, raw slots of the tiles before, weight buffer and its phase
 #pragma unroll 1
         for (uint32_t i = grp; i < total; i += NG, c += NG) {
-            while (c >= nc) { c -= nc; base += spt; }
+            if (c >= nc) {
+                while (c >= nc) { c -= nc; base += spt; tile += gridDim.x; }
+                table_of(tile);
+            }
             const uint32_t cc = c % GC, slot_n = base + c / GC, slot = slot_n % NR, rs = sbase + L::RAW + slot * L::RAW_SLOT;
             ok = ok && mbar_wait_thread(bar_rfull + 8 * slot, (slot_n / NR) & 1u, GP_WAIT_LIMIT, s_abort);
             Raw<FMT> w;
@@ -288,10 +353,12 @@ __global__ void __launch_bounds__(GpLayout<FMT, N>::THREADS, 1) gemm_prompt_kern
         }
         if (!ok && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
     } else {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(L::R_MISC));
+    gp_registers<L::R_ALL, L::R_MISC>();
     if (warp == GP_EPI + GP_DEC) {
         // ------------------------------------------------------------------ products
-        const uint32_t idesc = (1u << 4) | ((args.width >> 3) << 17) | ((GP_M >> 4) << 24);
+        uint32_t width = N;
+        if constexpr (!EXP) width = args.width;
+        const uint32_t idesc = (1u << 4) | ((width >> 3) << 17) | ((GP_M >> 4) << 24);
         const uint64_t db0 = hf_desc(sbase + L::B);
         bool ok = true;
         uint32_t s = 0, ph = 0, b = 0, d = 0;
@@ -322,15 +389,75 @@ __global__ void __launch_bounds__(GpLayout<FMT, N>::THREADS, 1) gemm_prompt_kern
             }
             __syncwarp();
         }
-    } else if (warp == GP_EPI + GP_DEC + 1) {
-        if (lane == 0) {
+    } else if (warp == GP_EPI + GP_DEC + 1 || (EXP && warp == GP_EPI + GP_DEC + 3)) {
+        if constexpr (EXP) {
+            // ------------------------------------------------------------------ activations of the tile's pairs, widened on the way, the two warps chunk by chunk in
+            // turn: eight tokens x four 16-byte pieces per load, the next chunk's values on their way
+            const uint32_t piece = lane & 3u, r8 = lane >> 2, turn = warp == GP_EPI + GP_DEC + 1 ? 0u : 1u;
+            if (turn == 0 && lane == 0) pdl_trigger();
+            const __half2 add = __half2half2(__int2half_rn(-1152));
+            const float *xs = nullptr;
+            const uint8_t *xq[4];
+            auto rows_of = [&](uint32_t tile) {
+                const uint32_t own = tile < tiles ? __ldcg(args.tile_pairs + tile / args.row_tiles * N + lane) : HF_NO_PAIR;
+                xs = own == HF_NO_PAIR ? nullptr : a.xs + (size_t)(own / args.act_group) * nc;
+#pragma unroll
+                for (uint32_t j = 0; j < 4; ++j) {
+                    const uint32_t pair = __shfl_sync(0xffffffffu, own, j * 8 + r8);
+                    xq[j] = pair == HF_NO_PAIR ? nullptr : reinterpret_cast<const uint8_t *>(a.xq) + (size_t)(pair / args.act_group) * a.cols + piece * 16;
+                }
+            };
+            uint4 v[4];
+            float sc = 1.0f;
+            auto load = [&](uint32_t c) {
+                sc = xs != nullptr ? __ldcg(xs + c) : 1.0f;
+#pragma unroll
+                for (uint32_t j = 0; j < 4; ++j) v[j] = xq[j] != nullptr ? __ldcg(reinterpret_cast<const uint4 *>(xq[j] + (size_t)c * 64)) : make_uint4(0, 0, 0, 0);
+            };
+            uint32_t tile = blockIdx.x, c = turn;
+            auto settle = [&]() {          // the chunk's tile
+                if (c < nc) return;
+                while (c >= nc) { c -= nc; tile += gridDim.x; }
+                rows_of(tile);
+            };
+            rows_of(tile);
+            settle();
+            if (turn < total) load(c);
+            bool ok = true;
+            for (uint32_t i = turn; i < total; i += 2) {
+                const uint32_t b = i % NB, s = i % NA;
+                // the products that read the slot are done; a buffer's arrivals belong to one chunk
+                if (i >= NB) ok = ok && mbar_wait_thread(bar_bfree + 8 * b, (i / NB - 1u) & 1u, GP_WAIT_LIMIT, s_abort);
+                if (i >= NA) ok = ok && mbar_wait_thread(bar_full + 8 * s, (i / NA - 1u) & 1u, GP_WAIT_LIMIT, s_abort);
+                const uint32_t dst = sbase + L::B + b * (N * 128);
+#pragma unroll
+                for (uint32_t j = 0; j < 4; ++j) {
+                    const uint32_t t = j * 8 + r8;
+                    uint32_t o[8];
+                    hf_widen(v[j].x ^ 0x80808080u, add, o[0], o[1]);
+                    hf_widen(v[j].y ^ 0x80808080u, add, o[2], o[3]);
+                    hf_widen(v[j].z ^ 0x80808080u, add, o[4], o[5]);
+                    hf_widen(v[j].w ^ 0x80808080u, add, o[6], o[7]);
+                    hf_sts128(dst + t * 128 + (((2 * piece) ^ (t & 7u)) << 4), o[0], o[1], o[2], o[3]);
+                    hf_sts128(dst + t * 128 + (((2 * piece + 1) ^ (t & 7u)) << 4), o[4], o[5], o[6], o[7]);
+                }
+                asm volatile("st.shared.f32 [%0], %1;" ::"r"(sbase + L::XS + (i % (2 * NB)) * L::XS_CHUNK + lane * 4), "f"(sc) : "memory");
+                c += 2;
+                settle();
+                if (i + 2 < total) load(c);
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0 && ok) hf_arrive(bar_full + 8 * s);
+            }
+            if (!ok && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
+        } else if (lane == 0) {
             // ------------------------------------------------------------------ activations and their scales
             const size_t pitch = (size_t)args.tok_pad * 128, xpitch = (size_t)(args.tok_pad / 32) * HF_REC;
             pdl_wait();
             pdl_trigger();
             bool ok = true;
             uint32_t i = 0, b = 0, ph = 1, xsl = 0;
-            for (uint32_t tile = blockIdx.x; ok && tile < args.tiles; tile += gridDim.x) {
+            for (uint32_t tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
                 const uint32_t tok0 = (tile % args.tok_tiles) * args.width, x0 = tok0 % 32, bytes = min(args.width, (args.n_tok - tok0 + 7u) & ~7u) * 128;          // whole groups of eight tokens; what lies behind is not stored
                 const uint32_t xbytes = (x0 + bytes / 128 + 31) / 32 * HF_REC;
                 const uint8_t *src = args.img + (size_t)tok0 * 128, *xsrc = args.xs_img + (size_t)(tok0 / 32) * HF_REC;
@@ -362,8 +489,10 @@ __global__ void __launch_bounds__(GpLayout<FMT, N>::THREADS, 1) gemm_prompt_kern
         const uint32_t j2 = lane & 1u, r16 = lane >> 1, d8 = r16 * GC * 8 + (j2 ^ ((r16 >> 2) & 1u)) * 16;          // among pairs of them
         bool ok = true;
         uint32_t n_slot = 0;
-        for (uint32_t tile = blockIdx.x; ok && tile < args.tiles; tile += gridDim.x) {
-            const uint32_t row0 = (tile / args.tok_tiles) * GP_M;
+        for (uint32_t tile = blockIdx.x; ok && tile < tiles; tile += gridDim.x) {
+            const uint32_t row0 = first_row(tile);
+            ptrdiff_t image = 0;          // this expert's image behind the first one's
+            if constexpr (EXP) image = args.bases[__ldcg(args.tile_expert + tile / args.row_tiles)] - args.base0;
             for (uint32_t c0 = 0; c0 < nc; c0 += GC, ++n_slot) {
                 const uint32_t slot = n_slot % NR, rs = sbase + L::RAW + slot * L::RAW_SLOT;
                 if (n_slot >= NR) {
@@ -372,9 +501,9 @@ __global__ void __launch_bounds__(GpLayout<FMT, N>::THREADS, 1) gemm_prompt_kern
                 }
                 const uint32_t p = c0 >> 5, n = tile_chunks(nc, p), cc = (c0 & 31u) + j;
                 if (n == 32 && row0 + GP_M <= a.rows_pad) {          // a full pass: the strides are constants, and pairs of 8-byte pieces lie on 16 bytes
-                    const uint8_t *p0 = a.plane[0] + tile_code_off(a.rows_pad, B0, p) + (size_t)(row0 + r8) * (32 * B0) + cc * B0;
-                    const uint8_t *p1 = a.plane[1] + tile_code_off(a.rows_pad, B1, p) + (size_t)(row0 + (B1 == 8 ? r16 : r8)) * (32 * B1) + (B1 == 8 ? (c0 & 31u) * 8 + j2 * 16 : cc * B1);
-                    const uint8_t *p2 = a.plane[2] + tile_code_off(a.rows_pad, B2, p) + (size_t)(row0 + (B2 == 8 ? r16 : r8)) * (32 * B2) + (B2 == 8 ? (c0 & 31u) * 8 + j2 * 16 : cc * B2);
+                    const uint8_t *p0 = a.plane[0] + image + tile_code_off(a.rows_pad, B0, p) + (size_t)(row0 + r8) * (32 * B0) + cc * B0;
+                    const uint8_t *p1 = a.plane[1] + image + tile_code_off(a.rows_pad, B1, p) + (size_t)(row0 + (B1 == 8 ? r16 : r8)) * (32 * B1) + (B1 == 8 ? (c0 & 31u) * 8 + j2 * 16 : cc * B1);
+                    const uint8_t *p2 = a.plane[2] + image + tile_code_off(a.rows_pad, B2, p) + (size_t)(row0 + (B2 == 8 ? r16 : r8)) * (32 * B2) + (B2 == 8 ? (c0 & 31u) * 8 + j2 * 16 : cc * B2);
 #pragma unroll
                     for (uint32_t r = 0; r < GP_M; r += STEP) {
                         hf_cp_async16(rs + d16 + r * GC * B0, p0 + r * 32 * B0);
@@ -389,8 +518,8 @@ __global__ void __launch_bounds__(GpLayout<FMT, N>::THREADS, 1) gemm_prompt_kern
                         }
                     }
                 } else if (cc < n) {
-                    const uint8_t *p0 = a.plane[0] + tile_code_off(a.rows_pad, B0, p) + cc * B0, *p1 = a.plane[1] + tile_code_off(a.rows_pad, B1, p) + cc * B1,
-                                  *p2 = a.plane[2] + tile_code_off(a.rows_pad, B2, p) + cc * B2;
+                    const uint8_t *p0 = a.plane[0] + image + tile_code_off(a.rows_pad, B0, p) + cc * B0, *p1 = a.plane[1] + image + tile_code_off(a.rows_pad, B1, p) + cc * B1,
+                                  *p2 = a.plane[2] + image + tile_code_off(a.rows_pad, B2, p) + cc * B2;
                     auto row = [&](uint32_t r, const uint8_t *q0, const uint8_t *q1, const uint8_t *q2) {
                         hf_cp_async16(rs + d16 + r * GC * B0, q0);
                         if (B1 == 16) hf_cp_async16(rs + GP_M * GC * B0 + d16 + r * GC * 16, q1);
@@ -398,6 +527,16 @@ __global__ void __launch_bounds__(GpLayout<FMT, N>::THREADS, 1) gemm_prompt_kern
                         if (B2 == 16) hf_cp_async16(rs + GP_M * GC * (B0 + B1) + d16 + r * GC * 16, q2);
                         if (B2 == 8) hf_cp_async8(rs + GP_M * GC * (B0 + B1) + e8 + r * GC * 8, q2);
                     };
+                    if (EXP && row0 + GP_M <= a.rows_pad) {
+                        const size_t at = (size_t)(row0 + r8) * n;
+                        const uint32_t step = STEP * n;
+                        p0 += at * B0; p1 += at * B1; p2 += at * B2;
+#pragma unroll
+                        for (uint32_t r = 0; r < GP_M; r += STEP) {
+                            row(r, p0, p1, p2);
+                            p0 += step * B0; p1 += step * B1; p2 += step * B2;
+                        }
+                    } else
 #pragma unroll 2
                     for (uint32_t r = 0; r < GP_M; r += STEP) {          // rows beyond the matrix repeat the last one (never stored)
                         const size_t at = (size_t)min(row0 + r8 + r, a.rows_pad - 1) * n;
@@ -407,7 +546,7 @@ __global__ void __launch_bounds__(GpLayout<FMT, N>::THREADS, 1) gemm_prompt_kern
                 {          // the words that hold the scales of these chunks
                     const uint32_t g0 = scale_group_of(a, p * 32), off0 = ((scale_group_of(a, c0) - g0) * 2u) & ~3u;
                     const uint32_t last = min(c0 + GC, nc) - 1, words = ((scale_group_of(a, last) - g0) * 2u - off0) / 4u + 1u, pitch = tile_scale_pitch(nc, a.sgc, p);
-                    const uint8_t *src = reinterpret_cast<const uint8_t *>(a.scales) + tile_scale_off(a.rows_pad, p) + off0;
+                    const uint8_t *src = reinterpret_cast<const uint8_t *>(a.scales) + image + tile_scale_off(a.rows_pad, p) + off0;
 #pragma unroll
                     for (uint32_t r = lane; r < GP_M; r += 32) {
                         const uint8_t *q = src + (size_t)min(row0 + r, a.rows_pad - 1) * pitch;
@@ -442,15 +581,24 @@ __global__ void __launch_bounds__(GpLayout<FMT, N>::THREADS, 1) gemm_prompt_kern
     }
 }
 
+template <int FMT> cudaError_t launch_gp_experts(cudaStream_t s, const GpExperts &args, uint32_t max_tiles, int sm_count, bool pdl) {
+    constexpr uint32_t smem = GpLayout<FMT, 32, true>::TOTAL;
+    static_assert(smem <= 227u * 1024u, "shared memory");
+    cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(gemm_prompt_kernel<FMT, 32, true>), smem);
+    if (e != cudaSuccess) return e;
+    return launch_kernel(gemm_prompt_kernel<FMT, 32, true>, dim3((unsigned)std::min<uint64_t>((uint64_t)max_tiles * args.row_tiles, (uint64_t)sm_count)), dim3(GpLayout<FMT, 32, true>::THREADS), smem, s,
+                         pdl, args);
+}
+
 template <int FMT, int N> cudaError_t launch_gp(cudaStream_t s, GpArgs args, int sm_count, bool pdl) {
     constexpr uint32_t smem = GpLayout<FMT, N>::TOTAL;
     static_assert(smem <= 227u * 1024u, "shared memory");
-    cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(gemm_prompt_kernel<FMT, N>), smem);
+    cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(gemm_prompt_kernel<FMT, N, false>), smem);
     if (e != cudaSuccess) return e;
     args.tok_tiles = (args.n_tok + N - 1) / N;
     args.width = std::min<uint32_t>(N, ((args.n_tok + args.tok_tiles - 1) / args.tok_tiles + 31) / 32 * 32);
     args.tiles = ((args.g.rows + GP_M - 1) / GP_M) * args.tok_tiles;
-    return launch_kernel(gemm_prompt_kernel<FMT, N>, dim3(std::min<uint32_t>(args.tiles, sm_count)), dim3(GpLayout<FMT, N>::THREADS), smem, s, pdl, args);
+    return launch_kernel(gemm_prompt_kernel<FMT, N, false>, dim3(std::min<uint32_t>(args.tiles, sm_count)), dim3(GpLayout<FMT, N>::THREADS), smem, s, pdl, args);
 }
 }  // namespace
 
@@ -490,6 +638,24 @@ cudaError_t launch_gemm_prompt(cudaStream_t stream, const GemvArgs &g, int fmt, 
         case FMT_NF5: return launch_gp_fmt<FMT_NF5>(stream, args, sm_count, pdl);
         case FMT_E8Q2: return launch_gp_fmt<FMT_E8Q2>(stream, args, sm_count, pdl);
         default: return cudaErrorNotSupported;
+    }
+}
+
+cudaError_t launch_gemm_experts(cudaStream_t stream, const DeviceMatrix &m0, int fmt, const ExpertCodebook *books, const uint8_t *const *bases, uint32_t n_experts,
+                                const ExpertTiles &t, uint32_t n_pair, uint32_t act_group, const int8_t *xq, const float *xs, float *out, int sm_count, uint32_t *err_flag, bool pdl) {
+    GpExperts args;
+    if (fill_gemv_args(m0, true, args.g) < 0) return cudaErrorNotSupported;
+    args.g.xq = xq; args.g.xs = xs; args.g.out = out; args.g.out_stride = m0.geom.rows; args.g.err_flag = err_flag;
+    args.n_tiles = t.n_tiles; args.tile_expert = t.expert; args.tile_pairs = t.pairs;
+    args.books = books; args.bases = bases; args.base0 = m0.d_base; args.act_group = act_group; args.row_tiles = (m0.geom.rows + GP_M - 1) / GP_M;
+    const uint32_t tiles = expert_tiles_max(n_pair, n_experts);
+    switch (fmt) {
+        case FMT_NF4: return launch_gp_experts<FMT_NF4>(stream, args, tiles, sm_count, pdl);
+        case FMT_NF4G: return launch_gp_experts<FMT_NF4G>(stream, args, tiles, sm_count, pdl);
+        case FMT_NF3: return launch_gp_experts<FMT_NF3>(stream, args, tiles, sm_count, pdl);
+        case FMT_NF5: return launch_gp_experts<FMT_NF5>(stream, args, tiles, sm_count, pdl);
+        case FMT_E8Q2: return launch_gp_experts<FMT_E8Q2>(stream, args, tiles, sm_count, pdl);
+        default: return cudaErrorNotSupported;       // experts are NF matrices (2..5 bits)
     }
 }
 
