@@ -2,8 +2,9 @@
 // bias per head, unquantized (bf16 or fp32) key and value rows in a ring per layer.
 //   * window_prep_kernel: per-head RMS norm of queries and keys of a prompt batch, cache rows, query rows (one warp per head).
 //   * window_flash_kernel (bf16 prompts): CTA = 128 query rows of one kv head - row = (token, head of the group), so all heads
-//     of a group share the key and value tiles - against 64-position tiles of the window, double-buffered with cp.async; both
-//     products on the tensor cores (bf16 operands, fp32 accumulators), scores, bias, online softmax and its sums in fp32.
+//     of a group share the key and value tiles.  S = Q K^T and O += P V by tcgen05.mma with S, P and O in tensor memory; scores,
+//     bias and softmax in fp32, one row per thread; the next S is computed while the softmax of this one runs, and O is rescaled
+//     only when a row's maximum has grown by more than 2^8.
 //   * window_row_kernel: one token and kv head per thread-block cluster.  The positions are split over the CTAs of the cluster,
 //     partial maxima, sums and outputs are merged through distributed shared memory, so a decode step is ONE launch: norms of
 //     the new query and key, the new cache row, attention and the activation of the output projection.  With fp32 rows the same
@@ -12,12 +13,12 @@
 
 #include "k2t_block_kernels.h"
 #include "k2t_dense.cuh"
+#include "k2t_flash_tc.cuh"
 
 namespace k2t {
 namespace {
 
 constexpr uint32_t ROW_MAX = 256;
-constexpr float LOG2E = 1.4426950408889634f;
 
 template <typename T> __device__ __forceinline__ void put(T *p, float v);
 template <> __device__ __forceinline__ void put<float>(float *p, float v) { *p = v; }
@@ -292,167 +293,249 @@ __global__ void __launch_bounds__(RW_THREADS) window_row_kernel(const AttnParams
 }
 
 // ------------------------------------------------------------------------------------------------ prompts, bf16
-constexpr uint32_t FL_M = 128, FL_N = 64, FL_THREADS = 256;
-__host__ __device__ constexpr uint32_t fl_pitch(uint32_t d) { return d * 2 + 16; }          // bytes; the pad spreads eight rows over all banks
-__host__ __device__ constexpr uint32_t fl_smem(uint32_t d) { return fl_pitch(d) * (FL_M + 4 * FL_N); }
+constexpr uint32_t FL_M = 128, FL_LOADERS = 96, FL_THREADS = 128 + FL_LOADERS + 32, FL_HEADER = 1024, FL_TMEM = 512, FL_WAIT = 1u << 22;
+__host__ __device__ constexpr uint32_t fl_tile(uint32_t d) { return d <= 128 ? 128 : 64; }          // keys per tile
+__host__ __device__ constexpr uint32_t fl_panels(uint32_t d) { return (d + 63) / 64; }
+__host__ __device__ constexpr uint32_t fl_smem(uint32_t d) { return 1024 + FL_HEADER + fl_panels(d) * 128 * (FL_M + 4 * fl_tile(d)); }
 
 __device__ __forceinline__ void fl_cp16(uint32_t dst, const void *src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
-__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t &a, uint32_t &b, uint32_t &c, uint32_t &d) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "r"(addr) : "memory");
-}
-__device__ __forceinline__ void ldsm4t(uint32_t addr, uint32_t &a, uint32_t &b, uint32_t &c, uint32_t &d) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(a), "=r"(b), "=r"(c), "=r"(d) : "r"(addr) : "memory");
-}
-__device__ __forceinline__ void mma_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
+template <int N> __device__ __forceinline__ void fl_cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void fl_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 
-__device__ __forceinline__ float fl_exp2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
-
+// Bound by the softmax warps: per tile a warp issues about nine instructions per key of its row (scale and bias, mask, maximum,
+// exponent, sum, packing), 128 keys at about 1300 issue cycles, against 1050 cycles of the tensor cores for both products.  The rows
+// of the ring are row-major, so the tiles come in by 16-byte asynchronous copies of three warps, which put chunk c of row r
+// at c ^ (r & 7) of its panel (the 128-byte swizzle) and fence them for the tensor cores; eight warps leave a softmax
+// thread the registers for its 128 scores (nine: 168 registers and spills).  Keys per tile: 128, or 64 where the rows above
+// 128 elements would not leave room for two tiles of keys and values.  The grid deals the rows of all kv heads in descending
+// order of their contexts: a wave of 256 CTAs in ascending order left the longest to the end.
+// 2048 tokens, 16 heads of 128 over 4 kv heads: 139 us with mma.sync and 64-key tiles, about 45 now (380 TFLOP/s of causal
+// work); a prompt of 12 blocks 5281 -> 4720 us, 300 tokens of 4 blocks 737 -> 648, 2 tokens behind 1000 positions 235 -> 207.
+// Warps 0 .. 3: queries, softmax and output, one row per thread; warps 4 .. 6: key and value tiles; warp 7: tensor-core issue.
+// Tensor memory: S of even and odd tiles (KT columns each, the softmax weights overwrite them as bf16 pairs), then O.
 template <int D>
-__global__ void __launch_bounds__(FL_THREADS) window_flash_kernel(const AttnParams p) {
-    extern __shared__ __align__(16) uint8_t sm8[];
+__global__ void __launch_bounds__(FL_THREADS, 1) window_flash_kernel(const AttnParams p) {
+    constexpr uint32_t KT = fl_tile(D), PD = fl_panels(D), CH = D / 8, Q_BYTES = PD * FL_M * 128, T_BYTES = PD * KT * 128;
+    extern __shared__ uint8_t smem_raw[];
     const WindowAttnArgs &a = p.a;
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = blockIdx.y, group = a.n_q / a.n_kv;
-    const uint32_t rows = p.n_tok * group, r0 = blockIdx.x * FL_M;
-    constexpr uint32_t P = fl_pitch(D), CH = D / 8;
-    const uint32_t s_q = (uint32_t)__cvta_generic_to_shared(sm8), s_kv = s_q + FL_M * P;       // K0 | V0 | K1 | V1
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = blockIdx.x, group = a.n_q / a.n_kv;
+    const uint32_t rows = p.n_tok * group, r0 = (gridDim.y - 1 - blockIdx.y) * FL_M;          // the longest rows first, of all heads
+    const uint32_t raw = (uint32_t)__cvta_generic_to_shared(smem_raw), sbase = (raw + 1023u) & ~1023u;
+    uint8_t *smem = smem_raw + (sbase - raw);
+    const uint32_t s_q = sbase + FL_HEADER, s_k = s_q + Q_BYTES, s_v = s_k + 2 * T_BYTES;
+    // barriers: queries, keys landed / free, values landed / free, S ready, weights ready, O updated, end
+    const uint32_t b_q = sbase, b_kf = sbase + 8, b_ke = sbase + 24, b_vf = sbase + 40, b_ve = sbase + 56, b_s = sbase + 72, b_p = sbase + 88, b_o = sbase + 104, b_end = sbase + 112;
+    volatile uint32_t *s_tmem = reinterpret_cast<volatile uint32_t *>(smem + 256), *s_abort = reinterpret_cast<volatile uint32_t *>(smem + 260);
+    if (tid == 0) {
+        mbar_init(b_q, 128);
+        for (uint32_t i = 0; i < 2; ++i) {
+            mbar_init(b_kf + 8 * i, FL_LOADERS); mbar_init(b_ke + 8 * i, 1); mbar_init(b_vf + 8 * i, FL_LOADERS); mbar_init(b_ve + 8 * i, 1);
+            mbar_init(b_s + 8 * i, 1); mbar_init(b_p + 8 * i, 128);
+        }
+        mbar_init(b_o, 1);
+        mbar_init(b_end, 1);
+        *s_abort = 0;
+        fence_mbar_init();
+    }
+    if (warp == 7) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + 256), "r"(FL_TMEM) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *s_tmem, t_o = tmem + 2 * KT;
     pdl_wait();
     pdl_trigger();
     const uint32_t pos0 = __ldcg(a.pos), r_last = min(rows, r0 + FL_M) - 1;
     const uint32_t p_first = pos0 + r0 / group, p_last = pos0 + r_last / group;
-    const uint32_t lo = p_first + 1 - a.ring.active_len(p_first + 1);
-    const __nv_bfloat16 *kc = static_cast<const __nv_bfloat16 *>(a.k_cache) + (size_t)g * p.ring_rows * D, *vc = static_cast<const __nv_bfloat16 *>(a.v_cache) + (size_t)g * p.ring_rows * D;
-    for (uint32_t i = tid; i < FL_M * CH; i += FL_THREADS) {
-        const uint32_t r = min(r0 + i / CH, rows - 1), c = i % CH;
-        fl_cp16(s_q + (i / CH) * P + c * 16, static_cast<const __nv_bfloat16 *>(a.q) + ((size_t)(r / group) * a.n_q + g * group + r % group) * D + c * 8);
-    }
-    auto fetch = [&](uint32_t j0, uint32_t buf) {           // positions beyond the last are clamped (masked below, rows finite)
-        for (uint32_t i = tid; i < FL_N * CH; i += FL_THREADS) {
-            const uint32_t c = i % CH, slot = a.ring.slot_of_pos(min(j0 + i / CH, p_last));
-            const uint32_t dst = s_kv + buf * 2 * FL_N * P + (i / CH) * P + c * 16;
-            fl_cp16(dst, kc + (size_t)slot * D + c * 8);
-            fl_cp16(dst + FL_N * P, vc + (size_t)slot * D + c * 8);
-        }
-    };
-    fetch(lo, 0);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    // the two query rows of this thread
-    uint32_t qpos[2];
-    float sc[2], sl[2], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f};
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const uint32_t r = min(r0 + warp * 16 + (lane >> 2) + 8 * i, rows - 1);
-        qpos[i] = pos0 + r / group;
-        sc[i] = __ldg(a.head_scale + g * group + r % group) * LOG2E;
-        sl[i] = __ldg(a.head_slope + g * group + r % group) * LOG2E;
-    }
-    const uint32_t window = a.ring.window ? a.ring.window : 0x7fffffffu;
-    // positions some row of this warp can see
-    const uint32_t w_first = pos0 + min(r0 + warp * 16, rows - 1) / group, w_last = pos0 + min(r0 + warp * 16 + 15, rows - 1) / group;
-    const uint32_t w_lo = w_first + 1 - a.ring.active_len(w_first + 1);
-    float o[D / 8][4];
-#pragma unroll
-    for (int i = 0; i < D / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
-    uint32_t buf = 0;
-    for (uint32_t j0 = lo; j0 <= p_last; j0 += FL_N, buf ^= 1) {
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();                                     // the tile has landed; everyone is done with the other buffer
-        if (j0 + FL_N <= p_last) fetch(j0 + FL_N, buf ^ 1);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        if (j0 > w_last || j0 + FL_N <= w_lo) continue;
-        const uint32_t s_k = s_kv + buf * 2 * FL_N * P, s_v = s_k + FL_N * P;
-        float s[FL_N / 8][4];
-#pragma unroll
-        for (int i = 0; i < (int)FL_N / 8; ++i) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.0f;
-#pragma unroll
-        for (uint32_t k = 0; k < D / 16; ++k) {
-            uint32_t a0, a1, a2, a3;
-            ldsm4(s_q + (warp * 16 + (lane & 15u)) * P + k * 32 + (lane >> 4) * 16, a0, a1, a2, a3);
-#pragma unroll
-            for (uint32_t n = 0; n < FL_N / 16; ++n) {
-                uint32_t b0, b1, b2, b3;       // keys n*16 .. +7 (k halves b0, b1), +8 .. +15 (b2, b3)
-                ldsm4(s_k + (n * 16 + (lane & 7u) + ((lane >> 4) << 3)) * P + k * 32 + ((lane >> 3) & 1u) * 16, b0, b1, b2, b3);
-                mma_bf16(s[2 * n], a0, a1, a2, a3, b0, b1);
-                mma_bf16(s[2 * n + 1], a0, a1, a2, a3, b2, b3);
+    const uint32_t lo = p_first + 1 - a.ring.active_len(p_first + 1), n_tiles = (p_last - lo) / KT + 1;
+
+    if (warp >= 4 && warp < 7) {
+        const uint32_t lt = tid - 128;
+        const __nv_bfloat16 *kc = static_cast<const __nv_bfloat16 *>(a.k_cache) + (size_t)g * p.ring_rows * D, *vc = static_cast<const __nv_bfloat16 *>(a.v_cache) + (size_t)g * p.ring_rows * D;
+        // one tile of rows into the panels; positions beyond the last are clamped to it (masked below, rows finite)
+        auto fetch = [&](const __nv_bfloat16 *src, uint32_t dst, uint32_t j) {
+            const uint32_t j0 = lo + j * KT, slot0 = a.ring.slot_of_pos(j0), last = p_last - j0;
+#pragma unroll 4
+            for (uint32_t i = lt; i < KT * CH; i += FL_LOADERS) {
+                const uint32_t r = i / CH, c = i % CH;
+                uint32_t slot = slot0 + min(r, last);
+                if (slot >= p.ring_rows) slot -= p.ring_rows;
+                fl_cp16(dst + (c >> 3) * (KT * 128) + r * 128 + (((c & 7u) ^ (r & 7u)) << 4), src + (size_t)slot * D + c * 8);
             }
-        }
-        float mx[2] = {-INFINITY, -INFINITY};
-        // bias of the tile's first key of this thread, the others follow in exact steps (small integers times the slope)
-        const float f0[2] = {(float)(int)(j0 + (lane & 3u) * 2 - qpos[0]), (float)(int)(j0 + (lane & 3u) * 2 - qpos[1])};
-#pragma unroll
-        for (uint32_t n = 0; n < FL_N / 8; ++n)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const uint32_t i = e >> 1;
-                s[n][e] = __fmaf_rn(s[n][e], sc[i], sl[i] * (f0[i] + (float)(n * 8 + (e & 1))));
+            fl_cp_commit();
+        };
+        // Every thread waits for its own copies, makes them visible to the tensor cores and announces them.  The keys of a tile are
+        // announced as soon as they have landed, its values once the keys of the next tile have been requested.
+        bool ok = true;
+        for (uint32_t j = 0; j < n_tiles; ++j) {
+            const uint32_t b = j & 1u;
+            if (j >= 2) ok = mbar_wait_warp(b_ke + 8 * b, ((j >> 1) - 1u) & 1u, FL_WAIT, s_abort);
+            if (!ok) break;
+            fetch(kc, s_k + b * T_BYTES, j);
+            if (j >= 1) {
+                fl_cp_wait<1>();
+                fence_proxy_async();
+                mbar_arrive(b_vf + 8 * (b ^ 1u));
             }
-        if (j0 + FL_N - 1 > w_first || w_last >= j0 + window) {            // some key of the tile is out of some row's sight
+            fl_cp_wait<0>();
+            fence_proxy_async();
+            mbar_arrive(b_kf + 8 * b);
+            if (j >= 2) ok = mbar_wait_warp(b_ve + 8 * b, ((j >> 1) - 1u) & 1u, FL_WAIT, s_abort);
+            if (!ok) break;
+            fetch(vc, s_v + b * T_BYTES, j);
+        }
+        fl_cp_wait<0>();                       // also after a wait that gave up: the copies land before the CTA leaves
+        fence_proxy_async();
+        if (ok) mbar_arrive(b_vf + 8 * ((n_tiles - 1) & 1u));
+        else if (lane == 0 && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
+    } else if (warp == 7) {
+        if (lane == 0) {
+            // fp32 accumulators, bf16 operands; A and B K-major for S, B with its columns consecutive for O
+            constexpr uint32_t id_s = (1u << 4) | (1u << 7) | (1u << 10) | ((KT >> 3) << 17) | ((FL_M >> 4) << 24);
+            constexpr uint32_t id_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((D >> 3) << 17) | ((FL_M >> 4) << 24);
+            auto scores = [&](uint32_t j) {
+                const uint32_t b = j & 1u, kb = s_k + b * T_BYTES;
+                if (!mbar_wait_thread(b_kf + 8 * b, (j >> 1) & 1u, FL_WAIT, s_abort)) return false;
+                tc_fence_after();
 #pragma unroll
-            for (uint32_t n = 0; n < FL_N / 8; ++n)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const uint32_t i = e >> 1, j = j0 + n * 8 + (lane & 3u) * 2 + (e & 1);
-                    if (j > qpos[i] || qpos[i] - j >= window) s[n][e] = -INFINITY;
+                for (uint32_t i = 0; i < D / 16; ++i)
+                    mma_ss(tmem + b * KT, desc_k(s_q + (i / 4) * FL_M * 128 + (i % 4) * 32), desc_k(kb + (i / 4) * KT * 128 + (i % 4) * 32), id_s, i != 0 ? 1u : 0u);
+                tc_commit(b_s + 8 * b);
+                tc_commit(b_ke + 8 * b);
+                return true;
+            };
+            bool ok = mbar_wait_thread(b_q, 0, FL_WAIT, s_abort) && scores(0);
+            for (uint32_t j = 0; j < n_tiles && ok; ++j) {
+                const uint32_t b = j & 1u;
+                if (j + 1 < n_tiles) {
+                    if (j >= 1) ok = mbar_wait_thread(b_o, (j - 1) & 1u, FL_WAIT, s_abort);      // the weights of tile j - 1 lie where S of tile j + 1 goes
+                    ok = ok && scores(j + 1);
+                    if (!ok) break;
                 }
-        }
+                ok = mbar_wait_thread(b_p + 8 * b, (j >> 1) & 1u, FL_WAIT, s_abort) && mbar_wait_thread(b_vf + 8 * b, (j >> 1) & 1u, FL_WAIT, s_abort);
+                if (!ok) break;
+                tc_fence_after();
 #pragma unroll
-        for (uint32_t n = 0; n < FL_N / 8; ++n)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) mx[e >> 1] = fmaxf(mx[e >> 1], s[n][e]);
-        float al[2];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 1));
-            mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 2));
-            const float m_new = fmaxf(m[i], mx[i]);
-            al[i] = m_new == -INFINITY ? 1.0f : fl_exp2(m[i] - m_new);
-            m[i] = m_new;
-            l[i] *= al[i];
-        }
-        const float mm[2] = {m[0] == -INFINITY ? 0.0f : m[0], m[1] == -INFINITY ? 0.0f : m[1]};        // a row that has seen nothing yet: exp2(-inf) = 0
-#pragma unroll
-        for (uint32_t n = 0; n < FL_N / 8; ++n)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float v = fl_exp2(s[n][e] - mm[e >> 1]);
-                s[n][e] = v;
-                l[e >> 1] += v;
+                for (uint32_t k = 0; k < KT / 16; ++k)
+                    mma_ts(t_o, tmem + b * KT + k * 8, desc_mn(s_v + b * T_BYTES + k * 16 * 128, KT * 128), id_o, (j | k) != 0 ? 1u : 0u);
+                tc_commit(b_ve + 8 * b);
+                tc_commit(b_o);
             }
+            tc_commit(b_end);                 // also after a wait that gave up: completes when the issued products have
+            if (!ok && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
+            for (uint32_t spin = 0; spin < FL_WAIT && !mbar_try_wait(b_end, 0u); ++spin) {}
+        }
+    } else {
+        for (uint32_t i = tid; i < FL_M * CH; i += 128) {          // rows beyond the last repeat it
+            const uint32_t r = i / CH, c = i % CH, rr = min(r0 + r, rows - 1);
+            fl_cp16(s_q + (c >> 3) * (FL_M * 128) + r * 128 + (((c & 7u) ^ (r & 7u)) << 4), static_cast<const __nv_bfloat16 *>(a.q) + ((size_t)(rr / group) * a.n_q + g * group + rr % group) * D + c * 8);
+        }
+        fl_cp_commit();
+        const uint32_t r = r0 + tid, rr = min(r, rows - 1), t = rr / group, head = g * group + rr % group, qpos = pos0 + t, lanes = (warp * 32u) << 16;
+        const uint32_t w_first = pos0 + min(r0 + warp * 32, rows - 1) / group, w_last = pos0 + min(r0 + warp * 32 + 31, rows - 1) / group;
+        const uint32_t window = a.ring.window ? min(a.ring.window, 0x3fffffffu) : 0x3fffffffu;
+        const float sc = __ldg(a.head_scale + head) * LOG2E, sl = __ldg(a.head_slope + head) * LOG2E;
+        fl_cp_wait<0>();
+        fence_proxy_async();
+        mbar_arrive(b_q);
+        float m = -INFINITY, l = 0.0f;         // maximum the weights are taken against, and their sum
+        bool ok = true;
+        for (uint32_t j = 0; j < n_tiles; ++j) {
+            const uint32_t b = j & 1u, t_s = tmem + b * KT + lanes, j0 = lo + j * KT;
+            ok = mbar_wait_warp(b_s + 8 * b, (j >> 1) & 1u, FL_WAIT, s_abort);
+            if (!ok) break;
+            tc_fence_after();
+            uint32_t v[KT];
 #pragma unroll
-        for (int i = 0; i < D / 8; ++i) { o[i][0] *= al[0]; o[i][1] *= al[0]; o[i][2] *= al[1]; o[i][3] *= al[1]; }
+            for (int c = 0; c < (int)KT; c += 32) tm_ld32(t_s + c, v + c);
+            tm_ld_wait();
+            // bias of the tile's first key, the others follow in exact steps (small integers times the slope)
+            const int rel = (int)(qpos - j0);
+            const float f0 = (float)-rel;
 #pragma unroll
-        for (uint32_t k = 0; k < FL_N / 16; ++k) {
-            const uint32_t a0 = pack_bf16(s[2 * k][0], s[2 * k][1]), a1 = pack_bf16(s[2 * k][2], s[2 * k][3]), a2 = pack_bf16(s[2 * k + 1][0], s[2 * k + 1][1]),
-                           a3 = pack_bf16(s[2 * k + 1][2], s[2 * k + 1][3]);
+            for (int c = 0; c < (int)KT; ++c) v[c] = __float_as_uint(__fmaf_rn(__uint_as_float(v[c]), sc, sl * (f0 + (float)c)));
+            if (j0 + KT - 1 > w_first || w_last >= j0 + window) {            // some key of the tile is out of some row's sight
+                const int from = rel - (int)window;
 #pragma unroll
-            for (uint32_t d = 0; d < D / 16; ++d) {
-                uint32_t b0, b1, b2, b3;
-                ldsm4t(s_v + (k * 16 + (lane & 15u)) * P + d * 32 + (lane >> 4) * 16, b0, b1, b2, b3);
-                mma_bf16(o[2 * d], a0, a1, a2, a3, b0, b1);
-                mma_bf16(o[2 * d + 1], a0, a1, a2, a3, b2, b3);
+                for (int c = 0; c < (int)KT; ++c)
+                    if (c > rel || c <= from) v[c] = 0xff800000u;
             }
+            float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+            for (int c = 0; c < (int)KT; ++c) mx[c & 3] = fmaxf(mx[c & 3], __uint_as_float(v[c]));
+            const float m_new = fmaxf(m, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])));
+            if (j == 0) {
+                m = m_new;
+            } else if (__any_sync(0xffffffffu, m_new > m + 8.0f)) {
+                ok = mbar_wait_warp(b_o, (j - 1) & 1u, FL_WAIT, s_abort);
+                if (!ok) break;
+                tc_fence_after();
+                const float al = m_new == -INFINITY ? 1.0f : exp2_approx(m - m_new);
+#pragma unroll 1
+                for (uint32_t c = 0; c < D; c += 16) {
+                    uint32_t o[16];
+                    tm_ld16(t_o + lanes + c, o);
+                    tm_ld_wait();
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * al);
+                    tm_st16(t_o + lanes + c, o);
+                }
+                l *= al;
+                m = m_new;
+            }
+            const float mm = m == -INFINITY ? 0.0f : m;          // a row that has seen nothing yet: exp2(-inf) = 0
+            float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+            for (int c = 0; c < (int)KT; c += 2) {
+                const float x = exp2_approx(__uint_as_float(v[c]) - mm), y = exp2_approx(__uint_as_float(v[c + 1]) - mm);
+                sum[(c >> 1) & 3] += x + y;
+                v[c >> 1] = pack_bf16(x, y);
+            }
+            l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+#pragma unroll
+            for (int c = 0; c < (int)KT / 2; c += 32) tm_st32(t_s + c, v + c);
+            tm_st_wait();
+            tc_fence_before();
+            mbar_arrive(b_p + 8 * b);
+        }
+        // the last update by a barrier of its own: the phases of b_o may still be two behind here, and a parity tells only neighbours apart
+        if (ok) ok = __all_sync(0xffffffffu, mbar_wait_thread(b_end, 0u, FL_WAIT, s_abort) && *s_abort == 0);
+        tc_fence_after();
+        if (ok) {
+            const float inv = 1.0f / l;
+#pragma unroll 1
+            for (uint32_t c = 0; c < D; c += 16) {
+                uint32_t o[16];
+                tm_ld16(t_o + lanes + c, o);
+                tm_ld_wait();
+                if (r < rows) {
+                    float f[16];
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) f[i] = __uint_as_float(o[i]) * inv;
+                    const uint32_t k = head * a.vdim + c;
+                    if (c + 16 <= a.vdim && (k & 7u) == 0) {
+#pragma unroll
+                        for (int i = 0; i < 16; i += 8)
+                            *reinterpret_cast<uint4 *>(static_cast<__nv_bfloat16 *>(a.out.p) + panel_index(a.out.ld, t, k + i)) =
+                                make_uint4(pack_bf16(f[i], f[i + 1]), pack_bf16(f[i + 2], f[i + 3]), pack_bf16(f[i + 4], f[i + 5]), pack_bf16(f[i + 6], f[i + 7]));
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i)
+                            if (c + i < a.vdim) act_store<false>(a.out, t, k + i, f[i]);
+                    }
+                }
+            }
+        } else if (lane == 0 && a.err_flag != nullptr) {
+            atomicExch(a.err_flag, 1u);
         }
     }
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        l[i] += __shfl_xor_sync(0xffffffffu, l[i], 1);
-        l[i] += __shfl_xor_sync(0xffffffffu, l[i], 2);
-        const uint32_t r = r0 + warp * 16 + (lane >> 2) + 8 * i;
-        if (r >= rows) continue;
-        const float inv = 1.0f / l[i];
-        const uint32_t t = r / group, base = (g * group + r % group) * a.vdim;
-#pragma unroll
-        for (int d = 0; d < D / 8; ++d) {
-            const uint32_t k = d * 8 + (lane & 3u) * 2;
-            if (k + 1 < a.vdim && (base & 1u) == 0)
-                *reinterpret_cast<uint32_t *>(static_cast<__nv_bfloat16 *>(a.out.p) + panel_index(a.out.ld, t, base + k)) = pack_bf16(o[d][2 * i] * inv, o[d][2 * i + 1] * inv);
-            else {
-                if (k < a.vdim) act_store<false>(a.out, t, base + k, o[d][2 * i] * inv);
-                if (k + 1 < a.vdim) act_store<false>(a.out, t, base + k + 1, o[d][2 * i + 1] * inv);
-            }
-        }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 7) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(FL_TMEM) : "memory");
     }
 }
 
@@ -482,7 +565,7 @@ cudaError_t flash_launch(cudaStream_t s, const AttnParams &p, bool pdl) {
     const uint32_t rows = p.n_tok * (p.a.n_q / p.a.n_kv);
     cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(window_flash_kernel<D>), fl_smem(D));
     if (e != cudaSuccess) return e;
-    return launch_kernel(window_flash_kernel<D>, dim3((rows + FL_M - 1) / FL_M, p.a.n_kv), dim3(FL_THREADS), fl_smem(D), s, pdl, p);
+    return launch_kernel(window_flash_kernel<D>, dim3(p.a.n_kv, (rows + FL_M - 1) / FL_M), dim3(FL_THREADS), fl_smem(D), s, pdl, p);
 }
 
 }  // namespace

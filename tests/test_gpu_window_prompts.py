@@ -1,0 +1,61 @@
+"""Window attention of prompt batches with bf16 rows, at the edges of its tiles: 128 rows (token, head of the group) of a key/value
+head, 128 or (heads above 128) 64 keys.  Every head size has its own kernel; groups that do not divide 128 leave tiles that end
+inside a token; windows narrower than the tokens of a tile leave rows whose keys begin after the first tile."""
+import numpy as np
+import pytest
+
+import folizen_models as fm
+import folizen_ref as ref
+
+pytestmark = pytest.mark.gpu
+TOL = 5e-2          # bf16 engine against the restatement in 64 bits, as for the other bf16 prompts of this design
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    import kronos_2t_b200 as k2
+    c = k2.Context(0)
+    yield c
+    c.close()
+
+
+def limit(eng, toks, want):
+    """Where a position's logits hang on the rounding alone, the bound is three times what decoding token by token gives there: it
+    rounds keys and values to bf16, a prompt rounds queries and softmax weights as well (worst case of the list: position 76 of
+    the 192 / 130 heads, 0.024 token by token and 0.053 as a prompt, by tensor-memory products and by mma.sync alike)."""
+    one = np.stack([eng.forward_token_ids([t], pos_start=i) for i, t in enumerate(toks)])
+    return np.maximum(TOL, 3 * fm.error(one, want))
+
+
+def check(ctx, folder, model, toks, cuts, max_seq, want):
+    from kronos_2t_b200 import models
+    eng = models.load_engine(ctx, fm.write(model, folder), "bfloat16", max_seq)
+    try:
+        out, at = [], 0
+        for n in cuts:
+            out.append(eng.forward_token_ids(toks[at:at + n], pos_start=at, want_all=True))
+            at += n
+        err = fm.error(np.concatenate(out), want)
+        assert (err < (limit(eng, toks, want) if err.max() >= TOL else TOL)).all(), (err.max(), err.argmax())
+    finally:
+        eng.close()
+
+
+# heads, kv heads, dim, vdim, window, tokens of the batches
+@pytest.mark.parametrize("heads,kv,dim,vdim,window,cuts", [
+    (4, 1, 32, 32, 4096, [2]), (4, 1, 64, 64, 4096, [32]), (4, 1, 64, 64, 4096, [33, 95]), (3, 1, 96, 80, 4096, [129, 42]), (8, 2, 128, 128, 4096, [255, 2, 128]),
+    (8, 2, 128, 120, 40, [200, 131]), (2, 2, 128, 128, 17, [128, 129]), (5, 1, 192, 192, 100, [27, 150]), (2, 2, 192, 130, 4096, [64, 65]), (1, 1, 256, 256, 4096, [127, 64]),
+    (2, 2, 256, 250, 9, [128, 130]), (6, 2, 32, 20, 70, [300, 86])])
+def test_tiles_of_a_prompt(ctx, tmp_path, heads, kv, dim, vdim, window, cuts):
+    model = fm.make(96, 61, [fm.attention(heads, kv, dim, vdim, window, ff=64), fm.attention(heads, kv, dim, vdim, window)], seed=dim + window)
+    toks = np.random.default_rng(len(cuts)).integers(0, 61, sum(cuts))
+    check(ctx, str(tmp_path / "m"), model, toks, cuts, sum(cuts) + 8, ref.forward(model, toks)[0])
+
+
+def test_rows_of_many_tiles(ctx, tmp_path):
+    """16 tiles of keys, a window that ends inside one, and a batch that begins in the middle: the same rows whole and in portions."""
+    model = fm.make(96, 61, [fm.attention(4, 2, 128, 128, 900, ff=64), fm.attention(4, 2, 128, 128, 4096)], seed=5)
+    toks = np.random.default_rng(3).integers(0, 61, 2000)
+    want = ref.forward(model, toks)[0]
+    for k, cuts in enumerate(([2000], [1000, 1000], [700, 65, 1235])):
+        check(ctx, str(tmp_path / f"m{k}"), model, toks, cuts, 2048, want)
