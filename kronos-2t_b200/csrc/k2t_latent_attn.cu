@@ -531,6 +531,8 @@ struct FlashParams {
     uint32_t n_tok, pd, pr, pv, vn, tmem;
 };
 
+// The grid deals the 128-token rows of ALL heads in descending order of their contexts (heads innermost): with the rows innermost
+// the last heads' longest CTAs began when the others were done.  2048 tokens, 4 blocks of 16 heads: 1966 -> 1918 us per prompt.
 // Warps 0 .. 3: softmax, one row (token) per thread; warp 4: bulk copies; warp 5: tensor-core issue.
 // Tensor memory: S of even and odd tiles (KT columns each, the softmax weights overwrite them as bf16 pairs), then O.
 template <int KT>
@@ -538,7 +540,7 @@ __global__ void __launch_bounds__(FL_THREADS, 1) latent_flash_kernel(const Flash
     extern __shared__ uint8_t smem_raw[];
     const LatentAttnArgs &a = p.a;
     const LatentShape &d = a.d;
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y, t0 = (gridDim.x - 1 - blockIdx.x) * FL_M;      // longest rows first
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.x, t0 = (gridDim.y - 1 - blockIdx.y) * FL_M;      // longest rows first, of all heads
     const uint32_t raw = (uint32_t)__cvta_generic_to_shared(smem_raw), sbase = (raw + 1023u) & ~1023u;
     uint8_t *smem = smem_raw + (sbase - raw);
     const uint32_t pq = p.pd + p.pr, k_bytes = pq * KT * 128, v_bytes = p.pv * KT * 128;
@@ -763,7 +765,7 @@ template <int RB> cudaError_t split_launch(cudaStream_t s, const SplitParams &p,
 template <int KT> cudaError_t flash_launch(cudaStream_t s, const FlashParams &p, size_t smem, bool pdl) {
     cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(latent_flash_kernel<KT>), smem);
     if (e != cudaSuccess) return e;
-    return launch_kernel(latent_flash_kernel<KT>, dim3((p.n_tok + FL_M - 1) / FL_M, p.a.d.heads), dim3(FL_THREADS), smem, s, pdl, p);
+    return launch_kernel(latent_flash_kernel<KT>, dim3(p.a.d.heads, (p.n_tok + FL_M - 1) / FL_M), dim3(FL_THREADS), smem, s, pdl, p);
 }
 
 }  // namespace
