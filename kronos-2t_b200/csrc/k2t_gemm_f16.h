@@ -47,9 +47,11 @@ cudaError_t launch_expert_tiles(cudaStream_t stream, const uint32_t *route_ids, 
 // of one expert and the cost of its decode.  Measured with 2048 columns, 2 layers: tokens at which tiles (first) and GEMVs take the same, by
 // experts / routes / width / bits: 128 / 8 / 768 / 3 60 (56: 953 and 909 us, 64: 962 and 1040), 4 39, 5 15; 64 / 6 / 768 / 3 47, 4 30, 5 and 2 fewer
 // than 16; 64 / 6 / 1408 / 3 54; 16 / 4 / 2816 / 3 20, 4 14; 8 / 2 / 4096 / 4 18; 4 / 2 / 2048 / 3 22; 256 / 8 / 768 / 2 fewer than 8.
+// Those lines are of tiles expanded into shared memory; in tensor memory (k2t_gemm_prompt.cu) a tile takes 0.72 to 0.78 of that, so at
+// the lines tiles are by now the faster form.
 bool experts_grouped(uint32_t n_tok, uint32_t n_pair, uint32_t n_experts, uint32_t hidden, uint32_t d_ff, uint32_t bits);
 
-// The expert projections of all pairs of `t`, an expert's weights expanded once per 32 pairs; out = [n_pair][rows].  Same bits as
+// (k2t_gemm_prompt.cu) The expert projections of all pairs of `t`, an expert's weights expanded once per 32 pairs; out = [n_pair][rows].  Same bits as
 // launch_gemv_experts, for activations in the form the library's own quantizers leave them.
 cudaError_t launch_gemm_experts(cudaStream_t stream, const DeviceMatrix &m0, int fmt, const ExpertCodebook *books, const uint8_t *const *bases, uint32_t n_experts,
                                 const ExpertTiles &t, uint32_t n_pair, uint32_t act_group, const int8_t *xq, const float *xs, float *out, int sm_count, uint32_t *err_flag, bool pdl);

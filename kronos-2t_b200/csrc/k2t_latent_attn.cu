@@ -532,7 +532,8 @@ struct FlashParams {
 };
 
 // The grid deals the 128-token rows of ALL heads in descending order of their contexts (heads innermost): with the rows innermost
-// the last heads' longest CTAs began when the others were done.  2048 tokens, 4 blocks of 16 heads: 1966 -> 1918 us per prompt.
+// the last heads' longest CTAs began when the others were done.  2048 tokens, 16 heads: 56 -> 36.7 us; a
+// prompt of 4 blocks 1966 -> 1918 us.
 // Warps 0 .. 3: softmax, one row (token) per thread; warp 4: bulk copies; warp 5: tensor-core issue.
 // Tensor memory: S of even and odd tiles (KT columns each, the softmax weights overwrite them as bf16 pairs), then O.
 template <int KT>

@@ -302,14 +302,16 @@ __device__ __forceinline__ void fl_cp16(uint32_t dst, const void *src) { asm vol
 template <int N> __device__ __forceinline__ void fl_cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void fl_cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 
-// Bound by the softmax warps: per tile a warp issues about nine instructions per key of its row (scale and bias, mask, maximum,
-// exponent, sum, packing), 128 keys at about 1300 issue cycles, against 1050 cycles of the tensor cores for both products.  The rows
-// of the ring are row-major, so the tiles come in by 16-byte asynchronous copies of three warps, which put chunk c of row r
-// at c ^ (r & 7) of its panel (the 128-byte swizzle) and fence them for the tensor cores; eight warps leave a softmax
-// thread the registers for its 128 scores (nine: 168 registers and spills).  Keys per tile: 128, or 64 where the rows above
+// A tile of 128 keys takes a CTA about 5000 cycles: 1050 are the tensor cores' for both products, about 1300 the issue slots of a
+// softmax warp (nine instructions per key of a row).  Two softmax warps per row, half of the keys each, changed nothing (a prompt
+// 4723 us against 4720), so what is left is the fetch of 64 KB of keys and values per tile and the hand-offs between the roles;
+// 256 rows per CTA over the same tiles would halve that fetch.  A value row that is not finite reaches, as 0 x inf, rows of its
+// tile that do not see it.  The rows of the ring are row-major, so the tiles come in by
+// 16-byte asynchronous copies of three warps, which put chunk c of row r at c ^ (r & 7) of its panel (the 128-byte swizzle) and
+// fence them for the tensor cores; eight warps leave a softmax thread the registers for its 128 scores (nine: 168 and spills).  Keys per tile: 128, or 64 where the rows above
 // 128 elements would not leave room for two tiles of keys and values.  The grid deals the rows of all kv heads in descending
 // order of their contexts: a wave of 256 CTAs in ascending order left the longest to the end.
-// 2048 tokens, 16 heads of 128 over 4 kv heads: 139 us with mma.sync and 64-key tiles, about 45 now (380 TFLOP/s of causal
+// 2048 tokens, 16 heads of 128 over 4 kv heads: 139 us with mma.sync and 64-key tiles, 45.5 now (378 TFLOP/s of causal
 // work); a prompt of 12 blocks 5281 -> 4720 us, 300 tokens of 4 blocks 737 -> 648, 2 tokens behind 1000 positions 235 -> 207.
 // Warps 0 .. 3: queries, softmax and output, one row per thread; warps 4 .. 6: key and value tiles; warp 7: tensor-core issue.
 // Tensor memory: S of even and odd tiles (KT columns each, the softmax weights overwrite them as bf16 pairs), then O.
