@@ -81,7 +81,7 @@ struct DeltaArgs {
     uint32_t *err_flag;
 };
 uint32_t delta_row(uint32_t dim);      // dim rounded up to 64; 0 = larger than the kernels support
-size_t delta_record_floats(uint32_t n_tok, uint32_t heads, uint32_t drow, float decay_scale);
+size_t delta_record_floats(uint32_t n_tok, uint32_t heads, uint32_t drow);
 bool delta_step_fits(const DeltaArgs &a);
 cudaError_t launch_delta_step(cudaStream_t s, bool f32, const DeltaArgs &a, bool pdl);                                   // one token, one launch
 cudaError_t launch_delta_tanh(cudaStream_t s, bool f32, const DeltaArgs &a, const Act &out, uint32_t n_tok, bool pdl);   // activation of the decay product

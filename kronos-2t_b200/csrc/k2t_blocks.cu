@@ -498,7 +498,7 @@ extern "C" KronosCudaEngine *kronos_cuda_engine_create_blocks(KronosCudaContext 
             z_cols = std::max(z_cols, rows);
             s_cols = std::max(s_cols, B.rank);
             logit_cols = std::max(logit_cols, hd);
-            rec_floats = std::max(rec_floats, delta_record_floats(MB, B.heads, B.row, B.decay_scale));
+            rec_floats = std::max(rec_floats, delta_record_floats(MB, B.heads, B.row));
             o_floats = std::max(o_floats, (size_t)B.heads * B.row);
         } else if (d.mixer == KRONOS_CUDA_MIXER_LATENT_ATTENTION) {
             if (B.vdim == 0 || d.q_rank == 0 || d.kv_rank == 0 || d.rot_dim == 0 || d.rot_dim % 2) return bad(at + "latent attention: a size is 0, or rot_dim is odd");

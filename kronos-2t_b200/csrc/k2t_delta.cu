@@ -5,10 +5,10 @@
 //   * delta_step_kernel (one token): a cluster per head.  The state is requested before the dependency wait (only the same
 //     layer's previous step wrote it), then coefficients, recurrence, per-head norm, output gate and the activation of the output
 //     projection in one launch.
-//   * prompts: delta_chunk_kernel turns sixteen tokens of a head into one record of coefficients, delta_scan_kernel walks the records -
-//     a CTA holds sixteen columns of a head's state - and delta_post_kernel norms and gates.
+//   * prompts: delta_prep_kernel writes the coefficients of every head and group of four tokens as one record,
+//     delta_scan_kernel walks the groups - a warp holds two or four columns, its lanes share the keys - with the records streamed through
+//     a ring of bulk copies and packed fp32 pairs (fma.rn.f32x2), delta_post_kernel norms and gates.
 #include <algorithm>
-#include <cmath>
 
 #include "k2t_block_kernels.h"
 #include "k2t_dense.cuh"
@@ -20,6 +20,11 @@ __device__ __forceinline__ float sigmoidf(float x) { return 1.0f / (1.0f + expf(
 // Decays are kept as w - 1: a channel that decays by a hair per token would lose that hair in the rounding of w, the same way
 // at every token, and a state carried over thousands of tokens would show it.
 __device__ __forceinline__ float decay_minus_one(float scale, float logit) { return expm1f(-scale * sigmoidf(logit)); }
+
+// ---- packed fp32 pairs
+__device__ __forceinline__ uint64_t pk(float a, float b) { uint64_t r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ void upk(uint64_t v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) { uint64_t r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
 
 // ------------------------------------------------------------------------------------------------ one token
 // A cluster of drow / 32 CTAs per head, CTA = 32 columns: thread = (four columns, KPS = drow / 32 keys).  Every CTA makes the
@@ -146,299 +151,241 @@ __global__ void __launch_bounds__(256) delta_tanh_kernel(const float *__restrict
     act_store<F32>(out, i / rank, i % rank, tanhf(__ldcg(in + (i / rank) * in_stride + i % rank)));
 }
 
-// Prompts run in chunks of sixteen tokens, each a step of matrix products.  With S the state ahead of a chunk, W_t = w_1 .. w_t by key channel,
-//   c_t = u_t^T S_(t-1) = U_t^T S + sum over s < t of (G_ts v_s - H_ts c_s),     U_t = u_t W_(t-1),
-//   o_t = S_t^T r_t     = R_t^T S + sum over s <= t of (P_ts v_s - Q_ts c_s),    R_t = r_t W_t,
-// G, H, P, Q the products by key channel of U or R with k_s / W_s and (a u)_s / W_s.  The triangular system for the c is solved ahead
-// of the scan, on the coefficients: c = A1 S + B1 v, o = A2 S + B2 v, and S <- W S + K^T v - A^T c, K_s = k_s w_(s+1) .. w_last, A alike.
-// What is left in sequence is one step of three products per sixteen tokens, where groups of four took a round of shuffles and 26 dependent
-// multiply-adds each.  The error against 64 bits stays that of groups of four (2048 random tokens, outputs: 1.1e-7 both; slow decays and
-// alike keys 2.5e-7 and 2.6e-7; fast decays 1.0e-7 both): W is a product and W - 1 a sum of its own, neither is had from the other.
-// A chunk's record: [drow + 16][32] (A1 | A2 by key, then B1 | B2 by source token), [32][drow] (K, then -A), W - 1 [drow],
-// v [drow / 16][16][16].  A decay is at least exp(-decay_scale), so W stays above exp(-40) over the tokens chunk_len allows a chunk.
-constexpr uint32_t CHUNK = 16, CCOLS = 16;
-__host__ __device__ constexpr uint32_t chunk_shared_floats(uint32_t drow) { return (drow + CHUNK) * 2 * CHUNK + 2 * CHUNK * drow + drow; }      // what every column group reads
-__host__ __device__ constexpr uint32_t chunk_floats(uint32_t drow) { return chunk_shared_floats(drow) + CHUNK * drow; }
+// Prompts run in groups of four tokens.  With S the state ahead of a group, the products c_t = u_t^T S_(t-1) the removals need are
+//   c_t = U_t^T S + sum over s < t of (G_ts v_s - H_ts c_s),   U_t = u_t w_0 .. w_(t-1),
+//   G_ts = (u_t w_(s+1) .. w_(t-1))^T k_s,   H_ts = (u_t w_(s+1) .. w_(t-1))^T (a u)_s   (products by key channel),
+// so the four reductions over the keys of a column go side by side and one round of shuffles serves four tokens.  A group's
+// record: four times [w - 1 | a u | U | k | r | v] of drow floats, then G and H of the pairs (1,0) (2,0) (2,1) (3,0) (3,1) (3,2).
+constexpr uint32_t GROUP = 4;
+__host__ __device__ constexpr uint32_t group_floats(uint32_t drow) { return GROUP * 6 * drow + 16; }
 
-// One CTA per (chunk, head), thread = key channel.  2048 tokens of 16 heads of 128: 103 us (with the 1 / W, 90 MB of records and loads whose
-// latency four CTAs an SM do not hide); the records of groups of four took 71.
-template <int D>
-__global__ void __launch_bounds__(D, 512 / D) delta_chunk_kernel(const DeltaArgs a, uint32_t n_tok, uint32_t len) {
-    extern __shared__ __align__(16) float cm[];
-    constexpr uint32_t PITCH = D + 4, SP = 36;          // rows 16 bytes apart in the banks
-    float *sa = cm, *sb = sa + 32 * PITCH, *sp = sb + 32 * PITCH, *s_inv = sp + 32 * SP, *sd = s_inv + CHUNK, *su = sd + CHUNK * D;          // sd, su: a thread's own decays and removals
-    const uint32_t c = threadIdx.x, lane = c & 31, warp = c >> 5, h = blockIdx.y, tok0 = blockIdx.x * len, dim = a.dim, HD = a.heads * dim;
+template <int NI>       // drow = 32 NI; one warp per (group, head)
+__global__ void __launch_bounds__(256) delta_prep_kernel(const DeltaArgs a, uint32_t n_tok) {
+    constexpr uint32_t D = 32 * NI;
+    const uint32_t lane = threadIdx.x & 31, h = blockIdx.y, g = blockIdx.x * 8 + (threadIdx.x >> 5), dim = a.dim, HD = a.heads * dim, groups = (n_tok + GROUP - 1) / GROUP;
     pdl_wait();
     pdl_trigger();
-    float *rec = a.rec + ((size_t)h * gridDim.x + blockIdx.x) * chunk_floats(D);
-    const float *in = a.in + (size_t)tok0 * a.in_stride + h * dim + c;
-    const uint32_t n = min(len, n_tok - tok0);
-    float k[CHUNK];
+    if (g >= groups) return;
+    float *rec = a.rec + ((size_t)h * groups + g) * group_floats(D);
+    float k[GROUP][NI], inv_k[GROUP], sums[12];
 #pragma unroll
-    for (uint32_t t = 0; t < CHUNK; ++t) {
-        const bool on = t < n && c < dim;
-        k[t] = on ? __ldcg(in + t * a.in_stride + HD) : 0.0f;
-        sd[t * D + c] = on ? __ldcg(a.decay_logit + (size_t)(tok0 + t) * a.logit_stride + h * dim + c) : 0.0f;
-        su[t * D + c] = on ? __ldcg(in + t * a.in_stride + 4 * HD) : 0.0f;
-        sb[t * PITCH + c] = k[t];
-    }
-    __syncthreads();
-#pragma unroll
-    for (uint32_t t = warp; t < CHUNK; t += D / 32) {
+    for (uint32_t t = 0; t < GROUP; ++t) {
+        const uint32_t tok = g * GROUP + t;
+        const float *in = a.in + tok * a.in_stride + h * dim;
         float kk = 0.0f;
 #pragma unroll
-        for (uint32_t i = 0; i < D / 32; ++i) { const float x = sb[t * PITCH + lane + 32 * i]; kk = __fmaf_rn(x, x, kk); }
-        kk = warp_sum(kk);
-        if (lane == 0) s_inv[t] = 1.0f / sqrtf(kk + a.unit_eps);
-    }
-    __syncthreads();
-    const float bias = c < dim ? __ldg(a.decay_bias + h * dim + c) : 0.0f, rate = c < dim ? __ldg(a.rate_bias + h * dim + c) : 0.0f;
-    float w = 1.0f, e = 0.0f;                // W_t, W_t - 1
-#pragma unroll 4
-    for (uint32_t t = 0; t < CHUNK; ++t) {
-        const bool on = t < n && c < dim;
-        const float kt = sb[t * PITCH + c], u = kt * s_inv[t], r = on ? __ldcg(in + t * a.in_stride) : 0.0f, v = on ? __ldcg(in + t * a.in_stride + 2 * HD) : 0.0f;
-        const float d = on ? decay_minus_one(a.decay_scale, sd[t * D + c] + bias) : 0.0f, au = on ? sigmoidf(su[t * D + c] + rate) * u : 0.0f;
-        sd[t * D + c] = d; su[t * D + c] = au;
-        sa[t * PITCH + c] = u * w;
-        e = __fmaf_rn(e, d, e + d);
-        w = fmaxf(w * (1.0f + d), 1e-30f);          // what decays further in one token leaves nothing of what was there
-        const float iw = 1.0f / w;
-        sa[(CHUNK + t) * PITCH + c] = r * w;
-        sb[t * PITCH + c] = kt * iw; sb[(CHUNK + t) * PITCH + c] = au * iw;
-        rec[chunk_shared_floats(D) + (c / CCOLS) * CHUNK * CCOLS + t * CCOLS + c % CCOLS] = v;
-    }
-    {
-        float *m2 = rec + (D + CHUNK) * 2 * CHUNK + c, suffix = 1.0f;
-        m2[2 * CHUNK * D] = e;
-#pragma unroll
-        for (int t = CHUNK - 1; t >= 0; --t) {
-            m2[t * D] = k[t] * suffix; m2[(CHUNK + t) * D] = -su[t * D + c] * suffix;
-            suffix *= 1.0f + sd[t * D + c];
+        for (int i = 0; i < NI; ++i) {
+            const uint32_t c = lane + 32 * i;
+            k[t][i] = tok < n_tok && c < dim ? __ldcg(in + HD + c) : 0.0f;
+            kk = __fmaf_rn(k[t][i], k[t][i], kk);
         }
+        inv_k[t] = 1.0f / sqrtf(warp_sum(kk) + a.unit_eps);
     }
-    __syncthreads();
-    {          // the 32 x 32 products: a thread's rows lie 8 apart, its columns next to one another
-        constexpr uint32_t NJ = D >= 256 ? 1 : D >= 128 ? 2 : 4, LJ = 32 / NJ;          // 4 x NJ products a thread, 8 LJ threads
-        static_assert(8 * LJ <= D, "every product has a thread");
-        const uint32_t i0 = c / LJ, j0 = (c % LJ) * NJ;
-        if (c < 8 * LJ) {
-            float acc[4][NJ];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+    for (int j = 0; j < 12; ++j) sums[j] = 0.0f;
 #pragma unroll
-                for (int j = 0; j < (int)NJ; ++j) acc[i][j] = 0.0f;
-#pragma unroll 2
-            for (uint32_t x = 0; x < D; x += 4) {
-                float4 q[4];
+    for (int i = 0; i < NI; ++i) {
+        const uint32_t c = lane + 32 * i;
+        float w[GROUP], au[GROUP];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) q[i] = *reinterpret_cast<const float4 *>(sa + (i0 + 8 * i) * PITCH + x);
-#pragma unroll
-                for (int j = 0; j < (int)NJ; ++j) {
-                    const float4 y = *reinterpret_cast<const float4 *>(sb + (j0 + j) * PITCH + x);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) acc[i][j] = __fmaf_rn(q[i].w, y.w, __fmaf_rn(q[i].z, y.z, __fmaf_rn(q[i].y, y.y, __fmaf_rn(q[i].x, y.x, acc[i][j]))));
-                }
+        for (uint32_t t = 0; t < GROUP; ++t) {
+            const uint32_t tok = g * GROUP + t;
+            const float *in = a.in + tok * a.in_stride + h * dim;
+            float d = 0.0f, r = 0.0f, v = 0.0f;
+            au[t] = 0.0f;
+            float u = k[t][i] * inv_k[t];
+            if (tok < n_tok && c < dim) {
+                d = decay_minus_one(a.decay_scale, __ldcg(a.decay_logit + tok * a.logit_stride + h * dim + c) + __ldg(a.decay_bias + h * dim + c));
+                au[t] = sigmoidf(__ldcg(in + 4 * HD + c) + __ldg(a.rate_bias + h * dim + c)) * u;
+                r = __ldcg(in + c);
+                v = __ldcg(in + 2 * HD + c);
             }
+            w[t] = 1.0f + d;
+            // u w_(t-1) .. w_(s+1) against k_s and (a u)_s, s from t - 1 down
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < (int)NJ; ++j) sp[(i0 + 8 * i) * SP + j0 + j] = acc[i][j];
-        }
-    }
-    __syncthreads();
-    // rows of sp: U_t, then R_t; columns: k_s / W_s, then (a u)_s / W_s.  x1 solves the system (a row of H at a time), x2 follows from it;
-    // both go to `to`, 32 floats in 16-byte pieces: A1 | A2
-    auto solve = [&](auto first, auto second, auto to) {
-        float x1[CHUNK];
-        auto less = [&](float x, const float *row, uint32_t count) {
-#pragma unroll
-            for (uint32_t q = 0; q < CHUNK; q += 4)
-                if (q < count) {
-                    const float4 m = *reinterpret_cast<const float4 *>(row + q);
-                    x = __fmaf_rn(-m.x, x1[q], x);
-                    if (q + 1 < count) x = __fmaf_rn(-m.y, x1[q + 1], x);
-                    if (q + 2 < count) x = __fmaf_rn(-m.z, x1[q + 2], x);
-                    if (q + 3 < count) x = __fmaf_rn(-m.w, x1[q + 3], x);
+            for (int s = GROUP - 2; s >= 0; --s)
+                if (s < (int)t) {
+                    const int pair = (int)t * ((int)t - 1) / 2 + s;
+                    sums[pair] = __fmaf_rn(u, k[s][i], sums[pair]);
+                    sums[6 + pair] = __fmaf_rn(u, au[s], sums[6 + pair]);
+                    u *= w[s];
                 }
-            return x;
-        };
-#pragma unroll
-        for (uint32_t t = 0; t < CHUNK; ++t) {
-            x1[t] = less(first(t), sp + t * SP + CHUNK, t);
-            if (t % 4 == 3) { to(t / 4, make_float4(x1[t - 3], x1[t - 2], x1[t - 1], x1[t])); asm volatile("" ::: "memory"); }
+            float *q = rec + t * 6 * D + c;
+            q[0] = d; q[D] = au[t]; q[2 * D] = u; q[3 * D] = k[t][i]; q[4 * D] = r; q[5 * D] = v;
         }
-#pragma unroll
-        for (uint32_t t = 0; t < CHUNK; t += 4) {
-            float x2[4];
-#pragma unroll
-            for (uint32_t i = 0; i < 4; ++i) x2[i] = less(second(t + i), sp + (CHUNK + t + i) * SP + CHUNK, t + i + 1);
-            to(4 + t / 4, make_float4(x2[0], x2[1], x2[2], x2[3]));
-            asm volatile("" ::: "memory");
-        }
-    };
-    // nobody reads sb any more: the key's 32 coefficients, pieces swizzled by key
-    solve([&](uint32_t t) { return sa[t * PITCH + c]; }, [&](uint32_t t) { return sa[(CHUNK + t) * PITCH + c]; },
-          [&](uint32_t q, float4 v) { *reinterpret_cast<float4 *>(sb + c * 2 * CHUNK + ((q ^ (c & 7u)) * 4)) = v; });
-    if (c < CHUNK)          // the same for the values: source token c
-        solve([&](uint32_t t) { return c < t ? sp[t * SP + c] : 0.0f; }, [&](uint32_t t) { return c <= t ? sp[(CHUNK + t) * SP + c] : 0.0f; },
-              [&](uint32_t q, float4 v) { *reinterpret_cast<float4 *>(rec + (D + c) * 2 * CHUNK + q * 4) = v; });
-    __syncthreads();
-#pragma unroll
-    for (uint32_t i = 0; i < 8; ++i) {
-        const uint32_t at = i * D + c, key = at >> 3, q = at & 7u;
-        reinterpret_cast<float4 *>(rec)[at] = *reinterpret_cast<const float4 *>(sb + key * 2 * CHUNK + ((q ^ (key & 7u)) * 4));
     }
+    float mine = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 12; ++j) {
+        const float v = warp_sum(sums[j]);
+        if ((int)lane == j) mine = v;
+    }
+    if (lane < 16) rec[GROUP * 6 * D + lane] = mine;
 }
 
-constexpr uint32_t SC_WAIT_LIMIT = 1u << 22, SC_THREADS = 256, SC_PITCH = 20;          // pitch: rows of 16 floats, four of them 16 banks on
-template <int D> struct ScanLayout {
-    static constexpr uint32_t STAGES = D > 192 ? 2 : 3, SHARED = chunk_shared_floats(D), STAGE = SHARED + CHUNK * CCOLS;
-    static constexpr uint32_t X = STAGES * STAGE;                                      // [D + 48][20]: the state, v of two chunks, c
-    static constexpr uint32_t PART = X + (D + 48) * SC_PITCH;                          // [8][32][20]: partial sums of c and o
-    static constexpr uint32_t TOTAL = (PART + 8 * 32 * SC_PITCH) * 4;
-};
+constexpr uint32_t SC_STAGES = 3;
+constexpr uint32_t SC_WAIT_LIMIT = 1u << 22;
+__host__ __device__ constexpr uint32_t stage_groups(uint32_t drow) { return drow >= 256 ? 1u : 256u / drow; }
 
-// CTA = 16 columns of a head's state.  Per chunk: 8 warps share the rows of (A1 | A2)^T S + (B1 | B2)^T v, 4 x 4 products a lane; the warps' sums
-// are added; then S takes its 32 updates, four keys x two columns at a time, those of v while the sums meet.  Bound by shared-memory reads
-// (0.76 of wavefronts): 4 x 4 products per two 16-byte reads.  2048 tokens of 16 heads of 128: 216 us, in groups of four 337.
-template <int D>
-__global__ void __launch_bounds__(SC_THREADS, 1) delta_scan_kernel(const float *__restrict__ rec, uint32_t n_tok, uint32_t len, float *__restrict__ state, float *__restrict__ o, uint32_t heads,
-                                                                   uint32_t *__restrict__ err_flag) {
+// Twice N values per lane (N = 8 or 16) summed over the warp side by side: lane l returns the sums of a[l N / 32] and b[l N / 32]
+// (an exchange halves the values per step).
+template <int N> __device__ __forceinline__ float2 warp_sum_many(float (&a)[N], float (&b)[N], uint32_t lane) {
+    constexpr int SPREAD = 32 / N;
+#pragma unroll
+    for (int w = N / 2; w > 0; w >>= 1) {
+        const bool up = (lane & (w * SPREAD)) != 0;
+#pragma unroll
+        for (int i = 0; i < w; ++i) {
+            const float ga = up ? a[i] : a[i + w], ka = up ? a[i + w] : a[i], gb = up ? b[i] : b[i + w], kb = up ? b[i + w] : b[i];
+            a[i] = __fadd_rn(ka, __shfl_xor_sync(0xffffffffu, ga, w * SPREAD));
+            b[i] = __fadd_rn(kb, __shfl_xor_sync(0xffffffffu, gb, w * SPREAD));
+        }
+    }
+    float ra = a[0], rb = b[0];
+#pragma unroll
+    for (int m = SPREAD / 2; m > 0; m >>= 1) { ra = __fadd_rn(ra, __shfl_xor_sync(0xffffffffu, ra, m)); rb = __fadd_rn(rb, __shfl_xor_sync(0xffffffffu, rb, m)); }
+    return make_float2(ra, rb);
+}
+__device__ __forceinline__ uint64_t lds64(uint32_t saddr) {        // kept in program order: a group's loads are issued ahead of its reductions
+    uint64_t v;
+    asm volatile("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(saddr) : "memory");
+    return v;
+}
+
+// CTA = four warps, warp = NC (two or four) columns of a head; the 32 lanes share the keys: lane l holds the key pairs
+// 2 (32 i + l), i < KP (drow = 64 KP), so a record vector is read once per warp, 256 consecutive bytes per load.  Two columns
+// give the SMs twice the warps to hide latencies with where there are few heads, four halve the shared-memory reads.
+template <int KP, int NC>
+__global__ void __launch_bounds__(128) delta_scan_kernel(const float *__restrict__ rec, uint32_t n_tok, float *__restrict__ state, float *__restrict__ o, uint32_t heads,
+                                                        uint32_t *__restrict__ err_flag) {
     extern __shared__ __align__(128) float ring[];
-    __shared__ __align__(8) uint64_t bars[3];
-    using L = ScanLayout<D>;
-    constexpr uint32_t NU = (2 * D + SC_THREADS - 1) / SC_THREADS, ROWS = (D + CHUNK) / 8, KG = D / 4;
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h = blockIdx.y, col0 = blockIdx.x * CCOLS;
+    __shared__ __align__(8) uint64_t bars[SC_STAGES];
+    constexpr uint32_t D = 64 * KP, GF = group_floats(D), SG = stage_groups(D), STAGE = SG * GF;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h = blockIdx.y, col = (blockIdx.x * 4 + warp) * NC;
     const uint32_t bar = (uint32_t)__cvta_generic_to_shared(bars), rb = (uint32_t)__cvta_generic_to_shared(ring);
-    const uint32_t chunks = (n_tok + len - 1) / len;
-    const float *src = rec + (size_t)h * chunks * chunk_floats(D);
-    float *X = ring + L::X, *part = ring + L::PART;
+    const uint32_t groups = (n_tok + GROUP - 1) / GROUP, chunks = (groups + SG - 1) / SG;
+    const float *src = rec + (size_t)h * groups * GF;
     if (tid == 0) {
-        for (uint32_t i = 0; i < L::STAGES; ++i) mbar_init(bar + 8 * i, 1);
+        for (uint32_t i = 0; i < SC_STAGES; ++i) mbar_init(bar + 8 * i, 1);
         fence_mbar_init();
     }
-    // this thread's part of the state: keys 4 kg .., columns 2 cp, 2 cp + 1 of unit u (a warp: four key groups x eight column pairs)
-    const uint32_t cp = lane & 7u, kg0 = warp * 4 + (lane >> 3);
-    float *sp = state + (size_t)h * D * D + col0 + 2 * cp;
-    float2 st[NU][4];
+    float *sp = state + (size_t)h * D * D + col;
+    uint64_t s[NC][KP];
 #pragma unroll
-    for (uint32_t u = 0; u < NU; ++u) {
-        const uint32_t kg = kg0 + 32 * u;
+    for (int i = 0; i < KP; ++i) {
+        const float *q = sp + (size_t)((i * 32 + lane) * 2) * D;
 #pragma unroll
-        for (uint32_t i = 0; i < 4; ++i) {
-            st[u][i] = kg < KG ? __ldcg(reinterpret_cast<const float2 *>(sp + (size_t)(4 * kg + i) * D)) : make_float2(0.0f, 0.0f);
-            if (kg < KG) *reinterpret_cast<float2 *>(X + (4 * kg + i) * SC_PITCH + 2 * cp) = st[u][i];
+        for (int c = 0; c < NC; c += 2) {
+            const float2 e = __ldcg(reinterpret_cast<const float2 *>(q + c)), f = __ldcg(reinterpret_cast<const float2 *>(q + D + c));
+            s[c][i] = pk(e.x, f.x); s[c + 1][i] = pk(e.y, f.y);
         }
     }
     pdl_wait();
     pdl_trigger();
     __syncthreads();
-    auto request = [&](uint32_t c) {
-        const uint32_t b = bar + 8 * (c % L::STAGES), dst = rb + (c % L::STAGES) * L::STAGE * 4;
-        const float *q = src + (size_t)c * chunk_floats(D);
-        mbar_expect_tx(b, L::STAGE * 4);
-        bulk_g2s(dst, q, L::SHARED * 4, b);
-        bulk_g2s(dst + L::SHARED * 4, q + L::SHARED + blockIdx.x * CHUNK * CCOLS, CHUNK * CCOLS * 4, b);
+    float oo[GROUP * NC];                       // outputs of the group before, not reduced yet
+#pragma unroll
+    for (int i = 0; i < (int)GROUP * NC; ++i) oo[i] = 0.0f;
+    uint32_t tok_o = n_tok;                     // its first token; n_tok = none
+    auto store = [&](uint32_t tok0, float sum) {
+        constexpr uint32_t LPV = 32 / (GROUP * NC);          // lanes that hold the same value
+        const uint32_t tok = tok0 + (lane >> 3);
+        if (lane % LPV == 0 && tok < n_tok) o[((size_t)tok * heads + h) * D + col + (lane / LPV) % NC] = sum;
     };
-    auto landed = [&](uint32_t c) {          // and v of chunk c beside the state; false: gave up
-        bool ok = mbar_try_wait(bar + 8 * (c % L::STAGES), (c / L::STAGES) & 1u);
-        for (uint32_t spin = 0; spin < SC_WAIT_LIMIT && !ok; ++spin) ok = mbar_try_wait(bar + 8 * (c % L::STAGES), (c / L::STAGES) & 1u);
-        X[(D + CHUNK * (c & 1u) + (tid >> 4)) * SC_PITCH + (tid & 15u)] = ring[(c % L::STAGES) * L::STAGE + L::SHARED + tid];
-        return ok;
+    auto request = [&](uint32_t c) {
+        const uint32_t bytes = min(SG, groups - c * SG) * GF * 4;
+        mbar_expect_tx(bar + 8 * (c % SC_STAGES), bytes);
+        bulk_g2s(rb + (c % SC_STAGES) * STAGE * 4, src + (size_t)c * STAGE, bytes, bar + 8 * (c % SC_STAGES));
     };
     if (tid == 0)
-        for (uint32_t c = 0; c < min(L::STAGES, chunks); ++c) request(c);
-    bool ok = landed(0);
-    const uint32_t oi = lane >> 2, cj = lane & 3u;
+        for (uint32_t c = 0; c < min(SC_STAGES, chunks); ++c) request(c);
     for (uint32_t c = 0; c < chunks; ++c) {
+        bool ok = false;
+        for (uint32_t spin = 0; spin < SC_WAIT_LIMIT && !ok; ++spin) ok = mbar_try_wait(bar + 8 * (c % SC_STAGES), (c / SC_STAGES) & 1u);
         if (__syncthreads_or(!ok)) {            // a copy did not land: report, let the others in flight land, leave
             if (tid == 0 && err_flag != nullptr) atomicExch(err_flag, 1u);
-            for (uint32_t d = c; d < min(c + L::STAGES, chunks); ++d)
-                for (uint32_t spin = 0; spin < SC_WAIT_LIMIT && !mbar_try_wait(bar + 8 * (d % L::STAGES), (d / L::STAGES) & 1u); ++spin) {}
+            for (uint32_t d = c + 1; d < min(c + SC_STAGES, chunks); ++d)
+                for (uint32_t spin = 0; spin < SC_WAIT_LIMIT && !mbar_try_wait(bar + 8 * (d % SC_STAGES), (d / SC_STAGES) & 1u); ++spin) {}
             return;
         }
-        const float *stage = ring + (c % L::STAGES) * L::STAGE, *vrow = X + (D + CHUNK * (c & 1u)) * SC_PITCH;
-        {          // partial sums of outputs 4 oi .. (c, then o) and columns 4 cj ..
-            float acc[4][4];
+        const uint32_t n = min(SG, groups - c * SG);
+        const float *at = ring + (c % SC_STAGES) * STAGE;
+        uint32_t sa = rb + (c % SC_STAGES) * STAGE * 4 + lane * 8;
+#pragma unroll 1
+        for (uint32_t gi = 0; gi < n; ++gi, at += GF, sa += GF * 4) {
+            uint64_t part[5][GROUP][KP];        // U, then w - 1, a u, k, r
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int j = 0; j < 5; ++j)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
-            const float *m1 = stage + warp * ROWS * 2 * CHUNK + 4 * oi;
+                for (uint32_t t = 0; t < GROUP; ++t)
 #pragma unroll
-            for (uint32_t r = 0; r < ROWS; ++r) {
-                const uint32_t row = warp * ROWS + r;
-                const float4 m = *reinterpret_cast<const float4 *>(m1 + r * 2 * CHUNK);
-                const float4 x = *reinterpret_cast<const float4 *>((row < D ? X + row * SC_PITCH : vrow + (row - D) * SC_PITCH) + 4 * cj);
-                const float mv[4] = {m.x, m.y, m.z, m.w}, xv[4] = {x.x, x.y, x.z, x.w};
+                    for (int i = 0; i < KP; ++i) part[j][t][i] = lds64(sa + ((t * 6 + (j == 0 ? 2 : j <= 2 ? j - 1 : j)) * (D / 2) + i * 32) * 8);
+            float d[GROUP * NC], v[GROUP * NC];
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
+            for (uint32_t t = 0; t < GROUP; ++t) {
+                uint64_t p[NC];
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) acc[i][j] = __fmaf_rn(mv[i], xv[j], acc[i][j]);
-            }
+                for (int i = 0; i < KP; ++i)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) *reinterpret_cast<float4 *>(part + (warp * 32 + 4 * oi + i) * SC_PITCH + 4 * cj) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-        }
-        const float *m2 = stage + (D + CHUNK) * 2 * CHUNK, *crow = X + (D + 2 * CHUNK) * SC_PITCH;
-        // updates s0 .. s0 + 15 of the state: v, then c
-        auto update = [&](float2 (&add)[4], uint32_t kg, const float *y0, uint32_t s0) {
+                    for (int c2 = 0; c2 < NC; ++c2) p[c2] = fma2(part[0][t][i], s[c2][i], i == 0 ? 0ull : p[c2]);
 #pragma unroll
-            for (uint32_t s = 0; s < CHUNK; ++s) {
-                const float4 m = *reinterpret_cast<const float4 *>(m2 + (s0 + s) * D + 4 * kg);
-                const float2 y = *reinterpret_cast<const float2 *>(y0 + s * SC_PITCH + 2 * cp);
-                const float mv[4] = {m.x, m.y, m.z, m.w};
-#pragma unroll
-                for (int i = 0; i < 4; ++i) { add[i].x = __fmaf_rn(mv[i], y.x, add[i].x); add[i].y = __fmaf_rn(mv[i], y.y, add[i].y); }
-            }
-        };
-        float2 add[NU][4];
-#pragma unroll
-        for (uint32_t u = 0; u < NU; ++u) {          // what needs no c goes on while the sums meet
-            const uint32_t kg = kg0 + 32 * u;
-            if (kg < KG) {
-                const float4 e = *reinterpret_cast<const float4 *>(m2 + 2 * CHUNK * D + 4 * kg);
-                const float ev[4] = {e.x, e.y, e.z, e.w};
-#pragma unroll
-                for (int i = 0; i < 4; ++i) add[u][i] = make_float2(ev[i] * st[u][i].x, ev[i] * st[u][i].y);
-                update(add[u], kg, vrow, 0);
-            }
-        }
-        __syncthreads();
-        {
-            const uint32_t out = tid >> 3;
-            float2 sum = make_float2(0.0f, 0.0f);
-#pragma unroll
-            for (uint32_t w = 0; w < 8; ++w) {
-                const float2 p = *reinterpret_cast<const float2 *>(part + (w * 32 + out) * SC_PITCH + 2 * (tid & 7u));
-                sum.x += p.x; sum.y += p.y;
-            }
-            if (out < CHUNK) *reinterpret_cast<float2 *>(X + (D + 2 * CHUNK + out) * SC_PITCH + 2 * (tid & 7u)) = sum;
-            else if (out - CHUNK < len && c * len + out - CHUNK < n_tok) *reinterpret_cast<float2 *>(o + ((size_t)(c * len + out - CHUNK) * heads + h) * D + col0 + 2 * (tid & 7u)) = sum;
-        }
-        __syncthreads();
-#pragma unroll
-        for (uint32_t u = 0; u < NU; ++u) {
-            const uint32_t kg = kg0 + 32 * u;
-            if (kg < KG) {
-                update(add[u], kg, crow, CHUNK);
-#pragma unroll
-                for (uint32_t i = 0; i < 4; ++i) {
-                    st[u][i].x += add[u][i].x; st[u][i].y += add[u][i].y;
-                    *reinterpret_cast<float2 *>(X + (4 * kg + i) * SC_PITCH + 2 * cp) = st[u][i];
+                for (int c2 = 0; c2 < NC; c2 += 2) {
+                    const float2 e = *reinterpret_cast<const float2 *>(at + (t * 6 + 5) * D + col + c2);
+                    v[t * NC + c2] = e.x; v[t * NC + c2 + 1] = e.y;
                 }
+#pragma unroll
+                for (int c2 = 0; c2 < NC; ++c2) { float e0, e1; upk(p[c2], e0, e1); d[t * NC + c2] = __fadd_rn(e0, e1); }
+            }
+            // the products of this group and the outputs of the one before are reduced side by side
+            const float2 sums = warp_sum_many<GROUP * NC>(d, oo, lane);
+            store(tok_o, sums.y);
+            tok_o = (c * SG + gi) * GROUP;
+#pragma unroll
+            for (int i = 0; i < (int)GROUP * NC; ++i) d[i] = __shfl_sync(0xffffffffu, sums.x, 32 / (GROUP * NC) * i);
+            const float *gh = at + GROUP * 6 * D;
+#pragma unroll
+            for (uint32_t t = 1; t < GROUP; ++t)
+#pragma unroll
+                for (uint32_t q = 0; q < t; ++q) {
+                    const float g = gh[t * (t - 1) / 2 + q], hh = -gh[6 + t * (t - 1) / 2 + q];
+#pragma unroll
+                    for (int c2 = 0; c2 < NC; ++c2) d[t * NC + c2] = __fmaf_rn(hh, d[q * NC + c2], __fmaf_rn(g, v[q * NC + c2], d[t * NC + c2]));
+                }
+#pragma unroll
+            for (uint32_t t = 0; t < GROUP; ++t) {
+                uint64_t v2[NC], c2n[NC], p[NC];
+#pragma unroll
+                for (int c2 = 0; c2 < NC; ++c2) { v2[c2] = pk(v[t * NC + c2], v[t * NC + c2]); c2n[c2] = pk(-d[t * NC + c2], -d[t * NC + c2]); }
+#pragma unroll
+                for (int i = 0; i < KP; ++i)
+#pragma unroll
+                    for (int c2 = 0; c2 < NC; ++c2) {
+                        s[c2][i] = fma2(part[2][t][i], c2n[c2], fma2(part[1][t][i], s[c2][i], fma2(part[3][t][i], v2[c2], s[c2][i])));
+                        p[c2] = fma2(part[4][t][i], s[c2][i], i == 0 ? 0ull : p[c2]);
+                    }
+#pragma unroll
+                for (int c2 = 0; c2 < NC; ++c2) { float e0, e1; upk(p[c2], e0, e1); oo[t * NC + c2] = __fadd_rn(e0, e1); }
             }
         }
-        if (c + 1 < chunks) ok = landed(c + 1);
         __syncthreads();                        // the stage is free
-        if (tid == 0 && c + L::STAGES < chunks) request(c + L::STAGES);
+        if (tid == 0 && c + SC_STAGES < chunks) request(c + SC_STAGES);
+    }
+    {
+        float none[GROUP * NC];
+#pragma unroll
+        for (int i = 0; i < (int)GROUP * NC; ++i) none[i] = 0.0f;
+        store(tok_o, warp_sum_many<GROUP * NC>(none, oo, lane).y);
     }
 #pragma unroll
-    for (uint32_t u = 0; u < NU; ++u) {
-        const uint32_t kg = kg0 + 32 * u;
+    for (int i = 0; i < KP; ++i) {
+        float *q = sp + (size_t)((i * 32 + lane) * 2) * D;
 #pragma unroll
-        for (uint32_t i = 0; i < 4; ++i)
-            if (kg < KG) *reinterpret_cast<float2 *>(sp + (size_t)(4 * kg + i) * D) = st[u][i];
+        for (int c = 0; c < NC; c += 2) {
+            float2 e, f;
+            upk(s[c][i], e.x, f.x); upk(s[c + 1][i], e.y, f.y);
+            *reinterpret_cast<float2 *>(q + c) = e;
+            *reinterpret_cast<float2 *>(q + D + c) = f;
+        }
     }
 }
 
@@ -455,30 +402,23 @@ __global__ void __launch_bounds__(256) delta_post_kernel(const DeltaArgs a, uint
     for (uint32_t j = lane; j < dim; j += 32) act_store<F32>(a.out, t, h * dim + j, __ldcg(o + j) * inv * __ldg(a.norm + h * dim + j) * sigmoidf(__ldcg(g + j)));
 }
 
-// tokens of a chunk: all sixteen for decay scales up to 2.5
-uint32_t chunk_len(float decay_scale) {
-    const float x = 40.0f / std::fabs(decay_scale);
-    return x >= 1.0f && x < (float)CHUNK ? (uint32_t)x : x < 1.0f ? 1u : CHUNK;
-}
-
-template <int D> cudaError_t scan(cudaStream_t s, const DeltaArgs &a, uint32_t n_tok, bool pdl) {
-    constexpr size_t prep_smem = ((size_t)64 * (D + 4) + 32 * 36 + CHUNK + 2 * CHUNK * D) * 4;
-    static_assert(ScanLayout<D>::TOTAL <= 227 * 1024, "shared memory");
-    cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(delta_chunk_kernel<D>), prep_smem);
-    if (e == cudaSuccess) e = allow_dynamic_smem(reinterpret_cast<const void *>(delta_scan_kernel<D>), ScanLayout<D>::TOTAL);
-    const uint32_t len = chunk_len(a.decay_scale);
-    if (e == cudaSuccess) e = launch_kernel(delta_chunk_kernel<D>, dim3((n_tok + len - 1) / len, a.heads), dim3(D), prep_smem, s, pdl, a, n_tok, len);
+template <int KP, int NC> cudaError_t scan_nc(cudaStream_t s, const DeltaArgs &a, uint32_t n_tok, bool pdl) {
+    constexpr size_t smem = (size_t)SC_STAGES * stage_groups(64 * KP) * group_floats(64 * KP) * 4;
+    cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(delta_scan_kernel<KP, NC>), smem);
     if (e != cudaSuccess) return e;
-    return launch_kernel(delta_scan_kernel<D>, dim3(D / CCOLS, a.heads), dim3(SC_THREADS), ScanLayout<D>::TOTAL, s, pdl, a.rec, n_tok, len, a.state, a.o, a.heads, a.err_flag);
+    return launch_kernel(delta_scan_kernel<KP, NC>, dim3(64 * KP / (4 * NC), a.heads), dim3(128), smem, s, pdl, a.rec, n_tok, a.state, a.o, a.heads, a.err_flag);
+}
+template <int KP> cudaError_t scan_kp(cudaStream_t s, const DeltaArgs &a, uint32_t n_tok, int sm_count, bool pdl) {
+    const uint32_t groups = (n_tok + GROUP - 1) / GROUP;
+    cudaError_t e = launch_kernel(delta_prep_kernel<2 * KP>, dim3((groups + 7) / 8, a.heads), dim3(256), 0, s, pdl, a, n_tok);
+    if (e != cudaSuccess) return e;
+    return 4u * KP * a.heads <= (uint32_t)sm_count ? scan_nc<KP, 2>(s, a, n_tok, pdl) : scan_nc<KP, 4>(s, a, n_tok, pdl);
 }
 
 }  // namespace
 
 uint32_t delta_row(uint32_t dim) { return dim <= 256 ? (dim + 63u) & ~63u : 0u; }
-size_t delta_record_floats(uint32_t n_tok, uint32_t heads, uint32_t drow, float decay_scale) {
-    const uint32_t len = chunk_len(decay_scale);
-    return ((size_t)n_tok + len - 1) / len * heads * chunk_floats(drow);
-}
+size_t delta_record_floats(uint32_t n_tok, uint32_t heads, uint32_t drow) { return (size_t)((n_tok + GROUP - 1) / GROUP) * heads * group_floats(drow); }
 bool delta_step_fits(const DeltaArgs &a) { return step_vec_smem(a.drow, (a.rank + 63) / 64 * 64) <= 200 * 1024; }
 
 template <bool F32, bool STAGED> static cudaError_t step_launch(cudaStream_t s, const DeltaArgs &a, size_t vec, size_t smem, bool pdl) {
@@ -499,10 +439,10 @@ cudaError_t launch_delta_prompt(cudaStream_t s, bool f32, const DeltaArgs &a, ui
     const dim3 grid((n_tok + 7) / 8, a.heads);
     cudaError_t e = cudaErrorInvalidValue;
     switch (a.drow / 64) {
-        case 1: e = scan<64>(s, a, n_tok, pdl); break;
-        case 2: e = scan<128>(s, a, n_tok, pdl); break;
-        case 3: e = scan<192>(s, a, n_tok, pdl); break;
-        case 4: e = scan<256>(s, a, n_tok, pdl); break;
+        case 1: e = scan_kp<1>(s, a, n_tok, sm_count, pdl); break;
+        case 2: e = scan_kp<2>(s, a, n_tok, sm_count, pdl); break;
+        case 3: e = scan_kp<3>(s, a, n_tok, sm_count, pdl); break;
+        case 4: e = scan_kp<4>(s, a, n_tok, sm_count, pdl); break;
         default: break;
     }
     if (e != cudaSuccess) return e;
