@@ -474,7 +474,8 @@ __global__ void __launch_bounds__(FL_THREADS, 1) window_flash_kernel(const AttnP
                 ok = mbar_wait_warp(b_o, (j - 1) & 1u, FL_WAIT, s_abort);
                 if (!ok) break;
                 tc_fence_after();
-                const float al = m_new == -INFINITY ? 1.0f : exp2_approx(m - m_new);
+                const bool grown = m_new > m + 8.0f;          // row by row: a row's bits do not depend on the rows beside it
+                const float al = grown ? exp2_approx(m - m_new) : 1.0f;
 #pragma unroll 1
                 for (uint32_t c = 0; c < D; c += 16) {
                     uint32_t o[16];
@@ -485,7 +486,7 @@ __global__ void __launch_bounds__(FL_THREADS, 1) window_flash_kernel(const AttnP
                     tm_st16(t_o + lanes + c, o);
                 }
                 l *= al;
-                m = m_new;
+                m = grown ? m_new : m;
             }
             const float mm = m == -INFINITY ? 0.0f : m;          // a row that has seen nothing yet: exp2(-inf) = 0
             float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
