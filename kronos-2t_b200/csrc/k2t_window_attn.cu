@@ -3,8 +3,8 @@
 //   * window_prep_kernel: per-head RMS norm of queries and keys of a prompt batch, cache rows, query rows (one warp per head).
 //   * window_flash_kernel (bf16 prompts): CTA = 128 query rows of one kv head - row = (token, head of the group), so all heads
 //     of a group share the key and value tiles.  S = Q K^T and O += P V by tcgen05.mma with S, P and O in tensor memory; scores,
-//     bias and softmax in fp32, one row per thread; the next S is computed while the softmax of this one runs, and O is rescaled
-//     only when a row's maximum has grown by more than 2^8.
+//     bias and softmax in fp32, one row per thread; the next S is computed while the softmax of this one runs, and a row
+//     of O is rescaled only when its maximum has grown by more than 2^8 - row by row, so that its bits depend on its keys alone.
 //   * window_row_kernel: one token and kv head per thread-block cluster.  The positions are split over the CTAs of the cluster,
 //     partial maxima, sums and outputs are merged through distributed shared memory, so a decode step is ONE launch: norms of
 //     the new query and key, the new cache row, attention and the activation of the output projection.  With fp32 rows the same
@@ -304,7 +304,7 @@ __device__ __forceinline__ void fl_cp_commit() { asm volatile("cp.async.commit_g
 
 // A tile of 128 keys takes a CTA about 5000 cycles: 1050 are the tensor cores' for both products, about 1300 the issue slots of a
 // softmax warp (nine instructions per key of a row).  Two softmax warps per row, half of the keys each, changed nothing (a prompt
-// 4723 us against 4720), so what is left is the fetch of 64 KB of keys and values per tile and the hand-offs between the roles;
+// of 12 blocks within 3 us), so what is left is the fetch of 64 KB of keys and values per tile and the hand-offs between the roles;
 // 256 rows per CTA over the same tiles would halve that fetch.  A value row that is not finite reaches, as 0 x inf, rows of its
 // tile that do not see it.  The rows of the ring are row-major, so the tiles come in by
 // 16-byte asynchronous copies of three warps, which put chunk c of row r at c ^ (r & 7) of its panel (the 128-byte swizzle) and
@@ -312,7 +312,7 @@ __device__ __forceinline__ void fl_cp_commit() { asm volatile("cp.async.commit_g
 // 128 elements would not leave room for two tiles of keys and values.  The grid deals the rows of all kv heads in descending
 // order of their contexts: a wave of 256 CTAs in ascending order left the longest to the end.
 // 2048 tokens, 16 heads of 128 over 4 kv heads: 139 us with mma.sync and 64-key tiles, 45.5 now (378 TFLOP/s of causal
-// work); a prompt of 12 blocks 5281 -> 4720 us, 300 tokens of 4 blocks 737 -> 648, 2 tokens behind 1000 positions 235 -> 207.
+// work); a prompt of 12 blocks 6552 -> about 5990 us, 300 tokens of 4 blocks 737 -> 648, 2 tokens behind 1000 positions 235 -> 207.
 // Warps 0 .. 3: queries, softmax and output, one row per thread; warps 4 .. 6: key and value tiles; warp 7: tensor-core issue.
 // Tensor memory: S of even and odd tiles (KT columns each, the softmax weights overwrite them as bf16 pairs), then O.
 template <int D>
