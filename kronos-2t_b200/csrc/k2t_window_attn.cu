@@ -312,7 +312,7 @@ __device__ __forceinline__ void fl_cp_commit() { asm volatile("cp.async.commit_g
 // 128 elements would not leave room for two tiles of keys and values.  The grid deals the rows of all kv heads in descending
 // order of their contexts: a wave of 256 CTAs in ascending order left the longest to the end.
 // 2048 tokens, 16 heads of 128 over 4 kv heads: 139 us with mma.sync and 64-key tiles, 45.5 now (378 TFLOP/s of causal
-// work); a prompt of 12 blocks 6552 -> about 5990 us, 300 tokens of 4 blocks 737 -> 648, 2 tokens behind 1000 positions 235 -> 207.
+// work); a prompt of 12 blocks 6632 -> 6015 us, 300 tokens of 4 blocks 737 -> 648, 2 tokens behind 1000 positions 235 -> 207.
 // Warps 0 .. 3: queries, softmax and output, one row per thread; warps 4 .. 6: key and value tiles; warp 7: tensor-core issue.
 // Tensor memory: S of even and odd tiles (KT columns each, the softmax weights overwrite them as bf16 pairs), then O.
 template <int D>
