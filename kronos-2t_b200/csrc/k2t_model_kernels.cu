@@ -373,8 +373,8 @@ __global__ void __launch_bounds__(ROUTER_THREADS) router_logits_kernel(const Rou
     bool ok = true;
     for (uint32_t c = 0; c < slices; ++c) {
         bool here = mbar_try_wait(bar + 8 * (c % RL_STAGES), (c / RL_STAGES) & 1u);
-        for (uint32_t spin = 0; ok && !here && spin < (1u << 22); ++spin) here = mbar_try_wait(bar + 8 * (c % RL_STAGES), (c / RL_STAGES) & 1u);
-        ok = ok && here;
+        for (uint32_t spin = 0; !here && spin < (1u << 22); ++spin) here = mbar_try_wait(bar + 8 * (c % RL_STAGES), (c / RL_STAGES) & 1u);
+        ok = ok && here;          // also behind a wait that gave up: the slices still in flight are waited for before the CTA leaves
         const float *x = s_dyn + ((c % RL_STAGES) * 32 + warp * 4 + (tile & 1u) * 2) * RL_PITCH + 4 * q, *w = s_dyn + ((c % RL_STAGES) * 32 + RL_TOKENS + (tile >> 1) * 4) * RL_PITCH + 4 * q;
         const uint32_t n = min(RL_SLICE, a.hidden - c * RL_SLICE);
         float4 xv[2][2], wv[2][4];
@@ -407,7 +407,7 @@ __global__ void __launch_bounds__(ROUTER_THREADS) router_logits_kernel(const Rou
         __syncthreads();
         if (warp == 0 && c + RL_STAGES < slices) request(c + RL_STAGES);
     }
-    if (!ok && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);          // every copy that was asked for has been waited for
+    if (!ok && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll

@@ -93,3 +93,11 @@ def test_a_wait_that_gives_up_does_not_split_its_warp(source):
 def test_the_reading_itself(role, found):
     assert bool(splits("void kernel() { if (warp < 4) { for (;;) { " + role + " } } }")) is found
     assert splits("void kernel() { if (lane == 0) { for (;;) { " + role + " } } }") == []
+
+
+@pytest.mark.parametrize("source", sorted(f for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh"))))
+def test_a_wait_is_not_cut_short_by_an_earlier_one(source):
+    """A role that asks for its next copy whatever the last wait said polls for each of them up to the limit: a loop that an earlier answer ends
+    would let the CTA leave while copies into its shared memory are in flight."""
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, source)).read())
+    assert re.findall(r"for \([^;]*\bspin\b[^;]*;[^;]*(?<![!\w])ok\b[^;]*;[^)]*\)", text) == []
