@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(RW_THREADS) window_row_kernel(const AttnParams
 }
 
 // ------------------------------------------------------------------------------------------------ prompts, bf16
-constexpr uint32_t FL_M = 128, FL_LOADERS = 96, FL_THREADS = 128 + FL_LOADERS + 32, FL_HEADER = 1024, FL_TMEM = 512, FL_WAIT = 1u << 22;
+constexpr uint32_t FL_M = 128, FL_LOADERS = 96, FL_THREADS = 128 + FL_LOADERS + 32, FL_HEADER = 1024, FL_TMEM = 512, FL_MARKS = 4096, FL_WAIT = 1u << 22;
 __host__ __device__ constexpr uint32_t fl_tile(uint32_t d) { return d <= 128 ? 128 : 64; }          // keys per tile
 __host__ __device__ constexpr uint32_t fl_panels(uint32_t d) { return (d + 63) / 64; }
 __host__ __device__ constexpr uint32_t fl_smem(uint32_t d) { return 1024 + FL_HEADER + fl_panels(d) * 128 * (FL_M + 4 * fl_tile(d)); }
@@ -305,8 +305,9 @@ __device__ __forceinline__ void fl_cp_commit() { asm volatile("cp.async.commit_g
 // A tile of 128 keys takes a CTA about 5000 cycles: 1050 are the tensor cores' for both products, about 1300 the issue slots of a
 // softmax warp (nine instructions per key of a row).  Two softmax warps per row, half of the keys each, changed nothing (a prompt
 // of 12 blocks within 3 us), so what is left is the fetch of 64 KB of keys and values per tile and the hand-offs between the roles;
-// 256 rows per CTA over the same tiles would halve that fetch.  A value row that is not finite reaches, as 0 x inf, rows of its
-// tile that do not see it.  The rows of the ring are row-major, so the tiles come in by
+// 256 rows per CTA over the same tiles would halve that fetch.  A value that is not finite would reach, as 0 x inf, all 128 rows: where
+// an output is not finite the CTA goes over its tiles once more, with zeros for such values, and adds them to the rows that see them.
+// The rows of the ring are row-major, so the tiles come in by
 // 16-byte asynchronous copies of three warps, which put chunk c of row r at c ^ (r & 7) of its panel (the 128-byte swizzle) and
 // fence them for the tensor cores; eight warps leave a softmax thread the registers for its 128 scores (nine: 168 and spills).  Keys per tile: 128, or 64 where the rows above
 // 128 elements would not leave room for two tiles of keys and values.  The grid deals the rows of all kv heads in descending
@@ -315,43 +316,23 @@ __device__ __forceinline__ void fl_cp_commit() { asm volatile("cp.async.commit_g
 // work); a prompt of 12 blocks 6632 -> 6015 us, 300 tokens of 4 blocks 737 -> 648, 2 tokens behind 1000 positions 235 -> 207.
 // Warps 0 .. 3: queries, softmax and output, one row per thread; warps 4 .. 6: key and value tiles; warp 7: tensor-core issue.
 // Tensor memory: S of even and odd tiles (KT columns each, the softmax weights overwrite them as bf16 pairs), then O.
-template <int D>
-__global__ void __launch_bounds__(FL_THREADS, 1) window_flash_kernel(const AttnParams p) {
-    constexpr uint32_t KT = fl_tile(D), PD = fl_panels(D), CH = D / 8, Q_BYTES = PD * FL_M * 128, T_BYTES = PD * KT * 128;
-    extern __shared__ uint8_t smem_raw[];
+// A pass of the CTA over its tiles: whether an output of the thread is not finite.  AGAIN: the second one; the phases of the barriers go on, tile j is tile
+// base + j of the CTA.
+template <int D, bool AGAIN>
+__device__ __forceinline__ bool flash_pass(const AttnParams &p, uint8_t *smem, uint32_t sbase, uint32_t tmem) {
+    constexpr uint32_t KT = fl_tile(D), PD = fl_panels(D), CH = D / 8, Q_BYTES = PD * FL_M * 128, T_BYTES = PD * KT * 128, PASS = AGAIN ? 1 : 0;
     const WindowAttnArgs &a = p.a;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = blockIdx.x, group = a.n_q / a.n_kv;
     const uint32_t rows = p.n_tok * group, r0 = (gridDim.y - 1 - blockIdx.y) * FL_M;          // the longest rows first, of all heads
-    const uint32_t raw = (uint32_t)__cvta_generic_to_shared(smem_raw), sbase = (raw + 1023u) & ~1023u;
-    uint8_t *smem = smem_raw + (sbase - raw);
-    const uint32_t s_q = sbase + FL_HEADER, s_k = s_q + Q_BYTES, s_v = s_k + 2 * T_BYTES;
-    // barriers: queries, keys landed / free, values landed / free, S ready, weights ready, O updated, end
+    const uint32_t s_q = sbase + FL_HEADER, s_k = s_q + Q_BYTES, s_v = s_k + 2 * T_BYTES, t_o = tmem + 2 * KT;
+    // barriers: queries, keys landed / free, values landed / free, S ready, weights ready, O updated, end of a pass
     const uint32_t b_q = sbase, b_kf = sbase + 8, b_ke = sbase + 24, b_vf = sbase + 40, b_ve = sbase + 56, b_s = sbase + 72, b_p = sbase + 88, b_o = sbase + 104, b_end = sbase + 112;
-    volatile uint32_t *s_tmem = reinterpret_cast<volatile uint32_t *>(smem + 256), *s_abort = reinterpret_cast<volatile uint32_t *>(smem + 260);
-    if (tid == 0) {
-        mbar_init(b_q, 128);
-        for (uint32_t i = 0; i < 2; ++i) {
-            mbar_init(b_kf + 8 * i, FL_LOADERS); mbar_init(b_ke + 8 * i, 1); mbar_init(b_vf + 8 * i, FL_LOADERS); mbar_init(b_ve + 8 * i, 1);
-            mbar_init(b_s + 8 * i, 1); mbar_init(b_p + 8 * i, 128);
-        }
-        mbar_init(b_o, 1);
-        mbar_init(b_end, 1);
-        *s_abort = 0;
-        fence_mbar_init();
-    }
-    if (warp == 7) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + 256), "r"(FL_TMEM) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = *s_tmem, t_o = tmem + 2 * KT;
-    pdl_wait();
-    pdl_trigger();
+    volatile uint32_t *s_abort = reinterpret_cast<volatile uint32_t *>(smem + 260);
+    uint32_t *s_marked = reinterpret_cast<uint32_t *>(smem + 512);
     const uint32_t pos0 = __ldcg(a.pos), r_last = min(rows, r0 + FL_M) - 1;
     const uint32_t p_first = pos0 + r0 / group, p_last = pos0 + r_last / group;
-    const uint32_t lo = p_first + 1 - a.ring.active_len(p_first + 1), n_tiles = (p_last - lo) / KT + 1;
+    const uint32_t lo = p_first + 1 - a.ring.active_len(p_first + 1), n_tiles = (p_last - lo) / KT + 1, base = AGAIN ? n_tiles : 0;
+    bool again = false;
 
     if (warp >= 4 && warp < 7) {
         const uint32_t lt = tid - 128;
@@ -368,38 +349,56 @@ __global__ void __launch_bounds__(FL_THREADS, 1) window_flash_kernel(const AttnP
             }
             fl_cp_commit();
         };
+        // the thread's pieces of a tile of values without what is not finite; the tile is marked
+        auto clean = [&](uint32_t dst, uint32_t j) {
+            for (uint32_t i = lt; i < KT * CH; i += FL_LOADERS) {
+                const uint32_t x = i / CH, c = i % CH, at = dst + (c >> 3) * (KT * 128) + x * 128 + (((c & 7u) ^ (x & 7u)) << 4);
+                uint32_t w[4], mark = 0;
+                asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(at));
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    if ((w[k] & 0x7F80u) == 0x7F80u) { w[k] &= 0xFFFF0000u; mark = 1; }
+                    if ((w[k] & 0x7F800000u) == 0x7F800000u) { w[k] &= 0x0000FFFFu; mark = 1; }
+                }
+                if (mark == 0) continue;
+                asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(at), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
+                atomicOr(s_marked + j % FL_MARKS / 32, 1u << (j % 32));
+            }
+        };
         // Every thread waits for its own copies, makes them visible to the tensor cores and announces them.  The keys of a tile are
         // announced as soon as they have landed, its values once the keys of the next tile have been requested.
         bool ok = true;
         for (uint32_t j = 0; j < n_tiles; ++j) {
-            const uint32_t b = j & 1u;
-            if (j >= 2) ok = mbar_wait_warp(b_ke + 8 * b, ((j >> 1) - 1u) & 1u, FL_WAIT, s_abort);
+            const uint32_t i = base + j, b = i & 1u;
+            if (i >= 2) ok = mbar_wait_warp(b_ke + 8 * b, ((i >> 1) - 1u) & 1u, FL_WAIT, s_abort);
             if (!ok) break;
             fetch(kc, s_k + b * T_BYTES, j);
             if (j >= 1) {
                 fl_cp_wait<1>();
+                if (AGAIN) clean(s_v + (b ^ 1u) * T_BYTES, j - 1);
                 fence_proxy_async();
                 mbar_arrive(b_vf + 8 * (b ^ 1u));
             }
             fl_cp_wait<0>();
             fence_proxy_async();
             mbar_arrive(b_kf + 8 * b);
-            if (j >= 2) ok = mbar_wait_warp(b_ve + 8 * b, ((j >> 1) - 1u) & 1u, FL_WAIT, s_abort);
+            if (i >= 2) ok = mbar_wait_warp(b_ve + 8 * b, ((i >> 1) - 1u) & 1u, FL_WAIT, s_abort);
             if (!ok) break;
             fetch(vc, s_v + b * T_BYTES, j);
         }
         fl_cp_wait<0>();                       // also after a wait that gave up: the copies land before the CTA leaves
+        if (ok && AGAIN) clean(s_v + ((base + n_tiles - 1) & 1u) * T_BYTES, n_tiles - 1);
         fence_proxy_async();
-        if (ok) mbar_arrive(b_vf + 8 * ((n_tiles - 1) & 1u));
+        if (ok) mbar_arrive(b_vf + 8 * ((base + n_tiles - 1) & 1u));
         else if (lane == 0 && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
     } else if (warp == 7) {
         if (lane == 0) {
             // fp32 accumulators, bf16 operands; A and B K-major for S, B with its columns consecutive for O
             constexpr uint32_t id_s = (1u << 4) | (1u << 7) | (1u << 10) | ((KT >> 3) << 17) | ((FL_M >> 4) << 24);
             constexpr uint32_t id_o = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | ((D >> 3) << 17) | ((FL_M >> 4) << 24);
-            auto scores = [&](uint32_t j) {
-                const uint32_t b = j & 1u, kb = s_k + b * T_BYTES;
-                if (!mbar_wait_thread(b_kf + 8 * b, (j >> 1) & 1u, FL_WAIT, s_abort)) return false;
+            auto scores = [&](uint32_t i_tile) {
+                const uint32_t b = i_tile & 1u, kb = s_k + b * T_BYTES;
+                if (!mbar_wait_thread(b_kf + 8 * b, (i_tile >> 1) & 1u, FL_WAIT, s_abort)) return false;
                 tc_fence_after();
 #pragma unroll
                 for (uint32_t i = 0; i < D / 16; ++i)
@@ -408,15 +407,15 @@ __global__ void __launch_bounds__(FL_THREADS, 1) window_flash_kernel(const AttnP
                 tc_commit(b_ke + 8 * b);
                 return true;
             };
-            bool ok = mbar_wait_thread(b_q, 0, FL_WAIT, s_abort) && scores(0);
+            bool ok = mbar_wait_thread(b_q, 0, FL_WAIT, s_abort) && scores(base);
             for (uint32_t j = 0; j < n_tiles && ok; ++j) {
-                const uint32_t b = j & 1u;
+                const uint32_t i = base + j, b = i & 1u;
                 if (j + 1 < n_tiles) {
-                    if (j >= 1) ok = mbar_wait_thread(b_o, (j - 1) & 1u, FL_WAIT, s_abort);      // the weights of tile j - 1 lie where S of tile j + 1 goes
-                    ok = ok && scores(j + 1);
+                    if (i >= 1) ok = mbar_wait_thread(b_o, (i - 1) & 1u, FL_WAIT, s_abort);      // the weights of tile i - 1 lie where S of tile i + 1 goes
+                    ok = ok && scores(i + 1);
                     if (!ok) break;
                 }
-                ok = mbar_wait_thread(b_p + 8 * b, (j >> 1) & 1u, FL_WAIT, s_abort) && mbar_wait_thread(b_vf + 8 * b, (j >> 1) & 1u, FL_WAIT, s_abort);
+                ok = mbar_wait_thread(b_p + 8 * b, (i >> 1) & 1u, FL_WAIT, s_abort) && mbar_wait_thread(b_vf + 8 * b, (i >> 1) & 1u, FL_WAIT, s_abort);
                 if (!ok) break;
                 tc_fence_after();
 #pragma unroll
@@ -426,11 +425,12 @@ __global__ void __launch_bounds__(FL_THREADS, 1) window_flash_kernel(const AttnP
                 tc_commit(b_o);
             }
             tc_commit(b_end);                 // also after a wait that gave up: completes when the issued products have
+            mbar_arrive(b_end);               // with this thread's view of the marks
             if (!ok && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
-            for (uint32_t spin = 0; spin < FL_WAIT && !mbar_try_wait(b_end, 0u); ++spin) {}
+            for (uint32_t spin = 0; spin < FL_WAIT && !mbar_try_wait(b_end, PASS); ++spin) {}
         }
     } else {
-        for (uint32_t i = tid; i < FL_M * CH; i += 128) {          // rows beyond the last repeat it
+        for (uint32_t i = tid; i < FL_M * CH && !AGAIN; i += 128) {          // rows beyond the last repeat it
             const uint32_t r = i / CH, c = i % CH, rr = min(r0 + r, rows - 1);
             fl_cp16(s_q + (c >> 3) * (FL_M * 128) + r * 128 + (((c & 7u) ^ (r & 7u)) << 4), static_cast<const __nv_bfloat16 *>(a.q) + ((size_t)(rr / group) * a.n_q + g * group + rr % group) * D + c * 8);
         }
@@ -441,12 +441,12 @@ __global__ void __launch_bounds__(FL_THREADS, 1) window_flash_kernel(const AttnP
         const float sc = __ldg(a.head_scale + head) * LOG2E, sl = __ldg(a.head_slope + head) * LOG2E;
         fl_cp_wait<0>();
         fence_proxy_async();
-        mbar_arrive(b_q);
+        if (!AGAIN) mbar_arrive(b_q);
         float m = -INFINITY, l = 0.0f;         // maximum the weights are taken against, and their sum
         bool ok = true;
         for (uint32_t j = 0; j < n_tiles; ++j) {
-            const uint32_t b = j & 1u, t_s = tmem + b * KT + lanes, j0 = lo + j * KT;
-            ok = mbar_wait_warp(b_s + 8 * b, (j >> 1) & 1u, FL_WAIT, s_abort);
+            const uint32_t i_tile = base + j, b = i_tile & 1u, t_s = tmem + b * KT + lanes, j0 = lo + j * KT;
+            ok = mbar_wait_warp(b_s + 8 * b, (i_tile >> 1) & 1u, FL_WAIT, s_abort);
             if (!ok) break;
             tc_fence_after();
             uint32_t v[KT];
@@ -471,7 +471,7 @@ __global__ void __launch_bounds__(FL_THREADS, 1) window_flash_kernel(const AttnP
             if (j == 0) {
                 m = m_new;
             } else if (__any_sync(0xffffffffu, m_new > m + 8.0f)) {
-                ok = mbar_wait_warp(b_o, (j - 1) & 1u, FL_WAIT, s_abort);
+                ok = mbar_wait_warp(b_o, (i_tile - 1) & 1u, FL_WAIT, s_abort);
                 if (!ok) break;
                 tc_fence_after();
                 const bool grown = m_new > m + 8.0f;          // row by row: a row's bits do not depend on the rows beside it
@@ -504,10 +504,11 @@ __global__ void __launch_bounds__(FL_THREADS, 1) window_flash_kernel(const AttnP
             mbar_arrive(b_p + 8 * b);
         }
         // the last update by a barrier of its own: the phases of b_o may still be two behind here, and a parity tells only neighbours apart
-        if (ok) ok = __all_sync(0xffffffffu, mbar_wait_thread(b_end, 0u, FL_WAIT, s_abort) && *s_abort == 0);
+        if (ok) ok = __all_sync(0xffffffffu, mbar_wait_thread(b_end, PASS, FL_WAIT, s_abort) && *s_abort == 0);
         tc_fence_after();
         if (ok) {
             const float inv = 1.0f / l;
+            float finite[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};          // NaN once an output is not finite
 #pragma unroll 1
             for (uint32_t c = 0; c < D; c += 16) {
                 uint32_t o[16];
@@ -516,7 +517,22 @@ __global__ void __launch_bounds__(FL_THREADS, 1) window_flash_kernel(const AttnP
                 if (r < rows) {
                     float f[16];
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) f[i] = __uint_as_float(o[i]) * inv;
+                    for (int i = 0; i < 16; ++i) { f[i] = __uint_as_float(o[i]) * inv; finite[i & 7] = __fmaf_rn(f[i], 0.0f, finite[i & 7]); }
+                    if (AGAIN) {
+                        const __nv_bfloat16 *vc = static_cast<const __nv_bfloat16 *>(a.v_cache) + (size_t)g * p.ring_rows * D + c;
+#pragma unroll 1
+                        for (uint32_t x = lo; x <= qpos; ++x) {
+                            const uint32_t j = (x - lo) / KT;
+                            if ((s_marked[j % FL_MARKS / 32] >> (j % 32) & 1u) == 0) { x = lo + j * KT + KT - 1; continue; }
+                            if (qpos - x >= window) continue;
+                            float v[16];
+                            get8(vc + (size_t)a.ring.slot_of_pos(x) * D, *reinterpret_cast<float(*)[8]>(v));
+                            get8(vc + (size_t)a.ring.slot_of_pos(x) * D + 8, *reinterpret_cast<float(*)[8]>(v + 8));
+#pragma unroll
+                            for (int i = 0; i < 16; ++i)
+                                if ((__float_as_uint(v[i]) & 0x7F800000u) == 0x7F800000u) f[i] += v[i];
+                        }
+                    }
                     const uint32_t k = head * a.vdim + c;
                     if (c + 16 <= a.vdim && (k & 7u) == 0) {
 #pragma unroll
@@ -530,12 +546,53 @@ __global__ void __launch_bounds__(FL_THREADS, 1) window_flash_kernel(const AttnP
                     }
                 }
             }
+            again = ((finite[0] + finite[1]) + (finite[2] + finite[3])) + ((finite[4] + finite[5]) + (finite[6] + finite[7])) != 0.0f;
         } else if (lane == 0 && a.err_flag != nullptr) {
             atomicExch(a.err_flag, 1u);
         }
     }
+    return again;
+}
+template <int D> __device__ __noinline__ void flash_again(const AttnParams &p, uint8_t *smem, uint32_t sbase, uint32_t tmem) { flash_pass<D, true>(p, smem, sbase, tmem); }
+
+template <int D>
+__global__ void __launch_bounds__(FL_THREADS, 1) window_flash_kernel(const __grid_constant__ AttnParams p) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t tid = threadIdx.x, warp = tid >> 5;
+    const uint32_t raw = (uint32_t)__cvta_generic_to_shared(smem_raw), sbase = (raw + 1023u) & ~1023u;
+    uint8_t *smem = smem_raw + (sbase - raw);
+    const uint32_t b_q = sbase, b_kf = sbase + 8, b_ke = sbase + 24, b_vf = sbase + 40, b_ve = sbase + 56, b_s = sbase + 72, b_p = sbase + 88, b_o = sbase + 104, b_end = sbase + 112;
+    volatile uint32_t *s_tmem = reinterpret_cast<volatile uint32_t *>(smem + 256), *s_abort = reinterpret_cast<volatile uint32_t *>(smem + 260);
+    if (tid < FL_MARKS / 32) reinterpret_cast<uint32_t *>(smem + 512)[tid] = 0;
+    if (tid == 0) {
+        mbar_init(b_q, 128);
+        for (uint32_t i = 0; i < 2; ++i) {
+            mbar_init(b_kf + 8 * i, FL_LOADERS); mbar_init(b_ke + 8 * i, 1); mbar_init(b_vf + 8 * i, FL_LOADERS); mbar_init(b_ve + 8 * i, 1);
+            mbar_init(b_s + 8 * i, 1); mbar_init(b_p + 8 * i, 128);
+        }
+        mbar_init(b_o, 1);
+        mbar_init(b_end, 2);
+        *s_abort = 0;
+        fence_mbar_init();
+    }
+    if (warp == 7) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(sbase + 256), "r"(FL_TMEM) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
     tc_fence_before();
     __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *s_tmem;
+    pdl_wait();
+    pdl_trigger();
+    const bool again = flash_pass<D, false>(p, smem, sbase, tmem);
+    tc_fence_before();
+    if (__syncthreads_or(again)) {
+        tc_fence_after();
+        flash_again<D>(p, smem, sbase, tmem);
+        tc_fence_before();
+        __syncthreads();
+    }
     if (warp == 7) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(FL_TMEM) : "memory");
