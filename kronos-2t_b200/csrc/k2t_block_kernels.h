@@ -59,6 +59,7 @@ struct WindowAttnArgs {
     float eps;
     Act out;                           // [n_tok][n_q * vdim]
     uint32_t *err_flag;
+    uint32_t ctx_bound;                // no token of the batch sees more positions than these; 0 = the host does not know
 };
 bool window_attn_fits(bool f32, uint32_t group, uint32_t row);       // queries of a group beside one another in shared memory
 uint32_t window_attn_row(uint32_t dim, uint32_t vdim);       // cache row in elements; 0 = larger than the kernels support

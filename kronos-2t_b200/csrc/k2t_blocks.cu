@@ -105,7 +105,7 @@ bool mix_attention(KronosCudaEngine *e, Block &B, uint32_t T, const Act &out) {
     a.qkv = b.z; a.qkv_stride = b.zs;
     a.q_norm = B.q_norm; a.k_norm = B.k_norm; a.head_scale = B.head_scale; a.head_slope = B.head_slope;
     a.k_cache = B.k; a.v_cache = B.v; a.q = b.q; a.pos = e->d_pos;
-    a.n_q = B.heads; a.n_kv = B.kv_heads; a.dim = B.dim; a.vdim = B.vdim; a.row = B.row; a.ring = B.ring; a.eps = e->cfg.rms_norm_eps; a.out = out; a.err_flag = e->ctx->d_err;
+    a.n_q = B.heads; a.n_kv = B.kv_heads; a.dim = B.dim; a.vdim = B.vdim; a.row = B.row; a.ring = B.ring; a.eps = e->cfg.rms_norm_eps; a.out = out; a.err_flag = e->ctx->d_err; a.ctx_bound = e->ctx_bound;
     uint32_t n = 0;
     const cudaError_t err = launch_window_attention(e->ctx->stream, b.f32, a, T, e->ctx->sm_count, &n, e->pdl);
     return engine_count(e, err, "attention", n);

@@ -1,4 +1,4 @@
-"""Window attention of prompts (bf16) by itself: what a value that is not finite reaches."""
+"""Window attention of prompts (bf16) by itself: its bits under cuts of a prompt, what a value that is not finite reaches."""
 import ctypes as C
 
 import numpy as np
@@ -19,7 +19,7 @@ class Ring(C.Structure):
 
 class Args(C.Structure):
     _fields_ = [(n, C.c_size_t if n == "qkv_stride" else C.c_void_p) for n in "qkv qkv_stride q_norm k_norm head_scale head_slope k_cache v_cache q pos".split()] + [
-        (n, C.c_uint32) for n in "n_q n_kv dim vdim row".split()] + [("ring", Ring), ("eps", C.c_float), ("out", Act), ("err_flag", C.c_void_p)]
+        (n, C.c_uint32) for n in "n_q n_kv dim vdim row".split()] + [("ring", Ring), ("eps", C.c_float), ("out", Act), ("err_flag", C.c_void_p), ("ctx_bound", C.c_uint32)]
 
 
 class Layer:
@@ -51,7 +51,7 @@ class Layer:
         cols = self.H * self.vdim
         out = torch.full(((cols + 63) // 64, ld, 64), -3.0, dtype=torch.bfloat16, device="cuda")
         a = Args(x.data_ptr(), x.shape[1], self.ones.data_ptr(), self.ones.data_ptr(), self.scale.data_ptr(), self.slope.data_ptr(), self.k.data_ptr(), self.v.data_ptr(), q.data_ptr(),
-                 at.data_ptr(), self.H, self.G, self.dim, self.vdim, self.row, Ring(self.window, 0, self.ring_len), 1e-6, Act(out.data_ptr(), ld), err.data_ptr())
+                 at.data_ptr(), self.H, self.G, self.dim, self.vdim, self.row, Ring(self.window, 0, self.ring_len), 1e-6, Act(out.data_ptr(), ld), err.data_ptr(), pos + n)
         launches = C.c_uint32()
         launch = internal("launch_window_attention", C.c_int, C.c_void_p, C.c_bool, C.POINTER(Args), C.c_uint32, C.c_int, C.POINTER(C.c_uint32), C.c_bool)
         assert launch(torch.cuda.current_stream().cuda_stream, False, C.byref(a), n, 148, C.byref(launches), False) == 0
@@ -65,7 +65,7 @@ class Layer:
 
 
 # heads, kv heads, dim, vdim, window, portions: every head size, both tile heights, groups that end a tile inside a token, windows inside a tile
-SHAPES = [(4, 1, 32, 32, 0, [2, 300]), (4, 2, 64, 64, 0, [3, 9, 140]), (3, 1, 96, 80, 100, [129, 42]), (8, 2, 128, 128, 0, [255, 2, 600]), (8, 2, 128, 120, 40, [200, 131]), (2, 2, 128, 128, 17, [128, 129]),
+SHAPES = [(4, 1, 32, 32, 0, [2, 300]), (4, 1, 64, 64, 0, [32]), (6, 2, 128, 128, 0, [33]), (8, 1, 256, 256, 7, [20, 12, 31]), (4, 2, 64, 64, 0, [3, 9, 140]), (3, 1, 96, 80, 100, [129, 42]), (8, 2, 128, 128, 0, [255, 2, 600]), (8, 2, 128, 120, 40, [200, 131]), (2, 2, 128, 128, 17, [128, 129]),
           (5, 1, 192, 192, 100, [27, 150]), (2, 2, 192, 130, 0, [64, 65, 200]), (1, 1, 256, 256, 0, [16, 17, 300]), (2, 2, 256, 250, 9, [128, 130]), (6, 2, 128, 128, 900, [700, 1300])]
 
 def portions(layer, qkv, cuts):
@@ -74,6 +74,15 @@ def portions(layer, qkv, cuts):
         out.append(layer.run(qkv[at:at + n], at)[0])
         at += n
     return np.concatenate(out)
+
+
+@pytest.mark.parametrize("heads,kv,dim,vdim,cuts", [(4, 2, 64, 64, [2, 9, 140, 250]), (4, 2, 64, 64, [32, 369]), (8, 2, 128, 128, [255, 2, 600, 143]), (8, 2, 128, 128, [2, 18, 12, 33, 300]), (2, 2, 192, 130, [31, 2, 90]), (3, 1, 96, 80, [129, 42, 130]), (1, 1, 256, 256, [16, 17, 300, 65])])
+def test_bits_under_any_cut(heads, kv, dim, vdim, cuts):
+    """Without a window the tiles of keys begin at position 0, whatever the batch: a row's bits depend on its keys alone."""
+    total = sum(cuts)
+    whole, parts = (Layer(heads, kv, dim, vdim, 0, total, slope=0.01, scale=4.0, seed=3) for _ in "ab")
+    qkv = whole.inputs(total)
+    assert np.array_equal(whole.run(qkv, 0)[0], portions(parts, qkv, cuts))
 
 
 @pytest.mark.parametrize("heads,kv,dim,vdim,window,cuts", SHAPES)
