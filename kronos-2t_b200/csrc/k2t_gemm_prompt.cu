@@ -381,14 +381,12 @@ __global__ void __launch_bounds__(GpLayout<FMT, N, EXP>::THREADS, 1) gemm_prompt
             if (++d == ND) d = 0;
             if (++b == NB) b = 0;
         }
-        if (!ok) {          // what was issued ends before the tensor memory is given back
-            if (lane == 0) {
-                if (a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
-                hf_commit(bar_last);
-                for (uint32_t spin = 0; spin < WAIT_LIMIT && !mbar_try_wait(bar_last, 0u); ++spin) {}
-            }
-            __syncwarp();
+        if (!ok && lane == 0 && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
+        if (gp_elect()) {          // what this thread issued ends before the tensor memory is given back, whichever role gave up
+            hf_commit(bar_last);
+            for (uint32_t spin = 0; spin < WAIT_LIMIT && !mbar_try_wait(bar_last, 0u); ++spin) {}
         }
+        __syncwarp();
     } else if (warp == GP_EPI + GP_DEC + 1 || (EXP && warp == GP_EPI + GP_DEC + 3)) {
         if constexpr (EXP) {
             // ------------------------------------------------------------------ activations of the tile's pairs, widened on the way, the two warps chunk by chunk in
@@ -474,11 +472,9 @@ __global__ void __launch_bounds__(GpLayout<FMT, N, EXP>::THREADS, 1) gemm_prompt
                     if (++xsl == 2 * NB) xsl = 0;
                 }
             }
-            if (!ok) {          // copies in flight land before the CTA leaves
-                if (a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
-                for (uint32_t k = i > NB ? i - NB : 0; k < i; ++k)
-                    for (uint32_t spin = 0; spin < 4096 && !mbar_try_wait(bar_bfull + 8 * (k % NB), (k / NB) & 1u); ++spin) {}
-            }
+            if (!ok && a.err_flag != nullptr) atomicExch(a.err_flag, 1u);
+            for (uint32_t k = i > NB ? i - NB : 0; k < i; ++k)          // copies in flight land before the CTA leaves, whichever role gave up
+                for (uint32_t spin = 0; spin < GP_WAIT_LIMIT && !mbar_try_wait(bar_bfull + 8 * (k % NB), (k / NB) & 1u); ++spin) {}
         }
     } else if (warp == GP_EPI + GP_DEC + 2) {
         // ------------------------------------------------------------------ raw weights, GC chunks of 128 rows at a time: GC lanes a row

@@ -101,3 +101,13 @@ def test_a_wait_is_not_cut_short_by_an_earlier_one(source):
     would let the CTA leave while copies into its shared memory are in flight."""
     text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, source)).read())
     assert re.findall(r"for \([^;]*\bspin\b[^;]*;[^;]*(?<![!\w])ok\b[^;]*;[^)]*\)", text) == []
+
+
+def test_prompt_gemm_waits_for_what_it_issued():
+    """The threads that ask for activations and issue products wait for the last of them on every way out: a role that gives up elsewhere would otherwise
+    let the CTA leave, and its tensor memory go back, while these are in flight."""
+    text = re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, "k2t_gemm_prompt.cu")).read())
+    drains = list(re.finditer(r"spin < \w*WAIT_LIMIT && !mbar_try_wait\((bar_last|bar_bfull)", text))
+    assert [m.group(1) for m in drains] == ["bar_last", "bar_bfull"]
+    for m in drains:
+        assert not any("!ok" in h for h in headers(text, m.start()))
