@@ -335,7 +335,7 @@ __global__ void __launch_bounds__(ROUTER_THREADS) moe_router_kernel(RouterArgs a
     router_select(a);
 }
 
-// Prompt batches: the logits of 16 tokens x 16 experts per CTA, then the selection, a CTA per token.  Same sums: a lane owns four of the sixteen
+// Larger prompt batches (router_in_two): the logits of 16 tokens x 16 experts per CTA, then the selection, a CTA per token.  Same sums: a lane owns four of the sixteen
 // accumulators of eight (token, expert) pairs, so six 16-byte loads feed 32 multiply-adds, where a CTA per token and eight experts read
 // the router matrix again for every token (300 tokens, 128 experts of 2048: 51 us in the one launch, 25 + 9 in two).
 constexpr uint32_t RL_TOKENS = 16, RL_EXPERTS = 16, RL_SLICE = 256, RL_PITCH = RL_SLICE + 8, RL_STAGES = 3;          // floats of a row per stage; rows two apart 16 banks apart
@@ -1076,16 +1076,27 @@ cudaError_t launch_rmsnorm_quant(cudaStream_t s, float *hidden, const float *del
                                  int8_t *q, float *scales, int32_t *sums, uint32_t n_tok, bool pdl) {
     return launch_rmsnorm_quant_x(s, hidden, delta, w, n, eps, q, scales, sums, nullptr, n_tok, pdl);
 }
+// staged form of the one launch: x and the CTA's eight rows in shared memory (rows padded by 16 floats); needs 16-byte rows
+static size_t router_staged_bytes(const RouterArgs &a) {
+    const size_t bytes = ((size_t)a.hidden + (size_t)ROUTER_EXPERTS_PER_CTA * (a.hidden + 16)) * 4;
+    return a.hidden % 4 == 0 && bytes <= 200 * 1024 && (reinterpret_cast<uintptr_t>(a.w) & 15u) == 0 ? bytes : 0;
+}
+// One launch takes a time that grows with its CTAs, a token and eight experts each, and with how few of them share an SM; two launches start at about
+// 7 us + 7.3 us per 1024 columns and grow little.  So a line by (token, expert) pairs.  One launch / two, us: hidden 2048, 128 experts, 16 tokens
+// 9.9 / 23.4, 96 20.8 / 23.7, 128 25.1 / 23.7, 300 48.3 / 28.0; 64 experts, 200 tokens 21.2 / 23.1, 300 28.2 / 23.1; 1024, 64, 200 14.7 / 15.6, 300 18.1 / 15.6;
+// two CTAs an SM: 3072, 64, 160 25.8 / 30.5, 256 37.3 / 30.6; one: 4096, 128, 64 37.1 / 39.0, 96 50.8 / 39.1; not staged: 7168, 128, 128 56.2 / 61.8, 160 68.4 / 62.0.
+// (256 experts of 768 columns and fewer would gain from some 8000 pairs on.)
 bool router_in_two(const RouterArgs &a, uint32_t n_tok) {
-    return n_tok >= 16 && a.hidden % 16 == 0 && (n_tok + RL_TOKENS - 1) / RL_TOKENS <= 0xFFFF && ((reinterpret_cast<uintptr_t>(a.w) | reinterpret_cast<uintptr_t>(a.x)) & 15u) == 0;
+    const size_t staged = router_staged_bytes(a), ctas = (228 * 1024) / (staged + 2560);          // beside static shared memory and the system's share
+    const size_t pairs = staged == 0 ? 18432 : ctas < 2 ? 9216 : ctas < 3 ? 12800 : 14336;
+    return (size_t)n_tok * a.n_experts >= pairs && a.hidden % 16 == 0 && (n_tok + RL_TOKENS - 1) / RL_TOKENS <= 0xFFFF &&
+           ((reinterpret_cast<uintptr_t>(a.w) | reinterpret_cast<uintptr_t>(a.x)) & 15u) == 0;
 }
 cudaError_t launch_moe_router(cudaStream_t s, const RouterArgs &a_in, bool pdl, uint32_t n_tok) {
     RouterArgs a = a_in;
     if (a.n_experts > ROUTER_MAX_EXPERTS || a.top_k > ROUTER_MAX_TOPK || a.hidden * 4 > 160 * 1024) return cudaErrorInvalidValue;
-    // staged form: x and the CTA's eight rows in shared memory (rows padded by 16 floats); needs 16-byte rows
-    const size_t staged_bytes = ((size_t)a.hidden + (size_t)ROUTER_EXPERTS_PER_CTA * (a.hidden + 16)) * 4;
-    a.staged = (a.hidden % 4 == 0 && staged_bytes <= 200 * 1024 && (reinterpret_cast<uintptr_t>(a.w) & 15u) == 0) ? 1u : 0u;
-    const size_t smem = a.staged ? staged_bytes : (size_t)a.hidden * 4;
+    const size_t staged = router_staged_bytes(a), smem = staged ? staged : (size_t)a.hidden * 4;
+    a.staged = staged ? 1u : 0u;
     {
         cudaError_t e = allow_dynamic_smem(reinterpret_cast<const void *>(moe_router_kernel), smem + 4096);      // beside 3 KiB of static shared memory
         if (e != cudaSuccess) return e;

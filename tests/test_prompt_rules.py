@@ -104,3 +104,23 @@ def test_rows_of_an_attention_tile():
     last = lambda d, r: max(ctx for ctx in range(128, 8192) if rows(d, ctx) >= r)  # noqa: E731
     assert [last(64, 16), last(128, 16), last(64, 8), last(128, 8)] == [3424, 3344, 6944, 6864]
     assert rows(96, 128) == 0
+
+
+class RouterArgs(C.Structure):
+    _fields_ = [("w", C.c_void_p), ("bias", C.c_void_p), ("x", C.c_void_p), ("n_experts", C.c_uint32), ("hidden", C.c_uint32), ("top_k", C.c_uint32), ("norm_topk", C.c_int32),
+                ("scoring", C.c_uint32), ("route_ids", C.c_void_p), ("route_w", C.c_void_p), ("logits", C.c_void_p), ("done", C.c_void_p), ("route_stride", C.c_uint32),
+                ("staged", C.c_uint32), ("err_flag", C.c_void_p)]
+
+
+# hidden, experts: tokens at which one launch was faster, at which two were
+@pytest.mark.parametrize("hidden,n_experts,one,two", [
+    (512, 64, (16, 64, 200), (256, 512)), (1024, 8, (16, 512), ()), (1024, 64, (16, 128, 200), (256, 300)), (1024, 128, (16, 64, 96), (128, 512)), (1536, 64, (16, 200), (256, 400)),
+    (1536, 256, (16, 48), (64, 128)), (2048, 16, (16, 512), ()), (2048, 32, (16, 300), (512,)), (2048, 64, (16, 128, 200), (300, 512)), (2048, 128, (16, 24, 48, 64, 96), (128, 300, 512)),
+    (2048, 256, (16, 48), (64, 128)), (2560, 64, (16, 160), (200, 300)), (3072, 64, (16, 160), (256, 300)), (3072, 128, (16, 96), (128, 200)), (3584, 128, (16, 64), (96, 128)),
+    (4096, 64, (16, 96, 128), (200, 300)), (4096, 128, (16, 64), (96, 200)), (5120, 128, (16, 64), (96, 128)), (6144, 64, (16, 256), (300, 512)), (7168, 128, (16, 128), (160, 300)),
+    (8192, 256, (16, 64), (96, 128))])
+def test_router_takes_the_faster_form(hidden, n_experts, one, two):
+    in_two = internal("router_in_two", C.c_bool, C.POINTER(RouterArgs), C.c_uint32)
+    a = RouterArgs(w=256, x=256, n_experts=n_experts, hidden=hidden, top_k=min(8, n_experts))
+    assert {t: in_two(C.byref(a), t) for t in one + two} == {**dict.fromkeys(one, False), **dict.fromkeys(two, True)}
+    assert not any(in_two(C.byref(a), t) for t in range(1, 16))
