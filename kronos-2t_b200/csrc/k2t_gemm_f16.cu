@@ -9,7 +9,8 @@
 // tokens per instruction: 1.3 instructions per (row, token, chunk) where the int32 accumulators of k2t_gemm_tc.cu take 4.75
 // (integer correction, conversion, multiply, fma).
 //
-// Rows of 32 chunks and more go to k2t_gemm_prompt.cu; here are the shorter ones, the conversion of the activations, and the sorting of the experts' pairs.
+// Rows of 32 chunks and more go to k2t_gemm_prompt.cu where that is the faster one (gemm_prompt_takes); here are the others, the conversion of the
+// activations, and the sorting of the experts' pairs.
 //
 // The activations come as an operand image (act_half_kernel below): per chunk 128 bytes per token in the 128-byte-swizzled
 // K-major layout, so a tile of tokens is one contiguous run, plus the tokens' scales.  One CTA = 128 rows x N tokens:
@@ -452,7 +453,7 @@ cudaError_t launch_gemm_f16(cudaStream_t stream, const DeviceMatrix &m, const in
     args.img = h.img; args.xs_img = h.scales; args.zero = image_ready ? h.zero : nullptr; args.n_tok = n_tok; args.tok_pad = tok_pad;
     cudaError_t e = image_ready ? cudaSuccess : launch_kernel(act_half_kernel, dim3((m.geom.nc + 3) / 4, tok_pad / 32), dim3(256), 0, stream, pdl, xq, xs, n_tok, m.geom.nc, tok_pad, h.img, h.scales);
     if (e != cudaSuccess) return e;
-    if (gemm_prompt_takes(m.geom.nc)) {
+    if (gemm_prompt_takes(fmt, m.geom.rows, m.geom.nc, n_tok, sm_count)) {
         e = launch_gemm_prompt(stream, args.g, fmt, h, image_ready, n_tok, sm_count, pdl);
         if (e == cudaSuccess && launches) *launches = image_ready ? 1 : 2;
         return e;

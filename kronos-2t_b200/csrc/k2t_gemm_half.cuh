@@ -107,8 +107,13 @@ template <int FMT> __device__ __forceinline__ void hf_expand(const Raw<FMT> &w, 
 
 // k2t_gemm_prompt.cu: the product for rows of 32 chunks and more whose last pass is not a stub of a few chunks (its fetch weighs as much as a
 // whole one's); shorter rows end before the longer start of that kernel pays (576 x 960, 200 tokens 5.8 against 5.9 us, 576 x 3072 7.2 against
-// 7.7; 4160 x 160 b5 29.5 against 32.5; from 2048 columns on it is the faster one at every width, 0 to 37%).
-bool gemm_prompt_takes(uint32_t nc);
+// 7.7; 4160 x 160 b5 29.5 against 32.5).  Of the others, rows of one whole pass and a part (nf5: of any passes and a part) stay with k2t_gemm_f16.cu while
+// its tiles of 32 tokens (b5: 64) fit one wave: the part comes by copies of single chunks, 8 bytes each for b5, nf3 and nf5, of one warp, and nothing is
+// shared yet.  There / here, us, image ready, cold weights: 3584 x 4608 b5, 77 tokens 29.1 / 31.7, 256 31.9 / 34.2, 300 43.6 / 38.1; 3584 x 4096 (rows) nf5,
+// 128 32.6 / 36.4, 300 41.4 / 39.5; nf3 25.9 / 27.9, 200 30.4 / 29.6; nf4 26.1 / 27.5, 300 31.5 / 30.6; nf4g128 26.0 / 26.7.  b4, b6 and e8q2 are within 2% or
+// faster here, and so are the other formats from nc = 64 on (4096 rows x 7168, 16 to 512 tokens: b5 55 to 83 / 53 to 72, nf3 49 to 78 / 46 to 70;
+// nf5, 128 tokens 60.6 / 63.2, x 18944 147 / 153) and whole passes (2048, 4096, 8192 columns: 0.99 to 1.5 times as fast).
+bool gemm_prompt_takes(int fmt, uint32_t rows, uint32_t nc, uint32_t n_tok, int sm_count);
 cudaError_t launch_gemm_prompt(cudaStream_t stream, const GemvArgs &g, int fmt, const ActHalf &h, bool image_ready, uint32_t n_tok, int sm_count, bool pdl);
 
 }  // namespace k2t

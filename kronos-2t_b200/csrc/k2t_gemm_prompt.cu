@@ -619,7 +619,12 @@ template <int FMT> static cudaError_t launch_gp_fmt(cudaStream_t s, const GpArgs
     }
 }
 
-bool gemm_prompt_takes(uint32_t nc) { return nc >= 32 && (nc % 32 == 0 || nc % 32 >= 8); }
+bool gemm_prompt_takes(int fmt, uint32_t rows, uint32_t nc, uint32_t n_tok, int sm_count) {
+    if (nc < 32 || (nc % 32 != 0 && nc % 32 < 8)) return false;
+    if (nc % 32 == 0 || (nc >= 64 && fmt != FMT_NF5)) return true;
+    const uint32_t shared = fmt == FMT_BP5 ? 64 : fmt == FMT_NF3 || fmt == FMT_NF4 || fmt == FMT_NF4G || fmt == FMT_NF5 ? 32 : 0;          // tokens of the other kernel's tile
+    return shared == 0 || (uint64_t)((rows + GP_M - 1) / GP_M) * ((n_tok + shared - 1) / shared) > (uint64_t)sm_count;
+}
 
 cudaError_t launch_gemm_prompt(cudaStream_t stream, const GemvArgs &g, int fmt, const ActHalf &h, bool image_ready, uint32_t n_tok, int sm_count, bool pdl) {
     GpArgs args;

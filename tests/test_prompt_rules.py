@@ -124,3 +124,17 @@ def test_router_takes_the_faster_form(hidden, n_experts, one, two):
     a = RouterArgs(w=256, x=256, n_experts=n_experts, hidden=hidden, top_k=min(8, n_experts))
     assert {t: in_two(C.byref(a), t) for t in one + two} == {**dict.fromkeys(one, False), **dict.fromkeys(two, True)}
     assert not any(in_two(C.byref(a), t) for t in range(1, 16))
+
+
+# format, rows, columns: tokens at which the GEMM of shorter rows was faster, at which the one of long rows was (148 SMs; rows of a whole pass of 32 chunks and a part)
+FMT = dict(b4=0, b5=1, b6=2, nf4=3, nf3=4, nf5=5)
+
+
+@pytest.mark.parametrize("fmt,rows,cols,short,long", [
+    ("b5", 4608, 3584, (16, 77, 256), (300, 512)), ("b5", 3584, 3584, (16, 300), (400, 512)), ("b5", 2880, 2880, (16, 300), (400,)), ("b5", 4096, 4096, (), (16, 512)), ("b5", 3584, 18944, (), (16, 77, 512)),
+    ("b5", 12288, 3584, (32, 64), (96, 512)), ("nf5", 3584, 3584, (16, 160), (200, 512)), ("nf5", 4096, 7168, (32, 128), (160, 512)), ("nf5", 3584, 18944, (32, 160), (200, 512)), ("nf5", 2048, 8192, (), (16, 512)), ("nf3", 3584, 3584, (32, 160), (200, 512)),
+    ("nf3", 4096, 7168, (), (16, 512)), ("nf4", 4096, 2880, (32, 128), (160, 512)), ("nf4", 2048, 3584, (32, 256), (300, 512)), ("nf4", 2048, 4096, (), (16, 300)), ("b6", 4608, 3584, (), (16, 512)),
+    ("b4", 37888, 3584, (), (16, 77)), ("b5", 260, 4160, (16, 512), ()), ("nf4", 960, 1984, (16, 512), ())])
+def test_long_rows_take_the_faster_kernel(fmt, rows, cols, short, long):
+    takes = internal("gemm_prompt_takes", C.c_bool, C.c_int, C.c_uint32, C.c_uint32, C.c_uint32, C.c_int)
+    assert {t: takes(FMT[fmt], rows, cols // 64, t, 148) for t in short + long} == {**dict.fromkeys(short, False), **dict.fromkeys(long, True)}
