@@ -4,7 +4,9 @@
 //   * window_flash_kernel (bf16 prompts): CTA = 128 query rows of one kv head - row = (token, head of the group), so all heads
 //     of a group share the key and value tiles.  S = Q K^T and O += P V by tcgen05.mma with S, P and O in tensor memory; scores,
 //     bias and softmax in fp32, one row per thread; the next S is computed while the softmax of this one runs, and a row
-//     of O is rescaled only when its maximum has grown by more than 2^8 - row by row, so that its bits depend on its keys alone.
+//     of O is rescaled only when its own maximum has grown by more than 2^8.  Without a window the tiles of keys begin at position 0
+//     and a row's bits depend on its keys alone; with one they begin at the first key that the CTA's first row sees, so that where a
+//     prompt is cut moves them, and with them the last bits of a row (sums in another order).
 //   * window_row_kernel: one token and kv head per thread-block cluster.  The positions are split over the CTAs of the cluster,
 //     partial maxima, sums and outputs are merged through distributed shared memory, so a decode step is ONE launch: norms of
 //     the new query and key, the new cache row, attention and the activation of the output projection.  With fp32 rows the same
@@ -474,7 +476,7 @@ __device__ __forceinline__ bool flash_pass(const AttnParams &p, uint8_t *smem, u
                 ok = mbar_wait_warp(b_o, (i_tile - 1) & 1u, FL_WAIT, s_abort);
                 if (!ok) break;
                 tc_fence_after();
-                const bool grown = m_new > m + 8.0f;          // row by row: a row's bits do not depend on the rows beside it
+                const bool grown = m_new > m + 8.0f;          // row by row, whatever the rows beside it do
                 const float al = grown ? exp2_approx(m - m_new) : 1.0f;
 #pragma unroll 1
                 for (uint32_t c = 0; c < D; c += 16) {

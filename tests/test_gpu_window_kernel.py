@@ -1,4 +1,5 @@
-"""Window attention of prompts (bf16) by itself: its bits under cuts of a prompt, what a value that is not finite reaches."""
+"""Window attention of prompts (bf16) by itself: the launch against 64-bit attention over the rows that it reads, key by key, its bits under cuts of a
+prompt, and what a value that is not finite reaches."""
 import ctypes as C
 
 import numpy as np
@@ -63,10 +64,31 @@ class Layer:
         assert (o[n:] == -3).all() and (o[:, cols:] == -3).all()
         return o[:n, :cols].float().cpu().numpy().reshape(n, self.H, self.vdim), q.float().cpu().numpy()[:, :, :self.dim]
 
+    def exact(self, q, pos):
+        """64-bit attention of the batch's queries over the cached rows: outputs, and the sums of weights times |values|."""
+        n = len(q)
+        seen = np.arange(max(0, pos + 1 - (self.window or pos + 1)), pos + n)
+        k, v = (c[:, seen % self.ring_len].float().cpu().numpy().astype(np.float64) for c in (self.k, self.v))
+        out, size = np.empty((n, self.H, self.vdim)), np.empty((n, self.H, self.vdim))
+        away = (pos + np.arange(n))[:, None] - seen[None]
+        hide = (away < 0) | (away >= self.window if self.window else False)
+        sc, sl = self.scale.cpu().numpy().astype(np.float64), self.slope.cpu().numpy().astype(np.float64)
+        for h in range(self.H):
+            g = h // (self.H // self.G)
+            s = (q[:, h].astype(np.float64) @ k[g, :, :self.dim].T) * sc[h] - sl[h] * away
+            s[hide] = -np.inf
+            w = np.exp(s - s.max(1, keepdims=True))
+            w /= w.sum(1, keepdims=True)
+            out[:, h], size[:, h] = w @ v[g, :, :self.vdim], w @ np.abs(v[g, :, :self.vdim])
+        return out, size
+
 
 # heads, kv heads, dim, vdim, window, portions: every head size, both tile heights, groups that end a tile inside a token, windows inside a tile
 SHAPES = [(4, 1, 32, 32, 0, [2, 300]), (4, 1, 64, 64, 0, [32]), (6, 2, 128, 128, 0, [33]), (8, 1, 256, 256, 7, [20, 12, 31]), (4, 2, 64, 64, 0, [3, 9, 140]), (3, 1, 96, 80, 100, [129, 42]), (8, 2, 128, 128, 0, [255, 2, 600]), (8, 2, 128, 120, 40, [200, 131]), (2, 2, 128, 128, 17, [128, 129]),
           (5, 1, 192, 192, 100, [27, 150]), (2, 2, 192, 130, 0, [64, 65, 200]), (1, 1, 256, 256, 0, [16, 17, 300]), (2, 2, 256, 250, 9, [128, 130]), (6, 2, 128, 128, 900, [700, 1300])]
+# One rounding of a weight and one of the result to bf16 (8 bits: 2^-8 each of what it rounds); scores (sums of 256 products in fp32) and exp2 add 1e-4 at most.
+BOUND = 2.0 ** -7 * 1.05
+
 
 def portions(layer, qkv, cuts):
     out, at = [], 0
@@ -74,6 +96,34 @@ def portions(layer, qkv, cuts):
         out.append(layer.run(qkv[at:at + n], at)[0])
         at += n
     return np.concatenate(out)
+
+
+@pytest.mark.parametrize("slope", [0.0, 0.02])
+@pytest.mark.parametrize("heads,kv,dim,vdim,window,cuts", SHAPES)
+def test_against_64_bits(heads, kv, dim, vdim, window, cuts, slope):
+    total = sum(cuts)
+    layer = Layer(heads, kv, dim, vdim, window, window + max(cuts) if window else total, slope=slope, seed=dim + window)          # a ring that wraps, where there is a window
+    qkv, at = layer.inputs(total), 0
+    for n in cuts:
+        got, q = layer.run(qkv[at:at + n], at)
+        want, size = layer.exact(q, at)
+        assert (np.abs(got - want) <= BOUND * size + 1e-30).all(), (np.abs(got - want) / size).max()
+        at += n
+
+
+@pytest.mark.parametrize("heads,kv,dim,vdim,window,cuts", SHAPES)
+def test_every_key_once(heads, kv, dim, vdim, window, cuts):
+    """Value columns that add up the weights of every vdim-th position, near-uniform weights: a key that is missing, there twice or in sight of a row that must not
+    see it changes a column by a tenth or more (some twenty positions a column at most)."""
+    total = sum(cuts)
+    layer = Layer(heads, kv, dim, vdim, window, window + max(cuts) if window else total, scale=0.1, seed=heads)
+    qkv, at = layer.inputs(total), 0
+    layer.values(qkv)[:] = (np.arange(total)[:, None] % vdim == np.arange(vdim)[None])[:, None, :]
+    for n in cuts:
+        got, q = layer.run(qkv[at:at + n], at)
+        want, size = layer.exact(q, at)
+        assert (np.abs(got - want) <= BOUND * size).all()
+        at += n
 
 
 @pytest.mark.parametrize("heads,kv,dim,vdim,cuts", [(4, 2, 64, 64, [2, 9, 140, 250]), (4, 2, 64, 64, [32, 369]), (8, 2, 128, 128, [255, 2, 600, 143]), (8, 2, 128, 128, [2, 18, 12, 33, 300]), (2, 2, 192, 130, [31, 2, 90]), (3, 1, 96, 80, [129, 42, 130]), (1, 1, 256, 256, [16, 17, 300, 65])])

@@ -8,6 +8,9 @@ import folizen_models as fm
 import folizen_ref as ref
 
 pytestmark = pytest.mark.gpu
+# A row behind a window has its tiles elsewhere in a portion: sums in another order and weights taken against another maximum, both rounded to bf16 in front of the
+# next product.  0.021 of the logits' spread at most where the whole prompt is 0.023 from 64 bits (2000 positions).
+PORTIONS = 3e-2
 TOL = 5e-2          # bf16 engine against the restatement in 64 bits, as for the other bf16 prompts of this design
 
 
@@ -20,11 +23,11 @@ def ctx():
 
 
 def limit(eng, toks, want):
-    """Where a position's logits hang on the rounding alone, the bound is three times what decoding token by token gives there: it
+    """Where a position's logits hang on the rounding alone, the bound is three times what decoding token by token gives there, 0.06 at most: it
     rounds keys and values to bf16, a prompt rounds queries and softmax weights as well (worst case of the list: position 76 of
     the 192 / 130 heads, 0.024 token by token and 0.053 as a prompt, by tensor-memory products and by mma.sync alike)."""
     one = np.stack([eng.forward_token_ids([t], pos_start=i) for i, t in enumerate(toks)])
-    return np.maximum(TOL, 3 * fm.error(one, want))
+    return np.clip(3 * fm.error(one, want), TOL, 0.06)
 
 
 def check(ctx, folder, model, toks, cuts, max_seq, want):
@@ -37,6 +40,7 @@ def check(ctx, folder, model, toks, cuts, max_seq, want):
             at += n
         err = fm.error(np.concatenate(out), want)
         assert (err < (limit(eng, toks, want) if err.max() >= TOL else TOL)).all(), (err.max(), err.argmax())
+        return np.concatenate(out)
     finally:
         eng.close()
 
@@ -53,9 +57,12 @@ def test_tiles_of_a_prompt(ctx, tmp_path, heads, kv, dim, vdim, window, cuts):
 
 
 def test_rows_of_many_tiles(ctx, tmp_path):
-    """16 tiles of keys, a window that ends inside one, and a batch that begins in the middle: the same rows whole and in portions."""
+    """16 tiles of keys, a window that ends inside one, and a batch that begins in the middle: the same rows whole and in portions.  Where the window
+    has cut keys off, the portions' tiles lie elsewhere; up to there the same bits."""
     model = fm.make(96, 61, [fm.attention(4, 2, 128, 128, 900, ff=64), fm.attention(4, 2, 128, 128, 4096)], seed=5)
     toks = np.random.default_rng(3).integers(0, 61, 2000)
     want = ref.forward(model, toks)[0]
-    for k, cuts in enumerate(([2000], [1000, 1000], [700, 65, 1235])):
-        check(ctx, str(tmp_path / f"m{k}"), model, toks, cuts, 2048, want)
+    whole, *parts = [check(ctx, str(tmp_path / f"m{k}"), model, toks, cuts, 2048, want) for k, cuts in enumerate(([2000], [1000, 1000], [700, 65, 1235]))]
+    for part in parts:
+        assert np.array_equal(part[:900], whole[:900])
+        assert fm.error(part, whole).max() < PORTIONS
