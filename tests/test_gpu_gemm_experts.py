@@ -13,10 +13,14 @@ pytestmark = pytest.mark.gpu
     (4, 1, 70, 3, 320, 192, 41),      # odd chunk counts, most experts with one or two pairs, some with none
     (5, 1, 6, 2, 64, 64, 33),         # one chunk
     (2, 2, 4, 4, 384, 128, 34),       # every token takes every expert: 34 pairs each
-    (3, 1, 33, 1, 2112, 64, 16),      # a pass boundary of 32 chunks
+    (3, 1, 33, 2, 2112, 64, 64),      # a pass boundary of 32 chunks
 ])
 def test_prompt_pairs_by_expert(oracle, bits, sgc, n_experts, top_k, hidden, d_ff, n_tok):
+    import ctypes as C
+
     import kronos_2t_b200 as k2
+    from k2t_internal import internal
+    assert internal("experts_grouped", C.c_bool, *[C.c_uint32] * 6)(n_tok, n_tok * top_k, n_experts, hidden, d_ff, bits), "a GEMV per pair"
     cfg = dict(hidden=hidden, layers=2, n_q=4, n_kv=2, head_dim=64, inter=256, vocab=320, max_seq=96, eps=1e-6, theta=1e6)
     spec = km.build(oracle, cfg, "nf4", seed=bits + n_experts, moe=dict(layers=[0, 1], n_experts=n_experts, top_k=top_k, d_ff=d_ff, bits=bits, sgc=sgc))
     if hidden > 64:
