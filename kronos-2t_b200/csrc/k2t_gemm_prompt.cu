@@ -15,7 +15,8 @@
 // Tiles of up to 192 tokens share one expansion (2.4 thousand warp instructions per chunk of 128 rows x 128 tokens instead of 3.0, half of
 // the rest of them expansion and waits).  Measured on B200, nf4g128, image ready, k2t_gemm_f16.cu -> here: 2048 x 6144, 512 tokens
 // 48.5 -> 32.5 us; 2048 x 16384 97.9 -> 82.6; 8192 x 2048 65.1 -> 59.3; b4, 77 tokens: 3584 x 37888 78.2 -> 57.7, 18944 x 3584 112.7 -> 104.1.
-// Bound: 0.6 instructions per scheduler and cycle; what a chunk needs at least, packed chain steps, is a quarter of its time.
+// Bound: 0.6 instructions per scheduler and cycle; what a chunk needs at least, packed chain steps, is a quarter of its time.  The instances of 192
+// tokens spill 5 to 13 words of registers (80 a thread at launch), those of nf3, nf5 and b5 at 32 to 128 tokens 1 to 8.
 // The experts of a prompt (EXP) run in the same kernel: a tile is 128 rows of one expert and up to 32 of its (token, route) pairs, which
 // expert_tiles_kernel has gathered; two warps fetch the pairs' int8 rows where they lie and widen them on the way (one warp that did so
 // held two CTAs an SM to a tile's chunk per 0.59 us).  2400 pairs of 128 experts, 3 bits: 1536 x 2048 202 -> 158 us, 2048 x 768 131 -> 94.
@@ -64,7 +65,7 @@ struct GpArgs {
     GemvArgs g;
     const uint8_t *img, *xs_img;
     const uint32_t *zero;              // image left by the kernel that quantized: not zero where any of its scales is; else null
-    uint32_t n_tok, tok_pad, tok_tiles, tiles, width;          // width: tokens of a tile, a multiple of 16
+    uint32_t n_tok, tok_pad, tok_tiles, tiles, width;          // width: tokens of a tile, a multiple of 32
 };
 
 // The pairs of a batch sorted into tiles of one expert each (k2t_gemm_f16.cu), and the experts' images.

@@ -397,12 +397,10 @@ __global__ void __launch_bounds__(ROUTER_THREADS) router_logits_kernel(const Rou
         load(0, 0);
 #pragma unroll 2
         for (uint32_t s = 0; s < n; s += 32) {          // the next sixteen are on their way while sixteen are added
-            if (s + 16 < n) load(s + 16, 1);
+            load(s + 16, 1);
             step(0);
-            if (s + 16 < n) {
-                if (s + 32 < n) load(s + 32, 0);
-                step(1);
-            }
+            if (s + 32 < n) load(s + 32, 0);
+            step(1);
         }
         __syncthreads();
         if (warp == 0 && c + RL_STAGES < slices) request(c + RL_STAGES);
@@ -1089,7 +1087,7 @@ static size_t router_staged_bytes(const RouterArgs &a) {
 bool router_in_two(const RouterArgs &a, uint32_t n_tok) {
     const size_t staged = router_staged_bytes(a), ctas = (228 * 1024) / (staged + 2560);          // beside static shared memory and the system's share
     const size_t pairs = staged == 0 ? 18432 : ctas < 2 ? 9216 : ctas < 3 ? 12800 : 14336;
-    return (size_t)n_tok * a.n_experts >= pairs && a.hidden % 16 == 0 && (n_tok + RL_TOKENS - 1) / RL_TOKENS <= 0xFFFF &&
+    return (size_t)n_tok * a.n_experts >= pairs && a.hidden % 32 == 0 && (n_tok + RL_TOKENS - 1) / RL_TOKENS <= 0xFFFF &&
            ((reinterpret_cast<uintptr_t>(a.w) | reinterpret_cast<uintptr_t>(a.x)) & 15u) == 0;
 }
 cudaError_t launch_moe_router(cudaStream_t s, const RouterArgs &a_in, bool pdl, uint32_t n_tok) {
