@@ -421,8 +421,8 @@ template <int FMT> cudaError_t launch_hf_fmt(cudaStream_t s, const HfArgs &args,
 bool experts_grouped(uint32_t n_tok, uint32_t n_pair, uint32_t n_experts, uint32_t hidden, uint32_t d_ff, uint32_t bits) {
     const uint32_t min_tok = gemm_tc_min_tokens();
     if (min_tok == 0 || n_tok < min_tok || n_experts == 0 || bits < 2 || bits > 5) return false;
-    // in units of a tile form's time per million weights (0.5 us)
-    constexpr float START = 120.0f, PAIR[4] = {6.0f, 1.4f, 2.2f, 4.2f}, PAIR_PER_WEIGHT[4] = {0.6f, 0.25f, 0.38f, 0.55f};          // 2 .. 5 bits
+    // in units of a tile form's time per million weights (0.35 us)
+    constexpr float START = 75.0f, PAIR[4] = {8.0f, 2.05f, 2.8f, 5.6f}, PAIR_PER_WEIGHT[4] = {0.8f, 0.326f, 0.5f, 0.73f};          // 2 .. 5 bits
     const float w = 3e-6f * (float)hidden * (float)d_ff, met = (float)n_experts * (1.0f - std::exp(-(float)n_pair / (float)n_experts));
     return (float)n_pair * std::max(PAIR[bits - 2], PAIR_PER_WEIGHT[bits - 2] * w) >= START + met * w;
 }

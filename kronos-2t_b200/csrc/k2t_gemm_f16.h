@@ -44,11 +44,9 @@ cudaError_t launch_expert_tiles(cudaStream_t stream, const uint32_t *route_ids, 
 
 // Whether the expert projections of a batch run in tiles (below) or as a GEMV per pair.  Tiles are a tensor-core form: only for batches that
 // gemm_tc_min_tokens() hands over.  Their time goes with the weights of the experts that the pairs meet, a GEMV's per pair, with the weights
-// of one expert and the cost of its decode.  Measured with 2048 columns, 2 layers: tokens at which tiles (first) and GEMVs take the same, by
-// experts / routes / width / bits: 128 / 8 / 768 / 3 60 (56: 953 and 909 us, 64: 962 and 1040), 4 39, 5 15; 64 / 6 / 768 / 3 47, 4 30, 5 and 2 fewer
-// than 16; 64 / 6 / 1408 / 3 54; 16 / 4 / 2816 / 3 20, 4 14; 8 / 2 / 4096 / 4 18; 4 / 2 / 2048 / 3 22; 256 / 8 / 768 / 2 fewer than 8.
-// Those lines are of tiles expanded into shared memory; in tensor memory (k2t_gemm_prompt.cu) a tile takes 0.72 to 0.78 of that, so at
-// the lines tiles are by now the faster form.
+// of one expert and the cost of its decode.  Measured with 2048 columns, prompts of 2 layers: tokens at which tiles (first) and GEMVs take the same, by
+// experts / routes / width / bits: 128 / 8 / 768 / 3 38 (32: 619 and 565 us, 48: 654 and 720), 4 24; 64 / 6 / 768 / 3 29, 4 20; 64 / 6 / 1408 / 3 36 (32: 610
+// and 560, 40: 624 and 667); fewer than 16: 5 and 2 bits of both, 16 / 4 / 2816 / 3 (16: 440 and 446) and 4, 8 / 2 / 4096 / 4, 4 / 2 / 2048 / 3.
 bool experts_grouped(uint32_t n_tok, uint32_t n_pair, uint32_t n_experts, uint32_t hidden, uint32_t d_ff, uint32_t bits);
 
 // (k2t_gemm_prompt.cu) The expert projections of all pairs of `t`, an expert's weights expanded once per 32 pairs; out = [n_pair][rows].  Same bits as

@@ -74,10 +74,10 @@ def test_which_batches_are_converted():
 
 # experts, routes, width, bits: tokens at which a GEMV per pair was faster, at which tiles were (2048 columns)
 @pytest.mark.parametrize("n_experts,k,d_ff,bits,gemv,tiles", [
-    (128, 8, 768, 3, (16, 32, 48, 56), (64, 72, 128)), (128, 8, 768, 4, (16, 32), (48, 64)), (128, 8, 768, 5, (), (20, 32, 64)), (128, 8, 768, 2, (), (16, 32, 64)),
-    (64, 6, 768, 3, (16, 32, 40), (56, 64)), (64, 6, 768, 4, (16, 24), (32, 48)), (64, 6, 768, 5, (), (16, 24)), (64, 6, 768, 2, (), (16, 24)),
-    (64, 6, 1408, 3, (16, 32, 48), (64, 80)), (16, 4, 2816, 3, (16,), (24, 32)), (16, 4, 2816, 4, (), (16, 20)), (16, 4, 2816, 5, (), (16,)),
-    (8, 2, 4096, 4, (16,), (20, 32)), (4, 2, 2048, 3, (16, 20), (32, 48)), (256, 8, 768, 2, (), (16, 32))])
+    (128, 8, 768, 3, (16, 24, 32), (48, 56, 64, 72, 128)), (128, 8, 768, 4, (16, 20), (28, 32, 48, 64)), (128, 8, 768, 5, (), (16, 20, 32, 64)), (128, 8, 768, 2, (), (16, 32, 64)),
+    (64, 6, 768, 3, (16, 20, 24), (32, 40, 56, 64)), (64, 6, 768, 4, (16,), (24, 32, 48)), (64, 6, 768, 5, (), (16, 24)), (64, 6, 768, 2, (), (16, 24)),
+    (64, 6, 1408, 3, (16, 24, 32), (40, 48, 64, 80)), (16, 4, 2816, 3, (), (16, 20, 24, 32)), (16, 4, 2816, 4, (), (16, 20)), (16, 4, 2816, 5, (), (16,)),
+    (8, 2, 4096, 4, (), (16, 20, 32)), (4, 2, 2048, 3, (), (16, 20, 32, 48)), (256, 8, 768, 2, (), (16, 32))])
 def test_experts_take_the_faster_form(n_experts, k, d_ff, bits, gemv, tiles):
     grouped = internal("experts_grouped", C.c_bool, *[C.c_uint32] * 6)
     form = {t: grouped(t, t * k, n_experts, 2048, d_ff, bits) for t in gemv + tiles}
