@@ -17,11 +17,12 @@ struct ActHalf {
 inline size_t act_half_tokens(size_t n_tok) { return (n_tok + 127) & ~(size_t)127; }
 bool gemm_f16_takes(size_t n_tok);          // batches whose padded tokens, 32 to a CTA of either launch, fit a grid
 // Whether a batch of int8 activations is better off converted and multiplied here than by the integer GEMM, which needs no conversion
-// launch.  Rotation + product of both, integer -> this one: as long as the integer GEMM fills less than half the SMs with its tiles of
-// 16 tokens it is 8 to 25% faster (2048 columns x 2048 rows, 128 tokens 19.4 -> 21.3 us; 18944 x 3584, 64 tokens 127 -> 138 us; 576 x 960,
-// 100 tokens 8.4 -> 9.9 us), beyond that slower (2048 x 6144, 33 tokens 22.5 -> 20.4 us; 18944 x 3584, 65 tokens 165 -> 139 us; 2048 x
-// 49152, 512 tokens 528 -> 276 us) - but for few chunks, whose launches weigh more (576 x 960, 512 tokens 12.2 -> 13.5 us in tiles of 32;
-// 576 x 1536 12.9 -> 11.9 us in tiles of 64).
+// launch.  Product of both, conversion included, cold weights, integer -> this one: as long as the integer GEMM fills less than half the SMs with
+// its tiles of 16 tokens it is up to 40% faster for rows of up to 64 chunks (576 columns x 960 rows, 100 tokens 5.7 -> 7.9 us; 2048 x 2048, 128 tokens 16.6 ->
+// 17.6; 3584 x 4608, 32 tokens 29.0 -> 29.9), beyond that slower (2048 x 6144, 33 tokens 20.4 -> 17.9; 18944 x 3584, 65 tokens 265 -> 135; 2048 x 49152,
+// 512 tokens 605 -> 253) - but for few chunks, whose launches weigh more (576 x 960, 512 tokens 9.2 -> 9.4 in tiles of 32; 576 x 1536 9.7 -> 8.4
+// in tiles of 64).  The line is older than k2t_gemm_prompt.cu: on the integer side of it rows of 96 chunks and more would gain 2 to 15% by that kernel (8192 x 2048 b4,
+// 64 tokens 56.9 -> 56.0; 18944 x 3584 151 -> 135; b6 x 8192 65 -> 56), and 2048 x 49152, 16 tokens 51 -> 40; nf5 (65 -> 73) and rows below a tile would lose.
 bool gemm_f16_pays(uint32_t rows, uint32_t nc, size_t n_tok, int sm_count);
 size_t act_half_bytes(size_t n_tok, uint32_t cols);
 size_t act_half_scale_bytes(size_t n_tok, uint32_t cols);
